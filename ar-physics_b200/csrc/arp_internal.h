@@ -99,6 +99,7 @@ struct SceneP {
     float rcut, rcut2, r_geom;        // 8h, (8h)^2, h*h/(8h)
     float contact_slack;              // r_cut - largest in-stencil |dx|, 0 when unbounded
     uint32_t solid_branch;            // the scene has more than one solid (shaders/mod.rs:51)
+    double code_inv;                  // kCodeUnits / h: scale of the quantised positions (scan_code)
 };
 
 // The fields of a material the fluid pair loop reads (32 B).
@@ -107,12 +108,27 @@ struct FluidMat {
     uint32_t eos, stiff, pad;
 };
 
+// What the fluid pair terms read of a pair of materials (16 B, one load): the
+// neighbor's mass, the sum of the viscosities (zero when the particle itself
+// is elastic, fluid.rs:203), the artificial viscosity coefficient (the sum of
+// the bulk viscosities of one material, the interaction's dampening of two;
+// both viscosities zero with an immobile neighbor, fluid.rs:201)
+// and the pair's contact potential id with the elastic flags.
+struct PairMat {
+    float mass, visc, bulk;
+    uint32_t bits;
+};
+constexpr uint32_t kPairPotential = 0xFFu;    // bits: contact potential id
+constexpr uint32_t kPairElastic1 = 0x100u;    // the particle's own material is elastic
+constexpr uint32_t kPairElastic2 = 0x200u;    // the neighbor's material is elastic
+
 // Kernel-wide view of the batch tables.
 struct Tables {
     const SceneP* scenes;
     const DevMat* mats;
     const FluidMat* fmats;
     const DevInter* inter;
+    const PairMat* pmats;             // laid out as `inter`
     uint32_t ncells;                  // total search cells of all scenes (the non-finite bucket follows)
     uint32_t max_nmat;                // largest per-scene material count
     uint32_t nscenes;
@@ -124,6 +140,15 @@ struct DevStats {
     uint32_t overflow_cells;
     uint32_t nonfinite_positions;
     uint32_t clamped_coordinates;
+};
+
+// Where a kernel that writes a state counts it into search cells, the first
+// pass of that state's grid build (all null: it does not).
+struct CellBins {
+    uint32_t* key = nullptr;    // search cell of each slot
+    uint32_t* rank = nullptr;   // arrival rank inside the cell
+    uint32_t* count = nullptr;  // histogram
+    uint2* coord = nullptr;     // packed reference-cell coordinates of each slot
 };
 
 // One stage of the Runge-Kutta epilogue (fused into the fluid kernel).
@@ -156,6 +181,7 @@ struct StageBuffers {
     const float4* prev1_vm;
     const float4* prev2_pd;
     const float4* prev2_vm;
+    CellBins bin;            // where the next state is counted into cells (count null: it is not)
 };
 
 // Record `msg` as the calling thread's last error and return `code`.
@@ -173,21 +199,23 @@ struct GridBuffers {
     uint32_t block_sums_cap;
 };
 
-// Build cell_start / perm for `n` positions.  Counting sort: keys and
-// histogram, exclusive scan, scatter, then ascending slot order within each
-// cell.  Returns the number of kernel launches issued.
+// Builds cell_start / perm for `n` positions.  Counting sort: keys and
+// histogram, exclusive scan (bin_cells; a kernel that writes the state may do
+// the first of the two through CellBins, then scan_cells), scatter, then
+// ascending slot order within each cell (sort_cells).  build_grid is both.
+// Each returns the number of kernel launches issued.
 // The scene of item i is mats[material].scene, the material read from
 // vm[i].w (bits) when vm is given, else from mat_u32[i].
-// Counters a stage's later kernels start from zero (the fluid kernel's
-// overflow counts and tile counter, the self-contact gate): the grid build's
-// first kernel clears them, which saves a memset per counter per stage.
-struct StageCounters {
-    uint32_t* p[3] = {nullptr, nullptr, nullptr};
-    uint32_t n[3] = {0, 0, 0};  // words at each pointer (at most 2)
-};
+inline CellBins cell_bins(const GridBuffers& gb) { return CellBins{gb.key, gb.rank, gb.count, gb.coord}; }
+int bin_cells(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
+              GridBuffers& gb, cudaStream_t st);
+int scan_cells(const Tables& T, GridBuffers& gb, cudaStream_t st);
+// `stats` (may be null) receives the occupancy counters; `zero2` (may be
+// null) points at two counters to clear for the stage's later kernels.
+int sort_cells(uint32_t n, const Tables& T, GridBuffers& gb, DevStats* stats, const uint32_t* boundary_start,
+               uint32_t* zero2, cudaStream_t st);
 int build_grid(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
-               GridBuffers& gb, DevStats* stats, const uint32_t* boundary_start, cudaStream_t st,
-               const StageCounters& zero = StageCounters{});
+               GridBuffers& gb, cudaStream_t st);
 
 // Exclusive scan of `len` counts into out (len entries); clears `count`.
 int exclusive_scan(uint32_t* count, uint32_t len, uint32_t* out, uint32_t* block_sums, cudaStream_t st);
@@ -200,7 +228,9 @@ int gather_sorted(const uint32_t* perm, uint32_t n, const float4* a_in, float4* 
                   cudaStream_t st);
 // Gather a state into sorted order (out[k] = in[perm[k]]) and evaluate the
 // pressure term p / rho^2 of every gathered particle (fluid.rs:45-52,
-// :128,165).  Any pointer pair may be null.
+// :128,165).  Any pointer pair may be null.  With `stats`, counts the
+// non-finite positions and the coordinates on the box's upper faces.  `out`:
+// what the fluid kernel reads (see FluidArgs).
 // Solid-order copies a gather writes on the side: for a gathered particle
 // whose solid id (sid_of_slot at its source slot) is valid, sx/sv/sc[sid] =
 // its state and cell coordinates, and slot_of[sid] = its new index (when
@@ -213,10 +243,16 @@ struct SolidScatter {
     uint2* sc = nullptr;
     uint32_t* slot_of = nullptr;
 };
+struct PairOut {
+    float4* rec = nullptr;
+    uint32_t* code = nullptr;
+    uint8_t* mat8 = nullptr;
+    uint32_t* mat = nullptr;  // may be null
+};
 int gather_state(const uint32_t* perm, uint32_t n, const float4* pd_in, float4* pd_out, const float4* vm_in,
                  float4* vm_out, const uint32_t* a_in, uint32_t* a_out, const uint32_t* b_in, uint32_t* b_out,
-                 const uint2* c_in, uint2* c_out, float* ps_out, const DevMat* mats, cudaStream_t st,
-                 const SolidScatter& sol = SolidScatter{});
+                 const uint2* c_in, uint2* c_out, float* ps_out, const Tables& T, cudaStream_t st,
+                 const SolidScatter& sol = SolidScatter{}, DevStats* stats = nullptr, const PairOut& out = PairOut{});
 
 // Particle records (caller order) to structure of arrays in caller order, and
 // back from cell order into caller order (the state exchange of the C ABI).
@@ -238,55 +274,43 @@ int count_neighbors(const float4* xs, const float4* vs, const uint32_t* start, u
 
 // ---- fluid forces + stage update (fluid.cu) ---------------------------------
 struct FluidArgs {
-    const float4* xs;        // sorted stage positions/density
-    const float4* vs;        // sorted stage velocity/material
+    // mobile particles in cell order, [0, n), then boundary particles in theirs
+    const float4* rec;       // [2k] position, density; [2k + 1] velocity, p / rho^2
+    const uint32_t* code;    // quantised positions (scan_code), readable kScanPad entries past the end
+    const uint8_t* mat8;     // material id inside the scene
+    const uint32_t* mat;     // material id (mobile particles only)
     const uint32_t* start;   // mobile cell start (ncells + 1)
-    const float4* bxs;       // boundary sorted
-    const float4* bvs;
-    const uint32_t* bstart;  // boundary cell start
+    const uint32_t* bstart;  // boundary cell start (first boundary particle: 0)
     const uint32_t* perm;    // sorted -> storage slot (nullptr = identity)
     const uint32_t* sid;     // storage-order solid id
-    const uint32_t* sid_of_boundary_index;  // per boundary caller id: solid id of the scene's mobile particle
-                                            // with the same in-scene index, or invalid
-    const uint32_t* borig;   // boundary caller ids, sorted
-    const float* ps;         // p / rho^2 of each sorted particle
-    const float* bps;        // p / rho^2 of each sorted boundary particle
     const float4* ksol;      // per-solid solid-term acceleration (nullptr when the solid branch is off)
-    uint32_t* overflow;        // [2n] two queues: particles whose hit list filled up ([0, n)), and those
-                               // whose list filled up inside one row ([n, 2n))
-    uint32_t* overflow_count;  // [2] their numbers (cleared before each launch)
     uint32_t n;
     int solid_branch;
-    int any_stiff_immobile;
-    int counters_cleared;  // the stage's grid build cleared overflow_count and the tile counter
 };
 // Launch shapes of the fluid kernel the autotuner chooses between: threads
-// per block, hit-list capacity, one tile per block or persistent blocks
-// taking tiles from an atomic work counter, and whether a warp empties its
-// lists by a vote before each search row (suited to dense scenes, where
-// lists overflow).  Every shape evaluates the same pairs in the same order
-// (a particle whose list fills up is finished by an overflow kernel in
-// candidate order), so results do not depend on the choice.
+// per block and hit-list capacity of the block form (one thread per particle
+// scans, four evaluate), or the threads per particle of the group form.
+// Every shape adds the same pair terms in the same order, so results do not
+// depend on the choice.
 struct FluidVariant {
     int block;       // threads per block
-    int cap;         // hit-list entries per thread
-    int persistent;  // tile-queue form
-    int flush;       // warp-voted list flushes (kFlush) instead of pass 1 then pass 2
-    int staged;      // candidates staged in shared memory per tile before the scan
-                     // (1: cooperative loads, 2: bulk copies on an mbarrier)
+    int cap;         // hit-list entries per particle
+    int lanes;       // group form: threads that share one particle; 0: the block form
 };
 constexpr int kNumFluidVariants = 15;
 extern const FluidVariant kFluidVariants[kNumFluidVariants];
-// `tile_counter` (one uint32 on the device) is used by persistent variants.
+constexpr uint32_t kScanPad = 32;
 int launch_fluid(const FluidArgs& a, const Tables& T, int kdim, const StageCoefs& c, const StageBuffers& b,
-                 int variant, uint32_t* tile_counter, cudaStream_t st);
+                 int variant, cudaStream_t st);
 
 // Velocity Verlet's kick and drift, in storage order: v' = v + (dt/2) a,
 // rho' = rho + (dt/2) drho/dt, x' = x + dt v' from the derivative record
-// (fpd, fvm) of the previous force evaluation; and the kick of a 4-float4
-// per-solid field (the plastic strain).  Return the launches issued.
+// (fpd, fvm) of the previous force evaluation, the drifted state counted into
+// cells; and the kick of a 4-float4 per-solid field (the plastic strain).
+// Return the launches issued.
 int verlet_kick_drift(const float4* pd, const float4* vm, const float4* fpd, const float4* fvm, uint32_t n, float half,
-                      float full, float4* out_pd, float4* out_vm, cudaStream_t st);
+                      float full, float4* out_pd, float4* out_vm, const Tables& T, const CellBins& bin,
+                      cudaStream_t st);
 int verlet_kick4(const float4* e, const float4* k4, uint32_t count, float half, float4* out, cudaStream_t st);
 
 // ---- solids (solid.cu) ------------------------------------------------------
@@ -320,8 +344,8 @@ struct SolidArgs {
     float4* A;                // [3*ns] sigma * L columns (stage scratch)
     float4* ksol;             // [ns] solid-term acceleration
     uint32_t* contact_bound;  // [2] max |u_i - u_0| bits, outside-box flag (cleared per stage)
-    const float4* xs;         // sorted stage positions (current-neighbor loop)
-    const float4* vs;
+    const float4* rec;        // sorted stage state (current-neighbor loop, see FluidArgs)
+    const uint32_t* mat;
     const uint32_t* start;
     const uint32_t* sid_sorted;
     float4* sx;               // [ns] stage position + density in solid-id order (gathered per stage)

@@ -8,7 +8,10 @@
 // search cell (the reference cell halved along x) and walks 3 (2D) or 9 (3D)
 // contiguous x-rows of 5 half-width cells, so neighbor loads are coalesced
 // across a warp (consecutive threads sit in the same or adjacent cells) and
-// 5/6 of the candidates of the 3x3x3 reference cells are tested.
+// 5/6 of the candidates of the 3x3x3 reference cells are tested; the pair
+// terms of the hits are then evaluated by four threads per particle (k_fluid).
+// Scenes too small to fill the GPU that way give each particle 4 to 16
+// threads throughout (k_fluid_group).
 //
 // Per pair the math is the shader's, term by term: continuity density rate,
 // symmetric pressure force with the equation of state evaluated for both
@@ -53,100 +56,134 @@ __device__ __forceinline__ float contact_potential(uint32_t eq, float r, float s
     }
 }
 
+// The particle a pair term is evaluated for.
 struct Self {
     float3 x, v;
-    float d1, m1, pterm1, f1, bf1;
-    uint32_t mat;     // global material id
-    bool elastic;
-    // material table and interaction row of the particle's scene, indexed by
-    // the neighbor's global material id (shared-memory copies for the block's
-    // first scene, the global tables otherwise)
-    const FluidMat* mt;
-    const DevInter* it;
+    float d1, m1, pterm1;
+    uint32_t mat;       // material id in the scene
+    const PairMat* pm;  // pair constants, indexed by the neighbor's material id in the scene (a shared-memory copy for
+                        // the block's first scene, the global table otherwise)
+};
+
+// The scene scalars the pair terms read, held in registers.
+struct PairK {
+    float h2, kg, eps_hh;  // kg = -6 kconst
 };
 
 struct Acc {
     float den;
-    float3 f;
+    float3 f, c;  // force without and with contact terms only
 };
 
-// One neighbor pair inside the kernel radius (the caller has tested it).
-// `ptj` is p_j / rho_j^2 of the neighbor, precomputed per particle.
-// The scene scalars the pair terms read, held in registers.
-struct PairK {
-    float h2, kconst, eps_hh;
+// What the pair terms read of a particle, one 32-byte sector and one load:
+// (x, y, z, rho), (vx, vy, vz, p / rho^2).
+struct PairRec {
+    float4 x, v;
 };
+__device__ __forceinline__ PairRec load_rec(const float4* rec, uint32_t j) {
+    PairRec r;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.x.x), "=f"(r.x.y), "=f"(r.x.z), "=f"(r.x.w), "=f"(r.v.x), "=f"(r.v.y), "=f"(r.v.z), "=f"(r.v.w)
+        : "l"(rec + 2 * (size_t)j));
+    return r;
+}
 
-template <int DIM, bool BOUNDARY>
-__device__ __forceinline__ void pair(const Self& s, float4 xj, float4 vj, float ptj, uint32_t mat2, bool elastic2,
-                                     const PairK& P, Acc& acc) {
-    const float rx = xj.x - s.x.x, ry = xj.y - s.x.y, rz = DIM == 3 ? xj.z - s.x.z : 0.0f;
-    const float r2 = DIM == 3 ? (rx * rx + ry * ry) + rz * rz : rx * rx + ry * ry;
-    const float diff = fmaxf(P.h2 - r2, 0.0f);
-    const float gws = -6.0f * P.kconst * diff * diff;
-    const float gx = gws * rx, gy = gws * ry, gz = gws * rz;
-    const float vx = vj.x - s.v.x, vy = vj.y - s.v.y, vz = DIM == 3 ? vj.z - s.v.z : 0.0f;
-    const float d2 = xj.w;
-    const FluidMat m2 = s.mt[mat2];
-    const float vgw = DIM == 3 ? (vx * gx + vy * gy) + vz * gz : vx * gx + vy * gy;
-    if (!BOUNDARY) acc.den += m2.mass * vgw;
-    const float pf = s.m1 * m2.mass * (s.pterm1 + ptj);
-    acc.f.x += pf * gx;
-    acc.f.y += pf * gy;
-    acc.f.z += pf * gz;
-    const DevInter it = s.it[mat2];
-    if (it.potential != ARP_CONTACT_ZERO) {
-        const float cp = contact_potential(it.potential, sqrtf(r2), it.radius, it.strength);
-        if (cp != 0.0f) {
-            const float cs = m2.mass * cp / d2;
-            const float cx = cs * gx, cy = cs * gy, cz = cs * gz;
-            if ((s.elastic || elastic2 || BOUNDARY) && s.mat != mat2) {
-                // fluid.rs:192-199: friction along the normalised tangential velocity
-                const float ix = rx / r2, iy = ry / r2, iz = rz / r2;
-                const float cr = DIM == 3 ? (cx * rx + cy * ry) + cz * rz : cx * rx + cy * ry;
-                const float nx = ix * cr, ny = iy * cr, nz = iz * cr;
-                const float vr = DIM == 3 ? (vx * rx + vy * ry) + vz * rz : vx * rx + vy * ry;
-                float tx = vx - ix * vr, ty = vy - iy * vr, tz = vz - iz * vr;
-                float tl = sqrtf(DIM == 3 ? (tx * tx + ty * ty) + tz * tz : tx * tx + ty * ty);
-                tx /= tl; ty /= tl; tz /= tl;
-                if (isfinite(tx) && isfinite(ty) && isfinite(tz)) {
-                    // normalize() applied a second time, as the shader does
-                    const float tl2 = sqrtf(DIM == 3 ? (tx * tx + ty * ty) + tz * tz : tx * tx + ty * ty);
-                    const float nl = sqrtf(DIM == 3 ? (nx * nx + ny * ny) + nz * nz : nx * nx + ny * ny);
-                    const float fr = it.friction * nl;
-                    acc.f.x += fr * (tx / tl2);
-                    acc.f.y += fr * (ty / tl2);
-                    acc.f.z += fr * (tz / tl2);
-                }
-            }
-            acc.f.x += cx;
-            acc.f.y += cy;
-            acc.f.z += cz;
+// What the terms of one neighbor pair share.  Every force term but the viscous
+// one and friction points along r = x_j - x_i, and every term carries
+// gws = |grad_w| / |r|, so the shader's sums of vectors
+// (pf grad_w - q grad_w + cs grad_w) are coefficients on r.
+struct PairGeom {
+    float3 r, v;
+    float r2, gws, vr;
+};
+template <int DIM>
+__device__ __forceinline__ PairGeom pair_geom(const Self& s, const PairRec& j, const PairK& P) {
+    PairGeom g;
+    g.r = make_float3(__fsub_rn(j.x.x, s.x.x), __fsub_rn(j.x.y, s.x.y), DIM == 3 ? __fsub_rn(j.x.z, s.x.z) : 0.0f);
+    const float rr = fmaf(g.r.y, g.r.y, __fmul_rn(g.r.x, g.r.x));
+    g.r2 = DIM == 3 ? fmaf(g.r.z, g.r.z, rr) : rr;
+    const float diff = fmaxf(__fsub_rn(P.h2, g.r2), 0.0f);
+    g.gws = __fmul_rn(__fmul_rn(P.kg, diff), diff);
+    g.v = make_float3(__fsub_rn(j.v.x, s.v.x), __fsub_rn(j.v.y, s.v.y), DIM == 3 ? __fsub_rn(j.v.z, s.v.z) : 0.0f);
+    const float vv = fmaf(g.v.y, g.r.y, __fmul_rn(g.v.x, g.r.x));
+    g.vr = DIM == 3 ? fmaf(g.v.z, g.r.z, vv) : vv;
+    return g;
+}
+
+// The terms of one pair inside the kernel radius (the caller has tested it),
+// contact aside: (density rate, force).  `ptj` is p_j / rho_j^2 of the
+// neighbor, precomputed per particle; v.r is shared by the continuity and the
+// artificial viscosity terms (v.grad_w = gws v.r).  Each operation is
+// separately rounded or an explicit fma, so every kernel that evaluates a pair
+// gets the same bits whatever the number of threads that share a particle.
+template <int DIM>
+__device__ __forceinline__ float4 pair_terms(const Self& s, const PairGeom& g, float d2, float ptj, bool boundary,
+                                             const PairMat& m, const PairK& P) {
+    const float mm = __fmul_rn(s.m1, m.mass);
+    const float denom = __fadd_rn(g.r2, P.eps_hh);
+    float p = __fadd_rn(s.pterm1, ptj);
+    // GLSL division carries 2.5 ulp; the 2-ulp hardware quotient is used in the viscosity terms
+    if (m.bulk != 0.0f)  // zero with a boundary particle
+        p = __fsub_rn(p, __fdividef(__fmul_rn(m.bulk, g.vr), __fmul_rn(__fadd_rn(s.d1, d2), denom)));
+    const float c = __fmul_rn(__fmul_rn(mm, p), g.gws);
+    float4 t;
+    t.x = __fmul_rn(boundary ? 0.0f : m.mass, __fmul_rn(g.gws, g.vr));
+    t.y = __fmul_rn(c, g.r.x);
+    t.z = __fmul_rn(c, g.r.y);
+    t.w = DIM == 3 ? __fmul_rn(c, g.r.z) : 0.0f;
+    if (m.visc != 0.0f) {  // zero for an elastic particle and with a boundary particle
+        const float q = __fmul_rn(__fmul_rn(mm, m.visc), __fmul_rn(g.gws, g.r2));
+        const float u = __fdividef(q, __fmul_rn(__fmul_rn(s.d1, d2), denom));
+        t.y = fmaf(-u, g.v.x, t.y);
+        t.z = fmaf(-u, g.v.y, t.z);
+        if (DIM == 3) t.w = fmaf(-u, g.v.z, t.w);
+    }
+    return t;
+}
+
+// The contact potential and friction of one pair (fluid.rs:176-199).  Few
+// pairs have one, and its registers would cost every pair a quarter of the
+// resident warps (94 registers against 64), so contacts are evaluated in a
+// second walk over the hits, taken only where some hit has one, and have sums
+// of their own.
+template <int DIM>
+__device__ __forceinline__ float3 contact_terms(const Self& s, const PairGeom& g, float d2, float mass2, uint32_t mat2,
+                                                bool rubs, const DevInter& it) {
+    float3 f = make_float3(0.0f, 0.0f, 0.0f);
+    const float cp = contact_potential(it.potential, sqrtf(g.r2), it.radius, it.strength);
+    if (cp == 0.0f) return f;
+    const float cs = __fmul_rn(__fdiv_rn(__fmul_rn(mass2, cp), d2), g.gws);
+    f = make_float3(__fmul_rn(cs, g.r.x), __fmul_rn(cs, g.r.y), __fmul_rn(cs, g.r.z));
+    if (it.friction != 0.0f && rubs && s.mat != mat2) {
+        // fluid.rs:192-199: friction along the normalised tangential velocity
+        const float ix = g.r.x / g.r2, iy = g.r.y / g.r2, iz = g.r.z / g.r2;
+        const float cr = __fmul_rn(cs, g.r2);  // contact force . r
+        const float nx = ix * cr, ny = iy * cr, nz = iz * cr;
+        float tx = g.v.x - ix * g.vr, ty = g.v.y - iy * g.vr, tz = g.v.z - iz * g.vr;
+        const float tl = sqrtf(DIM == 3 ? (tx * tx + ty * ty) + tz * tz : tx * tx + ty * ty);
+        tx /= tl; ty /= tl; tz /= tl;
+        if (isfinite(tx) && isfinite(ty) && isfinite(tz)) {
+            // normalize() applied a second time, as the shader does
+            const float tl2 = sqrtf(DIM == 3 ? (tx * tx + ty * ty) + tz * tz : tx * tx + ty * ty);
+            const float nl = sqrtf(DIM == 3 ? (nx * nx + ny * ny) + nz * nz : nx * nx + ny * ny);
+            const float fr = it.friction * nl;
+            f = make_float3(__fadd_rn(f.x, __fmul_rn(fr, tx / tl2)), __fadd_rn(f.y, __fmul_rn(fr, ty / tl2)),
+                            DIM == 3 ? __fadd_rn(f.z, __fmul_rn(fr, tz / tl2)) : 0.0f);
         }
     }
-    if (!BOUNDARY) {
-        const float denom = r2 + P.eps_hh;
-        if (!s.elastic) {
-            const float fsum = s.f1 + m2.visc;
-            if (fsum != 0.0f) {
-                const float rgw = DIM == 3 ? (rx * gx + ry * gy) + rz * gz : rx * gx + ry * gy;
-                const float q = s.m1 * m2.mass * fsum * rgw;
-                const float dd = s.d1 * d2 * denom;
-                // GLSL division carries 2.5 ulp; the 2-ulp hardware quotient is used here
-                acc.f.x -= __fdividef(q * vx, dd);
-                acc.f.y -= __fdividef(q * vy, dd);
-                acc.f.z -= __fdividef(q * vz, dd);
-            }
-        }
-        const float f_ = s.mat == mat2 ? s.bf1 + m2.bulk : it.dampening;
-        if (f_ != 0.0f) {
-            const float vr = DIM == 3 ? (vx * rx + vy * ry) + vz * rz : vx * rx + vy * ry;
-            const float q = s.m1 * m2.mass * __fdividef(f_ * vr, (s.d1 + d2) * denom);
-            acc.f.x -= q * gx;
-            acc.f.y -= q * gy;
-            acc.f.z -= q * gz;
-        }
-    }
+    return f;
+}
+
+__device__ __forceinline__ void add_terms(Acc& acc, float4 t) {
+    acc.den = __fadd_rn(acc.den, t.x);
+    acc.f.x = __fadd_rn(acc.f.x, t.y);
+    acc.f.y = __fadd_rn(acc.f.y, t.z);
+    acc.f.z = __fadd_rn(acc.f.z, t.w);
+}
+__device__ __forceinline__ void add_contact(Acc& acc, float3 t) {
+    acc.c.x = __fadd_rn(acc.c.x, t.x);
+    acc.c.y = __fadd_rn(acc.c.y, t.y);
+    acc.c.z = __fadd_rn(acc.c.z, t.z);
 }
 
 __device__ __forceinline__ float4 comb(float4 y0, float4 t, bool keep_w) {
@@ -162,44 +199,57 @@ __device__ __forceinline__ float4 axpy(float c, float4 k, float4 t) {
                        __fadd_rn(t.z, __fmul_rn(c, k.z)), __fadd_rn(t.w, __fmul_rn(c, k.w)));
 }
 
-constexpr uint32_t kBoundaryBit = 0x80000000u;
+// The scan and the evaluation see one array of particles: the n mobile ones in
+// cell order, then the boundary ones in theirs, so a neighbor is an index and
+// a boundary particle one of at least n.
 
-// Copy one scene's fluid materials and interaction block into shared memory.
-__device__ __forceinline__ void load_scene_tables(const Tables& T, uint32_t scene, FluidMat* sm, DevInter* si) {
-    const SceneP& sp = T.scenes[scene];
-    for (uint32_t i = threadIdx.x; i < sp.nmat; i += blockDim.x) sm[i] = T.fmats[sp.mat_base + i];
-    for (uint32_t i = threadIdx.x; i < sp.nmat * sp.nmat; i += blockDim.x) si[i] = T.inter[sp.inter_base + i];
-}
-
-// Pair terms of one hit: a boundary particle (index | kBoundaryBit) or a
-// mobile one.
+// Pair terms of neighbor j added to `acc` if j lies within the kernel radius
+// (the scan's test lets a few others through); the pair's material bits are
+// or-ed into `bits`.  r^2 < h^2 is h^2 - r^2 > 0, grad_w's max(.., 0) test:
+// without flush-to-zero a difference of finite floats is zero only when they
+// are equal.
 template <int DIM>
-__device__ __forceinline__ void eval_hit(uint32_t j, const Self& s, const FluidArgs& a, const PairK& K, Acc& acc) {
-    if (j & kBoundaryBit) {
-        const uint32_t jb = j & ~kBoundaryBit;
-        const float4 xj = a.bxs[jb];
-        const float4 vj = a.bvs[jb];
-        const uint32_t mat2 = __float_as_uint(vj.w);
-        bool elastic2 = false;
-        if (a.any_stiff_immobile && s.mt[mat2].stiff) {
-            // fluid.rs:141: the boundary index reads the mobile array's solid id
-            elastic2 = a.sid_of_boundary_index[a.borig[jb]] != kInvalid;
-        }
-        pair<DIM, true>(s, xj, vj, a.bps[jb], mat2, elastic2, K, acc);
-    } else {
-        const float4 xj = a.xs[j];
-        const float4 vj = a.vs[j];
-        const uint32_t mat2 = __float_as_uint(vj.w);
-        pair<DIM, false>(s, xj, vj, a.ps[j], mat2, s.mt[mat2].stiff != 0u, K, acc);
+__device__ __forceinline__ void add_hit(Acc& acc, uint32_t j, const PairRec& rj, uint32_t mat2, const Self& s,
+                                        const FluidArgs& a, const PairK& K, uint32_t& bits) {
+    const PairMat m = s.pm[mat2];
+    const PairGeom g = pair_geom<DIM>(s, rj, K);
+    const float4 t = pair_terms<DIM>(s, g, rj.x.w, rj.v.w, j >= a.n, m, K);
+    if (g.r2 < K.h2) {
+        add_terms(acc, t);
+        bits |= m.bits;
     }
+}
+// The contact terms of neighbor j, if there are any.  `it`: the interactions of
+// the particle's material.
+template <int DIM>
+__device__ __forceinline__ void add_hit_contact(Acc& acc, uint32_t j, const Self& s, const FluidArgs& a,
+                                                const DevInter* it, const PairK& K) {
+    const uint32_t mat2 = a.mat8[j];
+    const PairMat m = s.pm[mat2];
+    if ((m.bits & kPairPotential) == ARP_CONTACT_ZERO) return;
+    const PairRec rj = load_rec(a.rec, j);
+    const PairGeom g = pair_geom<DIM>(s, rj, K);
+    if (!(g.r2 < K.h2)) return;
+    const bool rubs = j >= a.n || (m.bits & (kPairElastic1 | kPairElastic2));
+    add_contact(acc, contact_terms<DIM>(s, g, rj.x.w, m.mass, mat2, rubs, it[mat2]));
 }
 
 // The derivative record of one particle (fluid.rs:243-247, plus the solid
 // term when active) and the Runge-Kutta stage epilogue: the store of k, the
-// b-weighted accumulator and the next stage state, in storage slot `slot`.
-__device__ __forceinline__ void stage_epilogue(const FluidArgs& a, const StageCoefs& c, const StageBuffers& b,
-                                               uint32_t slot, uint32_t sid, float4 vi, const Acc& acc, float d1,
-                                               float g_acc, bool solid_scene) {
+// b-weighted accumulator and the next stage state of sorted particle k, in its
+// storage slot.  With b.bin.count the new state is counted into its search
+// cell on the way (the first pass of the grid build that follows, which then
+// need not read the positions again).
+__device__ __forceinline__ void stage_epilogue(const FluidArgs& a, const Tables& T, const StageCoefs& c,
+                                               const StageBuffers& b, uint32_t k, const Acc& acc) {
+    const uint32_t slot = a.perm ? a.perm[k] : k;
+    const uint32_t sid = a.sid[slot];
+    const SceneP& P = T.scenes[T.mats[a.mat[k]].scene];
+    const PairRec self = load_rec(a.rec, k);
+    const float4 vi = self.v;
+    const float d1 = self.x.w;
+    const float g_acc = P.g;
+    const bool solid_scene = P.solid_branch != 0u;
     float4 kpd = make_float4(vi.x, vi.y, vi.z, acc.den);
     float4 kvm = make_float4(__fdiv_rn(acc.f.x, d1), __fadd_rn(__fdiv_rn(acc.f.y, d1), -g_acc),
                              __fdiv_rn(acc.f.z, d1), 0.0f);
@@ -236,8 +286,9 @@ __device__ __forceinline__ void stage_epilogue(const FluidArgs& a, const StageCo
         accp = b.acc_pd[slot];
         accv = b.acc_vm[slot];
     }
+    float4 np;
     if (c.last) {
-        float4 np = comb(y0p, accp, false);
+        np = comb(y0p, accp, false);
         if (c.kick) {  // a velocity-Verlet kick moves no particle: positions come from the drift
             np.x = y0p.x;
             np.y = y0p.y;
@@ -263,623 +314,513 @@ __device__ __forceinline__ void stage_epilogue(const FluidArgs& a, const StageCo
             tp = axpy(c.c_self, kpd, tp);
             tv = axpy(c.c_self, kvm, tv);
         }
-        b.next_pd[slot] = comb(y0p, tp, false);
+        np = comb(y0p, tp, false);
+        b.next_pd[slot] = np;
         b.next_vm[slot] = comb(y0v, tv, true);
     }
+    if (b.bin.count) bin_particle(np, P, T.ncells, slot, b.bin);
 }
 
-// The particle's own fields and table pointers for the pair loop; returns
-// its scene.  `sm`/`si` hold the tables of scene `scene0`.
-__device__ __forceinline__ const SceneP& init_self(uint32_t k, float4 xi, float4 vi, uint32_t sid, const FluidArgs& a,
-                                                   const Tables& T, const FluidMat* sm, const DevInter* si,
+// The particle's own fields for the pair terms; returns its scene.  `sm`: the
+// pair constants of scene `scene0` (kInvalid: none).
+__device__ __forceinline__ const SceneP& init_self(uint32_t k, const FluidArgs& a, const Tables& T, const PairMat* sm,
                                                    uint32_t scene0, Self& s) {
-    s.x = make_float3(xi.x, xi.y, xi.z);
-    s.v = make_float3(vi.x, vi.y, vi.z);
-    s.mat = __float_as_uint(vi.w);
-    const uint32_t scene = T.mats[s.mat].scene;
-    const SceneP& P = T.scenes[scene];
-    const uint32_t li = s.mat - P.mat_base;
-    // pre-offset so that [global id] lands on the scene's entry
-    s.mt = (scene == scene0 ? sm : T.fmats + P.mat_base) - P.mat_base;
-    s.it = (scene == scene0 ? si : T.inter + P.inter_base) + li * P.nmat - P.mat_base;
-    s.d1 = xi.w;
-    const FluidMat m1 = s.mt[s.mat];
-    s.m1 = m1.mass;
-    s.f1 = m1.visc;
-    s.bf1 = m1.bulk;
-    s.elastic = sid != kInvalid && m1.stiff;
-    s.pterm1 = a.ps[k];
+    const PairRec r = load_rec(a.rec, k);
+    const uint32_t mat = a.mat[k];
+    s.x = make_float3(r.x.x, r.x.y, r.x.z);
+    s.v = make_float3(r.v.x, r.v.y, r.v.z);
+    s.d1 = r.x.w;
+    s.pterm1 = r.v.w;
+    const DevMat& m = T.mats[mat];
+    const SceneP& P = T.scenes[m.scene];
+    s.mat = mat - P.mat_base;
+    s.m1 = m.mass;
+    s.pm = (m.scene == scene0 ? sm : T.pmats + P.inter_base) + s.mat * P.nmat;
     return P;
 }
 
-// How fluid_particle collects and evaluates the hits of a particle.  Every
-// mode sums the pairs in candidate order, so results do not depend on the
-// mode, CAP or the launch shape.
-enum FluidMode {
-    kTwoPass = 0,  // pass 1 fills the list, pass 2 evaluates it; a full list
-                   // queues the particle for kFlush (first overflow queue)
-    kFlush = 1,    // the warp agrees before each row whether some lane's list
-                   // could fill up in it and then evaluates and empties every
-                   // list; a row alone above CAP queues the particle for
-                   // kDirect (second overflow queue)
-    kDirect = 2,   // every hit evaluated during the scan (a row above even the
-                   // second queue's list)
+// The rows of search cells around a particle: row q (ascending z, then y; the
+// order of for_search_rows) spans `width` cells from search_row(q) on.
+struct SearchRows {
+    int y, z, x0, ry, nrows;
+    uint32_t width;
 };
-
-// Fluid forces and the stage update of sorted particle k.  `lst` is the
-// thread's column of the hit list ([CAP][BLOCK]); `sm`/`si` hold the
-// tables of scene `scene0`.  A particle handed to an overflow queue writes
-// nothing here.  `wmask` (kFlush): the lanes of this warp that run
-// fluid_particle, all of which take part in the per-row vote.  QUEUE false
-// (kFlush): a particle whose row holds more than CAP hits is not queued; the
-// call returns false, having written nothing, and the caller finishes it.
-template <int DIM, int BLOCK, int CAP, int MODE, bool QUEUE = true>
-__device__ __forceinline__ bool fluid_particle(uint32_t k, const FluidArgs& a, const Tables& T, const StageCoefs& c,
-                                               const StageBuffers& b, uint32_t* lst, const FluidMat* sm,
-                                               const DevInter* si, uint32_t scene0, unsigned wmask) {
-    const float4 xi = a.xs[k];
-    const float4 vi = a.vs[k];
-    const uint32_t slot = a.perm ? a.perm[k] : k;
-    const uint32_t sid = a.sid[slot];
-    Self s;
-    const SceneP& P = init_self(k, xi, vi, sid, a, T, sm, si, scene0, s);
-    const PairK K{P.h2, P.kconst, P.eps_hh};
-    const float g_acc = P.g;
-
-    Acc acc;
-    acc.den = 0.0f;
-    acc.f = make_float3(0.0f, 0.0f, 0.0f);
-    uint32_t* my = lst;
-    uint32_t cnt = 0;
-    bool full = false;
-    // pass 1: candidates of the search rows whose squared distance is inside
-    // h^2 (r^2 < h^2 is h^2 - r^2 > 0, grad_w's max(.., 0) test: without
-    // flush-to-zero a difference of finite floats is zero only when they are
-    // equal).  The particle itself passes the test and is dropped when the
-    // hits are evaluated, which keeps the index compare out of this loop.
-    auto hit = [&](float4 q) {
-        const float rx = q.x - xi.x, ry = q.y - xi.y;
-        const float r2 = DIM == 3 ? fmaf(q.z - xi.z, q.z - xi.z, fmaf(ry, ry, rx * rx)) : fmaf(ry, ry, rx * rx);
-        return r2 < K.h2;
-    };
-    constexpr bool DIRECT = MODE == kDirect;
-    auto take = [&](uint32_t j) {
-        if (DIRECT) {
-            if (j != k) eval_hit<DIM>(j, s, a, K, acc);
-        } else if (cnt < CAP) {
-            my[cnt++ * BLOCK] = j;
-        } else {
-            full = true;
-        }
-    };
-    // pass 2 over the hits collected so far, in candidate order
-    auto flush = [&]() {
-        for (uint32_t e = 0; e < cnt; ++e) {
-            const uint32_t j = my[e * BLOCK];
-            if (j != k) eval_hit<DIM>(j, s, a, K, acc);
-        }
-        cnt = 0;
-    };
-    if (MODE == kFlush) {
-        // The search rows (x-rows of the search cells within reach, see
-        // for_search_rows) in a fixed order and number for every lane, rows
-        // outside the grid (and every row of a non-finite particle) empty, so
-        // that the warp can vote before each row; the pass after the last row
-        // only evaluates what is left (one call site of the pair math keeps
-        // the registers down).
-        // (y reach: 2 rows for every lane, as dense scenes halve y; a lane
-        // whose scene does not skips the outer two as empty)
-        constexpr int RY = 2, RZ = 1 + (int)(kSearchHalve >> 2 & 1u);
-        constexpr int NY = 2 * RY + 1, NZ = DIM == 3 ? 2 * RZ + 1 : 1;
-        const bool fin = finite3(xi);
-        const Grid& g = P.sgrid;
-        const CellCoord cc = fin ? cell_coord(xi, g) : CellCoord{0, 0, 0};
-        const int rx = 1 + (int)P.halved[0], ry = 1 + (int)P.halved[1];
-        const int x0 = max(cc.x - rx, 0), x1 = min(cc.x + rx, (int)g.sub[0] - 1);
-        for (int r = 0;; ++r) {
-            const bool last = r == NY * NZ;
-            const int dy = r % NY - RY;
-            const int y = cc.y + dy;
-            const int z = DIM == 3 ? cc.z - RZ + r / NY : cc.z;
-            uint32_t bb = 0, be = 0, jb = 0, je = 0;
-            if (!last && fin && abs(dy) <= ry && y >= 0 && y < (int)g.sub[1] && z >= 0 && z < (int)g.sub[2]) {
-                const uint32_t row = P.cell_base + (uint32_t)y * g.sub[0] + (uint32_t)z * g.sub[0] * g.sub[1];
-                const uint32_t c0 = row + (uint32_t)x0, c1 = row + (uint32_t)x1 + 1u;
-                bb = a.bstart[c0];
-                be = a.bstart[c1];
-                jb = a.start[c0];
-                je = a.start[c1];
-            }
-            const bool fl = last || __any_sync(wmask, !full && cnt + (be - bb) + (je - jb) > (uint32_t)CAP);
-            if (fl && !full) flush();
-            if (last) break;
-            if (full) continue;
-            for (uint32_t j = bb; j < be; ++j)
-                if (hit(a.bxs[j])) take(j | kBoundaryBit);
-            for (uint32_t j = jb; j < je; ++j)
-                if (hit(a.xs[j])) take(j);
-        }
-        if (full) {
-            if (!QUEUE) return false;
-            a.overflow[a.n + atomicAdd(a.overflow_count + 1, 1u)] = k;
-            return true;
-        }
-    } else if (finite3(xi)) {
-        for_search_rows<DIM>(xi, P, [&](uint32_t c0, uint32_t c1) {
-            if (full) return;
-            const uint32_t bb = a.bstart[c0], be = a.bstart[c1];
-            for (uint32_t j = bb; j < be; ++j)
-                if (hit(a.bxs[j])) take(j | kBoundaryBit);
-            const uint32_t jb = a.start[c0], je = a.start[c1];
-            uint32_t j = jb;
-            for (; j + 3u < je; j += 4u) {  // four loads in flight
-                const float4 q0 = a.xs[j], q1 = a.xs[j + 1u], q2 = a.xs[j + 2u], q3 = a.xs[j + 3u];
-                const bool h0 = hit(q0), h1 = hit(q1), h2 = hit(q2), h3 = hit(q3);
-                if (h0) take(j);
-                if (h1) take(j + 1u);
-                if (h2) take(j + 2u);
-                if (h3) take(j + 3u);
-            }
-            for (; j < je; ++j)
-                if (hit(a.xs[j])) take(j);
-        });
-        if (MODE == kTwoPass) {
-            if (full) {
-                a.overflow[atomicAdd(a.overflow_count, 1u)] = k;
-                return true;
-            }
-            flush();  // pass 2
-        }
-    }
-
-    stage_epilogue(a, c, b, slot, sid, vi, acc, s.d1, g_acc, P.solid_branch != 0u);
-    return true;
+template <int DIM>
+__device__ __forceinline__ SearchRows search_rows(float4 x, bool scan, const SceneP& P) {
+    constexpr int RZ = 1 + (int)(kSearchHalve >> 2 & 1u);
+    const Grid& g = P.sgrid;
+    const CellCoord c = scan ? cell_coord(x, g) : CellCoord{0, 0, 0};
+    const int rx = 1 + (int)P.halved[0];
+    SearchRows r;
+    r.ry = 1 + (int)P.halved[1];
+    r.y = c.y - r.ry;
+    r.z = DIM == 3 ? c.z - RZ : c.z;
+    r.x0 = max(c.x - rx, 0);
+    r.width = (uint32_t)(min(c.x + rx, (int)g.sub[0] - 1) - r.x0) + 1u;
+    r.nrows = scan ? (2 * r.ry + 1) * (DIM == 3 ? 2 * RZ + 1 : 1) : 0;
+    return r;
+}
+// First cell of row q, or kInvalid outside the grid.
+__device__ __forceinline__ uint32_t search_row(const SearchRows& r, int q, const SceneP& P) {
+    const int qz = r.ry == 1 ? q / 3 : q / 5;
+    const int y = r.y + q - qz * (2 * r.ry + 1), z = r.z + qz;
+    const Grid& g = P.sgrid;
+    if (y < 0 || y >= (int)g.sub[1] || z < 0 || z >= (int)g.sub[2]) return kInvalid;
+    return P.cell_base + (uint32_t)r.x0 + (uint32_t)y * g.sub[0] + (uint32_t)z * g.sub[0] * g.sub[1];
 }
 
-// The flush form keeps the row loop's state live around the pair math; left
-// alone the compiler gives it 92 registers (5 blocks of 128 per SM), and
-// holding it to 7 blocks (72 registers, a few spilled) ran the batched
-// workload's fluid kernel 7 % faster.  The two-pass form keeps the
-// compiler's own choice (72 registers at 128 threads; an explicit minimum of
-// one block raises it to 80).
-constexpr int kFlushMinBlocks = 7;
+// How the terms of a particle's hits are added up, in every form: hit e of the
+// candidate order goes to partial sum e mod 4, each partial sum adds its hits
+// in order, and the total is (p0 + p1) + (p2 + p3); contact terms likewise in
+// sums of their own, whose total is added last.  Results therefore depend
+// neither on the launch shape nor on how lists are cut.
+constexpr int kPartials = 4;
+__device__ __forceinline__ float sum_partials(float v) {  // over the lanes that differ in their two lowest bits
+    v = __fadd_rn(v, __shfl_xor_sync(0xFFFFFFFFu, v, 1));
+    return __fadd_rn(v, __shfl_xor_sync(0xFFFFFFFFu, v, 2));
+}
 
-// One tile of BLOCK sorted particles per block.
-template <int DIM, int BLOCK, int CAP, int MODE>
-__device__ __forceinline__ void fluid_tile(const FluidArgs& a, const Tables& T, const StageCoefs& c,
-                                           const StageBuffers& b) {
+// ---- block form -----------------------------------------------------------------
+// BLOCK consecutive cell-sorted particles per block, in two phases per warp.
+//   * Scan, one thread per particle: the quantised candidates of its search
+//     rows, four to a load, tested into a bit mask of 32; the set bits are
+//     appended to its list of CAP entries in shared memory (an odd stride between
+//     lists, so lanes at equal counts hit different banks).
+//   * Evaluation, four threads per particle, eight particles of the warp at a
+//     time: thread q takes hits q, q + 4, ...  Consecutive hits of a particle are
+//     mostly consecutive slots of a search row, so the eight lanes that share
+//     one L1 pass read two particles' runs instead of eight unrelated places.
+// A lane whose list is full stops scanning; the warp then evaluates all lists
+// (whole rounds of four, the rest moves to the list's front), keeps the partial
+// sums in the tail of the lists of unfinished particles and scans on, so a
+// particle may have any number of hits.
+//
+// Bound: L1 data wavefronts (70 % of peak) and issue slots (64 %), with L1 and
+// L2 latency behind them (4.6 warps per issue on the long scoreboard); DRAM is
+// idle.  What it replaced, one thread per particle over 16-byte candidates
+// read from the positions, took 352 us per stage of the 1,048,576-particle
+// fluid and bar scene (RK2, 222 M warp instructions, 69 M wavefronts) and two
+// more launches for the particles whose lists overflowed; this takes 292 us
+// (202 M, 59 M), the next state's cell keys included.  On the way: 4 threads per
+// particle alone 372 us; + quantised candidates 345 us; + 32-byte records 330 us;
+// + the next row's bounds and a second hit's record in flight 292 us.
+// kBlocksPerSM 128-thread blocks per SM (72 registers): 8 (64 registers, spills)
+// take 6 % more, 6 (80 registers) 2 % more.
+constexpr int kBlocksPerSM = 7;
+template <int DIM, int BLOCK, int CAP>
+__global__ void __launch_bounds__(BLOCK, kBlocksPerSM * 128 / BLOCK) k_fluid(FluidArgs a, Tables T, StageCoefs c, StageBuffers b) {
+    constexpr int STRIDE = CAP + 1;
+    constexpr int TAIL = 7 * kPartials;  // words of saved partial sums
+    static_assert(CAP % 2 == 0 && CAP >= TAIL + 8, "odd stride; room to go on beside the saved sums");
+    constexpr unsigned FULL = 0xFFFFFFFFu;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint32_t* lst = reinterpret_cast<uint32_t*>(smem_raw);
-    FluidMat* sm = reinterpret_cast<FluidMat*>(smem_raw + sizeof(uint32_t) * CAP * BLOCK);
-    DevInter* si = reinterpret_cast<DevInter*>(reinterpret_cast<unsigned char*>(sm) + sizeof(FluidMat) * T.max_nmat);
+    uint32_t* const lists = reinterpret_cast<uint32_t*>(smem_raw);
+    PairMat* const sm = reinterpret_cast<PairMat*>(smem_raw + sizeof(uint32_t) * STRIDE * BLOCK);
     const uint32_t k0 = blockIdx.x * BLOCK;
-    const uint32_t scene0 = T.mats[__float_as_uint(a.vs[min(k0, a.n - 1u)].w)].scene;
-    load_scene_tables(T, scene0, sm, si);
+    const uint32_t scene0 = T.mats[a.mat[k0]].scene;  // k0 < n: one block per started tile
+    {
+        const SceneP& S0 = T.scenes[scene0];
+        for (uint32_t i = threadIdx.x; i < S0.nmat * S0.nmat; i += BLOCK) sm[i] = T.pmats[S0.inter_base + i];
+    }
     __syncthreads();
     const uint32_t k = k0 + threadIdx.x;
-    const unsigned wmask = MODE == kFlush ? __ballot_sync(0xFFFFFFFFu, k < a.n) : 0u;  // lanes with a particle
-    if (k < a.n) fluid_particle<DIM, BLOCK, CAP, MODE>(k, a, T, c, b, lst + threadIdx.x, sm, si, scene0, wmask);
-}
-
-// Persistent form: each block keeps taking the next tile of the cell-sorted,
-// scene-concatenated order from an atomic work counter, so scenes of very
-// different sizes share the SMs without a tail of idle blocks.  Blocks never
-// wait on each other.
-template <int DIM, int BLOCK, int CAP, int MODE>
-__device__ __forceinline__ void fluid_tiles_persistent(const FluidArgs& a, const Tables& T, const StageCoefs& c,
-                                                       const StageBuffers& b, uint32_t* tile_counter) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint32_t* lst = reinterpret_cast<uint32_t*>(smem_raw);
-    FluidMat* sm = reinterpret_cast<FluidMat*>(smem_raw + sizeof(uint32_t) * CAP * BLOCK);
-    DevInter* si = reinterpret_cast<DevInter*>(reinterpret_cast<unsigned char*>(sm) + sizeof(FluidMat) * T.max_nmat);
-    __shared__ uint32_t tile_s;
-    uint32_t loaded = kInvalid;
-    const uint32_t ntiles = (a.n + BLOCK - 1) / BLOCK;
-    for (;;) {
-        if (threadIdx.x == 0) tile_s = atomicAdd(tile_counter, 1u);
-        __syncthreads();
-        const uint32_t tile = tile_s;
-        if (tile >= ntiles) break;
-        const uint32_t k0 = tile * BLOCK;
-        const uint32_t scene0 = T.mats[__float_as_uint(a.vs[k0].w)].scene;
-        if (scene0 != loaded) {
-            load_scene_tables(T, scene0, sm, si);
-            loaded = scene0;
-        }
-        __syncthreads();
-        const uint32_t k = k0 + threadIdx.x;
-        const unsigned wmask = MODE == kFlush ? __ballot_sync(0xFFFFFFFFu, k < a.n) : 0u;  // lanes with a particle
-        if (k < a.n) fluid_particle<DIM, BLOCK, CAP, MODE>(k, a, T, c, b, lst + threadIdx.x, sm, si, scene0, wmask);
-        __syncthreads();
-    }
-}
-
-template <int DIM, int BLOCK, int CAP>
-__global__ void __launch_bounds__(BLOCK) k_fluid(FluidArgs a, Tables T, StageCoefs c, StageBuffers b) {
-    fluid_tile<DIM, BLOCK, CAP, kTwoPass>(a, T, c, b);
-}
-template <int DIM, int BLOCK, int CAP>
-__global__ void __launch_bounds__(BLOCK) k_fluid_persistent(FluidArgs a, Tables T, StageCoefs c, StageBuffers b,
-                                                            uint32_t* tile_counter) {
-    fluid_tiles_persistent<DIM, BLOCK, CAP, kTwoPass>(a, T, c, b, tile_counter);
-}
-template <int DIM, int BLOCK, int CAP>
-__global__ void __launch_bounds__(BLOCK, kFlushMinBlocks * 128 / BLOCK)
-    k_fluid_flush(FluidArgs a, Tables T, StageCoefs c, StageBuffers b) {
-    fluid_tile<DIM, BLOCK, CAP, kFlush>(a, T, c, b);
-}
-template <int DIM, int BLOCK, int CAP>
-__global__ void __launch_bounds__(BLOCK, kFlushMinBlocks * 128 / BLOCK)
-    k_fluid_flush_persistent(FluidArgs a, Tables T, StageCoefs c, StageBuffers b, uint32_t* tile_counter) {
-    fluid_tiles_persistent<DIM, BLOCK, CAP, kFlush>(a, T, c, b, tile_counter);
-}
-
-// The kernels of one launch shape (only the used ones are instantiated).
-template <int DIM, int BLOCK, int CAP, int MODE>
-struct FluidKernels {
-    static constexpr auto tile_kernel() {
-        if constexpr (MODE == kFlush) return k_fluid_flush<DIM, BLOCK, CAP>;
-        else return k_fluid<DIM, BLOCK, CAP>;
-    }
-    static constexpr auto persistent_kernel() {
-        if constexpr (MODE == kFlush) return k_fluid_flush_persistent<DIM, BLOCK, CAP>;
-        else return k_fluid_persistent<DIM, BLOCK, CAP>;
-    }
-    static constexpr auto tile = tile_kernel();
-    static constexpr auto persistent = persistent_kernel();
-};
-
-// First overflow queue: particles whose hit list filled up, evaluated with
-// list flushes (kFlush), grid-stride over the queue.
-constexpr int kFlushCap = 64;
-template <int DIM>
-__global__ void __launch_bounds__(128, kFlushMinBlocks) k_fluid_overflow_flush(FluidArgs a, Tables T, StageCoefs c,
-                                                                                StageBuffers b) {
-    __shared__ uint32_t lst[kFlushCap * 128];
-    const uint32_t cnt = a.overflow_count[0];
-    for (uint32_t i0 = blockIdx.x * 128u; i0 < cnt; i0 += gridDim.x * 128u) {  // uniform per block
-        const uint32_t i = i0 + threadIdx.x;
-        const unsigned wmask = __ballot_sync(0xFFFFFFFFu, i < cnt);  // lanes with a particle
-        if (i < cnt)
-            fluid_particle<DIM, 128, kFlushCap, kFlush>(a.overflow[i], a, T, c, b, lst + threadIdx.x, nullptr,
-                                                         nullptr, kInvalid, wmask);
-    }
-}
-
-// Second overflow queue: particles with more hits in one row than the list
-// that queued them holds.  The same flushing scan with lists of kWideCap
-// entries (64 threads per block, 40 KB of shared memory); a particle with
-// even more hits in one row is finished by its own thread evaluating its
-// pairs during the scan.
-constexpr int kWideCap = 160;
-template <int DIM>
-__global__ void __launch_bounds__(64) k_fluid_overflow(FluidArgs a, Tables T, StageCoefs c, StageBuffers b) {
-    __shared__ uint32_t lst[kWideCap * 64];
-    const uint32_t cnt = a.overflow_count[1];
-    for (uint32_t i0 = blockIdx.x * 64u; i0 < cnt; i0 += gridDim.x * 64u) {  // uniform per block
-        const uint32_t i = i0 + threadIdx.x;
-        const unsigned wmask = __ballot_sync(0xFFFFFFFFu, i < cnt);  // lanes with a particle
-        if (i < cnt) {
-            const uint32_t k = a.overflow[a.n + i];
-            if (!fluid_particle<DIM, 64, kWideCap, kFlush, false>(k, a, T, c, b, lst + threadIdx.x, nullptr,
-                                                                   nullptr, kInvalid, wmask))
-                fluid_particle<DIM, 64, 1, kDirect>(k, a, T, c, b, nullptr, nullptr, nullptr, kInvalid, 0u);
-        }
-    }
-}
-
-// ---- staged form -----------------------------------------------------------
-// One tile of BLOCK consecutive cell-sorted particles per block, with the
-// candidates of the tile staged in shared memory before the scan.  The tile's
-// particles lie in a few x-rows of search cells ("own rows"); for each own row
-// the NY x NZ neighbor rows it reaches are windows of contiguous cells, and
-// the positions of each window (a contiguous range of the sorted state) are
-// copied into shared memory once per block, instead of each thread reading
-// every candidate through L1 (a tile's particles share most candidates).
-// The scan then reads candidates from shared memory in the order the global
-// scan visits them (rows z-major, then y, cells ascending; boundary
-// candidates first in each row, read from global memory), so the pairs are
-// summed in the same order and the results are the same bits.  A tile with
-// more own rows than kMaxOwnRows or more candidates than kStageSlots sends its
-// particles to the first overflow queue.
-constexpr int kStageSlots = 1536;   // staged positions per block (24 KB)
-constexpr int kMaxOwnRows = 4;
-constexpr int kStageRY = 2;         // y reach of a dense scene (x-halved scenes use 1)
-constexpr int kStageRZ = 1 + (int)(kSearchHalve >> 2 & 1u);
-constexpr int kStageNY = 2 * kStageRY + 1;
-
-template <int DIM>
-struct StageShape {
-    static constexpr int NZ = DIM == 3 ? 2 * kStageRZ + 1 : 1;
-    static constexpr int NQ = kStageNY * NZ;   // windows per own row
-    static constexpr int NW = kMaxOwnRows * NQ;
-};
-
-// Shared-memory bytes of a staged launch.
-template <int DIM, int BLOCK, int CAP>
-constexpr size_t staged_smem_fixed() {
-    return 16 * (size_t)kStageSlots + sizeof(uint32_t) * (size_t)CAP * BLOCK;
-}
-
-// Bulk-copy staging (cp.async.bulk, global -> shared, one copy per window,
-// completion counted on an mbarrier).  Waits are bounded: a block whose
-// copies have not landed after kStageSpins polls sends its tile to the first
-// overflow queue (after waiting, again bounded, for the copies in flight), so
-// results never depend on the staging.
-constexpr uint32_t kStageSpins = 1u << 22;
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0u;
-}
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint32_t spins) {
-    for (uint32_t k = 0; k < spins; ++k)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
-
-template <int DIM, int BLOCK, int CAP, bool BULK>
-__global__ void __launch_bounds__(BLOCK) k_fluid_staged(FluidArgs a, Tables T, StageCoefs c, StageBuffers b) {
-    using SS = StageShape<DIM>;
-    static_assert(BLOCK >= SS::NW && BLOCK % 32 == 0, "one thread per window");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float4* stg = reinterpret_cast<float4*>(smem_raw);
-    uint32_t* lst = reinterpret_cast<uint32_t*>(smem_raw + 16 * (size_t)kStageSlots);
-    FluidMat* sm = reinterpret_cast<FluidMat*>(lst + CAP * BLOCK);
-    DevInter* si = reinterpret_cast<DevInter*>(reinterpret_cast<unsigned char*>(sm) + sizeof(FluidMat) * T.max_nmat);
-    __shared__ uint32_t s_row[BLOCK];          // global row id (first cell of the x-row) of each thread, or invalid
-    __shared__ uint32_t s_heads[BLOCK / 32];   // own-row heads per warp
-    __shared__ uint32_t r_scene[kMaxOwnRows], r_base[kMaxOwnRows], r_xa[kMaxOwnRows], r_xb[kMaxOwnRows];
-    __shared__ int r_y[kMaxOwnRows], r_z[kMaxOwnRows];
-    __shared__ uint32_t w_gstart[SS::NW], w_off[SS::NW + 1];
-    __shared__ uint32_t s_nrows;
-    __shared__ __align__(8) uint64_t s_bar;
-    __shared__ uint32_t s_landed;
-
-    const uint32_t k0 = blockIdx.x * BLOCK;
-    if (BULK && threadIdx.x == 0) mbar_init(&s_bar, 1);  // ordered before its use by the barriers below
-    const uint32_t k = k0 + threadIdx.x;
-    const uint32_t scene0 = T.mats[__float_as_uint(a.vs[min(k0, a.n - 1u)].w)].scene;
-    load_scene_tables(T, scene0, sm, si);
-
-    // own rows: consecutive threads of one x-row of search cells
     const bool valid = k < a.n;
-    float4 xi = make_float4(0.f, 0.f, 0.f, 0.f), vi = xi;
-    CellCoord cc{0, 0, 0};
-    uint32_t row = kInvalid;
-    const SceneP* Pp = nullptr;
-    if (valid) {
-        xi = a.xs[k];
-        vi = a.vs[k];
-        Pp = &T.scenes[T.mats[__float_as_uint(vi.w)].scene];
-        if (finite3(xi)) {
-            const Grid& g = Pp->sgrid;
-            cc = cell_coord(xi, g);
-            row = Pp->cell_base + (uint32_t)cc.y * g.sub[0] + (uint32_t)cc.z * g.sub[0] * g.sub[1];
-        }
-    }
-    s_row[threadIdx.x] = row;
-    __syncthreads();
-    const bool head = row != kInvalid && (threadIdx.x == 0 || s_row[threadIdx.x - 1] != row);
-    const bool tail = row != kInvalid && (threadIdx.x == BLOCK - 1 || s_row[threadIdx.x + 1] != row);
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned hb = __ballot_sync(0xFFFFFFFFu, head);
-    if (lane == 0) s_heads[warp] = __popc(hb);
-    __syncthreads();
-    uint32_t before = 0, nrows = 0;
-    for (uint32_t w = 0; w < BLOCK / 32; ++w) {
-        before += w < warp ? s_heads[w] : 0u;
-        nrows += s_heads[w];
-    }
-    // own-row index of this thread (rows are contiguous runs of threads)
-    const int rho = row == kInvalid ? -1 : (int)(before + __popc(hb & ((2u << lane) - 1u))) - 1;
-    if (head && rho < kMaxOwnRows) {
-        r_scene[rho] = T.mats[__float_as_uint(vi.w)].scene;
-        r_base[rho] = row;
-        r_y[rho] = cc.y;
-        r_z[rho] = cc.z;
-        r_xa[rho] = (uint32_t)cc.x;
-    }
-    if (tail && rho < kMaxOwnRows) r_xb[rho] = (uint32_t)cc.x;
-    if (threadIdx.x == 0) s_nrows = nrows;
-    __syncthreads();
-
-    // windows: own row r, neighbor row q = (dz + RZ) * NY + (dy + RY)
-    const uint32_t nwin = min(nrows, (uint32_t)kMaxOwnRows) * SS::NQ;
-    if (threadIdx.x < nwin) {
-        const uint32_t r = threadIdx.x / SS::NQ, q = threadIdx.x % SS::NQ;
-        const SceneP& P = T.scenes[r_scene[r]];
-        const Grid& g = P.sgrid;
-        const int dy = (int)(q % kStageNY) - kStageRY;
-        const int dz = DIM == 3 ? (int)(q / kStageNY) - kStageRZ : 0;
-        const int y = r_y[r] + dy, z = r_z[r] + dz;
-        const int ry = 1 + (int)P.halved[1], rx = 1 + (int)P.halved[0];
-        uint32_t wstart = 0, wlen = 0;
-        if (abs(dy) <= ry && y >= 0 && y < (int)g.sub[1] && z >= 0 && z < (int)g.sub[2]) {
-            const uint32_t rb = r_base[r] + (uint32_t)(dy * (int)g.sub[0]) + (uint32_t)(dz * (int)(g.sub[0] * g.sub[1]));
-            const uint32_t x0 = (uint32_t)max((int)r_xa[r] - rx, 0);
-            const uint32_t x1 = (uint32_t)min((int)r_xb[r] + rx, (int)g.sub[0] - 1);
-            wstart = a.start[rb + x0];
-            wlen = a.start[rb + x1 + 1u] - wstart;
-        }
-        w_gstart[threadIdx.x] = wstart;
-        w_off[threadIdx.x + 1] = wlen;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {  // at most NW (<= 60) windows: a serial prefix sum
-        uint32_t t = 0;
-        w_off[0] = 0;
-        for (uint32_t w = 1; w <= nwin; ++w) {
-            t += w_off[w];
-            w_off[w] = t;
-        }
-    }
-    __syncthreads();
-    const uint32_t total = w_off[nwin];
-    const bool staged = s_nrows <= (uint32_t)kMaxOwnRows && total <= (uint32_t)kStageSlots;
-    if (!staged) {
-        // too many rows or candidates for the staging area: the first overflow
-        // queue (global-memory scan with list flushes) takes the tile
-        if (valid) a.overflow[atomicAdd(a.overflow_count, 1u)] = k;
-        return;
-    }
-    if (BULK) {
-        // one elected thread issues a bulk copy per non-empty window (16-byte
-        // aligned float4 ranges) and arms the barrier with their bytes
-        if (threadIdx.x == 0) {
-            mbar_arrive_expect_tx(&s_bar, total * 16u);
-            for (uint32_t w = 0; w < nwin; ++w) {
-                const uint32_t o = w_off[w], len = w_off[w + 1] - o;
-                if (len) bulk_copy_g2s(stg + o, a.xs + w_gstart[w], len * 16u, &s_bar);
-            }
-        }
-        const bool landed = mbar_wait_bounded(&s_bar, 0u, kStageSpins);
-        if (threadIdx.x == 0) s_landed = 1u;
-        __syncthreads();
-        if (!landed) atomicAnd(&s_landed, 0u);
-        __syncthreads();
-        if (!s_landed) {
-            // copies still in flight may write the staging area: wait for them
-            // (bounded) before the block leaves, and let the global-memory scan
-            // of the first overflow queue take the tile
-            mbar_wait_bounded(&s_bar, 0u, kStageSpins);
-            if (valid) a.overflow[atomicAdd(a.overflow_count, 1u)] = k;
-            return;
-        }
-    } else {
-        for (uint32_t w = 0; w < nwin; ++w) {
-            const uint32_t o = w_off[w], len = w_off[w + 1] - o, gs = w_gstart[w];
-            for (uint32_t i = threadIdx.x; i < len; i += BLOCK) stg[o + i] = a.xs[gs + i];
-        }
-        __syncthreads();
-    }
-    if (!valid) return;
-
-    const uint32_t slot = a.perm ? a.perm[k] : k;
-    const uint32_t sid = a.sid[slot];
-    Self s;
-    const SceneP& P = init_self(k, xi, vi, sid, a, T, sm, si, scene0, s);
-    const PairK K{P.h2, P.kconst, P.eps_hh};
+    const uint32_t lane = threadIdx.x & 31u, q = lane & 3u;
+    const uint32_t my = threadIdx.x * STRIDE;            // first entry of the list
+    const uint32_t wlist = (threadIdx.x & ~31u) * STRIDE;  // of the warp's first list
+    uint32_t w = my;                // next free entry
+    uint32_t wend = my + CAP;       // where the list is full
+    uint32_t row = 0;               // next row to open
+    uint32_t jn = 0, hi = 0;        // what is left of the current range
+    uint32_t j2 = 0, hi2 = 0;       // the range after it in the same row (boundary, then mobile candidates)
+    uint32_t pend = 0, pbase = 0;   // hits not yet listed: bit 31 - i for candidate pbase + i
+    bool done = !valid;             // no candidates left
+    bool open = valid;              // the sums are not complete
+    bool saved = false;             // partial sums lie in the list's tail
     Acc acc;
     acc.den = 0.0f;
-    acc.f = make_float3(0.0f, 0.0f, 0.0f);
-    uint32_t* my = lst + threadIdx.x;
-    uint32_t cnt = 0;
-    bool full = false;
-    auto hit = [&](float4 q) {
-        const float rx = q.x - xi.x, ry = q.y - xi.y;
-        const float r2 = DIM == 3 ? fmaf(q.z - xi.z, q.z - xi.z, fmaf(ry, ry, rx * rx)) : fmaf(ry, ry, rx * rx);
-        return r2 < K.h2;
-    };
-    auto take = [&](uint32_t j) {
-        if (cnt < CAP) my[cnt++ * BLOCK] = j;
-        else full = true;
-    };
-    if (rho >= 0) {
-        const Grid& g = P.sgrid;
-        const int rx = 1 + (int)P.halved[0], ry = 1 + (int)P.halved[1];
-        const uint32_t x0 = (uint32_t)max(cc.x - rx, 0), x1 = (uint32_t)min(cc.x + rx, (int)g.sub[0] - 1);
-        for (int q = 0; q < SS::NQ; ++q) {
-            const int dy = q % kStageNY - kStageRY;
-            const int dz = DIM == 3 ? q / kStageNY - kStageRZ : 0;
-            const int y = cc.y + dy, z = cc.z + dz;
-            if (abs(dy) > ry || y < 0 || y >= (int)g.sub[1] || z < 0 || z >= (int)g.sub[2]) continue;
-            const uint32_t rb = row + (uint32_t)(dy * (int)g.sub[0]) + (uint32_t)(dz * (int)(g.sub[0] * g.sub[1]));
-            const uint32_t c0 = rb + x0, c1 = rb + x1 + 1u;
-            const uint32_t bb = a.bstart[c0], be = a.bstart[c1];
-            for (uint32_t j = bb; j < be; ++j)
-                if (hit(a.bxs[j])) take(j | kBoundaryBit);
-            const uint32_t w = (uint32_t)rho * SS::NQ + (uint32_t)q;
-            const uint32_t jb = a.start[c0], je = a.start[c1];
-            const int shift = (int)w_off[w] - (int)w_gstart[w];  // global index -> staging slot
-            uint32_t j = jb;
-            for (; j + 3u < je; j += 4u) {  // four shared-memory loads in flight
-                const int i0 = (int)j + shift;
-                const float4 q0 = stg[i0], q1 = stg[i0 + 1], q2 = stg[i0 + 2], q3 = stg[i0 + 3];
-                const bool h0 = hit(q0), h1 = hit(q1), h2 = hit(q2), h3 = hit(q3);
-                if (h0) take(j);
-                if (h1) take(j + 1u);
-                if (h2) take(j + 2u);
-                if (h3) take(j + 3u);
+    acc.f = make_float3(0.f, 0.f, 0.f);
+
+    for (;;) {
+        // scan until the candidates end or the list is full (what the scan
+        // needs of the particle is read again after an interruption, so that it
+        // need not stay in registers during the evaluation)
+        if (!done) {
+            const float4 xi = a.rec[2 * (size_t)k];
+            const SceneP& P = T.scenes[T.mats[a.mat[k]].scene];
+            const SearchRows rows = search_rows<DIM>(xi, finite3(xi), P);
+            const uint32_t own = own_code(xi, P);
+            const uint4* const code4 = reinterpret_cast<const uint4*>(a.code);
+            // the bounds of the next row are read while the current one is tested
+            uint32_t nb0 = 0, nb1 = 0, nm0 = 0, nm1 = 0;
+            auto fetch = [&]() {
+                const uint32_t c0 = row < (uint32_t)rows.nrows ? search_row(rows, (int)row, P) : kInvalid;
+                nb0 = nb1 = nm0 = nm1 = 0;
+                if (c0 != kInvalid) {
+                    nb0 = a.bstart[c0];
+                    nb1 = a.bstart[c0 + rows.width];
+                    nm0 = a.start[c0];
+                    nm1 = a.start[c0 + rows.width];
+                }
+            };
+            fetch();
+#pragma unroll 1
+            for (;;) {
+                while (pend && w < wend) {
+                    const uint32_t i = (uint32_t)__clz((int)pend);
+                    pend ^= 0x80000000u >> i;
+                    lists[w++] = pbase + i;
+                }
+                if (pend) break;
+                if (jn >= hi) {
+                    if (j2 < hi2) {
+                        jn = j2;
+                        hi = j2 = hi2;
+                    } else {
+                        if (row >= (uint32_t)rows.nrows) {
+                            done = true;
+                            break;
+                        }
+                        if (nb0 < nb1) {
+                            jn = a.n + nb0;
+                            hi = a.n + nb1;
+                            j2 = nm0;
+                            hi2 = nm1;
+                        } else {
+                            jn = nm0;
+                            hi = nm1;
+                        }
+                        ++row;
+                        fetch();
+                        if (jn >= hi) continue;
+                    }
+                }
+                // up to 32 candidates from the group of four that holds jn on
+                pbase = jn & ~3u;
+                const uint32_t g1 = (hi - pbase + 3u) >> 2;
+                const uint4* const p = code4 + (pbase >> 2);
+                uint32_t m = 0;
+                auto test4 = [&](uint4 v) {
+                    m = __funnelshift_l((uint32_t)code_test(v.x, own), m, 1);
+                    m = __funnelshift_l((uint32_t)code_test(v.y, own), m, 1);
+                    m = __funnelshift_l((uint32_t)code_test(v.z, own), m, 1);
+                    m = __funnelshift_l((uint32_t)code_test(v.w, own), m, 1);
+                };
+                {
+                    const uint4 v0 = p[0], v1 = p[1], v2 = p[2], v3 = p[3];  // the array is padded
+                    test4(v0);
+                    test4(v1);
+                    test4(v2);
+                    test4(v3);
+                }
+                if (g1 > 4u) {
+                    const uint4 v0 = p[4], v1 = p[5];
+                    uint4 v2 = make_uint4(0u, 0u, 0u, 0u), v3 = v2;
+                    if (g1 > 6u) {
+                        v2 = p[6];
+                        v3 = p[7];
+                    }
+                    test4(v0);
+                    test4(v1);
+                    if (g1 > 6u) {
+                        test4(v2);
+                        test4(v3);
+                    } else {
+                        m <<= 8;
+                    }
+                } else {
+                    m <<= 16;
+                }
+                const uint32_t end = min(hi - pbase, 32u);
+                pend = m & (FULL >> (jn - pbase)) & (FULL << (32u - end));
+                jn = pbase + 32u;
             }
-            for (; j < je; ++j)
-                if (hit(stg[(int)j + shift])) take(j);
         }
+        __syncwarp();
+        // evaluate: all of a finished list, whole rounds of four of another
+        const uint32_t cnt = w - my;
+        const uint32_t ev = !open ? 0u : done ? cnt : cnt & ~(uint32_t)(kPartials - 1);
+        const bool fin = open && done;
+        const uint32_t word = cnt << 16 | ev << 2 | (fin ? 2u : 0u) | (saved ? 1u : 0u);
+#pragma unroll 1
+        for (uint32_t pass = 0; pass < 4u; ++pass) {
+            const uint32_t owner = pass * 8u + (lane >> 2);
+            const uint32_t ow = __shfl_sync(FULL, word, owner);
+            const uint32_t n_ev = ow >> 2 & 0x3FFFu;
+            const uint32_t list = wlist + owner * STRIDE;
+            Acc part;
+            part.den = 0.0f;
+            part.f = part.c = make_float3(0.f, 0.f, 0.f);
+            if (ow & 1u) {
+                const uint32_t t = list + CAP - TAIL + 7u * q;
+                part.den = __uint_as_float(lists[t]);
+                part.f = make_float3(__uint_as_float(lists[t + 1]), __uint_as_float(lists[t + 2]),
+                                     __uint_as_float(lists[t + 3]));
+                part.c = make_float3(__uint_as_float(lists[t + 4]), __uint_as_float(lists[t + 5]),
+                                     __uint_as_float(lists[t + 6]));
+            }
+            if (n_ev > q) {
+                const uint32_t ko = k - lane + owner;
+                Self s;
+                const SceneP& P = init_self(ko, a, T, sm, scene0, s);
+                const PairK K{P.h2, -6.0f * P.kconst, P.eps_hh};
+                uint32_t bits = 0;
+#pragma unroll 1
+                for (uint32_t e = q; e < n_ev; e += 2 * kPartials) {  // two hits' loads in flight
+                    const bool two = e + kPartials < n_ev;
+                    const uint32_t j0 = lists[list + e], j1 = two ? lists[list + e + kPartials] : ko;
+                    const PairRec r0 = load_rec(a.rec, j0), r1 = load_rec(a.rec, j1);
+                    const uint32_t m0 = a.mat8[j0], m1 = a.mat8[j1];
+                    if (j0 != ko) add_hit<DIM>(part, j0, r0, m0, s, a, K, bits);
+                    if (j1 != ko) add_hit<DIM>(part, j1, r1, m1, s, a, K, bits);
+                }
+                if (bits & kPairPotential) {
+                    const DevInter* const it = T.inter + P.inter_base + s.mat * P.nmat;
+#pragma unroll 1
+                    for (uint32_t e = q; e < n_ev; e += kPartials) {
+                        const uint32_t j = lists[list + e];
+                        if (j != ko) add_hit_contact<DIM>(part, j, s, a, it, K);
+                    }
+                }
+            }
+            __syncwarp();
+            const bool unfinished = !(ow & 2u) && n_ev;
+            if (__any_sync(FULL, unfinished)) {
+                // the rest of the list (fewer than four entries) to its front, the sums to its tail
+                const uint32_t rest = (ow >> 16) - n_ev;
+                const uint32_t keep = unfinished && q < rest ? lists[list + n_ev + q] : 0u;
+                __syncwarp();
+                if (unfinished) {
+                    if (q < rest) lists[list + q] = keep;
+                    const uint32_t t = list + CAP - TAIL + 7u * q;
+                    lists[t] = __float_as_uint(part.den);
+                    lists[t + 1] = __float_as_uint(part.f.x);
+                    lists[t + 2] = __float_as_uint(part.f.y);
+                    lists[t + 3] = __float_as_uint(part.f.z);
+                    lists[t + 4] = __float_as_uint(part.c.x);
+                    lists[t + 5] = __float_as_uint(part.c.y);
+                    lists[t + 6] = __float_as_uint(part.c.z);
+                }
+            }
+            const float s0 = sum_partials(part.den);
+            float s1 = sum_partials(part.f.x), s2 = sum_partials(part.f.y), s3 = sum_partials(part.f.z);
+            if (__any_sync(FULL, part.c.x != 0.0f || part.c.y != 0.0f || part.c.z != 0.0f)) {
+                s1 = __fadd_rn(s1, sum_partials(part.c.x));
+                s2 = __fadd_rn(s2, sum_partials(part.c.y));
+                s3 = __fadd_rn(s3, sum_partials(part.c.z));
+            }
+            const uint32_t src = (lane & 7u) * 4u;
+            const float r0 = __shfl_sync(FULL, s0, src), r1 = __shfl_sync(FULL, s1, src),
+                        r2 = __shfl_sync(FULL, s2, src), r3 = __shfl_sync(FULL, s3, src);
+            if (fin && lane >> 3 == pass) {
+                acc.den = r0;
+                acc.f = make_float3(r1, r2, r3);
+            }
+        }
+        if (fin) open = false;
+        if (!__any_sync(FULL, open)) break;
+        __syncwarp();
+        saved = saved || ev > 0u;
+        w = my + (open ? cnt - ev : 0u);
+        wend = my + CAP - TAIL;
     }
-    if (full) {
-        a.overflow[atomicAdd(a.overflow_count, 1u)] = k;
-        return;
-    }
-    for (uint32_t e = 0; e < cnt; ++e) {
-        const uint32_t j = my[e * BLOCK];
-        if (j != k) eval_hit<DIM>(j, s, a, K, acc);
-    }
-    stage_epilogue(a, c, b, slot, sid, vi, acc, s.d1, P.g, P.solid_branch != 0u);
+    if (valid) stage_epilogue(a, T, c, b, k, acc);
 }
 
-template <int DIM, int BLOCK, int CAP, int MODE>
-void launch_variant(const FluidArgs& a, const Tables& T, const StageCoefs& c, const StageBuffers& b, bool persistent,
-                    uint32_t* tile_counter, cudaStream_t st) {
-    const size_t smem = sizeof(uint32_t) * CAP * BLOCK + sizeof(FluidMat) * T.max_nmat +
-                        sizeof(DevInter) * T.max_nmat * T.max_nmat;
-    if (smem > 48 * 1024) {
-        cudaFuncSetAttribute(FluidKernels<DIM, BLOCK, CAP, MODE>::tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-        cudaFuncSetAttribute(FluidKernels<DIM, BLOCK, CAP, MODE>::persistent,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// ---- group form --------------------------------------------------------------
+// LANES threads of a warp share one particle throughout.  In the block form a
+// launch takes at least as long as one thread's walk over ~170 candidates,
+// however few particles there are; here the walk is LANES times shorter and
+// there are LANES times as many warps, which pays until the SMs are full: the
+// 16,899-particle 3D scene 22 us per launch with 8 lanes against 58 in the block
+// form, the 126,464-particle one 62 us in the block form against 86 with 4 lanes.
+// Bound: the latency of the chain of dependent loads of one particle.
+//   * The bounds of all search rows are read at once, one row per lane, and
+//     turned into a list of non-empty segments of consecutive candidates
+//     (boundary, then mobile, row by row: the candidate order of the block
+//     form), so the scan is one flat loop with U loads in flight per lane.
+//   * Hits are compacted in candidate order by ballots into the particle's list
+//     in shared memory; when a list of the warp could fill up, the warp
+//     evaluates whole rounds of LANES hits of each and goes on.
+//   * Each lane evaluates one hit at a time; with more than four lanes the terms
+//     go through shared memory to the lanes that hold the partial sums (partial
+//     sum lane mod 4, 16 / LANES components each).
+constexpr int kGroupList = 96;   // list entries per particle
+constexpr int kGroupBlock = 128;
+
+template <int DIM, int LANES>
+__global__ void __launch_bounds__(kGroupBlock) k_fluid_group(FluidArgs a, Tables T, StageCoefs c, StageBuffers b) {
+    constexpr int NG = kGroupBlock / LANES;       // particles per block
+    constexpr int U = LANES >= 16 ? 2 : 4;        // candidate loads in flight per lane
+    constexpr int RZ = 1 + (int)(kSearchHalve >> 2 & 1u);
+    constexpr int MAXROWS = 5 * (DIM == 3 ? 2 * RZ + 1 : 1);
+    constexpr int CPL = 16 / LANES;               // components of the partial sum a lane holds
+    static_assert(LANES == 4 || LANES == 8 || LANES == 16, "four partial sums of four components over the lanes");
+    static_assert(kGroupList >= 2 * U * LANES, "the list holds what one scan iteration can add");
+    __shared__ uint32_t s_list[NG][kGroupList];
+    __shared__ uint2 s_seg[NG][2 * MAXROWS];      // (end, first index - first number) of each segment
+    __shared__ float4 s_term[LANES > 4 ? NG : 1][LANES];
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    constexpr unsigned GM = (1u << LANES) - 1u;
+    const uint32_t lane = threadIdx.x % LANES, gi = threadIdx.x / LANES;
+    const uint32_t gshift = (threadIdx.x & 31u) & ~(uint32_t)(LANES - 1);
+    const uint32_t kk = blockIdx.x * NG + gi;
+    const bool valid = kk < a.n;
+    const uint32_t k = valid ? kk : a.n - 1u;  // idle groups of the last block follow the last particle, without candidates
+    Self s;
+    const SceneP& P = init_self(k, a, T, nullptr, kInvalid, s);
+    const float4 xi = make_float4(s.x.x, s.x.y, s.x.z, 0.0f);
+    const PairK K{P.h2, -6.0f * P.kconst, P.eps_hh};
+    const uint32_t own = own_code(xi, P);
+    uint32_t* const list = s_list[gi];
+    uint2* const seg = s_seg[gi];
+
+    // segments of candidates, numbered 0 .. total over all rows
+    uint32_t total = 0, nseg = 0;
+    {
+        const SearchRows rows = search_rows<DIM>(xi, valid && finite3(xi), P);
+#pragma unroll
+        for (int q0 = 0; q0 < MAXROWS; q0 += LANES) {
+            const int q = q0 + (int)lane;
+            const uint32_t c0 = q < rows.nrows ? search_row(rows, q, P) : kInvalid;
+            uint32_t bb = 0, lb = 0, jb = 0, lm = 0;
+            if (c0 != kInvalid) {
+                const uint32_t c1 = c0 + rows.width;
+                bb = a.bstart[c0];
+                lb = a.bstart[c1] - bb;
+                jb = a.start[c0];
+                lm = a.start[c1] - jb;
+            }
+            uint32_t len = lb + lm, cnt = (lb ? 1u : 0u) + (lm ? 1u : 0u);
+#pragma unroll
+            for (int o = 1; o < LANES; o <<= 1) {
+                const uint32_t l2 = __shfl_up_sync(FULL, len, o, LANES), c2 = __shfl_up_sync(FULL, cnt, o, LANES);
+                if ((int)lane >= o) {
+                    len += l2;
+                    cnt += c2;
+                }
+            }
+            const uint32_t first = total + len - lb - lm;
+            uint32_t w = nseg + cnt - (lb ? 1u : 0u) - (lm ? 1u : 0u);
+            if (lb) seg[w++] = make_uint2(first + lb, a.n + bb - first);
+            if (lm) seg[w] = make_uint2(first + lb + lm, jb - first - lb);
+            total += __shfl_sync(FULL, len, LANES - 1, LANES);
+            nseg += __shfl_sync(FULL, cnt, LANES - 1, LANES);
+        }
     }
-    const uint32_t ntiles = (a.n + BLOCK - 1) / BLOCK;
-    if (!a.counters_cleared) cudaMemsetAsync(a.overflow_count, 0, 2 * sizeof(uint32_t), st);
-    if (!persistent) {
-        FluidKernels<DIM, BLOCK, CAP, MODE>::tile<<<ntiles, BLOCK, smem, st>>>(a, T, c, b);
-    } else {
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, FluidKernels<DIM, BLOCK, CAP, MODE>::persistent, BLOCK,
-                                                      smem);
-        per_sm = per_sm > 0 ? per_sm : 1;
-        int sms = 148;
-        int dev = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const uint32_t blocks = std::min<uint32_t>(ntiles, (uint32_t)(sms * per_sm));
-        if (!a.counters_cleared) cudaMemsetAsync(tile_counter, 0, sizeof(uint32_t), st);
-        FluidKernels<DIM, BLOCK, CAP, MODE>::persistent<<<blocks, BLOCK, smem, st>>>(a, T, c, b, tile_counter);
+    __syncwarp();
+
+    // components (lane / 4) * CPL + i of partial sum lane mod 4: (density rate,
+    // force) and (unused, contact force)
+    float acc[CPL], con[CPL];
+#pragma unroll
+    for (int i = 0; i < CPL; ++i) acc[i] = con[i] = 0.0f;
+    // adds one hit's terms per lane (zero where a lane has none: +0 leaves a
+    // sum that began at +0 as it is)
+    auto add = [&](float* to, float4 t) {
+        if (LANES == 4) {
+            to[0] = __fadd_rn(to[0], t.x);
+            to[1 % CPL] = __fadd_rn(to[1 % CPL], t.y);
+            to[2 % CPL] = __fadd_rn(to[2 % CPL], t.z);
+            to[3 % CPL] = __fadd_rn(to[3 % CPL], t.w);
+        } else {
+            float4* const term = s_term[LANES > 4 ? gi : 0];
+            term[lane] = t;
+            __syncwarp();
+            const float* f = reinterpret_cast<const float*>(term) + (lane >> 2) * CPL;
+#pragma unroll
+            for (int e = 0; e < LANES; e += kPartials)
+#pragma unroll
+                for (int i = 0; i < CPL; ++i) to[i] = __fadd_rn(to[i], f[4 * (e + (lane & 3u)) + i]);
+            __syncwarp();
+        }
+    };
+    bool any_con = false;
+    uint32_t t0 = 0, cnt = 0, si = 0;  // candidates tested, hits listed, the lane's current segment
+    for (;;) {
+        while (__any_sync(FULL, t0 < total)) {
+            uint32_t jj[U], code[U];
+            bool in[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const uint32_t t = t0 + (uint32_t)(u * LANES) + lane;
+                in[u] = t < total;
+                jj[u] = code[u] = 0u;
+                if (in[u]) {
+                    uint2 sg = seg[si];
+                    while (t >= sg.x) sg = seg[++si];  // the last segment ends at total > t
+                    jj[u] = sg.y + t;
+                    code[u] = a.code[jj[u]];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const bool h = in[u] && code_test(code[u], own) < 0;
+                const unsigned m = __ballot_sync(FULL, h) >> gshift & GM;
+                if (h) list[cnt + __popc(m & ((1u << lane) - 1u))] = jj[u];
+                cnt += __popc(m);
+            }
+            t0 += U * LANES;
+            if (__any_sync(FULL, cnt > (uint32_t)(kGroupList - U * LANES))) break;
+        }
+        __syncwarp();
+        const uint32_t ev = t0 < total ? cnt & ~(uint32_t)(LANES - 1) : cnt;
+        uint32_t bits = 0;
+#pragma unroll 1
+        for (uint32_t e0 = 0; __any_sync(FULL, e0 < ev); e0 += LANES) {
+            Acc t;
+            t.den = 0.0f;
+            t.f = make_float3(0.f, 0.f, 0.f);
+            if (e0 + lane < ev) {
+                const uint32_t j = list[e0 + lane];
+                if (j != k) add_hit<DIM>(t, j, load_rec(a.rec, j), a.mat8[j], s, a, K, bits);
+            }
+            add(acc, make_float4(t.den, t.f.x, t.f.y, t.f.z));
+        }
+        if (__any_sync(FULL, (bits & kPairPotential) != 0u)) {
+            any_con = true;
+            const DevInter* const it = T.inter + P.inter_base + s.mat * P.nmat;
+#pragma unroll 1
+            for (uint32_t e0 = 0; __any_sync(FULL, e0 < ev); e0 += LANES) {
+                Acc t;
+                t.c = make_float3(0.f, 0.f, 0.f);
+                if (e0 + lane < ev) {
+                    const uint32_t j = list[e0 + lane];
+                    if (j != k) add_hit_contact<DIM>(t, j, s, a, it, K);
+                }
+                add(con, make_float4(0.f, t.c.x, t.c.y, t.c.z));
+            }
+        }
+        if (!__any_sync(FULL, t0 < total)) break;
+        const uint32_t rest = cnt - ev;  // fewer than LANES
+        const uint32_t keep = lane < rest ? list[ev + lane] : 0u;
+        __syncwarp();
+        if (lane < rest) list[lane] = keep;
+        cnt = rest;
     }
-    // the overflow queues: grids of at most 1184 blocks striding over the
-    // queue, which usually is empty
-    const uint32_t oblocks = std::min<uint32_t>(ntiles * BLOCK / 128u + 1u, 1184u);
-    k_fluid_overflow_flush<DIM><<<oblocks, 128, 0, st>>>(a, T, c, b);
-    k_fluid_overflow<DIM><<<2u * oblocks, 64, 0, st>>>(a, T, c, b);
+#pragma unroll
+    for (int i = 0; i < CPL; ++i) {
+        acc[i] = sum_partials(acc[i]);
+        if (any_con) acc[i] = __fadd_rn(acc[i], sum_partials(con[i]));
+    }
+    Acc sum;
+    sum.den = __shfl_sync(FULL, acc[0], 0, LANES);
+    sum.f.x = __shfl_sync(FULL, acc[1 % CPL], 4 * (1 / CPL), LANES);
+    sum.f.y = __shfl_sync(FULL, acc[2 % CPL], 4 * (2 / CPL), LANES);
+    sum.f.z = __shfl_sync(FULL, acc[3 % CPL], 4 * (3 / CPL), LANES);
+    if (valid && lane == 0) stage_epilogue(a, T, c, b, k, sum);
 }
 
 // Velocity Verlet, first half of a step (kick, then drift), in storage
 // order: v' = v + (dt/2) a, rho' = rho + (dt/2) drho/dt, x' = x + dt v', with
 // (a, drho/dt) the derivative record kept from the previous force evaluation
 // (its position part is not used).  Each sum is formed as y + (0 + c k), the
-// order of the stage epilogue.
+// order of the stage epilogue.  The drifted state is counted into its search
+// cells on the way.
 __global__ void k_verlet_kick_drift(const float4* __restrict__ pd, const float4* __restrict__ vm,
                                     const float4* __restrict__ fpd, const float4* __restrict__ fvm, uint32_t n,
-                                    float half, float full, float4* __restrict__ out_pd, float4* __restrict__ out_vm) {
+                                    float half, float full, float4* __restrict__ out_pd, float4* __restrict__ out_vm,
+                                    Tables T, CellBins bin) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const float4 p = pd[k], v = vm[k], fp = fpd[k], fv = fvm[k];
@@ -887,8 +828,10 @@ __global__ void k_verlet_kick_drift(const float4* __restrict__ pd, const float4*
     const float4 vh = comb(v, axpy(half, fv, z), true);  // w holds the material bits
     const float rho = __fadd_rn(p.w, __fadd_rn(0.0f, __fmul_rn(half, fp.w)));
     const float4 dx = axpy(full, make_float4(vh.x, vh.y, vh.z, 0.0f), z);
-    out_pd[k] = make_float4(__fadd_rn(p.x, dx.x), __fadd_rn(p.y, dx.y), __fadd_rn(p.z, dx.z), rho);
+    const float4 np = make_float4(__fadd_rn(p.x, dx.x), __fadd_rn(p.y, dx.y), __fadd_rn(p.z, dx.z), rho);
+    out_pd[k] = np;
     out_vm[k] = vh;
+    bin_particle(np, T.scenes[T.mats[__float_as_uint(v.w)].scene], T.ncells, k, bin);
 }
 
 // The kick of the plastic strain (4 float4 per solid): e' = e + (0 + c k).
@@ -899,28 +842,13 @@ __global__ void k_verlet_kick4(const float4* __restrict__ e, const float4* __res
     out[i] = comb(e[i], axpy(half, k4[i], make_float4(0.f, 0.f, 0.f, 0.f)), false);
 }
 
-template <int DIM, int BLOCK, int CAP, bool BULK>
-int launch_staged(const FluidArgs& a, const Tables& T, const StageCoefs& c, const StageBuffers& b, cudaStream_t st) {
-    const size_t smem = staged_smem_fixed<DIM, BLOCK, CAP>() + sizeof(FluidMat) * T.max_nmat +
-                        sizeof(DevInter) * T.max_nmat * T.max_nmat;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_fluid_staged<DIM, BLOCK, CAP, BULK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    const uint32_t ntiles = (a.n + BLOCK - 1) / BLOCK;
-    if (!a.counters_cleared) cudaMemsetAsync(a.overflow_count, 0, 2 * sizeof(uint32_t), st);
-    k_fluid_staged<DIM, BLOCK, CAP, BULK><<<ntiles, BLOCK, smem, st>>>(a, T, c, b);
-    const uint32_t oblocks = std::min<uint32_t>(ntiles * BLOCK / 128u + 1u, 1184u);
-    k_fluid_overflow_flush<DIM><<<oblocks, 128, 0, st>>>(a, T, c, b);
-    k_fluid_overflow<DIM><<<2u * oblocks, 64, 0, st>>>(a, T, c, b);
-    return 3;
-}
-
 }  // namespace
 
 int verlet_kick_drift(const float4* pd, const float4* vm, const float4* fpd, const float4* fvm, uint32_t n, float half,
-                      float full, float4* out_pd, float4* out_vm, cudaStream_t st) {
+                      float full, float4* out_pd, float4* out_vm, const Tables& T, const CellBins& bin,
+                      cudaStream_t st) {
     if (n == 0) return 0;
-    k_verlet_kick_drift<<<(n + 255) / 256, 256, 0, st>>>(pd, vm, fpd, fvm, n, half, full, out_pd, out_vm);
+    k_verlet_kick_drift<<<(n + 255) / 256, 256, 0, st>>>(pd, vm, fpd, fvm, n, half, full, out_pd, out_vm, T, bin);
     return 1;
 }
 
@@ -931,41 +859,39 @@ int verlet_kick4(const float4* e, const float4* k4, uint32_t count, float half, 
 }
 
 const FluidVariant kFluidVariants[kNumFluidVariants] = {
-    {128, 48, 0, 0, 0}, {256, 48, 0, 0, 0}, {128, 48, 1, 0, 0}, {256, 48, 1, 0, 0},
-    {128, 96, 0, 0, 0}, {256, 96, 0, 0, 0}, {128, 96, 1, 0, 0}, {256, 96, 1, 0, 0},
-    {128, 48, 0, 1, 0}, {128, 48, 1, 1, 0},
-    {128, 48, 0, 0, 1}, {64, 48, 0, 0, 1}, {128, 48, 0, 0, 2},
-    {128, 40, 0, 1, 0}, {128, 32, 0, 1, 0},
+    {128, 40, 0}, {128, 44, 0}, {128, 48, 0}, {128, 56, 0}, {128, 64, 0}, {128, 96, 0},
+    {256, 40, 0}, {256, 44, 0}, {256, 48, 0}, {256, 56, 0}, {256, 64, 0}, {256, 96, 0},
+    {128, 96, 4}, {128, 96, 8}, {128, 96, 16},
 };
 
 int launch_fluid(const FluidArgs& a, const Tables& T, int kdim, const StageCoefs& c, const StageBuffers& b,
-                 int variant, uint32_t* tile_counter, cudaStream_t st) {
+                 int variant, cudaStream_t st) {
     if (a.n == 0) return 0;
     const FluidVariant v = kFluidVariants[variant < 0 || variant >= kNumFluidVariants ? 0 : variant];
-    const bool pers = v.persistent != 0;
-    if (v.staged == 1) {  // cooperative loads
-        if (kdim == 3 && v.block == 128) return launch_staged<3, 128, 48, false>(a, T, c, b, st);
-        if (kdim == 3 && v.block == 64) return launch_staged<3, 64, 48, false>(a, T, c, b, st);
-        if (kdim == 2 && v.block == 128) return launch_staged<2, 128, 48, false>(a, T, c, b, st);
-        if (kdim == 2 && v.block == 64) return launch_staged<2, 64, 48, false>(a, T, c, b, st);
-        return 0;
+    if (v.lanes) {
+        const uint32_t nb = (a.n + (uint32_t)(kGroupBlock / v.lanes) - 1u) / (uint32_t)(kGroupBlock / v.lanes);
+#define ARP_GROUP(D, L) \
+    if (kdim == D && v.lanes == L) k_fluid_group<D, L><<<nb, kGroupBlock, 0, st>>>(a, T, c, b);
+        ARP_GROUP(3, 4) ARP_GROUP(3, 8) ARP_GROUP(3, 16)
+        ARP_GROUP(2, 4) ARP_GROUP(2, 8) ARP_GROUP(2, 16)
+#undef ARP_GROUP
+        return 1;
     }
-    if (v.staged == 2) {  // bulk copies
-        if (kdim == 3 && v.block == 128) return launch_staged<3, 128, 48, true>(a, T, c, b, st);
-        if (kdim == 2 && v.block == 128) return launch_staged<2, 128, 48, true>(a, T, c, b, st);
-        return 0;
+    const size_t smem = sizeof(uint32_t) * (v.cap + 1) * v.block + sizeof(PairMat) * T.max_nmat * T.max_nmat;
+    const uint32_t nb = (a.n + (uint32_t)v.block - 1u) / (uint32_t)v.block;
+#define ARP_FLUID(D, B, C)                                                                                         \
+    if (kdim == D && v.block == B && v.cap == C) {                                                                 \
+        if (smem > 48 * 1024)                                                                                      \
+            cudaFuncSetAttribute(k_fluid<D, B, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);        \
+        k_fluid<D, B, C><<<nb, B, smem, st>>>(a, T, c, b);                                                         \
     }
-#define ARP_FLUID(D, B, C, M)                                               \
-    if (kdim == D && v.block == B && v.cap == C && v.flush == M && !v.staged) {  \
-        launch_variant<D, B, C, M>(a, T, c, b, pers, tile_counter, st);     \
-        return 3; /* the tile kernel and the two overflow kernels */       \
-    }
-    ARP_FLUID(3, 128, 48, 0) ARP_FLUID(3, 256, 48, 0) ARP_FLUID(3, 128, 96, 0) ARP_FLUID(3, 256, 96, 0)
-    ARP_FLUID(2, 128, 48, 0) ARP_FLUID(2, 256, 48, 0) ARP_FLUID(2, 128, 96, 0) ARP_FLUID(2, 256, 96, 0)
-    ARP_FLUID(3, 128, 48, 1) ARP_FLUID(2, 128, 48, 1)
-    ARP_FLUID(3, 128, 40, 1) ARP_FLUID(3, 128, 32, 1) ARP_FLUID(2, 128, 40, 1) ARP_FLUID(2, 128, 32, 1)
+#define ARP_FLUID_CAPS(D, B) \
+    ARP_FLUID(D, B, 40) ARP_FLUID(D, B, 44) ARP_FLUID(D, B, 48) ARP_FLUID(D, B, 56) \
+    ARP_FLUID(D, B, 64) ARP_FLUID(D, B, 96)
+    ARP_FLUID_CAPS(3, 128) ARP_FLUID_CAPS(3, 256) ARP_FLUID_CAPS(2, 128) ARP_FLUID_CAPS(2, 256)
+#undef ARP_FLUID_CAPS
 #undef ARP_FLUID
-    return 0;
+    return 1;
 }
 
 }  // namespace arp

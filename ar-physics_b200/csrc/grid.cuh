@@ -50,6 +50,60 @@ __host__ __device__ inline uint32_t cell_id(const CellCoord& c, const Grid& g) {
     return (uint32_t)c.x + (uint32_t)c.y * g.sub[0] + (uint32_t)c.z * g.sub[0] * g.sub[1];
 }
 
+// Counts slot i, at position p of scene P, into its search cell (the
+// non-finite bucket `ncells` for a non-finite position).
+__device__ __forceinline__ void bin_particle(float4 p, const SceneP& P, uint32_t ncells, uint32_t i,
+                                             const CellBins& b) {
+    uint32_t k = ncells;
+    uint2 coord = make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+    if (finite3(p)) {
+        const CellCoord fc = cell_coord(p, P.sgrid);
+        k = P.cell_base + cell_id(fc, P.sgrid);
+        // reference cell = search cell >> 1 on halved axes (exact, see SceneP)
+        coord = make_uint2((uint32_t)fc.x >> P.halved[0] | ((uint32_t)fc.y >> P.halved[1]) << 16,
+                           (uint32_t)fc.z >> P.halved[2]);
+    }
+    b.coord[i] = coord;
+    b.key[i] = k;
+    b.rank[i] = atomicAdd(&b.count[k], 1u);
+}
+
+// ---- quantised positions -------------------------------------------------------
+// The fluid kernel tests candidates on positions quantised to h / kCodeUnits,
+// one byte per axis modulo 256 (x lowest, the top byte 0): a candidate is 4
+// bytes instead of 16, and its test one subtraction, one four-way byte product
+// and one compare on integers.
+//
+// No pair within h may fail the test.  With X = (x - min) 63 / h per axis, a
+// candidate's code is rint(X_j); the particle's own code is rint(X_i) in x and
+// rint(X_i - 1/2) in y and z.  The codes are subtracted as 32-bit words, so a
+// negative lower byte borrows 1 from the next.  The difference then is
+// X_j - X_i plus an error of at most 1 in x and 1.5 in y and z (both roundings,
+// the half, the borrow), 2.345 in norm; the top byte is 0 or -1.  A pair within
+// h therefore has a sum of squares of at most (63 + 2.345)^2 + 1 = 4271.0; the
+// bound below leaves 2 for the roundings of X in double precision.  Differences past 127
+// wrap, which can only let far candidates through, and the evaluation of a
+// pair tests r < h again.
+constexpr double kCodeUnits = 63.0;
+constexpr int kCodeBound = 4273;
+
+__device__ __forceinline__ uint32_t code_axis(float p, float mn, double inv, double shift) {
+    return (uint32_t)__double2ll_rn(((double)p - (double)mn) * inv - shift) & 255u;
+}
+__device__ __forceinline__ uint32_t scan_code(float4 p, const SceneP& P) {
+    return code_axis(p.x, P.grid.min[0], P.code_inv, 0.0) | code_axis(p.y, P.grid.min[1], P.code_inv, 0.0) << 8 |
+           code_axis(p.z, P.grid.min[2], P.code_inv, 0.0) << 16;
+}
+__device__ __forceinline__ uint32_t own_code(float4 p, const SceneP& P) {
+    return code_axis(p.x, P.grid.min[0], P.code_inv, 0.0) | code_axis(p.y, P.grid.min[1], P.code_inv, 0.5) << 8 |
+           code_axis(p.z, P.grid.min[2], P.code_inv, 0.5) << 16;
+}
+// Negative when the candidate may lie within h.
+__device__ __forceinline__ int code_test(uint32_t candidate, uint32_t own) {
+    const int d = (int)(candidate - own);
+    return __dp4a(d, d, -kCodeBound - 1);
+}
+
 // ---- search grid -------------------------------------------------------------
 
 // Calls f(c0, c1) for the global search-cell ranges [c0, c1) (one x-row

@@ -39,40 +39,10 @@ __device__ __forceinline__ uint32_t scene_of(const float4* vm, const uint32_t* m
 }
 
 __global__ void k_cell_keys(const float4* __restrict__ pos, const float4* __restrict__ vm,
-                            const uint32_t* __restrict__ mat_u32, uint32_t n, Tables T, uint32_t* __restrict__ key,
-                            uint32_t* __restrict__ rank, uint32_t* __restrict__ count, uint2* __restrict__ coord,
-                            DevStats* stats, StageCounters zero) {
+                            const uint32_t* __restrict__ mat_u32, uint32_t n, Tables T, CellBins bin) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 3 && zero.p[i])
-        for (uint32_t q = 0; q < zero.n[i]; ++q) zero.p[i][q] = 0u;
     if (i >= n) return;
-    float4 p = pos[i];
-    uint32_t k;
-    if (!finite3(p)) {
-        k = T.ncells;
-        if (coord) coord[i] = make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
-        if (stats) atomicAdd(&stats->nonfinite_positions, 1u);
-    } else {
-        const SceneP& sp = T.scenes[scene_of(vm, mat_u32, i, T)];
-        const Grid& grid = sp.grid;
-        const CellCoord fc = cell_coord(p, sp.sgrid);
-        k = sp.cell_base + cell_id(fc, sp.sgrid);
-        if (coord) {
-            // reference cell = search cell >> 1 on halved axes (exact, see SceneP)
-            const uint32_t x = (uint32_t)fc.x >> sp.halved[0], y = (uint32_t)fc.y >> sp.halved[1],
-                           z = (uint32_t)fc.z >> sp.halved[2];
-            coord[i] = make_uint2(x | (y << 16), z);
-        }
-        if (stats) {
-            // a coordinate on the upper face would hash one past the last cell
-            bool face = (grid.dim[0] != 0.0f && p.x == grid.min[0] + grid.dim[0]) ||
-                        (grid.dim[1] != 0.0f && p.y == grid.min[1] + grid.dim[1]) ||
-                        (grid.dim[2] != 0.0f && p.z == grid.min[2] + grid.dim[2]);
-            if (face) atomicAdd(&stats->clamped_coordinates, 1u);
-        }
-    }
-    key[i] = k;
-    rank[i] = atomicAdd(&count[k], 1u);
+    bin_particle(pos[i], T.scenes[scene_of(vm, mat_u32, i, T)], T.ncells, i, bin);
 }
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
@@ -160,8 +130,10 @@ __global__ void k_scan_add(uint32_t* out, uint32_t len, const uint32_t* __restri
 }
 
 __global__ void k_scatter(const uint32_t* __restrict__ key, const uint32_t* __restrict__ rank, uint32_t n,
-                          const uint32_t* __restrict__ start, uint32_t* __restrict__ perm) {
+                          const uint32_t* __restrict__ start, uint32_t* __restrict__ perm,
+                          uint32_t* __restrict__ zero2) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (zero2 && i < 2u) zero2[i] = 0u;
     if (i >= n) return;
     perm[start[key[i]] + rank[i]] = i;
 }
@@ -407,8 +379,8 @@ __global__ void k_gather_state(const uint32_t* __restrict__ perm, uint32_t n, co
                                float4* __restrict__ vm_out, const uint32_t* __restrict__ a_in,
                                uint32_t* __restrict__ a_out, const uint32_t* __restrict__ b_in,
                                uint32_t* __restrict__ b_out, const uint2* __restrict__ c_in,
-                               uint2* __restrict__ c_out, float* __restrict__ ps_out,
-                               const DevMat* __restrict__ mats, SolidScatter sol) {
+                               uint2* __restrict__ c_out, float* __restrict__ ps_out, Tables T, SolidScatter sol,
+                               DevStats* stats, PairOut out) {
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t s = perm ? perm[k] : k;
@@ -428,10 +400,29 @@ __global__ void k_gather_state(const uint32_t* __restrict__ perm, uint32_t n, co
     if (a_out) a_out[k] = a_in[s];
     if (b_out) b_out[k] = b_in[s];
     if (c_out) c_out[k] = c_in[s];
-    if (ps_out) {
-        const DevMat& m = mats[__float_as_uint(vm.w)];
-        const float p = eos_pressure(m.state_eq, pd.w, m.sound_speed, m.target_den);
-        ps_out[k] = p / (pd.w * pd.w);
+    if (stats) {
+        if (!finite3(pd)) {
+            atomicAdd(&stats->nonfinite_positions, 1u);
+        } else {
+            // a coordinate on the upper face would hash one past the last cell
+            const Grid& g = T.scenes[T.mats[__float_as_uint(vm.w)].scene].grid;
+            const bool face = (g.dim[0] != 0.0f && pd.x == g.min[0] + g.dim[0]) ||
+                              (g.dim[1] != 0.0f && pd.y == g.min[1] + g.dim[1]) ||
+                              (g.dim[2] != 0.0f && pd.z == g.min[2] + g.dim[2]);
+            if (face) atomicAdd(&stats->clamped_coordinates, 1u);
+        }
+    }
+    const uint32_t mat = __float_as_uint(vm.w);
+    const DevMat& m = T.mats[mat];
+    const float p = eos_pressure(m.state_eq, pd.w, m.sound_speed, m.target_den);
+    const float ps = p / (pd.w * pd.w);
+    if (ps_out) ps_out[k] = ps;
+    if (out.rec) {
+        out.rec[2 * (size_t)k] = pd;
+        out.rec[2 * (size_t)k + 1] = make_float4(vm.x, vm.y, vm.z, ps);
+        out.code[k] = scan_code(pd, T.scenes[m.scene]);
+        out.mat8[k] = (uint8_t)m.local;
+        if (out.mat) out.mat[k] = mat;
     }
 }
 
@@ -557,28 +548,40 @@ cudaError_t noalloc_scratch(uint32_t** out) {
 
 }  // namespace
 
-int build_grid(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
-               GridBuffers& gb, DevStats* stats, const uint32_t* boundary_start, cudaStream_t st,
-               const StageCounters& zero) {
+int bin_cells(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
+              GridBuffers& gb, cudaStream_t st) {
     int launches = 0;
     if (n > 0) {
         // a single scene needs no material to find the scene: skip that read
         const bool one = T.nscenes == 1;
         k_cell_keys<<<blocks_for(n, kThreads), kThreads, 0, st>>>(pos, one ? nullptr : vm, one ? nullptr : mat_u32, n,
-                                                                  T, gb.key, gb.rank, gb.count, gb.coord, stats,
-                                                                  zero);
+                                                                  T, cell_bins(gb));
         ++launches;
     }
+    return launches + scan_cells(T, gb, st);
+}
+
+int scan_cells(const Tables& T, GridBuffers& gb, cudaStream_t st) {
     // cells, the non-finite bucket, and the total
-    launches += exclusive_scan(gb.count, T.ncells + 2, gb.start, gb.block_sums, st);
+    return exclusive_scan(gb.count, T.ncells + 2, gb.start, gb.block_sums, st);
+}
+
+int sort_cells(uint32_t n, const Tables& T, GridBuffers& gb, DevStats* stats, const uint32_t* boundary_start,
+               uint32_t* zero2, cudaStream_t st) {
+    int launches = 0;
     if (n > 0) {
-        k_scatter<<<blocks_for(n, kThreads), kThreads, 0, st>>>(gb.key, gb.rank, n, gb.start, gb.perm);
+        k_scatter<<<blocks_for(n, kThreads), kThreads, 0, st>>>(gb.key, gb.rank, n, gb.start, gb.perm, zero2);
         ++launches;
     }
     k_sort_runs<<<blocks_for(T.ncells + 1, kThreads), kThreads, 0, st>>>(gb.start, T.ncells, gb.perm, gb.rank,
                                                                          boundary_start, stats, T);
-    ++launches;
-    return launches;
+    return launches + 1;
+}
+
+int build_grid(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
+               GridBuffers& gb, cudaStream_t st) {
+    const int l = bin_cells(pos, vm, mat_u32, n, T, gb, st);
+    return l + sort_cells(n, T, gb, nullptr, nullptr, nullptr, st);
 }
 
 uint32_t scan_block_sums_needed(uint32_t len) { return blocks_for(len, kScanTile) + 1; }
@@ -601,11 +604,11 @@ int gather_sorted(const uint32_t* perm, uint32_t n, const float4* a_in, float4* 
 
 int gather_state(const uint32_t* perm, uint32_t n, const float4* pd_in, float4* pd_out, const float4* vm_in,
                  float4* vm_out, const uint32_t* a_in, uint32_t* a_out, const uint32_t* b_in, uint32_t* b_out,
-                 const uint2* c_in, uint2* c_out, float* ps_out, const DevMat* mats, cudaStream_t st,
-                 const SolidScatter& sol) {
+                 const uint2* c_in, uint2* c_out, float* ps_out, const Tables& T, cudaStream_t st,
+                 const SolidScatter& sol, DevStats* stats, const PairOut& out) {
     if (n == 0) return 0;
     k_gather_state<<<blocks_for(n, kThreads), kThreads, 0, st>>>(perm, n, pd_in, pd_out, vm_in, vm_out, a_in, a_out,
-                                                                 b_in, b_out, c_in, c_out, ps_out, mats, sol);
+                                                                 b_in, b_out, c_in, c_out, ps_out, T, sol, stats, out);
     return 1;
 }
 

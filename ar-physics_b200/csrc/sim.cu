@@ -226,7 +226,6 @@ struct arp_sim {
     Tableau tab{};
     float time = 0;
     bool initialized = false;
-    bool any_stiff_immobile = false;
     bool all_order2 = true;  // every stiff material uses strain order 2
     bool any_plastic = false;  // some stiff material is plastic
     uint32_t ncells = 0;     // search cells of all scenes
@@ -251,6 +250,7 @@ struct arp_sim {
     DevBuf<DevMat> d_mats;
     DevBuf<FluidMat> d_fmats;
     DevBuf<DevInter> d_inter;
+    DevBuf<PairMat> d_pmats;
     // mobile state: Y (y0), T (reorder target / y_new), S[2] (stage states)
     StateBuf Y, T, S[2], X, acc, kst[4];
     // velocity Verlet: the derivative record of the last force evaluation
@@ -261,23 +261,31 @@ struct arp_sim {
     bool vforce_valid = false;
     bool verlet() const { return integrator == ARP_INT_VERLET; }
     DevBuf<uint32_t> orig, orig_r, sid, sid_r, sid_sorted, slot_of;
-    DevBuf<float> ps, bps;  // p / rho^2 of sorted particles / boundary particles
+    DevBuf<float> bps;      // p / rho^2 of boundary particles
+    // what the fluid kernel reads of the stage's sorted particles, the boundary
+    // particles (put there by do_init) after them (see FluidArgs)
+    DevBuf<float4> p_rec;
+    DevBuf<uint32_t> p_code, p_mat;
+    DevBuf<uint8_t> p_mat8;
+    PairOut pair_out(size_t first) { return PairOut{p_rec.p + 2 * first, p_code.p + first, p_mat8.p + first, p_mat.p + first}; }
     DevBuf<arp_particle> records;      // device copy of caller-order Particle records (state exchange)
     DevBuf<uint32_t> sid_of_caller_d;  // caller id -> solid id
     DevBuf<uint32_t> mat_of_caller_d;  // caller id -> material id
     DevBuf<uint32_t> check_flag;
     // boundary (cell-sorted)
     DevBuf<float4> b_pd, b_vm;
-    DevBuf<uint32_t> b_orig, b_start, sid_of_bidx;
+    DevBuf<uint32_t> b_orig, b_start;
     // grid scratch
     GridBuffers gb{};
     DevBuf<uint32_t> g_key, g_rank, g_count, g_start, g_perm, g_bsums;
     DevBuf<uint2> g_coord;  // grid coordinates per slot
     DevBuf<uint32_t> contact_bound;
-    DevBuf<uint32_t> tile_counter;  // work queue of the persistent fluid kernel
-    DevBuf<uint32_t> overflow, overflow_count;  // the fluid kernel's two overflow queues (2n entries, 2 counts)
     int fluid_variant = 0;
     uint32_t grid_cap = 0;
+    // gb.start, key, rank and coord hold the state Y counted into cells: the
+    // last stage of a Runge-Kutta step does that for the next step's grid.
+    // False whenever Y or the grid buffers have changed otherwise.
+    bool binned = false;
     // solids
     DevBuf<float4> ref, L, F, A, ksol;
     DevBuf<float4> ep, ep_t, ep_s[2], ep_acc, ep_kst[4];
@@ -479,6 +487,7 @@ arp_status scene_params(arp_sim::SceneHost& H, uint32_t dim) {
     P.h = H.h;
     P.h2 = H.h * H.h;
     P.kconst = norm_const_f32(dim, H.h);
+    P.code_inv = kCodeUnits / (double)H.h;
     P.g = H.gravity;
     const float eps = 0.1f;
     volatile float t = eps * H.h;
@@ -561,22 +570,14 @@ arp_status do_init(arp_sim* S) {
             CUDA_TRY(cudaMemcpyAsync(tmp_vm.p, bvm.data(), nb * sizeof(float4), cudaMemcpyHostToDevice, st));
             CUDA_TRY(cudaMemcpyAsync(tmp_o.p, bo.data(), nb * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
         }
-        S->launches += build_grid(tmp_pd.p, tmp_vm.p, nullptr, nb, S->tables, S->gb, nullptr, nullptr, st);
+        S->launches += build_grid(tmp_pd.p, tmp_vm.p, nullptr, nb, S->tables, S->gb, st);
         S->launches += gather_state(S->gb.perm, nb, tmp_pd.p, S->b_pd.p, tmp_vm.p, S->b_vm.p, tmp_o.p,
-                                    S->b_orig.p, nullptr, nullptr, nullptr, nullptr, S->bps.p, S->d_mats.p, st);
+                                    S->b_orig.p, nullptr, nullptr, nullptr, nullptr, S->bps.p, S->tables, st, SolidScatter{}, nullptr, S->pair_out(n));
         CUDA_TRY(cudaMemcpyAsync(S->b_start.p, S->gb.start, (size_t(nc) + 2) * sizeof(uint32_t),
                                  cudaMemcpyDeviceToDevice, st));
         CUDA_TRY(cudaStreamSynchronize(st));
         ARP_TRY(check_launch("boundary grid"));
     }
-    if (S->any_stiff_immobile) {
-        // the scene's boundary index b read as an index into the scene's mobile particles
-        std::vector<uint32_t> sb(std::max(nb, 1u), kInvalid);
-        for (const auto& H : S->scenes)
-            for (uint32_t b = 0; b < H.nb; ++b) sb[H.b_base + b] = b < H.n ? S->sid_of_caller[H.p_base + b] : kInvalid;
-        CUDA_TRY(cudaMemcpy(S->sid_of_bidx.p, sb.data(), sb.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    }
-
     // solids: reference positions, plastic strain = 0, neighbor lists, L
     if (ns > 0) {
         // reference positions: the positions at creation, or carried over by
@@ -603,7 +604,7 @@ arp_status do_init(arp_sim* S) {
             S->host_ep.clear();
         }
         // grid over reference positions (neighbor_list.rs:266-275, mode 1)
-        S->launches += build_grid(S->ref.p, nullptr, S->mat_of_solid.p, ns, S->tables, S->gb, nullptr, nullptr, st);
+        S->launches += build_grid(S->ref.p, nullptr, S->mat_of_solid.p, ns, S->tables, S->gb, st);
         DevBuf<uint32_t> cnt;
         CUDA_TRY(cnt.alloc(size_t(ns) + 1));
         CUDA_TRY(cudaMemsetAsync(cnt.p, 0, (size_t(ns) + 1) * sizeof(uint32_t), st));
@@ -623,6 +624,7 @@ arp_status do_init(arp_sim* S) {
     }
     CUDA_TRY(cudaMemsetAsync(S->d_stats.p, 0, sizeof(DevStats), st));
     S->vforce_valid = false;
+    S->binned = false;
     S->initialized = true;
     return ARP_OK;
 }
@@ -670,6 +672,7 @@ arp_status save_checkpoint(arp_sim* S) {
 
 arp_status restore_checkpoint(arp_sim* S, const Checkpoint& c) {
     const size_t n = S->n;
+    S->binned = false;
     if (n) {
         CUDA_TRY(cudaMemcpyAsync(S->Y.pd.p, c.pd.p, n * sizeof(float4), cudaMemcpyDeviceToDevice, S->stream));
         CUDA_TRY(cudaMemcpyAsync(S->Y.vm.p, c.vm.p, n * sizeof(float4), cudaMemcpyDeviceToDevice, S->stream));
@@ -728,27 +731,24 @@ arp_status do_step(arp_sim* S, bool prime = false) {
     // 1. sort y0 into cell order
     arp_sim::Mark mk{};
     mark(S, mk, 0);
-    // each stage's grid build clears the counters the stage's kernels start from
-    StageCounters zero;
-    zero.p[0] = S->overflow_count.p;
-    zero.n[0] = 2;
-    zero.p[1] = S->tile_counter.p;
-    zero.n[1] = 1;
-    if (sb) {
-        zero.p[2] = S->contact_bound.p;
-        zero.n[2] = 2;
-    }
-    // velocity Verlet kicks and drifts first (storage order, into X); the grid
-    // and the force evaluation then see the drifted state
+    // a state is counted into cells where it is written: by the fluid kernel's
+    // epilogue, or by velocity Verlet's kick and drift (storage order, into X;
+    // the grid and the force evaluation then see the drifted state)
+    const CellBins bins = cell_bins(S->gb);
+    uint32_t* const zero2 = sb ? S->contact_bound.p : nullptr;  // cleared with each stage's sort
     const float4* src_pd = S->Y.pd.p;
     const float4* src_vm = S->Y.vm.p;
     if (verlet && !prime) {
         S->launches += verlet_kick_drift(S->Y.pd.p, S->Y.vm.p, S->vforce.pd.p, S->vforce.vm.p, n, half, S->dt_sub,
-                                         S->X.pd.p, S->X.vm.p, st);
+                                         S->X.pd.p, S->X.vm.p, S->tables, bins, st);
+        S->launches += scan_cells(S->tables, S->gb, st);
         src_pd = S->X.pd.p;
         src_vm = S->X.vm.p;
+    } else if (!S->binned) {
+        S->launches += bin_cells(src_pd, src_vm, nullptr, n, S->tables, S->gb, st);
     }
-    S->launches += build_grid(src_pd, src_vm, nullptr, n, S->tables, S->gb, S->d_stats.p, bstart, st, zero);
+    S->binned = false;
+    S->launches += sort_cells(n, S->tables, S->gb, S->d_stats.p, bstart, zero2, st);
     // the stage-0 solid copies and the solid -> slot map come out of the same gather
     SolidScatter sol0;
     if (ns) {
@@ -760,7 +760,8 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         sol0.slot_of = S->slot_of.p;
     }
     S->launches += gather_state(S->gb.perm, n, src_pd, S->T.pd.p, src_vm, S->T.vm.p, S->orig.p, S->orig_r.p,
-                                S->sid.p, S->sid_r.p, nullptr, nullptr, S->ps.p, S->d_mats.p, st, sol0);
+                                S->sid.p, S->sid_r.p, nullptr, nullptr, nullptr, S->tables, st, sol0, S->d_stats.p,
+                                S->pair_out(0));
     std::swap(S->Y, S->T);
     std::swap(S->orig, S->orig_r);
     std::swap(S->sid, S->sid_r);
@@ -817,7 +818,7 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         if (s > 0) {
             if (S->profiling && s > 0) mark(S, mk, 0);
             l0 = S->launches;
-            S->launches += build_grid(cur_pd, cur_vm, nullptr, n, S->tables, S->gb, S->d_stats.p, bstart, st, zero);
+            S->launches += sort_cells(n, S->tables, S->gb, S->d_stats.p, bstart, zero2, st);
             SolidScatter sol;  // this stage's solid copies
             if (sb && ns) {
                 sol.sid_of_slot = S->sid.p;
@@ -826,13 +827,11 @@ arp_status do_step(arp_sim* S, bool prime = false) {
                 sol.sv = S->sv.p;
                 sol.sc = S->sc.p;
             }
-            S->launches += gather_state(S->gb.perm, n, cur_pd, S->X.pd.p, cur_vm, S->X.vm.p, sb ? S->sid.p : nullptr,
-                                        sb ? S->sid_sorted.p : nullptr, nullptr, nullptr, nullptr, nullptr, S->ps.p,
-                                        S->d_mats.p, st, sol);
+            S->launches += gather_state(S->gb.perm, n, cur_pd, nullptr, cur_vm, nullptr, sb ? S->sid.p : nullptr,
+                                        sb ? S->sid_sorted.p : nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+                                        S->tables, st, sol, S->d_stats.p, S->pair_out(0));
             nl += S->launches - l0;
         }
-        const float4* xs = s == 0 ? S->Y.pd.p : S->X.pd.p;
-        const float4* vs = s == 0 ? S->Y.vm.p : S->X.vm.p;
         const uint32_t* perm = s == 0 ? nullptr : S->gb.perm;
         const uint32_t* sid_sorted = s == 0 ? S->sid.p : S->sid_sorted.p;
         float4* next_pd = last ? S->T.pd.p : S->S[s % 2].pd.p;
@@ -865,8 +864,8 @@ arp_status do_step(arp_sim* S, bool prime = false) {
             a.ksol = S->ksol.p;
             a.contact_bound = S->contact_bound.p;
             a.counters_cleared = n > 0 ? 1 : 0;
-            a.xs = xs;
-            a.vs = vs;
+            a.rec = S->p_rec.p;
+            a.mat = S->p_mat.p;
             a.start = S->gb.start;
             a.sid_sorted = sid_sorted;
             a.ns = ns;
@@ -892,28 +891,24 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         mark(S, mk, 2);
 
         FluidArgs f{};
-        f.xs = xs;
-        f.vs = vs;
+        f.rec = S->p_rec.p;
+        f.code = S->p_code.p;
+        f.mat8 = S->p_mat8.p;
+        f.mat = S->p_mat.p;
         f.start = S->gb.start;
-        f.bxs = S->b_pd.p;
-        f.bvs = S->b_vm.p;
         f.bstart = bstart;
         f.perm = perm;
         f.sid = S->sid.p;
-        f.sid_of_boundary_index = S->sid_of_bidx.p;
-        f.borig = S->b_orig.p;
-        f.ps = S->ps.p;
-        f.bps = S->bps.p;
         f.ksol = sb ? S->ksol.p : nullptr;
         f.n = n;
         f.solid_branch = sb ? 1 : 0;
-        f.overflow = S->overflow.p;
-        f.overflow_count = S->overflow_count.p;
-        f.counters_cleared = 1;  // by this stage's grid build
-        f.any_stiff_immobile = S->any_stiff_immobile ? 1 : 0;
         B.next_pd = next_pd;
         B.next_vm = next_vm;
-        const int fl = launch_fluid(f, S->tables, S->kdim, c, B, S->fluid_variant, S->tile_counter.p, st);
+        // the next state's cells: the next stage's grid, or the next step's
+        const bool bin_next = !verlet && !prime;
+        B.bin = bin_next ? bins : CellBins{};
+        int fl = launch_fluid(f, S->tables, S->kdim, c, B, S->fluid_variant, st);
+        if (bin_next) fl += scan_cells(S->tables, S->gb, st);
         S->launches += fl;
         mark(S, mk, 3);
         if (S->profiling) {
@@ -934,6 +929,7 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         if (sb && S->any_plastic) std::swap(S->ep, S->ep_t);  // without plastic materials ep stays zero
     }
     if (verlet) S->vforce_valid = true;
+    S->binned = !verlet && !prime;
     if (S->profiling) S->prof_steps++;
     return check_launch("step");
 }
@@ -1033,7 +1029,6 @@ arp_status append_scene(const arp_scene* sc, arp_sim* S) {
     for (uint32_t i = 0; i < M; ++i) {
         S->mats.push_back(mats[i]);
         S->scene_of_material.push_back(scene_idx);
-        if (mats[i].immobile && is_stiff(mats[i])) S->any_stiff_immobile = true;
         if (is_stiff(mats[i]) && mats[i].strain_order != 2) S->all_order2 = false;
         if (is_stiff(mats[i]) && mats[i].plastic) S->any_plastic = true;
     }
@@ -1137,7 +1132,10 @@ arp_status allocate(arp_sim* S) {
     CUDA_TRY(S->sid_r.alloc(n));
     CUDA_TRY(S->sid_sorted.alloc(n));
     CUDA_TRY(S->slot_of.alloc(ns));
-    CUDA_TRY(S->ps.alloc(n));
+    CUDA_TRY(S->p_rec.alloc(2 * (n + nb)));
+    CUDA_TRY(S->p_code.alloc(n + nb + kScanPad));
+    CUDA_TRY(S->p_mat8.alloc(n + nb));
+    CUDA_TRY(S->p_mat.alloc(n + nb));
     CUDA_TRY(S->sid_of_caller_d.alloc(n));
     CUDA_TRY(S->mat_of_caller_d.alloc(n));
     CUDA_TRY(S->check_flag.alloc(1));
@@ -1155,7 +1153,6 @@ arp_status allocate(arp_sim* S) {
     CUDA_TRY(S->b_vm.alloc(nb));
     CUDA_TRY(S->b_orig.alloc(nb));
     CUDA_TRY(S->b_start.alloc(nc + 2));
-    CUDA_TRY(S->sid_of_bidx.alloc(nb));
     CUDA_TRY(S->ref.alloc(ns));
     CUDA_TRY(S->mat_of_solid.alloc(ns));
     CUDA_TRY(S->L.alloc(3 * ns));
@@ -1163,9 +1160,6 @@ arp_status allocate(arp_sim* S) {
     CUDA_TRY(S->A.alloc(3 * ns));
     CUDA_TRY(S->ksol.alloc(ns));
     CUDA_TRY(S->contact_bound.alloc(2));
-    CUDA_TRY(S->tile_counter.alloc(1));
-    CUDA_TRY(S->overflow.alloc(2 * n));  // two queues of n entries
-    CUDA_TRY(S->overflow_count.alloc(2));
     CUDA_TRY(S->ep.alloc(4 * ns));
     CUDA_TRY(S->ep_t.alloc(4 * ns));
     CUDA_TRY(S->sx.alloc(ns));
@@ -1215,10 +1209,27 @@ arp_status allocate(arp_sim* S) {
     }
     CUDA_TRY(S->d_inter.alloc(di.size()));
     CUDA_TRY(cudaMemcpy(S->d_inter.p, di.data(), di.size() * sizeof(DevInter), cudaMemcpyHostToDevice));
+    std::vector<PairMat> pm(S->inter.size());
+    for (const auto& H : S->scenes)
+        for (uint32_t i = 0; i < H.nmat; ++i)
+            for (uint32_t j = 0; j < H.nmat; ++j) {
+                const arp_material& a = S->mats[H.mat_base + i];
+                const arp_material& b = S->mats[H.mat_base + j];
+                const arp_interaction& x = S->inter[H.inter_base + size_t(i) * H.nmat + j];
+                PairMat& o = pm[H.inter_base + size_t(i) * H.nmat + j];
+                o.mass = b.mass;
+                o.visc = is_stiff(a) || b.immobile ? 0.0f : a.visc + b.visc;
+                o.bulk = b.immobile ? 0.0f : i == j ? a.bulk_visc + b.bulk_visc : x.dampening;
+                o.bits = std::min(x.potential, kPairPotential) | (is_stiff(a) ? kPairElastic1 : 0u) |
+                         (is_stiff(b) ? kPairElastic2 : 0u);
+            }
+    CUDA_TRY(S->d_pmats.alloc(pm.size()));
+    CUDA_TRY(cudaMemcpy(S->d_pmats.p, pm.data(), pm.size() * sizeof(PairMat), cudaMemcpyHostToDevice));
     S->tables.scenes = S->d_scenes.p;
     S->tables.mats = S->d_mats.p;
     S->tables.fmats = S->d_fmats.p;
     S->tables.inter = S->d_inter.p;
+    S->tables.pmats = S->d_pmats.p;
     S->tables.ncells = S->ncells;
     S->tables.max_nmat = S->max_nmat;
     S->tables.nscenes = (uint32_t)S->scenes.size();
@@ -1262,9 +1273,11 @@ arp_status run_autotune(arp_sim* S, bool force) {
     if (n == 0) return ARP_OK;
     cudaStream_t st = S->stream;
     // stage-0 inputs: y0 sorted into cell order (the state itself is unchanged)
-    S->launches += build_grid(S->Y.pd.p, S->Y.vm.p, nullptr, n, S->tables, S->gb, nullptr, S->b_start.p, st);
+    S->binned = false;
+    S->launches += build_grid(S->Y.pd.p, S->Y.vm.p, nullptr, n, S->tables, S->gb, st);
     S->launches += gather_state(S->gb.perm, n, S->Y.pd.p, S->T.pd.p, S->Y.vm.p, S->T.vm.p, S->orig.p, S->orig_r.p,
-                                S->sid.p, S->sid_r.p, nullptr, nullptr, S->ps.p, S->d_mats.p, st);
+                                S->sid.p, S->sid_r.p, nullptr, nullptr, nullptr, S->tables, st, SolidScatter{},
+                                nullptr, S->pair_out(0));
     std::swap(S->Y, S->T);
     std::swap(S->orig, S->orig_r);
     std::swap(S->sid, S->sid_r);
@@ -1288,28 +1301,21 @@ arp_status run_autotune(arp_sim* S, bool force) {
     B.next_pd = last ? S->T.pd.p : S->S[0].pd.p;  // scratch at this point
     B.next_vm = last ? S->T.vm.p : S->S[0].vm.p;
     FluidArgs f{};
-    f.xs = S->Y.pd.p;
-    f.vs = S->Y.vm.p;
+    f.rec = S->p_rec.p;
+    f.code = S->p_code.p;
+    f.mat8 = S->p_mat8.p;
+    f.mat = S->p_mat.p;
     f.start = S->gb.start;
-    f.bxs = S->b_pd.p;
-    f.bvs = S->b_vm.p;
     f.bstart = S->b_start.p;
     f.sid = S->sid.p;
-    f.sid_of_boundary_index = S->sid_of_bidx.p;
-    f.borig = S->b_orig.p;
-    f.ps = S->ps.p;
-    f.bps = S->bps.p;
     f.n = n;
-    f.any_stiff_immobile = S->any_stiff_immobile ? 1 : 0;
-    f.overflow = S->overflow.p;
-    f.overflow_count = S->overflow_count.p;
     cudaEvent_t e0 = take_event(S), e1 = take_event(S);
     float best = 1e30f;
     int best_v = 0;
     for (int v = 0; v < kNumFluidVariants; ++v) {
-        S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, S->tile_counter.p, st);  // warm-up
+        S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, st);  // warm-up
         CUDA_TRY(cudaEventRecord(e0, st));
-        for (int r = 0; r < 3; ++r) S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, S->tile_counter.p, st);
+        for (int r = 0; r < 3; ++r) S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, st);
         CUDA_TRY(cudaEventRecord(e1, st));
         CUDA_TRY(cudaEventSynchronize(e1));
         float ms = 0;
@@ -1518,7 +1524,7 @@ arp_status arp_sim_fluid_variant(const arp_sim* sim, int* variant, int* block, i
     if (!sim) return fail(ARP_ERR_INVALID_ARG, "sim is null");
     if (variant) *variant = sim->fluid_variant;
     if (block) *block = kFluidVariants[sim->fluid_variant].block;
-    if (persistent) *persistent = kFluidVariants[sim->fluid_variant].persistent;
+    if (persistent) *persistent = 0;  // no shape uses a tile queue
     return ARP_OK;
 }
 
@@ -1606,6 +1612,12 @@ arp_status arp_sim_step(arp_sim* sim, uint32_t nsteps) {
         // plain launches before a graphed step (the graph replays only steps
         // that carry the record); a plain step makes it itself
         if (graphed && sim->verlet() && !sim->vforce_valid) ARP_TRY(do_step(sim, true));
+        // likewise the graph replays only steps that find their state counted
+        // into cells by the step before
+        if (graphed && !sim->verlet() && !sim->binned) {
+            sim->launches += bin_cells(sim->Y.pd.p, sim->Y.vm.p, nullptr, sim->n, sim->tables, sim->gb, sim->stream);
+            sim->binned = true;
+        }
         if (graphed) ARP_TRY(graph_step(sim));
         else ARP_TRY(do_step(sim));
     }
@@ -1753,6 +1765,7 @@ arp_status arp_sim_set_particles(arp_sim* sim, const arp_particle* in, uint32_t 
         sim->launches += records_to_soa(sim->records.p, n, sim->sid_of_caller_d.p, sim->mat_of_caller_d.p,
                                         sim->Y.pd.p, sim->Y.vm.p, sim->orig.p, sim->sid.p, st);
         sim->vforce_valid = false;  // a new state: velocity Verlet evaluates its forces again
+        sim->binned = false;
         CUDA_TRY(cudaStreamSynchronize(st));
         ARP_TRY(check_launch("set_particles"));
     }
@@ -1812,6 +1825,7 @@ arp_status arp_sim_set_particles_async(arp_sim* sim, const arp_particle* in, uin
                                     sim->Y.pd.p, sim->Y.vm.p, sim->orig.p, sim->sid.p, st);
     CUDA_TRY(cudaEventRecord(io.in_used[q], st));
     sim->vforce_valid = false;  // a new state: velocity Verlet evaluates its forces again
+    sim->binned = false;
     return check_launch("set_particles_async");
 }
 
@@ -2022,7 +2036,8 @@ arp_status arp_sim_neighbors(arp_sim* sim, uint32_t* cell_of, uint32_t* cell_sta
     ARP_TRY(need_init(sim));
     const uint32_t n = sim->n;
     cudaStream_t st = sim->stream;
-    sim->launches += build_grid(sim->Y.pd.p, sim->Y.vm.p, nullptr, n, sim->tables, sim->gb, nullptr, nullptr, st);
+    sim->binned = false;
+    sim->launches += build_grid(sim->Y.pd.p, sim->Y.vm.p, nullptr, n, sim->tables, sim->gb, st);
     sim->launches += gather_sorted(sim->gb.perm, n, sim->Y.pd.p, sim->X.pd.p, sim->Y.vm.p, sim->X.vm.p, nullptr,
                                    nullptr, nullptr, nullptr, st);
     DevBuf<uint32_t> cnt;

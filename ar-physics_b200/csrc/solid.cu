@@ -461,10 +461,10 @@ __global__ void __launch_bounds__(kThreads) k_solid_forces(SolidArgs a, Tables T
     if (maybe && finite3(xi)) {
         for_reference_block_rows(xi, P, [&](uint32_t c0, uint32_t c1) {
             for (uint32_t k = a.start[c0]; k < a.start[c1]; ++k) {
-                if (__float_as_uint(a.vs[k].w) != mat) continue;
+                if (a.mat[k] != mat) continue;
                 const uint32_t sj = a.sid_sorted[k];
                 if (sj == kInvalid) continue;
-                const float4 xj = a.xs[k];
+                const float4 xj = a.rec[2 * (size_t)k];
                 const float3 dx = sub3(xj, xi);
                 const float3 dX = sub3(a.ref[sj], Xi);
                 const float dXX = dot3(dX, dX), dxx = dot3(dx, dx);

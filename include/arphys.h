@@ -272,15 +272,16 @@ arp_status arp_sim_update(arp_sim* sim);
  * the un-vendored crate numerical-integration is not observable, so this is
  * a stated assumption, like the Runge-Kutta tableaus. */
 arp_status arp_sim_step(arp_sim* sim, uint32_t nsteps);
-/* Time every launch shape of the fluid kernel (128 or 256 threads per block,
- * 48 or 96 listed neighbors per thread, one tile per block or persistent
- * blocks on a tile queue, lists evaluated after the scan or emptied whenever
- * a warp's next row could overfill one, or the tile's candidates staged in
- * shared memory before the scan, 64 or 128 threads per block) on the current
+/* Time every launch shape of the fluid kernel (the block form: one thread per
+ * particle lists its neighbors, four evaluate them; 128 or 256 threads per
+ * block, lists of 40 to 96; and the group form: 4, 8 or 16 threads per particle
+ * throughout, for scenes too small to fill the GPU otherwise) on the current
  * state and keep the fastest; arp_sim_init does this once per (dimension,
  * particle count, h/spacing) bucket and reuses the choice afterwards.  The
  * shapes evaluate identical arithmetic, so results do not depend on it. */
 arp_status arp_sim_autotune(arp_sim* sim, int* variant);
+/* The shape in use: its id, threads per block, and 0 (no shape uses persistent
+ * blocks on a tile queue). */
 arp_status arp_sim_fluid_variant(const arp_sim* sim, int* variant, int* block, int* persistent);
 /* Pin the fluid kernel's launch shape (0 .. arp_fluid_variant_count() - 1). */
 arp_status arp_sim_set_fluid_variant(arp_sim* sim, int variant);
