@@ -19,7 +19,7 @@
 // thread writes only its own particle.  Not differentiated: self-contact
 // (flagged when a pair is active).
 #include "grid.cuh"
-#include "warp.cuh"
+#include "solid_rec.cuh"
 
 namespace arp {
 
@@ -71,6 +71,18 @@ __device__ __forceinline__ M3 m3_cols(const float4* c) {
     r.m[0][1] = c1.x; r.m[1][1] = c1.y; r.m[2][1] = c1.z;
     r.m[0][2] = c2.x; r.m[1][2] = c2.y; r.m[2][2] = c2.z;
     return r;
+}
+// A and F of a stress record; returns its cell coordinates
+__device__ __forceinline__ uint2 m3_stress(const float4* AF, uint32_t i, M3& A, M3& F) {
+    const StressRec r = load_stress(AF, i);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            A.m[k][c] = r.A[c][k];
+            F.m[k][c] = r.F[c][k];
+        }
+    return r.cell;
 }
 __device__ __forceinline__ void m3_store_cols(const M3& a, float4* c) {
 #pragma unroll
@@ -706,14 +718,6 @@ __device__ __forceinline__ void hg_vjp(float3 dx, float3 dX, const M3& Fa, const
     o.le = le;
 }
 
-__device__ __forceinline__ bool in_stencil2(uint2 a, uint2 b) {
-    const int dx = (int)(a.x & 0xFFFFu) - (int)(b.x & 0xFFFFu);
-    const int dy = (int)(a.x >> 16) - (int)(b.x >> 16);
-    const int dz = (int)a.y - (int)b.y;
-    return a.y != 0xFFFFFFFFu && b.y != 0xFFFFFFFFu && dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1 && dz >= -1 &&
-           dz <= 1;
-}
-
 // LANES threads share one solid: both reference-list loops are split over
 // them with stride LANES, their partial sums combined by group_sum; lane 0
 // finishes the particle.
@@ -727,7 +731,7 @@ __global__ void __launch_bounds__(kT) k_adj_solid(AdjArgs a, Tables T) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = t / LANES, lane = t % LANES;
     if (i >= a.ns) return;  // whole groups leave together
-    const float4 xi = a.st.sx[i], vi = a.st.sv[i];
+    const float4 xi = a.st.sx[2 * (size_t)i], vi = a.st.sv[i];
     const uint32_t mat = __float_as_uint(vi.w);
     const DevMat mm = T.mats[mat];
     const SceneP& P = T.scenes[mm.scene];
@@ -736,9 +740,9 @@ __global__ void __launch_bounds__(kT) k_adj_solid(AdjArgs a, Tables T) {
     const float d1 = xi.w, m1 = mm.mass, V1 = m1 / d1;
     const float3 w = mul(1.0f / d1, f3(a.mu_vm[slot]));
     const float3 wdm = mask_dim(w, P.dim);
-    const M3 Ai = m3_cols(a.st.A + 3 * i), Fi = m3_cols(a.st.F + 3 * i);
+    M3 Ai, Fi;
+    const uint2 ci = m3_stress(a.st.AF, i, Ai, Fi);
     const float3 Xi = f3(a.ref[i]);
-    const uint2 ci = a.st.sc[i];
     M3 lA = m3_zero(), lFh = m3_zero();
     float3 lx = make_float3(0.f, 0.f, 0.f), fs = lx;
     float lrho = 0.0f;
@@ -747,11 +751,15 @@ __global__ void __launch_bounds__(kT) k_adj_solid(AdjArgs a, Tables T) {
         const uint32_t e = a.rl.nbr[k];
         if (!(e & kSameMatBit)) continue;
         const uint32_t j = e & ~kSameMatBit;
-        const float3 g = ref_grad(a.ref, j, Xi, P);
-        const float4 xj = a.st.sx[j];
+        const SolidPos pj = load_pos(a.st.sx, j);
+        const float3 dX = sub(f3(pj.X), Xi);
+        const float diff = P.h2 - ((dX.x * dX.x + dX.y * dX.y) + dX.z * dX.z);
+        const float3 g = mul(-6.0f * P.kconst * diff * diff, dX);
+        const float4 xj = pj.x;
         const float d2 = xj.w;
         const float c = -V1 * (m1 / d2);
-        const M3 Aj = m3_cols(a.st.A + 3 * j);
+        M3 Aj, Fj;
+        const uint2 cj = m3_stress(a.st.AF, j, Aj, Fj);
         M3 As;
 #pragma unroll
         for (int r = 0; r < 3; ++r)
@@ -766,11 +774,8 @@ __global__ void __launch_bounds__(kT) k_adj_solid(AdjArgs a, Tables T) {
         const float3 wjd = mask_dim(wj, P.dim);
         m3_add_outer(lA, -c, wjd, g);
         lrho += (c / d1) * dot(wjd, Ag);
-        if (in_stencil2(a.st.sc[j], ci)) {
-            const M3 Fj = m3_cols(a.st.F + 3 * j);
+        if (in_stencil(cj, ci)) {
             const float3 dx = sub(f3(xj), f3(xi));
-            const float3 dX = sub(f3(a.ref[j]), Xi);
-            const float diff = P.h2 - dot(dX, dX);
             const float kern = P.kconst * diff * diff * diff;
             HgGrad o;
             hg_vjp(dx, dX, Fi, Fj, d1, d2, m1, kern, P, w, o);

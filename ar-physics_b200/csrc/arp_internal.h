@@ -232,7 +232,7 @@ int gather_sorted(const uint32_t* perm, uint32_t n, const float4* a_in, float4* 
 // non-finite positions and the coordinates on the box's upper faces.  `out`:
 // what the fluid kernel reads (see FluidArgs).
 // Solid-order copies a gather writes on the side: for a gathered particle
-// whose solid id (sid_of_slot at its source slot) is valid, sx/sv/sc[sid] =
+// whose solid id (sid_of_slot at its source slot) is valid, sx[2 sid]/sv/sc[sid] =
 // its state and cell coordinates, and slot_of[sid] = its new index (when
 // slot_of is given).
 struct SolidScatter {
@@ -329,7 +329,7 @@ int ref_lists_fill(const float4* ref, const uint32_t* mat_of_solid, uint32_t ns,
                    const Tables& T, SolidRefList& rl, float4* L, cudaStream_t st);
 
 struct SolidArgs {
-    const float4* ref;        // reference positions, w = rest volume m / rho0
+    const float4* ref;        // reference positions, w = rest volume m / rho0 (self-contact; pairs read them from sx)
     const float4* L;
     SolidRefList rl;
     const float4* ep;         // stage plastic strain (4 per solid)
@@ -340,15 +340,14 @@ struct SolidArgs {
     const float4* ep_prev0;   // stored k_0, k_1, k_2
     const float4* ep_prev1;
     const float4* ep_prev2;
-    float4* F;                // [3*ns] deformation gradient columns (stage scratch)
-    float4* A;                // [3*ns] sigma * L columns (stage scratch)
+    float4* AF;               // [6*ns] stress records (stage scratch, solid_rec.cuh)
     float4* ksol;             // [ns] solid-term acceleration
     uint32_t* contact_bound;  // [2] max |u_i - u_0| bits, outside-box flag (cleared per stage)
     const float4* rec;        // sorted stage state (current-neighbor loop, see FluidArgs)
     const uint32_t* mat;
     const uint32_t* start;
     const uint32_t* sid_sorted;
-    float4* sx;               // [ns] stage position + density in solid-id order (gathered per stage)
+    const float4* sx;         // [2*ns] position records in solid-id order (solid_rec.cuh)
     float4* sv;               // [ns] stage velocity + material bits in solid-id order
     uint2* sc;                // [ns] packed cell coordinates in solid-id order
     const float2* stiff;      // [ns] per-solid (normal, shear) stiffness overriding the material's, or null
@@ -397,11 +396,9 @@ struct AdjStage {
     const float4* vm;          // (vx, vy, vz, material bits)
     const uint32_t* perm;      // sorted index -> slot of the stage grid (null: identity)
     const uint32_t* start;     // cell starts of the stage grid
-    const float4* F;           // [3*ns] deformation gradient columns
-    const float4* A;           // [3*ns] sigma * L columns
-    const float4* sx;          // [ns] solid-order state
-    const float4* sv;
-    const uint2* sc;           // [ns] packed cell coordinates
+    const float4* AF;          // [6*ns] stress records (solid_rec.cuh)
+    const float4* sx;          // [2*ns] position records
+    const float4* sv;          // [ns] velocities, material bits
     const uint32_t* contact_bound;  // [2] self-contact gate of the stage
     const float4* ep;          // [4*ns] plastic strain of the stage (columns), null without plastic materials
 };

@@ -27,6 +27,7 @@
 #include <algorithm>
 
 #include "grid.cuh"
+#include "warp.cuh"
 
 namespace arp {
 
@@ -82,9 +83,7 @@ struct PairRec {
 };
 __device__ __forceinline__ PairRec load_rec(const float4* rec, uint32_t j) {
     PairRec r;
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(r.x.x), "=f"(r.x.y), "=f"(r.x.z), "=f"(r.x.w), "=f"(r.v.x), "=f"(r.v.y), "=f"(r.v.z), "=f"(r.v.w)
-        : "l"(rec + 2 * (size_t)j));
+    load8(rec + 2 * (size_t)j, r.x, r.v);
     return r;
 }
 

@@ -391,7 +391,7 @@ __global__ void k_gather_state(const uint32_t* __restrict__ perm, uint32_t n, co
     if (sol.sx) {
         const uint32_t sid = sol.sid_of_slot[s];
         if (sid != kInvalid) {
-            sol.sx[sid] = pd;
+            sol.sx[2 * (size_t)sid] = pd;
             sol.sv[sid] = vm;
             sol.sc[sid] = sol.coord_of_slot[s];
             if (sol.slot_of) sol.slot_of[sid] = k;

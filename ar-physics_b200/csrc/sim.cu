@@ -150,8 +150,7 @@ struct StepRecord {
     DevBuf<float4> pd[kMaxStages], vm[kMaxStages];      // stage states, storage order
     DevBuf<uint32_t> perm[kMaxStages], start[kMaxStages];
     bool has_perm[kMaxStages] = {false, false, false, false};
-    DevBuf<float4> F[kMaxStages], A[kMaxStages], sx[kMaxStages], sv[kMaxStages];
-    DevBuf<uint2> sc[kMaxStages];
+    DevBuf<float4> AF[kMaxStages], sx[kMaxStages], sv[kMaxStages];
     DevBuf<uint32_t> cb[kMaxStages];
     DevBuf<float4> ep[kMaxStages];                       // plastic strain of each stage (plastic scenes)
     DevBuf<uint32_t> orig, sid, slot_of;                 // of the step (after its reorder)
@@ -287,9 +286,9 @@ struct arp_sim {
     // False whenever Y or the grid buffers have changed otherwise.
     bool binned = false;
     // solids
-    DevBuf<float4> ref, L, F, A, ksol;
+    DevBuf<float4> ref, L, AF, ksol;
     DevBuf<float4> ep, ep_t, ep_s[2], ep_acc, ep_kst[4];
-    DevBuf<float4> sx, sv;  // stage state in solid-id order
+    DevBuf<float4> sx, sv;  // position records (2 per solid) and velocities of the stage in solid-id order
     DevBuf<uint2> sc;
     DevBuf<float2> stiff;   // per-solid (normal, shear) stiffness, when set
     bool have_stiff = false;
@@ -595,6 +594,9 @@ arp_status do_init(arp_sim* S) {
         std::vector<float4> ref_dev(S->host_ref);
         for (uint32_t s = 0; s < ns; ++s) ref_dev[s].w = S->mats[mos[s]].mass / S->mats[mos[s]].start_den;
         CUDA_TRY(cudaMemcpyAsync(S->ref.p, ref_dev.data(), ns * sizeof(float4), cudaMemcpyHostToDevice, st));
+        // and the constant half of the position records
+        CUDA_TRY(cudaMemcpy2DAsync(S->sx.p + 1, 2 * sizeof(float4), S->ref.p, sizeof(float4), sizeof(float4), ns,
+                                   cudaMemcpyDeviceToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(S->mat_of_solid.p, mos.data(), ns * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemsetAsync(S->ep.p, 0, size_t(ns) * 4 * sizeof(float4), st));
         if (!S->host_ep.empty()) {
@@ -859,8 +861,7 @@ arp_status do_step(arp_sim* S, bool prime = false) {
             a.ep_prev0 = cp[0] != 0.f ? S->ep_kst[0].p : nullptr;
             a.ep_prev1 = cp[1] != 0.f ? S->ep_kst[1].p : nullptr;
             a.ep_prev2 = cp[2] != 0.f ? S->ep_kst[2].p : nullptr;
-            a.F = S->F.p;
-            a.A = S->A.p;
+            a.AF = S->AF.p;
             a.ksol = S->ksol.p;
             a.contact_bound = S->contact_bound.p;
             a.counters_cleared = n > 0 ? 1 : 0;
@@ -879,11 +880,9 @@ arp_status do_step(arp_sim* S, bool prime = false) {
             S->launches += sl;
             cur_ep = a.ep_next;
             if (R) {
-                CUDA_TRY(keep(R->F[s], (const float4*)S->F.p, 3 * size_t(ns), st));
-                CUDA_TRY(keep(R->A[s], (const float4*)S->A.p, 3 * size_t(ns), st));
-                CUDA_TRY(keep(R->sx[s], (const float4*)S->sx.p, ns, st));
+                CUDA_TRY(keep(R->AF[s], (const float4*)S->AF.p, 6 * size_t(ns), st));
+                CUDA_TRY(keep(R->sx[s], (const float4*)S->sx.p, 2 * size_t(ns), st));
                 CUDA_TRY(keep(R->sv[s], (const float4*)S->sv.p, ns, st));
-                CUDA_TRY(keep(R->sc[s], (const uint2*)S->sc.p, ns, st));
                 CUDA_TRY(keep(R->cb[s], (const uint32_t*)S->contact_bound.p, 2, st));
                 if (S->any_plastic) CUDA_TRY(keep(R->ep[s], a.ep, 4 * size_t(ns), st));
             }
@@ -1156,13 +1155,12 @@ arp_status allocate(arp_sim* S) {
     CUDA_TRY(S->ref.alloc(ns));
     CUDA_TRY(S->mat_of_solid.alloc(ns));
     CUDA_TRY(S->L.alloc(3 * ns));
-    CUDA_TRY(S->F.alloc(3 * ns));
-    CUDA_TRY(S->A.alloc(3 * ns));
+    CUDA_TRY(S->AF.alloc(6 * ns));
     CUDA_TRY(S->ksol.alloc(ns));
     CUDA_TRY(S->contact_bound.alloc(2));
     CUDA_TRY(S->ep.alloc(4 * ns));
     CUDA_TRY(S->ep_t.alloc(4 * ns));
-    CUDA_TRY(S->sx.alloc(ns));
+    CUDA_TRY(S->sx.alloc(2 * ns));
     CUDA_TRY(S->sv.alloc(ns));
     CUDA_TRY(S->sc.alloc(ns));
     CUDA_TRY(S->ep_s[0].alloc(4 * ns));
@@ -2358,11 +2356,9 @@ arp_status arp_tape_backward(arp_sim* sim, const float* dl_dstate, float* grad_s
         a.st.perm = R.has_perm[q] ? R.perm[q].p : nullptr;
         a.st.start = R.start[q].p;
         const bool sb = sim->solid_branch();
-        a.st.F = sb ? R.F[q].p : nullptr;
-        a.st.A = sb ? R.A[q].p : nullptr;
+        a.st.AF = sb ? R.AF[q].p : nullptr;
         a.st.sx = sb ? R.sx[q].p : nullptr;
         a.st.sv = sb ? R.sv[q].p : nullptr;
-        a.st.sc = sb ? R.sc[q].p : nullptr;
         a.st.contact_bound = sb ? R.cb[q].p : nullptr;
         a.sid = R.sid.p;
         a.slot_of = R.slot_of.p;

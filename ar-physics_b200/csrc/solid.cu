@@ -11,26 +11,30 @@
 //   * once per particle set: a CSR list of reference neighbors within h
 //     (solid ids, same-material flag, gradW(X_j - X_i), V_j = m_j / rho0_j)
 //     and L (k_ref_count / k_ref_fill / k_ref_L);
-//   * per stage, one thread per solid: F, Fdot from the list, Seth-Hill
+//   * per stage, 2 or 4 threads per solid: F, Fdot from the list, Seth-Hill
 //     strain + Hooke stress (all strain orders, GLSL mat4 semantics),
 //     A = sigma L, the Johnson-Cook plastic rate and its stage update
 //     (k_solid_stress);
-//   * per stage, one thread per solid: elastic force -V_i V_j (A_i + A_j)
+//   * per stage, 2 or 4 threads per solid: elastic force -V_i V_j (A_i + A_j)
 //     gradW over the list, then hourglass control and self-contact over the
 //     current 3x3x3 cells (k_solid_forces).  A_j is read, not recomputed.
 #include "grid.cuh"
 #include "mat4.cuh"
-#include "warp.cuh"
+#include "solid_rec.cuh"
 
 namespace arp {
 
 namespace {
 
 constexpr int kThreads = 128;
-#ifndef ARP_SOLID_LANES
-#define ARP_SOLID_LANES 2
-#endif
-constexpr int kSolidLanes = ARP_SOLID_LANES;  // threads per solid in the stress and force kernels
+// Both stage kernels add up entry e of a solid's reference list in partial sum
+// e mod 4 and combine them as (p0 + p2) + (p1 + p3), whatever the number of
+// threads per solid: 4 hold one partial sum each, 2 hold two.  Four threads
+// halve the chain of dependent loads of one solid, which is what a scene with
+// few solids waits for; two repeat less of the work per solid.  Stress and force
+// kernels per stage (events on both sides), 4 / 2 threads: 1,274 solids 21 / 24 us,
+// 9,072 24 / 28, 15,872 24 / 28, 32,256 34 / 32, 129,024 96 / 82.
+constexpr uint32_t kFewSolids = 24576;
 constexpr uint32_t kSameMat = 0x80000000u;
 // The stage kernels recompute gradW(dX) and W(dX) of each reference pair from
 // the reference positions (a gather that neighboring solids share in L1/L2)
@@ -205,60 +209,190 @@ __device__ __forceinline__ float4 add4(float4 a, float4 b) {
     return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
 }
 
+// The four partial sums of a solid, LANES threads holding 4 / LANES each:
+// (p0 + p2) + (p1 + p3) on every lane.
+template <int LANES>
+__device__ __forceinline__ float sum4(const float* p) {
+    static_assert(LANES == 4 || LANES == 2, "four partial sums");
+    if (LANES == 4) return group_sum<4>(p[0]);  // lanes 0..3 hold p0..p3
+    return group_sum<2>(__fadd_rn(p[0], p[4 / LANES - 1]));  // lanes 0, 1 hold p0, p2 and p1, p3
+}
+
+// 3 x 3 stress chain of strain order 2 without plastic flow: the 4 x 4 forms
+// below with their zeros and the padded fourth axis left out.  [column][row].
+struct T3 {
+    float m[3][3];
+};
+__device__ __forceinline__ T3 t3_mul(const T3& a, const T3& b) {  // a b
+    T3 r;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) r.m[c][k] = (a.m[0][k] * b.m[c][0] + a.m[1][k] * b.m[c][1]) + a.m[2][k] * b.m[c][2];
+    return r;
+}
+__device__ __forceinline__ T3 t3_transpose(const T3& a) {
+    T3 r;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) r.m[c][k] = a.m[k][c];
+    return r;
+}
+__device__ __forceinline__ T3 stress_order2(const T3& F, const T3& Fd, float lam, float mu, float lam_d, float mu_d,
+                                            uint32_t dim) {
+    T3 E = t3_mul(t3_transpose(F), F);
+    T3 R = t3_mul(t3_transpose(Fd), F);
+    float tr = 0.0f, trd = 0.0f;
+    T3 S;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const bool unused = (uint32_t)c >= dim;
+            E.m[c][k] = c == k ? (unused ? 0.0f : 0.5f * (E.m[c][k] - 1.0f)) : 0.5f * E.m[c][k];
+            S.m[c][k] = 0.5f * (R.m[c][k] + R.m[k][c]);
+        }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        if ((uint32_t)c < dim) {
+            tr += E.m[c][c];
+            trd += S.m[c][c];
+        }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float d = c == k ? 1.0f : 0.0f;
+            S.m[c][k] = (d * (lam * tr) + 2.0f * mu * E.m[c][k]) + (d * (lam_d * trd) + 2.0f * mu_d * S.m[c][k]);
+        }
+    return t3_mul(F, t3_transpose(S));
+}
+
 // ORDER2: every solid material uses strain order 2 (Green-Lagrange), so the
 // log-series, square-root and inverse paths are compiled out.
 // PLASTIC: some solid material is plastic; otherwise the plastic strain is
 // zero throughout and its buffers are neither read nor written.
-// LANES threads share one solid: they walk its reference list with stride
-// LANES and combine their partial sums with shuffles (group_sum: a fixed
-// order, so the result is deterministic); lane 0 finishes the particle.
-
+// LANES (4 or 2) threads share one solid, each with two entries' records in
+// flight; lane 0 finishes the particle.
+// Bound: L1 and L2 latency of the neighbors' records (32 + 16 bytes each), and
+// for few solids the one thread that runs the stress chain.
 template <bool ORDER2, bool PLASTIC, int LANES>
 __global__ void __launch_bounds__(kThreads) k_solid_stress(SolidArgs a, Tables T, StageCoefs c) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = t / LANES, lane = t % LANES;
     if (i >= a.ns) return;  // whole groups leave together
-    const float4 xi = a.sx[i];
+    const SolidPos pi = load_pos(a.sx, i);
+    const float4 xi = pi.x, Xs = pi.X;
     const float4 vi = a.sv[i];
-    const DevMat mm = T.mats[__float_as_uint(vi.w)];
+    const uint32_t k1 = a.rl.off[i + 1];
+    uint32_t k = a.rl.off[i] + lane;
+    const DevMat& mm = T.mats[__float_as_uint(vi.w)];
     const SceneP& P = T.scenes[mm.scene];
     if (!P.solid_branch) return;  // a scene with a single solid skips the solid term
     const float4 L0 = a.L[3 * i], L1 = a.L[3 * i + 1], L2 = a.L[3 * i + 2];
-    const float4 Xs = a.ref[i];
+    const float h2 = P.h2, kg = -6.0f * P.kconst;
     // strain.rs:139-160: F = sum V dx (x) (L gradW), Fdot likewise with dv
-    float F[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-    float Fd[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-    for (uint32_t k = a.rl.off[i] + lane; k < a.rl.off[i + 1]; k += LANES) {
-        const uint32_t j = a.rl.nbr[k] & ~kSameMat;
-        const float4 vj = a.sv[j];
-        // gradW(X_j - X_i) as k_ref_fill computes it; V_j rides in ref.w
-        const float4 Xj = a.ref[j];
-        const float3 dX = sub3(Xj, Xs);
-        const float diff = P.h2 - dot3(dX, dX);
-        const float sg = -6.0f * P.kconst * diff * diff;
-        const float4 g = make_float4(sg * dX.x, sg * dX.y, sg * dX.z, Xj.w);
-        const float3 dx = sub3(a.sx[j], xi);
+    constexpr int SETS = 4 / LANES;  // partial sums this thread holds
+    float F[3][3], Fs[SETS][3][3] = {}, Fd[3][3], Fds[SETS][3][3] = {};
+    auto add = [&](int set, const SolidPos& pj, float4 vj) {
+        // gradW(X_j - X_i) as k_ref_fill computes it; V_j rides in X.w
+        const float3 dX = sub3(pj.X, Xs);
+        const float diff = h2 - dot3(dX, dX);
+        const float sg = kg * diff * diff;
+        const float3 g = make_float3(sg * dX.x, sg * dX.y, sg * dX.z);
+        const float3 dx = sub3(pj.x, xi);
         const float3 dv = sub3(vj, vi);
-        const float gr[3] = {(L0.x * g.x + L1.x * g.y) + L2.x * g.z, (L0.y * g.x + L1.y * g.y) + L2.y * g.z,
-                             (L0.z * g.x + L1.z * g.y) + L2.z * g.z};
+        const float gr[3] = {pj.X.w * ((L0.x * g.x + L1.x * g.y) + L2.x * g.z),
+                             pj.X.w * ((L0.y * g.x + L1.y * g.y) + L2.y * g.z),
+                             pj.X.w * ((L0.z * g.x + L1.z * g.y) + L2.z * g.z)};
         const float x[3] = {dx.x, dx.y, dx.z}, v[3] = {dv.x, dv.y, dv.z};
 #pragma unroll
         for (int cc = 0; cc < 3; ++cc)
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
-                F[cc][r] += g.w * (x[r] * gr[cc]);
-                Fd[cc][r] += g.w * (v[r] * gr[cc]);
+                Fs[set][cc][r] += x[r] * gr[cc];
+                Fds[set][cc][r] += v[r] * gr[cc];
             }
+    };
+    for (; k + LANES < k1; k += 2 * LANES) {
+        const uint32_t j0 = a.rl.nbr[k] & ~kSameMat, j1 = a.rl.nbr[k + LANES] & ~kSameMat;
+        const SolidPos p0 = load_pos(a.sx, j0), p1 = load_pos(a.sx, j1);
+        const float4 v0 = a.sv[j0], v1 = a.sv[j1];
+        add(0, p0, v0);
+        add(SETS - 1, p1, v1);
     }
-    if (LANES > 1) {
+    if (k < k1) {
+        const uint32_t j = a.rl.nbr[k] & ~kSameMat;
+        add(0, load_pos(a.sx, j), a.sv[j]);
+    }
+#pragma unroll
+    for (int cc = 0; cc < 3; ++cc)
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            float f[SETS], fd[SETS];
+#pragma unroll
+            for (int q = 0; q < SETS; ++q) {
+                f[q] = Fs[q][cc][r];
+                fd[q] = Fds[q][cc][r];
+            }
+            F[cc][r] = sum4<LANES>(f);
+            Fd[cc][r] = sum4<LANES>(fd);
+        }
+    if (lane != 0) return;
+    // Bound used to skip the self-contact scan: max |u_i - u_0| over solids
+    // (u = x - X) and whether any solid left the box.
+    {
+        const SolidPos p0 = load_pos(a.sx, 0);
+        const float ux = (xi.x - Xs.x) - (p0.x.x - p0.X.x), uy = (xi.y - Xs.y) - (p0.x.y - p0.X.y),
+                    uz = (xi.z - Xs.z) - (p0.x.z - p0.X.z);
+        const float du = sqrtf((ux * ux + uy * uy) + uz * uz);
+        bool outside = !finite3(xi) || !(du == du);
+        const float pc[3] = {xi.x, xi.y, xi.z};
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            const float d = P.grid.dim[ax];
+            if (d != 0.0f) {
+                const float t = (pc[ax] - P.grid.min[ax]) / d;
+                outside = outside || !(t >= 0.0f && t < 1.0f);
+            }
+        }
+        const uint32_t mx = __reduce_max_sync(__activemask(), outside ? 0x7F800000u : __float_as_uint(du));
+        const uint32_t any_out = __reduce_or_sync(__activemask(), outside ? 1u : 0u);
+        if ((threadIdx.x & 31) == __ffs(__activemask()) - 1) {
+            atomicMax(&a.contact_bound[0], mx);
+            if (any_out) atomicOr(&a.contact_bound[1], 1u);
+        }
+    }
+    const float2 lm = a.stiff ? a.stiff[i] : make_float2(mm.lam, mm.mu);
+    StressRec out;
+    out.cell = a.sc[i];
+    if (ORDER2 && !PLASTIC) {
+        T3 Fm, Fdm, Lm;
 #pragma unroll
         for (int cc = 0; cc < 3; ++cc)
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
-                F[cc][r] = group_sum<LANES>(F[cc][r]);
-                Fd[cc][r] = group_sum<LANES>(Fd[cc][r]);
+                Fm.m[cc][r] = F[cc][r];
+                Fdm.m[cc][r] = Fd[cc][r];
             }
-        if (lane != 0) return;
+        const float4 Lc[3] = {L0, L1, L2};
+#pragma unroll
+        for (int cc = 0; cc < 3; ++cc) {
+            Lm.m[cc][0] = Lc[cc].x;
+            Lm.m[cc][1] = Lc[cc].y;
+            Lm.m[cc][2] = Lc[cc].z;
+        }
+        const T3 A = t3_mul(stress_order2(Fm, Fdm, lm.x, lm.y, mm.lam_d, mm.mu_d, P.dim), Lm);
+#pragma unroll
+        for (int cc = 0; cc < 3; ++cc)
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                out.A[cc][r] = A.m[cc][r];
+                out.F[cc][r] = F[cc][r];
+            }
+        store_stress(a.AF, i, out);
+        return;
     }
     M4 Fm = m4_zero(), Fdm = m4_zero(), Lm = m4_zero(), EP;
 #pragma unroll
@@ -289,45 +423,21 @@ __global__ void __launch_bounds__(kThreads) k_solid_stress(SolidArgs a, Tables T
     } else {
         EP = m4_zero();
     }
-    // Bound used to skip the self-contact scan: max |u_i - u_0| over solids
-    // (u = x - X) and whether any solid left the box.
-    {
-        const float4 X0 = a.ref[0];
-        const float4 x0 = a.sx[0];
-        const float4 Xi = a.ref[i];
-        const float ux = (xi.x - Xi.x) - (x0.x - X0.x), uy = (xi.y - Xi.y) - (x0.y - X0.y),
-                    uz = (xi.z - Xi.z) - (x0.z - X0.z);
-        const float du = sqrtf((ux * ux + uy * uy) + uz * uz);
-        bool outside = !finite3(xi) || !(du == du);
-        const float pc[3] = {xi.x, xi.y, xi.z};
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            const float d = P.grid.dim[ax];
-            if (d != 0.0f) {
-                const float t = (pc[ax] - P.grid.min[ax]) / d;
-                outside = outside || !(t >= 0.0f && t < 1.0f);
-            }
-        }
-        const uint32_t mx = __reduce_max_sync(__activemask(), outside ? 0x7F800000u : __float_as_uint(du));
-        const uint32_t any_out = __reduce_or_sync(__activemask(), outside ? 1u : 0u);
-        if ((threadIdx.x & 31) == __ffs(__activemask()) - 1) {
-            atomicMax(&a.contact_bound[0], mx);
-            if (any_out) atomicOr(&a.contact_bound[1], 1u);
-        }
-    }
     // solid.rs:334-341
     const M4 strain = PLASTIC ? m4_add(seth_hill<ORDER2>(Fm, mm.strain_order, P.dim), EP)
                               : seth_hill<ORDER2>(Fm, mm.strain_order, P.dim);
     const M4 rate = seth_hill_rate<ORDER2>(Fm, Fdm, mm.strain_order, P.dim);
-    const float2 lm = a.stiff ? a.stiff[i] : make_float2(mm.lam, mm.mu);
     const M4 pk2 = m4_add(hooke(strain, lm.x, lm.y, P.dim), hooke(rate, mm.lam_d, mm.mu_d, P.dim));
     const M4 sigma = m4_mul(Fm, m4_transpose(pk2));
     const M4 A = m4_mul(sigma, Lm);
 #pragma unroll
-    for (int cc = 0; cc < 3; ++cc) {
-        a.F[3 * i + cc] = make_float4(Fm.m[cc][0], Fm.m[cc][1], Fm.m[cc][2], Fm.m[cc][3]);
-        a.A[3 * i + cc] = make_float4(A.m[cc][0], A.m[cc][1], A.m[cc][2], A.m[cc][3]);
-    }
+    for (int cc = 0; cc < 3; ++cc)
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            out.A[cc][r] = A.m[cc][r];
+            out.F[cc][r] = F[cc][r];
+        }
+    store_stress(a.AF, i, out);
     // solid.rs:499-517: plastic strain rate (relaxation towards the
     // Johnson-Cook yield surface); the equivalent-strain factor is the
     // shader's integer (dim-1)/dim
@@ -375,83 +485,85 @@ __global__ void __launch_bounds__(kThreads) k_solid_stress(SolidArgs a, Tables T
     }
 }
 
-__device__ __forceinline__ bool in_stencil(uint2 a, uint2 b) {
-    const int dx = (int)(a.x & 0xFFFFu) - (int)(b.x & 0xFFFFu);
-    const int dy = (int)(a.x >> 16) - (int)(b.x >> 16);
-    const int dz = (int)a.y - (int)b.y;
-    return a.y != 0xFFFFFFFFu && b.y != 0xFFFFFFFFu && dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1 && dz >= -1 &&
-           dz <= 1;
-}
-
+// Bound: L1 and L2 latency of the neighbors' records (32 + 80 bytes each, two in
+// flight per thread).  With separate arrays of float4 columns (position, reference
+// position, cell, A, F: ten loads a neighbor) and two threads per solid the two
+// kernels took 92 us per stage of 129,024 solids and 36 us for 1,274.
 template <int LANES>
 __global__ void __launch_bounds__(kThreads) k_solid_forces(SolidArgs a, Tables T) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = t / LANES, lane = t % LANES;
     if (i >= a.ns) return;  // whole groups leave together
-    const float4 xi = a.sx[i];
+    const SolidPos pi = load_pos(a.sx, i);
+    const float4 xi = pi.x, Xi = pi.X;
     const uint32_t mat = __float_as_uint(a.sv[i].w);
-    const DevMat mm = T.mats[mat];
+    const uint32_t k1 = a.rl.off[i + 1];
+    uint32_t k = a.rl.off[i] + lane;
+    const StressRec si = load_stress(a.AF, i);
+    const DevMat& mm = T.mats[mat];
     const SceneP& P = T.scenes[mm.scene];
     if (!P.solid_branch) return;
     const float m1 = mm.mass, d1 = xi.w;
     const float V1 = m1 / d1;
-    const float4 Ai0 = a.A[3 * i], Ai1 = a.A[3 * i + 1], Ai2 = a.A[3 * i + 2];
-    const float4 Xi = a.ref[i];
-    const float4 Fi0 = a.F[3 * i], Fi1 = a.F[3 * i + 1], Fi2 = a.F[3 * i + 2];
-    const uint2 ci = a.sc[i];
-    float fx = 0.f, fy = 0.f, fz = 0.f;
+    const float h2 = P.h2, kc = P.kconst, hg_h = P.hg_h, eps_hh = P.eps_hh, eps_h = P.eps_h;
+    const uint32_t dim = P.dim;
+    constexpr int SETS = 4 / LANES;
+    float fs[3][SETS] = {};
     // Reference neighbors of the same material: the elastic force
     // (solid.rs:343-374) and, when the neighbor also sits in the current
     // 3x3x3 cells, hourglass control (solid.rs:430-443; kernel(dX) is
     // non-zero exactly for these pairs).
-    for (uint32_t k = a.rl.off[i] + lane; k < a.rl.off[i + 1]; k += LANES) {
-        const uint32_t e = a.rl.nbr[k];
-        if (!(e & kSameMat)) continue;
-        const uint32_t j = e & ~kSameMat;
-        // dX = X_j - X_i, gradW(dX) as k_ref_fill computes it
-        const float3 dX = sub3(a.ref[j], Xi);
-        const float diff = P.h2 - dot3(dX, dX);
-        const float sg = -6.0f * P.kconst * diff * diff;
-        const float3 g = make_float3(sg * dX.x, sg * dX.y, sg * dX.z);
-        const float4 xj = a.sx[j];
-        const float d2 = xj.w;
+    auto add = [&](int set, const SolidPos& pj, const StressRec& sj) {
+        float &fx = fs[0][set], &fy = fs[1][set], &fz = fs[2][set];
+        // dX = X_j - X_i, gradW(dX) = sg dX as k_ref_fill computes it
+        const float3 dX = sub3(pj.X, Xi);
+        const float diff = h2 - dot3(dX, dX);
+        const float sg = -6.0f * kc * diff * diff;
+        const float d2 = pj.x.w;
         const float V2 = __fdividef(m1, d2);  // GLSL division carries 2.5 ulp; the 2-ulp hardware quotient is used
-        const float s = -V1 * V2;
-        const float4 Aj0 = a.A[3 * j], Aj1 = a.A[3 * j + 1], Aj2 = a.A[3 * j + 2];
-        const float4 c0 = make_float4(s * (Ai0.x + Aj0.x), s * (Ai0.y + Aj0.y), s * (Ai0.z + Aj0.z), 0.f);
-        const float4 c1 = make_float4(s * (Ai1.x + Aj1.x), s * (Ai1.y + Aj1.y), s * (Ai1.z + Aj1.z), 0.f);
-        const float4 c2 = make_float4(s * (Ai2.x + Aj2.x), s * (Ai2.y + Aj2.y), s * (Ai2.z + Aj2.z), 0.f);
+        const float s = (-V1 * V2) * sg;
         // components at or above dim are dropped (solid.rs:370)
-        fx += (c0.x * g.x + c1.x * g.y) + c2.x * g.z;
-        if (P.dim >= 2) fy += (c0.y * g.x + c1.y * g.y) + c2.y * g.z;
-        if (P.dim >= 3) fz += (c0.z * g.x + c1.z * g.y) + c2.z * g.z;
-        if (in_stencil(a.sc[j], ci)) {
-            const float3 dx = sub3(xj, xi);
+        fx += s * (((si.A[0][0] + sj.A[0][0]) * dX.x + (si.A[1][0] + sj.A[1][0]) * dX.y) +
+                   (si.A[2][0] + sj.A[2][0]) * dX.z);
+        if (dim >= 2)
+            fy += s * (((si.A[0][1] + sj.A[0][1]) * dX.x + (si.A[1][1] + sj.A[1][1]) * dX.y) +
+                          (si.A[2][1] + sj.A[2][1]) * dX.z);
+        if (dim >= 3)
+            fz += s * (((si.A[0][2] + sj.A[0][2]) * dX.x + (si.A[1][2] + sj.A[1][2]) * dX.y) +
+                          (si.A[2][2] + sj.A[2][2]) * dX.z);
+        if (in_stencil(sj.cell, si.cell)) {
+            const float3 dx = sub3(pj.x, xi);
             const float l = sqrtf(dot3(dx, dx));
-            const float4 Fj0 = a.F[3 * j], Fj1 = a.F[3 * j + 1], Fj2 = a.F[3 * j + 2];
-            const float ex = ((0.5f * (Fi0.x + Fj0.x)) * dX.x + (0.5f * (Fi1.x + Fj1.x)) * dX.y) +
-                             (0.5f * (Fi2.x + Fj2.x)) * dX.z - dx.x;
-            const float ey = ((0.5f * (Fi0.y + Fj0.y)) * dX.x + (0.5f * (Fi1.y + Fj1.y)) * dX.y) +
-                             (0.5f * (Fi2.y + Fj2.y)) * dX.z - dx.y;
-            const float ez = ((0.5f * (Fi0.z + Fj0.z)) * dX.x + (0.5f * (Fi1.z + Fj1.z)) * dX.y) +
-                             (0.5f * (Fi2.z + Fj2.z)) * dX.z - dx.z;
-            const float kern = P.kconst * diff * diff * diff;  // W(dX)
+            float e[3];
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+                e[r] = 0.5f * (((si.F[0][r] + sj.F[0][r]) * dX.x + (si.F[1][r] + sj.F[1][r]) * dX.y) +
+                               (si.F[2][r] + sj.F[2][r]) * dX.z);
+            const float ex = e[0] - dx.x, ey = e[1] - dx.y, ez = e[2] - dx.z;
+            const float kern = kc * diff * diff * diff;  // W(dX)
             const float sh = ((__fdividef(100000000.0f * m1 * m1, d1 * d2) *
-                               __fdividef(0.5f * ((ex * dx.x + ey * dx.y) + ez * dx.z), l + P.hg_h)) *
-                              __fdividef(1.0f, l * l + P.eps_hh)) *
+                               __fdividef(0.5f * ((ex * dx.x + ey * dx.y) + ez * dx.z), l + hg_h)) *
+                              __fdividef(1.0f, l * l + eps_hh)) *
                              kern;
-            const float den = l + P.eps_h;
-            fx -= __fdividef(sh * dx.x, den);
-            fy -= __fdividef(sh * dx.y, den);
-            fz -= __fdividef(sh * dx.z, den);
+            const float u = __fdividef(sh, l + eps_h);
+            fx -= u * dx.x;
+            fy -= u * dx.y;
+            fz -= u * dx.z;
         }
+    };
+    for (; k + LANES < k1; k += 2 * LANES) {
+        const uint32_t e0 = a.rl.nbr[k], e1 = a.rl.nbr[k + LANES];
+        const SolidPos p0 = load_pos(a.sx, e0 & ~kSameMat), p1 = load_pos(a.sx, e1 & ~kSameMat);
+        const StressRec s0 = load_stress(a.AF, e0 & ~kSameMat), s1 = load_stress(a.AF, e1 & ~kSameMat);
+        if (e0 & kSameMat) add(0, p0, s0);
+        if (e1 & kSameMat) add(SETS - 1, p1, s1);
     }
-    if (LANES > 1) {
-        fx = group_sum<LANES>(fx);
-        fy = group_sum<LANES>(fy);
-        fz = group_sum<LANES>(fz);
-        if (lane != 0) return;
+    if (k < k1) {
+        const uint32_t e = a.rl.nbr[k], j = e & ~kSameMat;
+        if (e & kSameMat) add(0, load_pos(a.sx, j), load_stress(a.AF, j));
     }
+    float fx = sum4<LANES>(fs[0]), fy = sum4<LANES>(fs[1]), fz = sum4<LANES>(fs[2]);
+    if (lane != 0) return;
     // Self-contact (solid.rs:428,445-450): same-material neighbors in the
     // current cells whose reference distance exceeds r_cut.  Skipped when
     // every solid is inside the box and r_cut - max|dx in stencil| exceeds
@@ -498,17 +610,24 @@ int ref_lists_fill(const float4* ref, const uint32_t* mat_of, uint32_t ns, const
     return 2;
 }
 
-int launch_solid(const SolidArgs& a, const Tables& T, const StageCoefs& c, cudaStream_t st) {
-    if (a.ns == 0) return 0;
-    if (!a.counters_cleared) cudaMemsetAsync(a.contact_bound, 0, 2 * sizeof(uint32_t), st);
-    // a.sx, a.sv, a.sc were written by the stage's gather (gather_state)
-    constexpr int L = kSolidLanes;
+namespace {
+template <int L>
+void launch_solid_lanes(const SolidArgs& a, const Tables& T, const StageCoefs& c, cudaStream_t st) {
     const uint32_t blocks = blocks_for(a.ns * L, kThreads);
     if (a.all_order2 && !a.any_plastic) k_solid_stress<true, false, L><<<blocks, kThreads, 0, st>>>(a, T, c);
     else if (a.all_order2) k_solid_stress<true, true, L><<<blocks, kThreads, 0, st>>>(a, T, c);
     else if (!a.any_plastic) k_solid_stress<false, false, L><<<blocks, kThreads, 0, st>>>(a, T, c);
     else k_solid_stress<false, true, L><<<blocks, kThreads, 0, st>>>(a, T, c);
     k_solid_forces<L><<<blocks, kThreads, 0, st>>>(a, T);
+}
+}  // namespace
+
+int launch_solid(const SolidArgs& a, const Tables& T, const StageCoefs& c, cudaStream_t st) {
+    if (a.ns == 0) return 0;
+    if (!a.counters_cleared) cudaMemsetAsync(a.contact_bound, 0, 2 * sizeof(uint32_t), st);
+    // a.sx (its stage half), a.sv and a.sc were written by the stage's gather (gather_state)
+    if (a.ns <= kFewSolids) launch_solid_lanes<4>(a, T, c, st);
+    else launch_solid_lanes<2>(a, T, c, st);
     return 2;
 }
 

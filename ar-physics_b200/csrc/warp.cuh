@@ -1,9 +1,16 @@
-// warp.cuh -- sums over the lanes of a thread group inside a warp.
+// warp.cuh -- sums over the lanes of a thread group inside a warp, 32-byte loads.
 #pragma once
 
 #include <cstdint>
 
 namespace arp {
+
+// One 32-byte sector in one load (p 32-byte aligned, read-only in the kernel).
+__device__ __forceinline__ void load8(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
 
 // Sum of v over the LANES consecutive lanes (LANES a power of two, at most
 // 32) that share one item: a butterfly of shuffles, the same order on every
