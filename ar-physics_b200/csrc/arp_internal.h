@@ -191,29 +191,31 @@ arp_status set_error(arp_status code, const std::string& msg);
 struct GridBuffers {
     uint32_t* key;         // [cap] cell id of each slot (ncells for non-finite)
     uint32_t* rank;        // [cap] arrival rank inside the cell
-    uint32_t* count;       // [ncells + 1] occupancy (zeroed by the scan)
+    uint32_t* count;       // [ncells + 2] occupancy, then its prefix inside tiles; cleared by the ordering
     uint32_t* start;       // [ncells + 2] exclusive prefix of count
     uint32_t* perm;        // [cap] sorted index -> slot
     uint2* coord;          // [cap] packed cell coordinates of each slot: x | y << 16, z
     uint32_t* block_sums;  // scan partials
     uint32_t block_sums_cap;
+    bool scattered;        // count holds a prefix that the ordering has not cleared yet (a graph replay of a step
+                           // begins and ends with the same value)
 };
 
-// Builds cell_start / perm for `n` positions.  Counting sort: keys and
-// histogram, exclusive scan (bin_cells; a kernel that writes the state may do
-// the first of the two through CellBins, then scan_cells), scatter, then
-// ascending slot order within each cell (sort_cells).  build_grid is both.
-// Each returns the number of kernel launches issued.
+// The grid of `n` positions: cell_start / perm by a counting sort.  Keys and
+// histogram (k_cell_keys, or the kernel that writes the state through
+// CellBins), cell starts and scatter (scatter_cells; bin_cells does both), then
+// ascending slot order within each cell: order_cells, or order_gather, which
+// gathers the state into that order as well.  build_grid is bin_cells and
+// order_cells.  Each returns the number of kernel launches issued.
 // The scene of item i is mats[material].scene, the material read from
 // vm[i].w (bits) when vm is given, else from mat_u32[i].
+// `zero2` (may be null) points at two counters to clear for the stage's later
+// kernels.
 inline CellBins cell_bins(const GridBuffers& gb) { return CellBins{gb.key, gb.rank, gb.count, gb.coord}; }
 int bin_cells(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
-              GridBuffers& gb, cudaStream_t st);
-int scan_cells(const Tables& T, GridBuffers& gb, cudaStream_t st);
-// `stats` (may be null) receives the occupancy counters; `zero2` (may be
-// null) points at two counters to clear for the stage's later kernels.
-int sort_cells(uint32_t n, const Tables& T, GridBuffers& gb, DevStats* stats, const uint32_t* boundary_start,
-               uint32_t* zero2, cudaStream_t st);
+              GridBuffers& gb, uint32_t* zero2, cudaStream_t st);
+int scatter_cells(uint32_t n, const Tables& T, GridBuffers& gb, uint32_t* zero2, cudaStream_t st);
+int order_cells(const Tables& T, GridBuffers& gb, cudaStream_t st);
 int build_grid(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
                GridBuffers& gb, cudaStream_t st);
 
@@ -226,11 +228,6 @@ uint32_t scan_block_sums_needed(uint32_t len);
 int gather_sorted(const uint32_t* perm, uint32_t n, const float4* a_in, float4* a_out, const float4* b_in,
                   float4* b_out, const uint32_t* c_in, uint32_t* c_out, const uint32_t* d_in, uint32_t* d_out,
                   cudaStream_t st);
-// Gather a state into sorted order (out[k] = in[perm[k]]) and evaluate the
-// pressure term p / rho^2 of every gathered particle (fluid.rs:45-52,
-// :128,165).  Any pointer pair may be null.  With `stats`, counts the
-// non-finite positions and the coordinates on the box's upper faces.  `out`:
-// what the fluid kernel reads (see FluidArgs).
 // Solid-order copies a gather writes on the side: for a gathered particle
 // whose solid id (sid_of_slot at its source slot) is valid, sx[2 sid]/sv/sc[sid] =
 // its state and cell coordinates, and slot_of[sid] = its new index (when
@@ -243,16 +240,25 @@ struct SolidScatter {
     uint2* sc = nullptr;
     uint32_t* slot_of = nullptr;
 };
+// What the fluid kernel reads (see FluidArgs).
 struct PairOut {
     float4* rec = nullptr;
     uint32_t* code = nullptr;
     uint8_t* mat8 = nullptr;
     uint32_t* mat = nullptr;  // may be null
 };
+// Gathers a state into sorted order (out[k] = in[perm[k]]) and evaluates the
+// pressure term p / rho^2 of every gathered particle (fluid.rs:45-52,
+// :128,165).  Null outputs are skipped.
 int gather_state(const uint32_t* perm, uint32_t n, const float4* pd_in, float4* pd_out, const float4* vm_in,
                  float4* vm_out, const uint32_t* a_in, uint32_t* a_out, const uint32_t* b_in, uint32_t* b_out,
-                 const uint2* c_in, uint2* c_out, float* ps_out, const Tables& T, cudaStream_t st,
-                 const SolidScatter& sol = SolidScatter{}, DevStats* stats = nullptr, const PairOut& out = PairOut{});
+                 float* ps_out, const Tables& T, cudaStream_t st, const PairOut& out = PairOut{});
+// order_cells and such a gather in one launch.  With `stats`, the occupancy
+// counters, the non-finite positions and the coordinates on the box's upper
+// faces are counted too.
+int order_gather(const Tables& T, GridBuffers& gb, const uint32_t* boundary_start, const float4* pd_in, float4* pd_out,
+                 const float4* vm_in, float4* vm_out, const uint32_t* a_in, uint32_t* a_out, const uint32_t* b_in,
+                 uint32_t* b_out, cudaStream_t st, const SolidScatter& sol, DevStats* stats, const PairOut& out);
 
 // Particle records (caller order) to structure of arrays in caller order, and
 // back from cell order into caller order (the state exchange of the C ABI).

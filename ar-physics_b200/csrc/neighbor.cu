@@ -6,16 +6,19 @@
 // atomics, so slot order is nondeterministic on a GPU and particles past 128
 // are dropped.  Here the grid is a counting sort with no capacity limit:
 //   1. cell key + histogram (one atomic per particle; the returned value is
-//      the particle's arrival rank inside its cell);
-//   2. exclusive scan of the histogram (warp-shuffle block scan, block sums,
-//      offsets), which also clears the histogram for the next build;
-//   3. scatter to perm[start[key] + rank];
-//   4. sort each cell's run by slot so the order is deterministic for every
-//      run length (short runs by one thread, long runs by the whole block);
-//      this also records the largest occupancy and cells over the
-//      reference's 128.
-// Memory traffic per particle: 16 B position read, 4+4 B key/rank write and
-// read, 4 B perm write, 4+4 B perm read/write in the run sort.
+//      the particle's arrival rank inside its cell), by the kernel that writes
+//      the state where there is one (CellBins), else by k_cell_keys;
+//   2. k_scan_tiles: exclusive prefix of the histogram inside tiles of 4096
+//      cells, in place, and the tile totals;
+//   3. k_scatter: every block turns the tile totals into tile bases itself,
+//      writes its share of the cell starts (prefix + base) and scatters its
+//      particles to perm[start[key] + rank];
+//   4. k_order_gather: per block of cells, the slots of each cell ascending (so
+//      the order is deterministic for every run length) and the state gathered
+//      into that order; it also clears the histogram and records the largest
+//      occupancy and cells over the reference's 128.
+// Memory traffic per particle: 16 B position, 4+4 B key/rank, 4+4 B perm, and
+// the state read and written once.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -73,29 +76,43 @@ __device__ __forceinline__ void block_excl_scan(uint32_t v, uint32_t& excl) {
     excl = warp_tot[warp] + inc - v;
 }
 
-// `count` and `out` may be the same array (the allocation-free build scans in
-// place), so they are not declared __restrict__.
-__global__ void k_scan_tiles(uint32_t* count, uint32_t len, uint32_t* out, uint32_t* __restrict__ block_sums) {
+// Exclusive prefix inside each tile of kScanTile counts and the tile totals.
+// `count` and `out` may be the same array, so they are not declared
+// __restrict__; with CLEAR (different arrays) the counts are left at zero for
+// the next histogram.  `wide`: both arrays are 16-byte aligned (the
+// allocation-free build scans a caller's array, which need not be).
+template <bool CLEAR>
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t* count, uint32_t len, uint32_t* out,
+                                                             uint32_t* __restrict__ block_sums, bool wide) {
     __shared__ uint32_t last_total;
     const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    uint32_t s = 0;
+    uint32_t v[kScanItems] = {0u, 0u, 0u, 0u};
+    static_assert(kScanItems == 4, "one 16-byte load per thread");
+    const bool whole = wide && base + kScanItems <= len;
+    if (whole) {
+        const uint4 q = *reinterpret_cast<const uint4*>(count + base);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+        if (CLEAR) *reinterpret_cast<uint4*>(count + base) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
 #pragma unroll
-    for (int j = 0; j < kScanItems; ++j) {
-        uint32_t idx = base + j;
-        v[j] = idx < len ? count[idx] : 0u;
-        if (idx < len) count[idx] = 0u;  // ready for the next histogram
-        s += v[j];
+        for (int j = 0; j < kScanItems; ++j)
+            if (base + j < len) {
+                v[j] = count[base + j];
+                if (CLEAR) count[base + j] = 0u;
+            }
     }
     uint32_t excl;
+    const uint32_t s = v[0] + v[1] + v[2] + v[3];
     block_excl_scan(s, excl);
     if (threadIdx.x == blockDim.x - 1) last_total = excl + s;
-    uint32_t run = excl;
+    const uint4 o = make_uint4(excl, excl + v[0], excl + v[0] + v[1], excl + v[0] + v[1] + v[2]);
+    if (whole) {
+        *reinterpret_cast<uint4*>(out + base) = o;
+    } else {
+        const uint32_t w[kScanItems] = {o.x, o.y, o.z, o.w};
 #pragma unroll
-    for (int j = 0; j < kScanItems; ++j) {
-        uint32_t idx = base + j;
-        if (idx < len) out[idx] = run;
-        run += v[j];
+        for (int j = 0; j < kScanItems; ++j)
+            if (base + j < len) out[base + j] = w[j];
     }
     __syncthreads();
     if (threadIdx.x == 0) block_sums[blockIdx.x] = last_total;
@@ -129,13 +146,57 @@ __global__ void k_scan_add(uint32_t* out, uint32_t len, const uint32_t* __restri
     }
 }
 
-__global__ void k_scatter(const uint32_t* __restrict__ key, const uint32_t* __restrict__ rank, uint32_t n,
-                          const uint32_t* __restrict__ start, uint32_t* __restrict__ perm,
-                          uint32_t* __restrict__ zero2) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+// Cell starts and scatter from the tile-local prefix `local` (k_scan_tiles in
+// place) and the tile totals, which every block sums up itself: at most
+// kBaseTiles of them (4 M cells), so no pass of its own finishes the scan.
+constexpr uint32_t kBaseTiles = 1024;
+__global__ void __launch_bounds__(kThreads) k_scatter(const uint32_t* __restrict__ key,
+                                                      const uint32_t* __restrict__ rank, uint32_t n,
+                                                      const uint32_t* __restrict__ local,
+                                                      const uint32_t* __restrict__ sums, uint32_t len,
+                                                      uint32_t* __restrict__ start, uint32_t* __restrict__ perm,
+                                                      uint32_t* __restrict__ zero2) {
+    __shared__ uint32_t tile_base[kBaseTiles];
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (zero2 && i < 2u) zero2[i] = 0u;
-    if (i >= n) return;
-    perm[start[key[i]] + rank[i]] = i;
+    // loads that do not need the bases first
+    const bool mine = i < n;
+    const uint32_t c = mine ? key[i] : 0u;
+    const uint32_t at = mine ? local[c] + rank[i] : 0u;
+    const uint32_t q = 4u * i;
+    uint4 st = make_uint4(0u, 0u, 0u, 0u);
+    if (q + 4u <= len) st = *reinterpret_cast<const uint4*>(local + q);
+    const uint32_t tiles = (len + kScanTile - 1) / kScanTile;
+    static_assert(kBaseTiles == 4 * kThreads, "four totals per thread");
+    {
+        uint32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = 4u * threadIdx.x + j < tiles ? sums[4u * threadIdx.x + j] : 0u;
+        uint32_t excl;
+        block_excl_scan(v[0] + v[1] + v[2] + v[3], excl);
+        tile_base[4u * threadIdx.x] = excl;
+        tile_base[4u * threadIdx.x + 1] = excl + v[0];
+        tile_base[4u * threadIdx.x + 2] = excl + v[0] + v[1];
+        tile_base[4u * threadIdx.x + 3] = excl + v[0] + v[1] + v[2];
+    }
+    __syncthreads();
+    if (mine) perm[at + tile_base[c / kScanTile]] = i;
+    if (q < len) {
+        const uint32_t b = tile_base[q / kScanTile];  // four entries of one tile
+        if (q + 4u <= len) {
+            *reinterpret_cast<uint4*>(start + q) = make_uint4(st.x + b, st.y + b, st.z + b, st.w + b);
+        } else {
+            for (uint32_t j = q; j < len; ++j) start[j] = local[j] + b;
+        }
+    }
+}
+// The same scatter from finished cell starts (grids of more tiles).
+__global__ void k_scatter_plain(const uint32_t* __restrict__ key, const uint32_t* __restrict__ rank, uint32_t n,
+                                const uint32_t* __restrict__ start, uint32_t* __restrict__ perm,
+                                uint32_t* __restrict__ zero2) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (zero2 && i < 2u) zero2[i] = 0u;
+    if (i < n) perm[start[key[i]] + rank[i]] = i;
 }
 
 // Occupancy (mobile + boundary) of the reference cell whose first search
@@ -287,33 +348,25 @@ __device__ void block_bitonic_run(uint32_t* perm, uint32_t b, uint32_t L, uint32
     __syncthreads();
 }
 
-// Sort each cell's run ascending, so the order inside a cell never depends
-// on the arrival order of the histogram's atomics: runs of at most kShortRun
-// by an insertion sort on their own thread, runs of at most kWarpRun by one
-// warp each (warp_sort_run; the block's warps share its runs), runs of at
-// most kBlockRun by the whole block in shared memory (block_bitonic_run), and
-// longer ones (cells that gather particles outside the box, which are
-// clamped into the edge cells) by the whole block through the scratch `tmp`,
-// free once the scatter has run (block_sort_run).
-// With `stats`, also the occupancy counters of the reference cells.
-__global__ void __launch_bounds__(kThreads) k_sort_runs(const uint32_t* __restrict__ start, uint32_t ncells,
-                                                        uint32_t* __restrict__ perm, uint32_t* __restrict__ tmp,
-                                                        const uint32_t* __restrict__ boundary_start, DevStats* stats,
-                                                        Tables T) {
+// Sorts the runs of the block's kThreads cells (cells past ncells are the
+// non-finite bucket, then nothing) ascending in global memory, so the order
+// inside a cell never depends on the arrival order of the histogram's atomics:
+// runs of at most kShortRun by an insertion sort on their own thread, runs of
+// at most kWarpRun by one warp each (warp_sort_run; the block's warps share its
+// runs), runs of at most kBlockRun by the whole block in shared memory
+// (block_bitonic_run), and longer ones (cells that gather particles outside the
+// box, which are clamped into the edge cells) by the whole block through the
+// scratch `tmp`, free once the scatter has run (block_sort_run).
+__device__ void sort_block_runs(const uint32_t* start, uint32_t ncells, uint32_t* perm, uint32_t* tmp,
+                                uint32_t* wbuf /* [kBlockRun] shared */) {
     __shared__ uint32_t long_cells[kThreads], mid_cells[kThreads];
     __shared__ uint32_t nlong, nmid;
-    __shared__ uint32_t wbuf[kBlockRun];  // kThreads / 32 warp buffers of kWarpRun, or one block buffer
     if (threadIdx.x == 0) nlong = nmid = 0;
     __syncthreads();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c <= ncells) {  // includes the non-finite bucket at index ncells
         const uint32_t b = start[c], e = start[c + 1];
         const uint32_t len = e - b;
-        if (stats && c < ncells) {
-            const uint32_t occ = reference_cell_occupancy(c, start, boundary_start, T);
-            if (occ > 0) atomicMax(&stats->max_cell_occupancy, occ);
-            if (occ > kBucketSlots) atomicAdd(&stats->overflow_cells, 1u);
-        }
         if (len > kWarpRun) {
             long_cells[atomicAdd(&nlong, 1u)] = c;
         } else if (len > kShortRun) {
@@ -344,6 +397,56 @@ __global__ void __launch_bounds__(kThreads) k_sort_runs(const uint32_t* __restri
         if (L <= kBlockRun) block_bitonic_run(perm, start[lc], L, wbuf);
         else block_sort_run(perm, tmp, start[lc], start[lc + 1]);
     }
+    __syncthreads();
+}
+
+// The runs of a block's cells ordered without moving data twice: when they
+// hold at most kStage slots and none is longer than kWarpRun, the slots are
+// staged in shared memory and every thread ranks its slot among its cell's by
+// counting the smaller ones (a handful of shared-memory reads for the few
+// particles of a search cell); f(position, slot) is called for each.  Other
+// blocks are sorted in global memory first.  Insertion sorts in global memory,
+// one thread per cell, took 14 us per stage of the 1 M-particle scene.
+constexpr uint32_t kStage = kBlockRun;
+// `key(slot)` is the slot's cell.
+template <class Key, class F>
+__device__ __forceinline__ void order_block(const uint32_t* start, uint32_t ncells, uint32_t* perm, uint32_t* tmp,
+                                            Key&& key, F&& f) {
+    __shared__ uint32_t buf[kStage];
+    __shared__ uint32_t cstart[kThreads + 1];
+    const uint32_t c0 = blockIdx.x * kThreads;
+    const uint32_t c = c0 + threadIdx.x;
+    // cells 0 .. ncells (the last is the non-finite bucket), start has ncells + 2 entries
+    const uint32_t s0 = start[min(c, ncells + 1u)], s1 = start[min(c + 1u, ncells + 1u)];
+    cstart[threadIdx.x] = s0;
+    if (threadIdx.x == kThreads - 1) cstart[kThreads] = s1;
+    const int lengthy = __syncthreads_or(s1 - s0 > kWarpRun);
+    const uint32_t p0 = cstart[0], m = cstart[kThreads] - p0;
+    if (m == 0u) return;
+    if (!lengthy && m <= kStage) {
+        for (uint32_t t = threadIdx.x; t < m; t += kThreads) buf[t] = perm[p0 + t];
+        __syncthreads();
+        for (uint32_t t = threadIdx.x; t < m; t += kThreads) {
+            const uint32_t v = buf[t];
+            const uint32_t q = key(v) - c0;
+            const uint32_t b = cstart[q] - p0, e = cstart[q + 1] - p0;
+            uint32_t at = b;
+            for (uint32_t j = b; j < e; ++j) at += buf[j] < v ? 1u : 0u;
+            f(p0 + at, v);
+        }
+        return;
+    }
+    sort_block_runs(start, ncells, perm, tmp, buf);
+    for (uint32_t t = threadIdx.x; t < m; t += kThreads) f(p0 + t, perm[p0 + t]);
+}
+
+__global__ void __launch_bounds__(kThreads) k_order(const uint32_t* __restrict__ start, uint32_t ncells, uint32_t* perm,
+                                                    uint32_t* tmp, const uint32_t* __restrict__ key,
+                                                    uint32_t* __restrict__ count) {
+    const uint32_t c = blockIdx.x * kThreads + threadIdx.x;
+    if (count && c < ncells + 2u) count[c] = 0u;  // ready for the next histogram
+    order_block(start, ncells, perm, tmp, [&](uint32_t v) { return key[v]; },
+                [&](uint32_t at, uint32_t v) { perm[at] = v; });
 }
 
 __global__ void k_gather(const uint32_t* __restrict__ perm, uint32_t n, const float4* __restrict__ a_in,
@@ -374,56 +477,89 @@ __device__ __forceinline__ float eos_pressure(uint32_t eq, float density, float 
     }
 }
 
-__global__ void k_gather_state(const uint32_t* __restrict__ perm, uint32_t n, const float4* __restrict__ pd_in,
-                               float4* __restrict__ pd_out, const float4* __restrict__ vm_in,
-                               float4* __restrict__ vm_out, const uint32_t* __restrict__ a_in,
-                               uint32_t* __restrict__ a_out, const uint32_t* __restrict__ b_in,
-                               uint32_t* __restrict__ b_out, const uint2* __restrict__ c_in,
-                               uint2* __restrict__ c_out, float* __restrict__ ps_out, Tables T, SolidScatter sol,
-                               DevStats* stats, PairOut out) {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const uint32_t s = perm ? perm[k] : k;
-    const float4 pd = pd_in[s];
-    const float4 vm = vm_in[s];
-    if (pd_out) pd_out[k] = pd;
-    if (vm_out) vm_out[k] = vm;
-    if (sol.sx) {
-        const uint32_t sid = sol.sid_of_slot[s];
+// What a gather of a state reads and writes: slot s of the source goes to
+// sorted position k.  Null pointers are skipped.
+struct GatherArgs {
+    const float4 *pd_in, *vm_in;
+    float4 *pd_out, *vm_out;
+    const uint32_t *a_in, *b_in;
+    uint32_t *a_out, *b_out;
+    float* ps_out;
+    SolidScatter sol;
+    DevStats* stats;
+    PairOut out;
+};
+__device__ __forceinline__ void gather_one(const GatherArgs& g, const Tables& T, uint32_t k, uint32_t s) {
+    const float4 pd = g.pd_in[s];
+    const float4 vm = g.vm_in[s];
+    if (g.pd_out) g.pd_out[k] = pd;
+    if (g.vm_out) g.vm_out[k] = vm;
+    if (g.sol.sx) {
+        const uint32_t sid = g.sol.sid_of_slot[s];
         if (sid != kInvalid) {
-            sol.sx[2 * (size_t)sid] = pd;
-            sol.sv[sid] = vm;
-            sol.sc[sid] = sol.coord_of_slot[s];
-            if (sol.slot_of) sol.slot_of[sid] = k;
+            g.sol.sx[2 * (size_t)sid] = pd;
+            g.sol.sv[sid] = vm;
+            g.sol.sc[sid] = g.sol.coord_of_slot[s];
+            if (g.sol.slot_of) g.sol.slot_of[sid] = k;
         }
     }
-    if (a_out) a_out[k] = a_in[s];
-    if (b_out) b_out[k] = b_in[s];
-    if (c_out) c_out[k] = c_in[s];
-    if (stats) {
-        if (!finite3(pd)) {
-            atomicAdd(&stats->nonfinite_positions, 1u);
-        } else {
-            // a coordinate on the upper face would hash one past the last cell
-            const Grid& g = T.scenes[T.mats[__float_as_uint(vm.w)].scene].grid;
-            const bool face = (g.dim[0] != 0.0f && pd.x == g.min[0] + g.dim[0]) ||
-                              (g.dim[1] != 0.0f && pd.y == g.min[1] + g.dim[1]) ||
-                              (g.dim[2] != 0.0f && pd.z == g.min[2] + g.dim[2]);
-            if (face) atomicAdd(&stats->clamped_coordinates, 1u);
-        }
-    }
+    if (g.a_out) g.a_out[k] = g.a_in[s];
+    if (g.b_out) g.b_out[k] = g.b_in[s];
     const uint32_t mat = __float_as_uint(vm.w);
     const DevMat& m = T.mats[mat];
+    if (g.stats) {
+        if (!finite3(pd)) {
+            atomicAdd(&g.stats->nonfinite_positions, 1u);
+        } else {
+            // a coordinate on the upper face would hash one past the last cell
+            const Grid& gr = T.scenes[m.scene].grid;
+            const bool face = (gr.dim[0] != 0.0f && pd.x == gr.min[0] + gr.dim[0]) ||
+                              (gr.dim[1] != 0.0f && pd.y == gr.min[1] + gr.dim[1]) ||
+                              (gr.dim[2] != 0.0f && pd.z == gr.min[2] + gr.dim[2]);
+            if (face) atomicAdd(&g.stats->clamped_coordinates, 1u);
+        }
+    }
     const float p = eos_pressure(m.state_eq, pd.w, m.sound_speed, m.target_den);
     const float ps = p / (pd.w * pd.w);
-    if (ps_out) ps_out[k] = ps;
-    if (out.rec) {
-        out.rec[2 * (size_t)k] = pd;
-        out.rec[2 * (size_t)k + 1] = make_float4(vm.x, vm.y, vm.z, ps);
-        out.code[k] = scan_code(pd, T.scenes[m.scene]);
-        out.mat8[k] = (uint8_t)m.local;
-        if (out.mat) out.mat[k] = mat;
+    if (g.ps_out) g.ps_out[k] = ps;
+    if (g.out.rec) {
+        g.out.rec[2 * (size_t)k] = pd;
+        g.out.rec[2 * (size_t)k + 1] = make_float4(vm.x, vm.y, vm.z, ps);
+        g.out.code[k] = scan_code(pd, T.scenes[m.scene]);
+        g.out.mat8[k] = (uint8_t)m.local;
+        if (g.out.mat) g.out.mat[k] = mat;
     }
+}
+
+__global__ void k_gather_state(const uint32_t* __restrict__ perm, uint32_t n, GatherArgs g, Tables T) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) gather_one(g, T, k, perm ? perm[k] : k);
+}
+
+// Orders the block's cells and gathers the state of their particles.  Also,
+// with `stats`, the occupancy counters of the reference cells.
+__global__ void __launch_bounds__(kThreads) k_order_gather(const uint32_t* __restrict__ start, uint32_t ncells,
+                                                           uint32_t* perm, uint32_t* tmp,
+                                                           const uint32_t* __restrict__ key,
+                                                           uint32_t* __restrict__ count,
+                                                           const uint32_t* __restrict__ boundary_start, DevStats* stats,
+                                                           GatherArgs g, Tables T) {
+    const uint32_t c = blockIdx.x * kThreads + threadIdx.x;
+    if (c < ncells + 2u) count[c] = 0u;  // ready for the next histogram
+    if (stats) {
+        const uint32_t occ = c < ncells ? reference_cell_occupancy(c, start, boundary_start, T) : 0u;
+        const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, occ);
+        const uint32_t over = __popc(__ballot_sync(0xFFFFFFFFu, occ > kBucketSlots));
+        if ((threadIdx.x & 31u) == 0u) {
+            if (most > 0u) atomicMax(&stats->max_cell_occupancy, most);
+            if (over > 0u) atomicAdd(&stats->overflow_cells, over);
+        }
+    }
+    order_block(start, ncells, perm, tmp, [&](uint32_t v) { return key[v]; },
+                [&](uint32_t at, uint32_t v) {
+                    perm[at] = v;
+                    gather_one(g, T, at, v);
+                });
 }
 
 // Particle records (48 B, caller order) -> structure of arrays in caller order.
@@ -524,6 +660,17 @@ __global__ void k_scatter_noalloc(const float4* __restrict__ pos, uint32_t n, Gr
     perm[start[k] + rank[i]] = i;
 }
 
+__global__ void __launch_bounds__(kThreads) k_order_noalloc(const float4* __restrict__ pos, Grid grid,
+                                                            const uint32_t* __restrict__ start, uint32_t* perm,
+                                                            uint32_t* tmp) {
+    order_block(start, grid.ncells, perm, tmp,
+                [&](uint32_t v) {
+                    const float4 p = pos[v];
+                    return finite3(p) ? cell_id(cell_coord(p, grid), grid) : grid.ncells;
+                },
+                [&](uint32_t at, uint32_t v) { perm[at] = v; });
+}
+
 // Device address of g_noalloc_scratch, looked up once per device with that
 // device current (host code may not use the symbol itself as an address).
 constexpr int kMaxDevices = 64;
@@ -549,8 +696,12 @@ cudaError_t noalloc_scratch(uint32_t** out) {
 }  // namespace
 
 int bin_cells(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
-              GridBuffers& gb, cudaStream_t st) {
+              GridBuffers& gb, uint32_t* zero2, cudaStream_t st) {
     int launches = 0;
+    // a state that was scattered and then replaced never reached the ordering,
+    // which clears the counts
+    if (gb.scattered) cudaMemsetAsync(gb.count, 0, (size_t(T.ncells) + 2) * sizeof(uint32_t), st);
+    gb.scattered = false;
     if (n > 0) {
         // a single scene needs no material to find the scene: skip that read
         const bool one = T.nscenes == 1;
@@ -558,37 +709,58 @@ int bin_cells(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint
                                                                   T, cell_bins(gb));
         ++launches;
     }
-    return launches + scan_cells(T, gb, st);
+    return launches + scatter_cells(n, T, gb, zero2, st);
 }
 
-int scan_cells(const Tables& T, GridBuffers& gb, cudaStream_t st) {
-    // cells, the non-finite bucket, and the total
-    return exclusive_scan(gb.count, T.ncells + 2, gb.start, gb.block_sums, st);
-}
-
-int sort_cells(uint32_t n, const Tables& T, GridBuffers& gb, DevStats* stats, const uint32_t* boundary_start,
-               uint32_t* zero2, cudaStream_t st) {
-    int launches = 0;
-    if (n > 0) {
-        k_scatter<<<blocks_for(n, kThreads), kThreads, 0, st>>>(gb.key, gb.rank, n, gb.start, gb.perm, zero2);
-        ++launches;
+int scatter_cells(uint32_t n, const Tables& T, GridBuffers& gb, uint32_t* zero2, cudaStream_t st) {
+    const uint32_t len = T.ncells + 2;  // cells, the non-finite bucket, and the total
+    const uint32_t tiles = blocks_for(len, kScanTile);
+    if (tiles > kBaseTiles) {
+        // exclusive_scan clears the counts
+        const int l = exclusive_scan(gb.count, len, gb.start, gb.block_sums, st);
+        k_scatter_plain<<<std::max(blocks_for(n, kThreads), 1u), kThreads, 0, st>>>(gb.key, gb.rank, n, gb.start,
+                                                                                    gb.perm, zero2);
+        return l + 1;
     }
-    k_sort_runs<<<blocks_for(T.ncells + 1, kThreads), kThreads, 0, st>>>(gb.start, T.ncells, gb.perm, gb.rank,
-                                                                         boundary_start, stats, T);
-    return launches + 1;
+    gb.scattered = true;
+    k_scan_tiles<false><<<tiles, kScanThreads, 0, st>>>(gb.count, len, gb.count, gb.block_sums, true);
+    const uint32_t work = std::max(n, (len + 3u) / 4u);
+    k_scatter<<<blocks_for(work, kThreads), kThreads, 0, st>>>(gb.key, gb.rank, n, gb.count, gb.block_sums, len,
+                                                               gb.start, gb.perm, zero2);
+    return 2;
+}
+
+int order_cells(const Tables& T, GridBuffers& gb, cudaStream_t st) {
+    gb.scattered = false;
+    k_order<<<blocks_for(T.ncells + 2, kThreads), kThreads, 0, st>>>(gb.start, T.ncells, gb.perm, gb.rank, gb.key,
+                                                                     gb.count);
+    return 1;
+}
+
+int order_gather(const Tables& T, GridBuffers& gb, const uint32_t* boundary_start, const float4* pd_in, float4* pd_out,
+                 const float4* vm_in, float4* vm_out, const uint32_t* a_in, uint32_t* a_out, const uint32_t* b_in,
+                 uint32_t* b_out, cudaStream_t st, const SolidScatter& sol, DevStats* stats, const PairOut& out) {
+    gb.scattered = false;
+    const GatherArgs g{pd_in, vm_in, pd_out, vm_out, a_in, b_in, a_out, b_out, nullptr, sol, stats, out};
+    k_order_gather<<<blocks_for(T.ncells + 2, kThreads), kThreads, 0, st>>>(gb.start, T.ncells, gb.perm, gb.rank,
+                                                                            gb.key, gb.count, boundary_start,
+                                                                            stats, g, T);
+    return 1;
 }
 
 int build_grid(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
                GridBuffers& gb, cudaStream_t st) {
-    const int l = bin_cells(pos, vm, mat_u32, n, T, gb, st);
-    return l + sort_cells(n, T, gb, nullptr, nullptr, nullptr, st);
+    const int l = bin_cells(pos, vm, mat_u32, n, T, gb, nullptr, st);
+    return l + order_cells(T, gb, st);
 }
 
 uint32_t scan_block_sums_needed(uint32_t len) { return blocks_for(len, kScanTile) + 1; }
 
 int exclusive_scan(uint32_t* count, uint32_t len, uint32_t* out, uint32_t* block_sums, cudaStream_t st) {
     const uint32_t tiles = blocks_for(len, kScanTile);
-    k_scan_tiles<<<tiles, kScanThreads, 0, st>>>(count, len, out, block_sums);
+    const bool wide = ((reinterpret_cast<uintptr_t>(count) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0u;
+    if (count == out) k_scan_tiles<false><<<tiles, kScanThreads, 0, st>>>(count, len, out, block_sums, wide);
+    else k_scan_tiles<true><<<tiles, kScanThreads, 0, st>>>(count, len, out, block_sums, wide);
     k_scan_add<<<tiles, kScanThreads, 0, st>>>(out, len, block_sums);
     return 2;
 }
@@ -604,11 +776,10 @@ int gather_sorted(const uint32_t* perm, uint32_t n, const float4* a_in, float4* 
 
 int gather_state(const uint32_t* perm, uint32_t n, const float4* pd_in, float4* pd_out, const float4* vm_in,
                  float4* vm_out, const uint32_t* a_in, uint32_t* a_out, const uint32_t* b_in, uint32_t* b_out,
-                 const uint2* c_in, uint2* c_out, float* ps_out, const Tables& T, cudaStream_t st,
-                 const SolidScatter& sol, DevStats* stats, const PairOut& out) {
+                 float* ps_out, const Tables& T, cudaStream_t st, const PairOut& out) {
     if (n == 0) return 0;
-    k_gather_state<<<blocks_for(n, kThreads), kThreads, 0, st>>>(perm, n, pd_in, pd_out, vm_in, vm_out, a_in, a_out,
-                                                                 b_in, b_out, c_in, c_out, ps_out, T, sol, stats, out);
+    const GatherArgs g{pd_in, vm_in, pd_out, vm_out, a_in, b_in, a_out, b_out, ps_out, SolidScatter{}, nullptr, out};
+    k_gather_state<<<blocks_for(n, kThreads), kThreads, 0, st>>>(perm, n, g, T);
     return 1;
 }
 
@@ -690,8 +861,7 @@ extern "C" arp_status arp_grid_build_noalloc(const void* pos_den, uint32_t n, co
     if (n > 0) k_rank_noalloc<<<blocks_for(n, kThreads), kThreads, 0, st>>>(pos, n, g, cell_start, rank);
     exclusive_scan(cell_start, len, cell_start, tile_sums, st);  // in place: counts become starts
     if (n > 0) k_scatter_noalloc<<<blocks_for(n, kThreads), kThreads, 0, st>>>(pos, n, g, cell_start, rank, perm);
-    k_sort_runs<<<blocks_for(g.ncells + 1, kThreads), kThreads, 0, st>>>(cell_start, g.ncells, perm, rank, nullptr,
-                                                                         nullptr, Tables{});
+    if (n > 0) k_order_noalloc<<<blocks_for(g.ncells + 1, kThreads), kThreads, 0, st>>>(pos, g, cell_start, perm, rank);
     e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(ARP_ERR_CUDA, std::string("grid build launch: ") + cudaGetErrorString(e));
     return ARP_OK;

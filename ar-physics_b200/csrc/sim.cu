@@ -281,8 +281,9 @@ struct arp_sim {
     DevBuf<uint32_t> contact_bound;
     int fluid_variant = 0;
     uint32_t grid_cap = 0;
-    // gb.start, key, rank and coord hold the state Y counted into cells: the
-    // last stage of a Runge-Kutta step does that for the next step's grid.
+    // gb holds the state Y counted and scattered into cells (all but the order
+    // inside them): the last stage of a Runge-Kutta step does that for the next
+    // step's grid.
     // False whenever Y or the grid buffers have changed otherwise.
     bool binned = false;
     // solids
@@ -571,7 +572,7 @@ arp_status do_init(arp_sim* S) {
         }
         S->launches += build_grid(tmp_pd.p, tmp_vm.p, nullptr, nb, S->tables, S->gb, st);
         S->launches += gather_state(S->gb.perm, nb, tmp_pd.p, S->b_pd.p, tmp_vm.p, S->b_vm.p, tmp_o.p,
-                                    S->b_orig.p, nullptr, nullptr, nullptr, nullptr, S->bps.p, S->tables, st, SolidScatter{}, nullptr, S->pair_out(n));
+                                    S->b_orig.p, nullptr, nullptr, S->bps.p, S->tables, st, S->pair_out(n));
         CUDA_TRY(cudaMemcpyAsync(S->b_start.p, S->gb.start, (size_t(nc) + 2) * sizeof(uint32_t),
                                  cudaMemcpyDeviceToDevice, st));
         CUDA_TRY(cudaStreamSynchronize(st));
@@ -743,14 +744,13 @@ arp_status do_step(arp_sim* S, bool prime = false) {
     if (verlet && !prime) {
         S->launches += verlet_kick_drift(S->Y.pd.p, S->Y.vm.p, S->vforce.pd.p, S->vforce.vm.p, n, half, S->dt_sub,
                                          S->X.pd.p, S->X.vm.p, S->tables, bins, st);
-        S->launches += scan_cells(S->tables, S->gb, st);
+        S->launches += scatter_cells(n, S->tables, S->gb, zero2, st);
         src_pd = S->X.pd.p;
         src_vm = S->X.vm.p;
     } else if (!S->binned) {
-        S->launches += bin_cells(src_pd, src_vm, nullptr, n, S->tables, S->gb, st);
+        S->launches += bin_cells(src_pd, src_vm, nullptr, n, S->tables, S->gb, zero2, st);
     }
     S->binned = false;
-    S->launches += sort_cells(n, S->tables, S->gb, S->d_stats.p, bstart, zero2, st);
     // the stage-0 solid copies and the solid -> slot map come out of the same gather
     SolidScatter sol0;
     if (ns) {
@@ -761,9 +761,8 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         sol0.sc = S->sc.p;
         sol0.slot_of = S->slot_of.p;
     }
-    S->launches += gather_state(S->gb.perm, n, src_pd, S->T.pd.p, src_vm, S->T.vm.p, S->orig.p, S->orig_r.p,
-                                S->sid.p, S->sid_r.p, nullptr, nullptr, nullptr, S->tables, st, sol0, S->d_stats.p,
-                                S->pair_out(0));
+    S->launches += order_gather(S->tables, S->gb, bstart, src_pd, S->T.pd.p, src_vm, S->T.vm.p, S->orig.p,
+                                S->orig_r.p, S->sid.p, S->sid_r.p, st, sol0, S->d_stats.p, S->pair_out(0));
     std::swap(S->Y, S->T);
     std::swap(S->orig, S->orig_r);
     std::swap(S->sid, S->sid_r);
@@ -820,7 +819,6 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         if (s > 0) {
             if (S->profiling && s > 0) mark(S, mk, 0);
             l0 = S->launches;
-            S->launches += sort_cells(n, S->tables, S->gb, S->d_stats.p, bstart, zero2, st);
             SolidScatter sol;  // this stage's solid copies
             if (sb && ns) {
                 sol.sid_of_slot = S->sid.p;
@@ -829,9 +827,9 @@ arp_status do_step(arp_sim* S, bool prime = false) {
                 sol.sv = S->sv.p;
                 sol.sc = S->sc.p;
             }
-            S->launches += gather_state(S->gb.perm, n, cur_pd, nullptr, cur_vm, nullptr, sb ? S->sid.p : nullptr,
-                                        sb ? S->sid_sorted.p : nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                        S->tables, st, sol, S->d_stats.p, S->pair_out(0));
+            S->launches += order_gather(S->tables, S->gb, bstart, cur_pd, nullptr, cur_vm, nullptr,
+                                        sb ? S->sid.p : nullptr, sb ? S->sid_sorted.p : nullptr, nullptr, nullptr, st,
+                                        sol, S->d_stats.p, S->pair_out(0));
             nl += S->launches - l0;
         }
         const uint32_t* perm = s == 0 ? nullptr : S->gb.perm;
@@ -907,7 +905,7 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         const bool bin_next = !verlet && !prime;
         B.bin = bin_next ? bins : CellBins{};
         int fl = launch_fluid(f, S->tables, S->kdim, c, B, S->fluid_variant, st);
-        if (bin_next) fl += scan_cells(S->tables, S->gb, st);
+        if (bin_next) fl += scatter_cells(n, S->tables, S->gb, zero2, st);
         S->launches += fl;
         mark(S, mk, 3);
         if (S->profiling) {
@@ -1274,8 +1272,7 @@ arp_status run_autotune(arp_sim* S, bool force) {
     S->binned = false;
     S->launches += build_grid(S->Y.pd.p, S->Y.vm.p, nullptr, n, S->tables, S->gb, st);
     S->launches += gather_state(S->gb.perm, n, S->Y.pd.p, S->T.pd.p, S->Y.vm.p, S->T.vm.p, S->orig.p, S->orig_r.p,
-                                S->sid.p, S->sid_r.p, nullptr, nullptr, nullptr, S->tables, st, SolidScatter{},
-                                nullptr, S->pair_out(0));
+                                S->sid.p, S->sid_r.p, nullptr, S->tables, st, S->pair_out(0));
     std::swap(S->Y, S->T);
     std::swap(S->orig, S->orig_r);
     std::swap(S->sid, S->sid_r);
@@ -1613,7 +1610,8 @@ arp_status arp_sim_step(arp_sim* sim, uint32_t nsteps) {
         // likewise the graph replays only steps that find their state counted
         // into cells by the step before
         if (graphed && !sim->verlet() && !sim->binned) {
-            sim->launches += bin_cells(sim->Y.pd.p, sim->Y.vm.p, nullptr, sim->n, sim->tables, sim->gb, sim->stream);
+            sim->launches += bin_cells(sim->Y.pd.p, sim->Y.vm.p, nullptr, sim->n, sim->tables, sim->gb,
+                                       sim->solid_branch() ? sim->contact_bound.p : nullptr, sim->stream);
             sim->binned = true;
         }
         if (graphed) ARP_TRY(graph_step(sim));
