@@ -751,7 +751,7 @@ __global__ void __launch_bounds__(kT) k_adj_solid(AdjArgs a, Tables T) {
         const uint32_t e = a.rl.nbr[k];
         if (!(e & kSameMatBit)) continue;
         const uint32_t j = e & ~kSameMatBit;
-        const SolidPos pj = load_pos(a.st.sx, j);
+        const SolidPos pj = load_pos_at(a.st.sx, j);
         const float3 dX = sub(f3(pj.X), Xi);
         const float diff = P.h2 - ((dX.x * dX.x + dX.y * dX.y) + dX.z * dX.z);
         const float3 g = mul(-6.0f * P.kconst * diff * diff, dX);

@@ -27,6 +27,7 @@
 #include <algorithm>
 
 #include "grid.cuh"
+#include "launch.cuh"
 #include "warp.cuh"
 
 namespace arp {
@@ -81,9 +82,14 @@ struct Acc {
 struct PairRec {
     float4 x, v;
 };
-__device__ __forceinline__ PairRec load_rec(const float4* rec, uint32_t j) {
+__device__ __forceinline__ PairRec load_rec(const float4* rec, uint32_t k) {
     PairRec r;
-    load8(rec + 2 * (size_t)j, r.x, r.v);
+    load8(rec + 2 * (size_t)k, r.x, r.v);
+    return r;
+}
+__device__ __forceinline__ PairRec load_hit(const float4* rec, uint32_t j) {  // j read from a list or a table
+    PairRec r;
+    load8_at(rec + 2 * (size_t)j, r.x, r.v);
     return r;
 }
 
@@ -226,7 +232,7 @@ __device__ __forceinline__ void add_hit_contact(Acc& acc, uint32_t j, const Self
     const uint32_t mat2 = a.mat8[j];
     const PairMat m = s.pm[mat2];
     if ((m.bits & kPairPotential) == ARP_CONTACT_ZERO) return;
-    const PairRec rj = load_rec(a.rec, j);
+    const PairRec rj = load_hit(a.rec, j);
     const PairGeom g = pair_geom<DIM>(s, rj, K);
     if (!(g.r2 < K.h2)) return;
     const bool rubs = j >= a.n || (m.bits & (kPairElastic1 | kPairElastic2));
@@ -415,6 +421,7 @@ __global__ void __launch_bounds__(BLOCK, kBlocksPerSM * 128 / BLOCK) k_fluid(Flu
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint32_t* const lists = reinterpret_cast<uint32_t*>(smem_raw);
     PairMat* const sm = reinterpret_cast<PairMat*>(smem_raw + sizeof(uint32_t) * STRIDE * BLOCK);
+    step_begin();
     const uint32_t k0 = blockIdx.x * BLOCK;
     const uint32_t scene0 = T.mats[a.mat[k0]].scene;  // k0 < n: one block per started tile
     {
@@ -568,7 +575,7 @@ __global__ void __launch_bounds__(BLOCK, kBlocksPerSM * 128 / BLOCK) k_fluid(Flu
                 for (uint32_t e = q; e < n_ev; e += 2 * kPartials) {  // two hits' loads in flight
                     const bool two = e + kPartials < n_ev;
                     const uint32_t j0 = lists[list + e], j1 = two ? lists[list + e + kPartials] : ko;
-                    const PairRec r0 = load_rec(a.rec, j0), r1 = load_rec(a.rec, j1);
+                    const PairRec r0 = load_hit(a.rec, j0), r1 = load_hit(a.rec, j1);
                     const uint32_t m0 = a.mat8[j0], m1 = a.mat8[j1];
                     if (j0 != ko) add_hit<DIM>(part, j0, r0, m0, s, a, K, bits);
                     if (j1 != ko) add_hit<DIM>(part, j1, r1, m1, s, a, K, bits);
@@ -633,7 +640,9 @@ __global__ void __launch_bounds__(BLOCK, kBlocksPerSM * 128 / BLOCK) k_fluid(Flu
 // there are LANES times as many warps, which pays until the SMs are full: the
 // 16,899-particle 3D scene 22 us per launch with 8 lanes against 58 in the block
 // form, the 126,464-particle one 62 us in the block form against 86 with 4 lanes.
-// Bound: the latency of the chain of dependent loads of one particle.
+// Bound: the latency of the chain of dependent loads of one particle, and whether
+// all blocks are resident at once: 8 blocks per SM with 16 lanes (16.5 us for 9,072
+// particles, 18.9 with 7), 7 with 4 and 8 (35.5 us for 32,256, 37 with 8, 42 with 6).
 //   * The bounds of all search rows are read at once, one row per lane, and
 //     turned into a list of non-empty segments of consecutive candidates
 //     (boundary, then mobile, row by row: the candidate order of the block
@@ -648,7 +657,7 @@ constexpr int kGroupList = 96;   // list entries per particle
 constexpr int kGroupBlock = 128;
 
 template <int DIM, int LANES>
-__global__ void __launch_bounds__(kGroupBlock) k_fluid_group(FluidArgs a, Tables T, StageCoefs c, StageBuffers b) {
+__global__ void __launch_bounds__(kGroupBlock, LANES == 16 ? 8 : 7) k_fluid_group(FluidArgs a, Tables T, StageCoefs c, StageBuffers b) {
     constexpr int NG = kGroupBlock / LANES;       // particles per block
     constexpr int U = LANES >= 16 ? 2 : 4;        // candidate loads in flight per lane
     constexpr int RZ = 1 + (int)(kSearchHalve >> 2 & 1u);
@@ -661,6 +670,7 @@ __global__ void __launch_bounds__(kGroupBlock) k_fluid_group(FluidArgs a, Tables
     __shared__ float4 s_term[LANES > 4 ? NG : 1][LANES];
     constexpr unsigned FULL = 0xFFFFFFFFu;
     constexpr unsigned GM = (1u << LANES) - 1u;
+    step_begin();
     const uint32_t lane = threadIdx.x % LANES, gi = threadIdx.x / LANES;
     const uint32_t gshift = (threadIdx.x & 31u) & ~(uint32_t)(LANES - 1);
     const uint32_t kk = blockIdx.x * NG + gi;
@@ -772,7 +782,7 @@ __global__ void __launch_bounds__(kGroupBlock) k_fluid_group(FluidArgs a, Tables
             t.f = make_float3(0.f, 0.f, 0.f);
             if (e0 + lane < ev) {
                 const uint32_t j = list[e0 + lane];
-                if (j != k) add_hit<DIM>(t, j, load_rec(a.rec, j), a.mat8[j], s, a, K, bits);
+                if (j != k) add_hit<DIM>(t, j, load_hit(a.rec, j), a.mat8[j], s, a, K, bits);
             }
             add(acc, make_float4(t.den, t.f.x, t.f.y, t.f.z));
         }
@@ -816,10 +826,11 @@ __global__ void __launch_bounds__(kGroupBlock) k_fluid_group(FluidArgs a, Tables
 // (its position part is not used).  Each sum is formed as y + (0 + c k), the
 // order of the stage epilogue.  The drifted state is counted into its search
 // cells on the way.
-__global__ void k_verlet_kick_drift(const float4* __restrict__ pd, const float4* __restrict__ vm,
-                                    const float4* __restrict__ fpd, const float4* __restrict__ fvm, uint32_t n,
-                                    float half, float full, float4* __restrict__ out_pd, float4* __restrict__ out_vm,
+__global__ void k_verlet_kick_drift(const float4* pd, const float4* vm,
+                                    const float4* fpd, const float4* fvm, uint32_t n,
+                                    float half, float full, float4* out_pd, float4* out_vm,
                                     Tables T, CellBins bin) {
+    step_begin();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const float4 p = pd[k], v = vm[k], fp = fpd[k], fv = fvm[k];
@@ -834,8 +845,9 @@ __global__ void k_verlet_kick_drift(const float4* __restrict__ pd, const float4*
 }
 
 // The kick of the plastic strain (4 float4 per solid): e' = e + (0 + c k).
-__global__ void k_verlet_kick4(const float4* __restrict__ e, const float4* __restrict__ k4, uint32_t count, float half,
-                               float4* __restrict__ out) {
+__global__ void k_verlet_kick4(const float4* e, const float4* k4, uint32_t count, float half,
+                               float4* out) {
+    step_begin();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     out[i] = comb(e[i], axpy(half, k4[i], make_float4(0.f, 0.f, 0.f, 0.f)), false);
@@ -847,13 +859,13 @@ int verlet_kick_drift(const float4* pd, const float4* vm, const float4* fpd, con
                       float full, float4* out_pd, float4* out_vm, const Tables& T, const CellBins& bin,
                       cudaStream_t st) {
     if (n == 0) return 0;
-    k_verlet_kick_drift<<<(n + 255) / 256, 256, 0, st>>>(pd, vm, fpd, fvm, n, half, full, out_pd, out_vm, T, bin);
+    launch_step(k_verlet_kick_drift, (n + 255) / 256, 256, 0, st, pd, vm, fpd, fvm, n, half, full, out_pd, out_vm, T, bin);
     return 1;
 }
 
 int verlet_kick4(const float4* e, const float4* k4, uint32_t count, float half, float4* out, cudaStream_t st) {
     if (count == 0) return 0;
-    k_verlet_kick4<<<(count + 255) / 256, 256, 0, st>>>(e, k4, count, half, out);
+    launch_step(k_verlet_kick4, (count + 255) / 256, 256, 0, st, e, k4, count, half, out);
     return 1;
 }
 
@@ -870,7 +882,7 @@ int launch_fluid(const FluidArgs& a, const Tables& T, int kdim, const StageCoefs
     if (v.lanes) {
         const uint32_t nb = (a.n + (uint32_t)(kGroupBlock / v.lanes) - 1u) / (uint32_t)(kGroupBlock / v.lanes);
 #define ARP_GROUP(D, L) \
-    if (kdim == D && v.lanes == L) k_fluid_group<D, L><<<nb, kGroupBlock, 0, st>>>(a, T, c, b);
+    if (kdim == D && v.lanes == L) launch_step(k_fluid_group<D, L>, nb, kGroupBlock, 0, st, a, T, c, b);
         ARP_GROUP(3, 4) ARP_GROUP(3, 8) ARP_GROUP(3, 16)
         ARP_GROUP(2, 4) ARP_GROUP(2, 8) ARP_GROUP(2, 16)
 #undef ARP_GROUP
@@ -882,7 +894,7 @@ int launch_fluid(const FluidArgs& a, const Tables& T, int kdim, const StageCoefs
     if (kdim == D && v.block == B && v.cap == C) {                                                                 \
         if (smem > 48 * 1024)                                                                                      \
             cudaFuncSetAttribute(k_fluid<D, B, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);        \
-        k_fluid<D, B, C><<<nb, B, smem, st>>>(a, T, c, b);                                                         \
+        launch_step(k_fluid<D, B, C>, nb, B, smem, st, a, T, c, b);                                                \
     }
 #define ARP_FLUID_CAPS(D, B) \
     ARP_FLUID(D, B, 40) ARP_FLUID(D, B, 44) ARP_FLUID(D, B, 48) ARP_FLUID(D, B, 56) \

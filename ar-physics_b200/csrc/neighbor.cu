@@ -26,6 +26,7 @@
 #include <string>
 
 #include "grid.cuh"
+#include "launch.cuh"
 
 namespace arp {
 
@@ -41,8 +42,9 @@ __device__ __forceinline__ uint32_t scene_of(const float4* vm, const uint32_t* m
     return T.mats[m].scene;
 }
 
-__global__ void k_cell_keys(const float4* __restrict__ pos, const float4* __restrict__ vm,
-                            const uint32_t* __restrict__ mat_u32, uint32_t n, Tables T, CellBins bin) {
+__global__ void k_cell_keys(const float4* pos, const float4* vm,
+                            const uint32_t* mat_u32, uint32_t n, Tables T, CellBins bin) {
+    step_begin();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     bin_particle(pos[i], T.scenes[scene_of(vm, mat_u32, i, T)], T.ncells, i, bin);
@@ -83,8 +85,9 @@ __device__ __forceinline__ void block_excl_scan(uint32_t v, uint32_t& excl) {
 // allocation-free build scans a caller's array, which need not be).
 template <bool CLEAR>
 __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t* count, uint32_t len, uint32_t* out,
-                                                             uint32_t* __restrict__ block_sums, bool wide) {
+                                                             uint32_t* block_sums, bool wide) {
     __shared__ uint32_t last_total;
+    step_begin();
     const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     uint32_t v[kScanItems] = {0u, 0u, 0u, 0u};
     static_assert(kScanItems == 4, "one 16-byte load per thread");
@@ -121,9 +124,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t* count, ui
 // Adds to each tile of the scan the sum of the totals of the tiles before it;
 // each block (one tile of kScanTile items) sums those totals itself, a block
 // reduction over at most a few hundred values, so no separate pass scans them.
-__global__ void k_scan_add(uint32_t* out, uint32_t len, const uint32_t* __restrict__ sums) {
+__global__ void k_scan_add(uint32_t* out, uint32_t len, const uint32_t* sums) {
     __shared__ uint32_t warp_part[kScanThreads / 32];
     __shared__ uint32_t prefix;
+    step_begin();
     uint32_t part = 0;
     for (uint32_t t = threadIdx.x; t < blockIdx.x; t += blockDim.x) part += sums[t];
 #pragma unroll
@@ -150,13 +154,14 @@ __global__ void k_scan_add(uint32_t* out, uint32_t len, const uint32_t* __restri
 // place) and the tile totals, which every block sums up itself: at most
 // kBaseTiles of them (4 M cells), so no pass of its own finishes the scan.
 constexpr uint32_t kBaseTiles = 1024;
-__global__ void __launch_bounds__(kThreads) k_scatter(const uint32_t* __restrict__ key,
-                                                      const uint32_t* __restrict__ rank, uint32_t n,
-                                                      const uint32_t* __restrict__ local,
-                                                      const uint32_t* __restrict__ sums, uint32_t len,
-                                                      uint32_t* __restrict__ start, uint32_t* __restrict__ perm,
-                                                      uint32_t* __restrict__ zero2) {
+__global__ void __launch_bounds__(kThreads) k_scatter(const uint32_t* key,
+                                                      const uint32_t* rank, uint32_t n,
+                                                      const uint32_t* local,
+                                                      const uint32_t* sums, uint32_t len,
+                                                      uint32_t* start, uint32_t* perm,
+                                                      uint32_t* zero2) {
     __shared__ uint32_t tile_base[kBaseTiles];
+    step_begin();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (zero2 && i < 2u) zero2[i] = 0u;
     // loads that do not need the bases first
@@ -191,9 +196,10 @@ __global__ void __launch_bounds__(kThreads) k_scatter(const uint32_t* __restrict
     }
 }
 // The same scatter from finished cell starts (grids of more tiles).
-__global__ void k_scatter_plain(const uint32_t* __restrict__ key, const uint32_t* __restrict__ rank, uint32_t n,
-                                const uint32_t* __restrict__ start, uint32_t* __restrict__ perm,
-                                uint32_t* __restrict__ zero2) {
+__global__ void k_scatter_plain(const uint32_t* key, const uint32_t* rank, uint32_t n,
+                                const uint32_t* start, uint32_t* perm,
+                                uint32_t* zero2) {
+    step_begin();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (zero2 && i < 2u) zero2[i] = 0u;
     if (i < n) perm[start[key[i]] + rank[i]] = i;
@@ -202,8 +208,8 @@ __global__ void k_scatter_plain(const uint32_t* __restrict__ key, const uint32_t
 // Occupancy (mobile + boundary) of the reference cell whose first search
 // cell is global cell c, or 0 when c is not the first search cell of its
 // reference cell.
-__device__ __forceinline__ uint32_t reference_cell_occupancy(uint32_t c, const uint32_t* __restrict__ start,
-                                                             const uint32_t* __restrict__ bstart, const Tables& T) {
+__device__ __forceinline__ uint32_t reference_cell_occupancy(uint32_t c, const uint32_t* start, const uint32_t* bstart,
+                                                             const Tables& T) {
     uint32_t lo = 0, hi = T.nscenes;  // scene with the largest cell_base <= c
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
@@ -440,9 +446,10 @@ __device__ __forceinline__ void order_block(const uint32_t* start, uint32_t ncel
     for (uint32_t t = threadIdx.x; t < m; t += kThreads) f(p0 + t, perm[p0 + t]);
 }
 
-__global__ void __launch_bounds__(kThreads) k_order(const uint32_t* __restrict__ start, uint32_t ncells, uint32_t* perm,
-                                                    uint32_t* tmp, const uint32_t* __restrict__ key,
-                                                    uint32_t* __restrict__ count) {
+__global__ void __launch_bounds__(kThreads) k_order(const uint32_t* start, uint32_t ncells, uint32_t* perm,
+                                                    uint32_t* tmp, const uint32_t* key,
+                                                    uint32_t* count) {
+    step_begin();
     const uint32_t c = blockIdx.x * kThreads + threadIdx.x;
     if (count && c < ncells + 2u) count[c] = 0u;  // ready for the next histogram
     order_block(start, ncells, perm, tmp, [&](uint32_t v) { return key[v]; },
@@ -538,12 +545,13 @@ __global__ void k_gather_state(const uint32_t* __restrict__ perm, uint32_t n, Ga
 
 // Orders the block's cells and gathers the state of their particles.  Also,
 // with `stats`, the occupancy counters of the reference cells.
-__global__ void __launch_bounds__(kThreads) k_order_gather(const uint32_t* __restrict__ start, uint32_t ncells,
+__global__ void __launch_bounds__(kThreads) k_order_gather(const uint32_t* start, uint32_t ncells,
                                                            uint32_t* perm, uint32_t* tmp,
-                                                           const uint32_t* __restrict__ key,
-                                                           uint32_t* __restrict__ count,
-                                                           const uint32_t* __restrict__ boundary_start, DevStats* stats,
+                                                           const uint32_t* key,
+                                                           uint32_t* count,
+                                                           const uint32_t* boundary_start, DevStats* stats,
                                                            GatherArgs g, Tables T) {
+    step_begin();
     const uint32_t c = blockIdx.x * kThreads + threadIdx.x;
     if (c < ncells + 2u) count[c] = 0u;  // ready for the next histogram
     if (stats) {
@@ -641,8 +649,9 @@ constexpr uint32_t kNoAllocMaxCells = (1u << 22) - 2;  // cell_start then holds 
 constexpr uint32_t kNoAllocMaxTiles = (kNoAllocMaxCells + 2 + kScanTile - 1) / kScanTile;
 __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocMaxParticles + kNoAllocMaxTiles];
 
-__global__ void k_rank_noalloc(const float4* __restrict__ pos, uint32_t n, Grid grid, uint32_t* __restrict__ count,
-                               uint32_t* __restrict__ rank) {
+__global__ void k_rank_noalloc(const float4* pos, uint32_t n, Grid grid, uint32_t* count,
+                               uint32_t* rank) {
+    step_begin();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = pos[i];
@@ -650,9 +659,10 @@ __global__ void k_rank_noalloc(const float4* __restrict__ pos, uint32_t n, Grid 
     rank[i] = atomicAdd(&count[k], 1u);
 }
 
-__global__ void k_scatter_noalloc(const float4* __restrict__ pos, uint32_t n, Grid grid,
-                                  const uint32_t* __restrict__ start, const uint32_t* __restrict__ rank,
-                                  uint32_t* __restrict__ perm) {
+__global__ void k_scatter_noalloc(const float4* pos, uint32_t n, Grid grid,
+                                  const uint32_t* start, const uint32_t* rank,
+                                  uint32_t* perm) {
+    step_begin();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = pos[i];
@@ -660,9 +670,10 @@ __global__ void k_scatter_noalloc(const float4* __restrict__ pos, uint32_t n, Gr
     perm[start[k] + rank[i]] = i;
 }
 
-__global__ void __launch_bounds__(kThreads) k_order_noalloc(const float4* __restrict__ pos, Grid grid,
-                                                            const uint32_t* __restrict__ start, uint32_t* perm,
+__global__ void __launch_bounds__(kThreads) k_order_noalloc(const float4* pos, Grid grid,
+                                                            const uint32_t* start, uint32_t* perm,
                                                             uint32_t* tmp) {
+    step_begin();
     order_block(start, grid.ncells, perm, tmp,
                 [&](uint32_t v) {
                     const float4 p = pos[v];
@@ -705,7 +716,7 @@ int bin_cells(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint
     if (n > 0) {
         // a single scene needs no material to find the scene: skip that read
         const bool one = T.nscenes == 1;
-        k_cell_keys<<<blocks_for(n, kThreads), kThreads, 0, st>>>(pos, one ? nullptr : vm, one ? nullptr : mat_u32, n,
+        launch_step(k_cell_keys, blocks_for(n, kThreads), kThreads, 0, st, pos, one ? nullptr : vm, one ? nullptr : mat_u32, n,
                                                                   T, cell_bins(gb));
         ++launches;
     }
@@ -718,21 +729,21 @@ int scatter_cells(uint32_t n, const Tables& T, GridBuffers& gb, uint32_t* zero2,
     if (tiles > kBaseTiles) {
         // exclusive_scan clears the counts
         const int l = exclusive_scan(gb.count, len, gb.start, gb.block_sums, st);
-        k_scatter_plain<<<std::max(blocks_for(n, kThreads), 1u), kThreads, 0, st>>>(gb.key, gb.rank, n, gb.start,
+        launch_step(k_scatter_plain, std::max(blocks_for(n, kThreads), 1u), kThreads, 0, st, gb.key, gb.rank, n, gb.start,
                                                                                     gb.perm, zero2);
         return l + 1;
     }
     gb.scattered = true;
-    k_scan_tiles<false><<<tiles, kScanThreads, 0, st>>>(gb.count, len, gb.count, gb.block_sums, true);
+    launch_step(k_scan_tiles<false>, tiles, kScanThreads, 0, st, gb.count, len, gb.count, gb.block_sums, true);
     const uint32_t work = std::max(n, (len + 3u) / 4u);
-    k_scatter<<<blocks_for(work, kThreads), kThreads, 0, st>>>(gb.key, gb.rank, n, gb.count, gb.block_sums, len,
+    launch_step(k_scatter, blocks_for(work, kThreads), kThreads, 0, st, gb.key, gb.rank, n, gb.count, gb.block_sums, len,
                                                                gb.start, gb.perm, zero2);
     return 2;
 }
 
 int order_cells(const Tables& T, GridBuffers& gb, cudaStream_t st) {
     gb.scattered = false;
-    k_order<<<blocks_for(T.ncells + 2, kThreads), kThreads, 0, st>>>(gb.start, T.ncells, gb.perm, gb.rank, gb.key,
+    launch_step(k_order, blocks_for(T.ncells + 2, kThreads), kThreads, 0, st, gb.start, T.ncells, gb.perm, gb.rank, gb.key,
                                                                      gb.count);
     return 1;
 }
@@ -742,7 +753,7 @@ int order_gather(const Tables& T, GridBuffers& gb, const uint32_t* boundary_star
                  uint32_t* b_out, cudaStream_t st, const SolidScatter& sol, DevStats* stats, const PairOut& out) {
     gb.scattered = false;
     const GatherArgs g{pd_in, vm_in, pd_out, vm_out, a_in, b_in, a_out, b_out, nullptr, sol, stats, out};
-    k_order_gather<<<blocks_for(T.ncells + 2, kThreads), kThreads, 0, st>>>(gb.start, T.ncells, gb.perm, gb.rank,
+    launch_step(k_order_gather, blocks_for(T.ncells + 2, kThreads), kThreads, 0, st, gb.start, T.ncells, gb.perm, gb.rank,
                                                                             gb.key, gb.count, boundary_start,
                                                                             stats, g, T);
     return 1;
@@ -759,9 +770,9 @@ uint32_t scan_block_sums_needed(uint32_t len) { return blocks_for(len, kScanTile
 int exclusive_scan(uint32_t* count, uint32_t len, uint32_t* out, uint32_t* block_sums, cudaStream_t st) {
     const uint32_t tiles = blocks_for(len, kScanTile);
     const bool wide = ((reinterpret_cast<uintptr_t>(count) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0u;
-    if (count == out) k_scan_tiles<false><<<tiles, kScanThreads, 0, st>>>(count, len, out, block_sums, wide);
-    else k_scan_tiles<true><<<tiles, kScanThreads, 0, st>>>(count, len, out, block_sums, wide);
-    k_scan_add<<<tiles, kScanThreads, 0, st>>>(out, len, block_sums);
+    if (count == out) launch_step(k_scan_tiles<false>, tiles, kScanThreads, 0, st, count, len, out, block_sums, wide);
+    else launch_step(k_scan_tiles<true>, tiles, kScanThreads, 0, st, count, len, out, block_sums, wide);
+    launch_step(k_scan_add, tiles, kScanThreads, 0, st, out, len, block_sums);
     return 2;
 }
 
@@ -858,10 +869,10 @@ extern "C" arp_status arp_grid_build_noalloc(const void* pos_den, uint32_t n, co
     e = cudaMemsetAsync(cell_start, 0, (size_t)len * sizeof(uint32_t), st);
     if (e != cudaSuccess) return set_error(ARP_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
     const float4* pos = static_cast<const float4*>(pos_den);
-    if (n > 0) k_rank_noalloc<<<blocks_for(n, kThreads), kThreads, 0, st>>>(pos, n, g, cell_start, rank);
+    if (n > 0) launch_step(k_rank_noalloc, blocks_for(n, kThreads), kThreads, 0, st, pos, n, g, cell_start, rank);
     exclusive_scan(cell_start, len, cell_start, tile_sums, st);  // in place: counts become starts
-    if (n > 0) k_scatter_noalloc<<<blocks_for(n, kThreads), kThreads, 0, st>>>(pos, n, g, cell_start, rank, perm);
-    if (n > 0) k_order_noalloc<<<blocks_for(g.ncells + 1, kThreads), kThreads, 0, st>>>(pos, g, cell_start, perm, rank);
+    if (n > 0) launch_step(k_scatter_noalloc, blocks_for(n, kThreads), kThreads, 0, st, pos, n, g, cell_start, rank, perm);
+    if (n > 0) launch_step(k_order_noalloc, blocks_for(g.ncells + 1, kThreads), kThreads, 0, st, pos, g, cell_start, perm, rank);
     e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(ARP_ERR_CUDA, std::string("grid build launch: ") + cudaGetErrorString(e));
     return ARP_OK;

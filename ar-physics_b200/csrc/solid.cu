@@ -19,6 +19,7 @@
 //     gradW over the list, then hourglass control and self-contact over the
 //     current 3x3x3 cells (k_solid_forces).  A_j is read, not recomputed.
 #include "grid.cuh"
+#include "launch.cuh"
 #include "mat4.cuh"
 #include "solid_rec.cuh"
 
@@ -279,6 +280,7 @@ __device__ __forceinline__ T3 stress_order2(const T3& F, const T3& Fd, float lam
 // for few solids the one thread that runs the stress chain.
 template <bool ORDER2, bool PLASTIC, int LANES>
 __global__ void __launch_bounds__(kThreads) k_solid_stress(SolidArgs a, Tables T, StageCoefs c) {
+    step_begin();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = t / LANES, lane = t % LANES;
     if (i >= a.ns) return;  // whole groups leave together
@@ -317,14 +319,14 @@ __global__ void __launch_bounds__(kThreads) k_solid_stress(SolidArgs a, Tables T
     };
     for (; k + LANES < k1; k += 2 * LANES) {
         const uint32_t j0 = a.rl.nbr[k] & ~kSameMat, j1 = a.rl.nbr[k + LANES] & ~kSameMat;
-        const SolidPos p0 = load_pos(a.sx, j0), p1 = load_pos(a.sx, j1);
+        const SolidPos p0 = load_pos_at(a.sx, j0), p1 = load_pos_at(a.sx, j1);
         const float4 v0 = a.sv[j0], v1 = a.sv[j1];
         add(0, p0, v0);
         add(SETS - 1, p1, v1);
     }
     if (k < k1) {
         const uint32_t j = a.rl.nbr[k] & ~kSameMat;
-        add(0, load_pos(a.sx, j), a.sv[j]);
+        add(0, load_pos_at(a.sx, j), a.sv[j]);
     }
 #pragma unroll
     for (int cc = 0; cc < 3; ++cc)
@@ -491,6 +493,7 @@ __global__ void __launch_bounds__(kThreads) k_solid_stress(SolidArgs a, Tables T
 // kernels took 92 us per stage of 129,024 solids and 36 us for 1,274.
 template <int LANES>
 __global__ void __launch_bounds__(kThreads) k_solid_forces(SolidArgs a, Tables T) {
+    step_begin();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = t / LANES, lane = t % LANES;
     if (i >= a.ns) return;  // whole groups leave together
@@ -553,14 +556,14 @@ __global__ void __launch_bounds__(kThreads) k_solid_forces(SolidArgs a, Tables T
     };
     for (; k + LANES < k1; k += 2 * LANES) {
         const uint32_t e0 = a.rl.nbr[k], e1 = a.rl.nbr[k + LANES];
-        const SolidPos p0 = load_pos(a.sx, e0 & ~kSameMat), p1 = load_pos(a.sx, e1 & ~kSameMat);
-        const StressRec s0 = load_stress(a.AF, e0 & ~kSameMat), s1 = load_stress(a.AF, e1 & ~kSameMat);
+        const SolidPos p0 = load_pos_at(a.sx, e0 & ~kSameMat), p1 = load_pos_at(a.sx, e1 & ~kSameMat);
+        const StressRec s0 = load_stress<true>(a.AF, e0 & ~kSameMat), s1 = load_stress<true>(a.AF, e1 & ~kSameMat);
         if (e0 & kSameMat) add(0, p0, s0);
         if (e1 & kSameMat) add(SETS - 1, p1, s1);
     }
     if (k < k1) {
         const uint32_t e = a.rl.nbr[k], j = e & ~kSameMat;
-        if (e & kSameMat) add(0, load_pos(a.sx, j), load_stress(a.AF, j));
+        if (e & kSameMat) add(0, load_pos_at(a.sx, j), load_stress<true>(a.AF, j));
     }
     float fx = sum4<LANES>(fs[0]), fy = sum4<LANES>(fs[1]), fz = sum4<LANES>(fs[2]);
     if (lane != 0) return;
@@ -614,11 +617,11 @@ namespace {
 template <int L>
 void launch_solid_lanes(const SolidArgs& a, const Tables& T, const StageCoefs& c, cudaStream_t st) {
     const uint32_t blocks = blocks_for(a.ns * L, kThreads);
-    if (a.all_order2 && !a.any_plastic) k_solid_stress<true, false, L><<<blocks, kThreads, 0, st>>>(a, T, c);
-    else if (a.all_order2) k_solid_stress<true, true, L><<<blocks, kThreads, 0, st>>>(a, T, c);
-    else if (!a.any_plastic) k_solid_stress<false, false, L><<<blocks, kThreads, 0, st>>>(a, T, c);
-    else k_solid_stress<false, true, L><<<blocks, kThreads, 0, st>>>(a, T, c);
-    k_solid_forces<L><<<blocks, kThreads, 0, st>>>(a, T);
+    if (a.all_order2 && !a.any_plastic) launch_step(k_solid_stress<true, false, L>, blocks, kThreads, 0, st, a, T, c);
+    else if (a.all_order2) launch_step(k_solid_stress<true, true, L>, blocks, kThreads, 0, st, a, T, c);
+    else if (!a.any_plastic) launch_step(k_solid_stress<false, false, L>, blocks, kThreads, 0, st, a, T, c);
+    else launch_step(k_solid_stress<false, true, L>, blocks, kThreads, 0, st, a, T, c);
+    launch_step(k_solid_forces<L>, blocks, kThreads, 0, st, a, T);
 }
 }  // namespace
 

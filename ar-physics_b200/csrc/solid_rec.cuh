@@ -18,6 +18,11 @@ __device__ __forceinline__ SolidPos load_pos(const float4* sx, uint32_t i) {
     load8(sx + 2 * (size_t)i, r.x, r.X);
     return r;
 }
+__device__ __forceinline__ SolidPos load_pos_at(const float4* sx, uint32_t j) {  // j read from a reference list
+    SolidPos r;
+    load8_at(sx + 2 * (size_t)j, r.x, r.X);
+    return r;
+}
 
 // Stress record, 6 float4 (SolidArgs::AF): the 3 x 3 matrices A = sigma L and F
 // by columns, then the packed cell coordinates (18 floats + 2 words, 96 bytes).
@@ -26,11 +31,17 @@ struct StressRec {
     float A[3][3], F[3][3];  // [column][row]
     uint2 cell;
 };
+template <bool AT = false>  // AT: i was read from a reference list
 __device__ __forceinline__ StressRec load_stress(const float4* AF, uint32_t i) {
     const float4* const p = AF + kStressRec * (size_t)i;
     float4 a, b, c, d;
-    load8(p, a, b);
-    load8(p + 2, c, d);
+    if (AT) {
+        load8_at(p, a, b);
+        load8_at(p + 2, c, d);
+    } else {
+        load8(p, a, b);
+        load8(p + 2, c, d);
+    }
     const float4 e = p[4];
     StressRec r;
     r.A[0][0] = a.x; r.A[0][1] = a.y; r.A[0][2] = a.z;

@@ -5,9 +5,16 @@
 
 namespace arp {
 
-// One 32-byte sector in one load (p 32-byte aligned, read-only in the kernel).
+// One 32-byte sector in one load (p 32-byte aligned).  load8 is volatile and so
+// stays behind the wait of step_begin(); load8_at may be moved and is for
+// addresses that depend on memory read after that wait.
 __device__ __forceinline__ void load8(const float4* p, float4& a, float4& b) {
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p));
+}
+__device__ __forceinline__ void load8_at(const float4* p, float4& a, float4& b) {
+    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
         : "l"(p));
 }
