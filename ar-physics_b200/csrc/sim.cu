@@ -315,7 +315,10 @@ struct arp_sim {
     // solid-id buffers (and the plastic strain's when it changes), so the
     // steps alternate between two sets of buffer pointers; a graph is kept
     // for each set, keyed by its pointers, and replayed with the step's
-    // host-side effects applied by hand.
+    // host-side effects applied by hand.  A force evaluation of its own
+    // (velocity Verlet after a new state) swaps the state's buffers once
+    // more, so a program that keeps setting states meets up to eight sets;
+    // capturing one anew takes 200 us.
     struct StepGraph {
         cudaGraph_t g = nullptr;
         cudaGraphExec_t exec = nullptr;
@@ -323,7 +326,9 @@ struct arp_sim {
         uint64_t launches = 0;  // kernels per replay
     };
     bool use_graph = false;
-    StepGraph graphs[2];
+    static constexpr int kStepGraphs = 8;
+    StepGraph graphs[kStepGraphs];
+    int next_graph = 0;  // slot to reuse when none is free
     cudaStream_t graph_stream = nullptr;
     void drop_graph() {
         for (auto& x : graphs) {
@@ -1238,6 +1243,10 @@ arp_status allocate(arp_sim* S) {
 // state.  All variants evaluate the same pairs in the same order, so the
 // choice changes speed, never results.  Choices are cached per (kernel
 // dimension, log2 particle count, quarter-octave of h / particle spacing).
+// Sizes at which a form cannot win are left out: the group form above
+// kGroupMost particles (126,464 in 3D: 86 us against 62; 1.05 M: 600 against
+// 290), the block form below kBlockLeast (9,072 in 3D: 58 us against 14).
+constexpr uint32_t kGroupMost = 131072, kBlockLeast = 12288;
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int>, int> g_tune_cache;
 
@@ -1308,6 +1317,8 @@ arp_status run_autotune(arp_sim* S, bool force) {
     float best = 1e30f;
     int best_v = 0;
     for (int v = 0; v < kNumFluidVariants; ++v) {
+        const FluidVariant& fv = kFluidVariants[v];
+        if (fv.lanes ? n > kGroupMost : n < kBlockLeast) continue;
         S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, st);  // warm-up
         CUDA_TRY(cudaEventRecord(e0, st));
         for (int r = 0; r < 3; ++r) S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, st);
@@ -1576,13 +1587,17 @@ arp_status graph_step(arp_sim* S) {
     const void* sig[4];
     step_signature(S, sig);
     int k = -1, free_slot = -1;
-    for (int q = 0; q < 2; ++q) {
+    for (int q = 0; q < arp_sim::kStepGraphs; ++q) {
         const auto& G = S->graphs[q];
         if (G.exec && std::equal(sig, sig + 4, G.sig)) k = q;
         if (!G.exec && free_slot < 0) free_slot = q;
     }
     if (k < 0) {  // capture; do_step's host side happens during the capture
-        k = free_slot >= 0 ? free_slot : 0;
+        k = free_slot;
+        if (k < 0) {
+            k = S->next_graph;
+            S->next_graph = (k + 1) % arp_sim::kStepGraphs;
+        }
         const float t = S->time;
         ARP_TRY(capture_step_graph(S, k));
         S->time = t;

@@ -272,10 +272,11 @@ arp_status arp_sim_update(arp_sim* sim);
  * the un-vendored crate numerical-integration is not observable, so this is
  * a stated assumption, like the Runge-Kutta tableaus. */
 arp_status arp_sim_step(arp_sim* sim, uint32_t nsteps);
-/* Time every launch shape of the fluid kernel (the block form: one thread per
- * particle lists its neighbors, four evaluate them; 128 or 256 threads per
- * block, lists of 40 to 96; and the group form: 4, 8 or 16 threads per particle
- * throughout, for scenes too small to fill the GPU otherwise) on the current
+/* Time the launch shapes of the fluid kernel that suit the particle count (the
+ * block form: one thread per particle lists its neighbors, four evaluate them;
+ * 128 or 256 threads per block, lists of 40 to 96; and the group form: 4, 8 or
+ * 16 threads per particle throughout, for scenes too small to fill the GPU
+ * otherwise) on the current
  * state and keep the fastest; arp_sim_init does this once per (dimension,
  * particle count, h/spacing) bucket and reuses the choice afterwards.  The
  * shapes evaluate identical arithmetic, so results do not depend on it. */
@@ -287,11 +288,11 @@ arp_status arp_sim_fluid_variant(const arp_sim* sim, int* variant, int* block, i
 arp_status arp_sim_set_fluid_variant(arp_sim* sim, int variant);
 /* The number of launch shapes of the fluid kernel. */
 int arp_fluid_variant_count(void);
-/* Replay each step from a CUDA graph captured on the handle's stream (two
- * graphs, one for each of the two buffer sets consecutive steps alternate
- * between; captured on first use and again after the stream or the buffers
- * change).  Steps sampled by arp_sim_profile_enable and steps on a tape run
- * as plain launches.  Off by default. */
+/* Replay each step from a CUDA graph captured on the handle's stream (one
+ * graph for each set of buffers that steps alternate between; captured on first
+ * use and again after the stream or the buffers change).  Steps sampled by
+ * arp_sim_profile_enable and steps on a tape run as plain launches.  Off by
+ * default. */
 arp_status arp_sim_set_graph(arp_sim* sim, int enable);
 
 /* ---- queries (FluidSim accessors, src/soft_body/mod.rs:168-178) ------------ */
