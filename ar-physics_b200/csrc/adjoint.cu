@@ -9,6 +9,8 @@
 //                   (strain.rs:139-160, solid.rs:147-204,334-341), plus the
 //                   gradient of the per-solid (normal, shear) stiffness;
 //   * k_adj_strain  F and dF/dt as sums over the reference neighbors;
+//   * k_adj_prep    the weights mu of the stage (from the later stages' adjoints)
+//                   and the records the other kernels read of each particle;
 //   * k_adj_fluid   every fluid pair term (continuity, pressure with the
 //                   state equation, contact potential, viscosity, artificial
 //                   viscosity, friction; fluid.rs:154-247) and dx/dt = v.
@@ -18,7 +20,8 @@
 // and of its neighbors' pairs (pairwise-symmetric gathers): no atomics, each
 // thread writes only its own particle.  Not differentiated: self-contact
 // (flagged when a pair is active).
-#include "grid.cuh"
+#include "group_scan.cuh"
+#include "launch.cuh"
 #include "solid_rec.cuh"
 
 namespace arp {
@@ -26,10 +29,18 @@ namespace arp {
 namespace {
 
 constexpr int kT = 128;
-#ifndef ARP_ADJ_SOLID_LANES
-#define ARP_ADJ_SOLID_LANES 4
-#endif
-constexpr int kAdjSolidLanes = ARP_ADJ_SOLID_LANES;  // threads per solid in k_adj_solid
+// Threads that share one solid in k_adj_solid: 8 up to kAdjFewSolids, 2 above
+// (cantilever bars, us a launch with 8 / 4 / 2: 3,840 solids 10.0 / 14.1 /
+// 23.3; 15,872: 22.2 / 18.4 / 24.3; 32,256: 38.9 / 34.0 / 29.8; 129,024: 146 /
+// 115 / 104).  k_adj_strain reads less a pair: 4 throughout (129,024 solids:
+// 50 us, 45 with 2; 3,840: 7.4, 10.3 with 2).
+constexpr uint32_t kAdjFewSolids = 16384;
+constexpr int kAdjStrainLanes = 4;
+// Threads that share one particle in k_adj_fluid, likewise 8 or 2 (3D bars and
+// fluid, us with 8 / 4 / 2: 3,840 particles 13.5 / 21.7 / 35; 15,872: 22.6 /
+// 23.5 / 35; 34,688: 41.2 / 38.6 / 33.2; 264,064: - / 244 / 193, 1 thread 224;
+// 2D, 16,384: 11.8 / 10.7 / 13.9; 302,891: 136 / 104 / 84, 1 thread 82).
+constexpr uint32_t kAdjFew = 24576;
 constexpr uint32_t kSameMatBit = 0x80000000u;
 
 inline uint32_t nblocks(uint32_t n, int t) { return (n + (uint32_t)t - 1u) / (uint32_t)t; }
@@ -44,9 +55,8 @@ __device__ __forceinline__ float3 neg(float3 a) { return make_float3(-a.x, -a.y,
 // gradW(X_j - X_i) of a reference pair, as the reference-list build computes
 // it: recomputed from the reference positions (shared by neighboring solids
 // in L1/L2) rather than streamed per list entry.
-__device__ __forceinline__ float3 ref_grad(const float4* __restrict__ ref, uint32_t j, float3 Xi, const SceneP& P) {
-    const float3 dX = sub(f3(ref[j]), Xi);
-    const float diff = P.h2 - ((dX.x * dX.x + dX.y * dX.y) + dX.z * dX.z);
+__device__ __forceinline__ float3 ref_grad(float3 dX, const SceneP& P, float& diff) {
+    diff = P.h2 - ((dX.x * dX.x + dX.y * dX.y) + dX.z * dX.z);
     const float s = -6.0f * P.kconst * diff * diff;
     return make_float3(s * dX.x, s * dX.y, s * dX.z);
 }
@@ -73,8 +83,9 @@ __device__ __forceinline__ M3 m3_cols(const float4* c) {
     return r;
 }
 // A and F of a stress record; returns its cell coordinates
+template <bool AT>
 __device__ __forceinline__ uint2 m3_stress(const float4* AF, uint32_t i, M3& A, M3& F) {
-    const StressRec r = load_stress(AF, i);
+    const StressRec r = load_stress<AT>(AF, i);
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -84,9 +95,18 @@ __device__ __forceinline__ uint2 m3_stress(const float4* AF, uint32_t i, M3& A, 
         }
     return r.cell;
 }
-__device__ __forceinline__ void m3_store_cols(const M3& a, float4* c) {
+// two matrices as such a record
+__device__ __forceinline__ void m3_store_pair(float4* AF, uint32_t i, const M3& A, const M3& F) {
+    StressRec r;
 #pragma unroll
-    for (int j = 0; j < 3; ++j) c[j] = make_float4(a.m[0][j], a.m[1][j], a.m[2][j], 0.0f);
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            r.A[c][k] = A.m[k][c];
+            r.F[c][k] = F.m[k][c];
+        }
+    r.cell = make_uint2(0u, 0u);
+    store_stress(AF, i, r);
 }
 __device__ __forceinline__ float3 m3_vec(const M3& a, float3 v) {
     return make_float3(a.m[0][0] * v.x + a.m[0][1] * v.y + a.m[0][2] * v.z,
@@ -188,11 +208,12 @@ struct PairGeom {
     float cp, dcp_over_R;
     bool contact;
 };
+// Adjoints gathered by particle `a` of a pair; force: its weight times its force.
 struct PairGrad {
-    float3 F;        // forward force contribution to the self particle
-    float3 lr;       // dL/dr, r = x_nbr - x_self
-    float3 lvv;      // dL/d(v_nbr - v_self)
-    float ld_self, ld_nbr, lpt;
+    float3 lr;     // dL/dr, r = x_b - x_a
+    float3 lvv;    // dL/d(v_b - v_a)
+    float ld, lpt; // dL/d its density and p / rho^2
+    float force;
 };
 
 template <int DIM>
@@ -231,81 +252,50 @@ __device__ __forceinline__ PairGeom flipped(const PairGeom& G) {
     return H;
 }
 
-// The fluid pair term of `a` with neighbor `b` (fluid.rs:154-214, as the
-// forward kernel evaluates it) and its vector-Jacobian product for weights
-// wd (on d rho/dt) and wF (on the force sum), friction (fluid.rs:192-199)
-// included.
-template <int DIM, bool BOUNDARY>
-__device__ __forceinline__ void pair_vjp(const PairGeom& G, const PairSide& a, const PairSide& b, float dampening,
-                                         float friction, float wd, float3 wF, PairGrad& o) {
+// d(g(r) . lg)/dr of g = gws(r) r, gws = -6 k (h^2 - r.r)^2
+__device__ __forceinline__ float3 through_grad(const PairGeom& G, float3 lg) {
+    return add(mul(G.gws, lg), mul(G.c24 * dot(lg, G.r), G.r));
+}
+
+// The pair term of `a` with `b` and that of `b` with `a` (fluid.rs:154-214, as
+// the forward kernel evaluates them, without contact), differentiated at once:
+// but for the masses of the continuity term and the viscosity's condition the
+// second is the first with r, vv and g negated, so its vector-Jacobian product
+// for weights wb is the first's for -wb, and both together are the first's for
+// the difference of the weights.  wds: the weights on both density rates, each
+// times the other's mass; wa, wb: those on the force sums.  A boundary particle
+// `b` enters the pressure term alone, with wds and wb zero.
+template <int DIM>
+__device__ __forceinline__ void pair_vjp(const PairGeom& G, const PairSide& a, const PairSide& b, bool boundary,
+                                         float dampening, float wds, float3 wa, float3 wb, PairGrad& o) {
     const float3 r = G.r, vv = G.vv, g = G.g;
-    float3 F = make_float3(0.f, 0.f, 0.f), lg = F, lr = F, lvv = F;
-    float ld1 = 0.f, ld2 = 0.f;
-    if (!BOUNDARY) {
-        lvv = mul(wd * b.m, g);
-        lg = mul(wd * b.m, vv);
-    }
+    const float3 W = sub(wa, wb);
     const float mm = a.m * b.m;
     const float pf = mm * (a.pt + b.pt);
-    F = mul(pf, g);
-    lg = add(lg, mul(pf, wF));
-    const float wg = dot(wF, g);
-    const float lpt = mm * wg;
-    if (G.contact) {
-        const float cs = b.m * G.cp * b.inv_d;
-        F = add(F, mul(cs, g));
-        lg = add(lg, mul(cs, wF));
-        ld2 -= wg * cs * b.inv_d;
-        lr = mul(wg * b.m * b.inv_d * G.dcp_over_R, r);
-        if (friction != 0.0f && (a.elastic || b.elastic || BOUNDARY) && a.mat != b.mat) {
-            // forward: the normal force r (cs g.r) / r.r = cs gws r has length
-            // N = |cs gws| R; the tangential velocity u = vv - r (vv.r) / r.r
-            // gives t = u / |u|, and the force gains friction N t (the second
-            // normalize of the shader leaves t as it is)
-            const float r2 = dot(r, r);
-            const float sv = dot(vv, r) / r2;
-            const float3 u = sub(vv, mul(sv, r));
-            const float ul = sqrtf(dot(u, u));
-            const float3 t = mul(1.0f / ul, u);
-            if (isfinite(t.x) && isfinite(t.y) && isfinite(t.z)) {
-                const float R = sqrtf(r2);
-                const float acs = fabsf(cs), ags = fabsf(G.gws);
-                const float N = acs * ags * R;
-                F = add(F, mul(friction * N, t));
-                const float wt = dot(wF, t);
-                // through t = u / |u| and u = (I - r r^T / r.r) vv
-                const float3 lu = mul(friction * N / ul, sub(wF, mul(wt, t)));
-                const float lur = dot(lu, r);
-                lvv = add(lvv, sub(lu, mul(lur / r2, r)));
-                lr = add(lr, sub(mul(-sv, lu), mul(lur / r2, sub(vv, mul(2.0f * sv, r)))));
-                // through N: |cs| ~ 1/rho_b; dN/dR from cp(R), gws(R) (d gws/dR = c24 R) and R
-                const float lN = friction * wt;
-                ld2 -= lN * N * b.inv_d;
-                const float dcs = copysignf(b.m * b.inv_d * G.dcp_over_R * R, cs);
-                const float dgs = copysignf(G.c24 * R, G.gws);
-                const float dN = dcs * ags * R + acs * dgs * R + acs * ags;
-                lr = add(lr, mul(lN * dN / R, r));
-            }
-        }
-    }
-    if (!BOUNDARY) {
+    const float wga = dot(wa, g), wg = dot(W, g);
+    float3 lg = add(mul(wds, vv), mul(pf, W));
+    float3 lvv = mul(wds, g), lr = make_float3(0.f, 0.f, 0.f);
+    float ld = 0.0f;
+    o.lpt = mm * wg;
+    o.force = pf * wga;
+    if (!boundary) {
         float ldenom = 0.0f;
-        if (!a.elastic) {
-            const float fsum = a.visc + b.visc;
-            if (fsum != 0.0f) {
-                const float rgw = dot(r, g);
-                const float idd = a.inv_d * b.inv_d * G.inv_denom;
-                const float t = mm * fsum * rgw * idd;
-                F = sub(F, mul(t, vv));
-                lvv = sub(lvv, mul(t, wF));
-                const float lt = -dot(wF, vv);
-                const float lrgw = lt * mm * fsum * idd;
-                ld1 -= lt * t * a.inv_d;
-                ld2 -= lt * t * b.inv_d;
-                ldenom -= lt * t * G.inv_denom;
-                lr = add(lr, mul(lrgw, g));
-                lg = add(lg, mul(lrgw, r));
-            }
+        const float fsum = a.visc + b.visc;
+        if (fsum != 0.0f) {  // no viscous force on solids
+            const float3 z = make_float3(0.f, 0.f, 0.f);
+            const float3 wva = a.elastic ? z : wa;
+            const float3 Wv = sub(wva, b.elastic ? z : wb);
+            const float rgw = dot(r, g);
+            const float idd = a.inv_d * b.inv_d * G.inv_denom;
+            const float t = mm * fsum * rgw * idd;
+            lvv = sub(lvv, mul(t, Wv));
+            const float lt = -dot(Wv, vv);
+            const float lrgw = lt * mm * fsum * idd;
+            ld -= lt * t * a.inv_d;
+            ldenom -= lt * t * G.inv_denom;
+            lr = add(lr, mul(lrgw, g));
+            lg = add(lg, mul(lrgw, r));
+            o.force -= t * dot(wva, vv);
         }
         const float f_ = a.mat == b.mat ? a.bulk + b.bulk : dampening;
         if (f_ != 0.0f) {
@@ -313,166 +303,236 @@ __device__ __forceinline__ void pair_vjp(const PairGeom& G, const PairSide& a, c
             const float ids = __fdividef(1.0f, a.d + b.d);
             const float q0 = mm * f_ * ids * G.inv_denom;
             const float Q = q0 * vr;
-            F = sub(F, mul(Q, g));
-            lg = sub(lg, mul(Q, wF));
+            lg = sub(lg, mul(Q, W));
             const float lQ = -wg;
             const float lvr = lQ * q0;
-            ld1 -= lQ * Q * ids;
-            ld2 -= lQ * Q * ids;
+            ld -= lQ * Q * ids;
             ldenom -= lQ * Q * G.inv_denom;
             lvv = add(lvv, mul(lvr, r));
             lr = add(lr, mul(lvr, vv));
+            o.force -= Q * wga;
         }
         lr = add(lr, mul(2.0f * ldenom, r));
     }
-    // g = gws(r) r, gws = -6 k (h^2 - r.r)^2
-    lr = add(lr, add(mul(G.gws, lg), mul(G.c24 * dot(lg, r), r)));
-    if (DIM == 2) {
-        lr.z = 0.0f;
-        lvv.z = 0.0f;
-    }
-    o.F = F;
-    o.lr = lr;
+    o.lr = add(lr, through_grad(G, lg));
     o.lvv = lvv;
-    o.ld_self = ld1;
-    o.ld_nbr = ld2;
-    o.lpt = lpt;
+    o.ld = ld;
 }
 
-// Per particle of the stage: the weights of its derivative record and its
-// state-equation terms, read by its own thread and by its neighbors':
-// w = (mu_v / rho, mu_rho), e = (p / rho^2, d(p / rho^2)/d rho, 1 / rho);
-// and the positions in cell order for the neighbor scan.  Thread k is cell
-// position k.
-__global__ void k_adj_prep(AdjArgs a, Tables T, float4* __restrict__ w, float4* __restrict__ e) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.n) return;
-    const uint32_t i = a.st.perm ? a.st.perm[k] : k;
-    const float4 xi = a.st.pd[i];
-    a.xs[k] = xi;
-    const FluidMat fm = T.fmats[__float_as_uint(a.st.vm[i].w)];
-    const float ir = 1.0f / xi.w;
-    const float4 mv = a.mu_vm[i];
-    w[i] = make_float4(mv.x * ir, mv.y * ir, mv.z * ir, a.mu_pd[i].w);
-    float pt, dpt;
-    eos_pt(fm.eos, xi.w, fm.c, fm.d0, pt, dpt);
-    e[i] = make_float4(pt, dpt, ir, 0.0f);
-}
-
-constexpr int kAdjCap = 48;                   // hit-list entries per thread of k_adj_fluid
-constexpr uint32_t kHitBoundary = 0x80000000u;  // list entry of a boundary particle
-
+// Contact and friction of `a` with `b` (fluid.rs:185-199) for weights wF on the
+// force of `a`; they read the density of `b` alone.  ld: dL/d that density.
 template <int DIM>
-__global__ void __launch_bounds__(kT) k_adj_fluid(AdjArgs a, Tables T, const float4* __restrict__ W,
-                                                  const float4* __restrict__ EQ) {
-    __shared__ uint32_t lst[kAdjCap * kT];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const float4 xi = a.st.pd[i], vi = a.st.vm[i];
-    const uint32_t mat = __float_as_uint(vi.w);
+__device__ __forceinline__ void contact_vjp(const PairGeom& G, const PairSide& a, const PairSide& b, bool boundary,
+                                            float friction, float3 wF, PairGrad& o) {
+    const float3 r = G.r, vv = G.vv, g = G.g;
+    float3 lvv = make_float3(0.f, 0.f, 0.f);
+    const float wg = dot(wF, g);
+    const float cs = b.m * G.cp * b.inv_d;
+    float force = cs * wg;
+    float ld = -wg * cs * b.inv_d;
+    float3 lr = mul(wg * b.m * b.inv_d * G.dcp_over_R, r);
+    if (friction != 0.0f && (a.elastic || b.elastic || boundary) && a.mat != b.mat) {
+        // forward: the normal force r (cs g.r) / r.r = cs gws r has length
+        // N = |cs gws| R; the tangential velocity u = vv - r (vv.r) / r.r
+        // gives t = u / |u|, and the force gains friction N t (the second
+        // normalize of the shader leaves t as it is)
+        const float r2 = dot(r, r);
+        const float sv = dot(vv, r) / r2;
+        const float3 u = sub(vv, mul(sv, r));
+        const float ul = sqrtf(dot(u, u));
+        const float3 t = mul(1.0f / ul, u);
+        if (isfinite(t.x) && isfinite(t.y) && isfinite(t.z)) {
+            const float R = sqrtf(r2);
+            const float acs = fabsf(cs), ags = fabsf(G.gws);
+            const float N = acs * ags * R;
+            const float wt = dot(wF, t);
+            force += friction * N * wt;
+            // through t = u / |u| and u = (I - r r^T / r.r) vv
+            const float3 lu = mul(friction * N / ul, sub(wF, mul(wt, t)));
+            const float lur = dot(lu, r);
+            lvv = sub(lu, mul(lur / r2, r));
+            lr = add(lr, sub(mul(-sv, lu), mul(lur / r2, sub(vv, mul(2.0f * sv, r)))));
+            // through N: |cs| ~ 1/rho_b; dN/dR from cp(R), gws(R) (d gws/dR = c24 R) and R
+            const float lN = friction * wt;
+            ld -= lN * N * b.inv_d;
+            const float dcs = copysignf(b.m * b.inv_d * G.dcp_over_R * R, cs);
+            const float dgs = copysignf(G.c24 * R, G.gws);
+            const float dN = dcs * ags * R + acs * dgs * R + acs * ags;
+            lr = add(lr, mul(lN * dN / R, r));
+        }
+    }
+    o.lr = add(lr, through_grad(G, mul(cs, wF)));
+    o.lvv = lvv;
+    o.ld = ld;
+    o.force = force;
+    o.lpt = 0.0f;
+}
+
+__device__ __forceinline__ float4 axpy4(float c, float4 x, float4 y) {
+    return make_float4(y.x + c * x.x, y.y + c * x.y, y.z + c * x.z, y.w + c * x.w);
+}
+
+constexpr uint32_t kAdjMat = 0xFFu, kAdjElastic = 0x100u;  // id bits of a record: material in its scene, elastic
+
+// What a stage's kernels read of each particle, thread k at cell position k
+// (boundary particles after the n mobile ones):
+//   * mu, the weights of the stage's derivative record, from the adjoint of the
+//     step's result and the later stages' (Runge-Kutta; given otherwise), and
+//     a cleared lam_Y when solids add to it;
+//   * rec: (x, rho), (v, id bits), (mu_v / rho, mu_rho), (p / rho^2,
+//     d(p / rho^2)/d rho, 1 / rho, material id bits): 64 bytes a neighbor is
+//     read with two loads;
+//   * the quantised position, and sw (velocity, mu_v / rho) of a solid.
+// One launch in place of six (a gather into storage order, the weights, two
+// clears, the records and positions in cell order); bound by its memory traffic,
+// 4.4 us for 32,256 particles, 12 for 302,891.
+__global__ void k_adj_prep(AdjArgs a, Tables T) {
+    step_begin();
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= a.n + a.nb) return;
+    const bool mobile = k < a.n;
+    const uint32_t i = mobile && a.st.perm ? a.st.perm[k] : k;
+    const float4 x = mobile ? a.st.pd[i] : a.bxs[k - a.n];
+    const float4 v = mobile ? a.st.vm[i] : a.bvs[k - a.n];
+    const uint32_t mat = __float_as_uint(v.w);
+    const DevMat& m = T.mats[mat];
+    const float ir = 1.0f / x.w;
+    float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+    float pt, dpt;
+    if (mobile) {
+        float4 mp, mv;
+        if (a.lc_p) {
+            const uint32_t c = a.orig[i];
+            const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+            mp = axpy4(a.cb, a.lc_p[c], z);
+            mv = axpy4(a.cb, a.lc_v[c], z);
+            for (int t = 0; t < a.later.n; ++t) {
+                mp = axpy4(a.later.c[t], a.later.pd[t][i], mp);
+                mv = axpy4(a.later.c[t], a.later.vm[t][i], mv);
+            }
+        } else {
+            mp = a.mu_pd[i];
+            mv = a.mu_vm[i];
+        }
+        a.mux[k] = mp;
+        w = make_float4(mv.x * ir, mv.y * ir, mv.z * ir, mp.w);
+        eos_pt(m.state_eq, x.w, m.sound_speed, m.target_den, pt, dpt);
+        if (a.solid_branch) {
+            const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+            a.lam_pd[i] = z;
+            a.lam_vm[i] = z;
+            const uint32_t sid = a.sid[i];
+            if (sid != kInvalid) {
+                a.sw[2 * (size_t)sid] = v;
+                a.sw[2 * (size_t)sid + 1] = w;
+            }
+        }
+    } else {
+        pt = a.bps[k - a.n];
+        dpt = 0.0f;
+    }
+    const uint32_t id = m.local | (mobile && m.stiff ? kAdjElastic : 0u);
+    float4* const r = a.rec + 4 * (size_t)k;
+    r[0] = x;
+    r[1] = make_float4(v.x, v.y, v.z, __uint_as_float(id));
+    r[2] = w;
+    r[3] = make_float4(pt, dpt, ir, v.w);
+    a.code[k] = scan_code(x, T.scenes[m.scene]);
+}
+
+// LANES threads share one particle, as in the forward kernel's group form: the
+// scan lists hits, the lanes take one pair at a time, both terms of it at once,
+// and their sums are combined at the end.  Bound by the pair arithmetic at 96
+// registers a thread (20 warps per SM; 16 without the bound: 4 % slower).  With
+// one thread per particle, separate arrays and each pair's two terms
+// differentiated in turn a launch took 72 us for 32,256 particles in 3D (now
+// 38) and 107 us for 302,891 in 2D (now 84).
+template <int DIM, int LANES>
+__global__ void __launch_bounds__(kT, 5) k_adj_fluid(AdjArgs a, Tables T) {
+    constexpr int NG = kT / LANES;  // particles per block
+    constexpr int LIST = LANES <= 2 ? 48 : kGroupList;
+    using Scan = GroupScan<DIM, LANES, LIST>;
+    __shared__ uint32_t s_list[NG][LIST];
+    __shared__ uint2 s_seg[NG][2 * Scan::MAXROWS];
+    step_begin();
+    const uint32_t lane = threadIdx.x % LANES, gi = threadIdx.x / LANES;
+    const uint32_t kk = blockIdx.x * NG + gi;
+    const bool valid = kk < a.n;
+    const uint32_t k = valid ? kk : a.n - 1u;  // idle groups of the last block follow the last particle, without candidates
+    float4 xi, vi, wi, ei;
+    load8(a.rec + 4 * (size_t)k, xi, vi);
+    load8(a.rec + 4 * (size_t)k + 2, wi, ei);
+    const uint32_t mat = __float_as_uint(ei.w);  // batch-wide
     const DevMat& mm = T.mats[mat];
     const SceneP& P = T.scenes[mm.scene];
-    const FluidMat fm = T.fmats[mat];
-    const uint32_t sid = a.sid[i];
-    const float4 ei = EQ[i], wi = W[i];
-    const PairSide si{f3(xi), f3(vi), xi.w, ei.z, ei.x, fm.mass, fm.visc, fm.bulk, mat,
-                      sid != kInvalid && fm.stiff != 0u};
+    const uint32_t id = __float_as_uint(vi.w), li = id & kAdjMat;
+    const PairSide si{f3(xi), f3(vi), xi.w, ei.z, ei.x, mm.mass, mm.visc, mm.bulk_visc, li, (id & kAdjElastic) != 0u};
     const float dpt_i = ei.y;
     const float wd = wi.w;
     const float3 wF = f3(wi);
-    const bool solid_term = a.solid_branch && sid != kInvalid && P.solid_branch;
-    float3 lx = make_float3(0.f, 0.f, 0.f);
-    float3 lv = mul(solid_term ? 2.0f : 1.0f, f3(a.mu_pd[i]));  // dx/dt = v (twice for solids in the solid branch)
-    float lrho = 0.0f;
-    float3 Fs = make_float3(0.f, 0.f, 0.f);
-    const uint32_t li = mat - P.mat_base;
-    const DevInter* row_i = T.inter + P.inter_base + li * P.nmat;
-    // Two passes, as in the forward kernel: the scan lists the hits (cell
-    // positions; boundary ones flagged) in shared memory, then the pair VJPs
-    // run over the list with nearly full warps.  A particle with more hits
-    // than the list holds scans again for the next kAdjCap of them (the pair
-    // math stays at one call site); the pairs are taken in scan order.
-    uint32_t* my = lst + threadIdx.x;
-    auto eval = [&](uint32_t h) {
-        if (h & kHitBoundary) {
-            const uint32_t jb = h & ~kHitBoundary;
-            const float4 xb = a.bxs[jb];
-            const float4 vb = a.bvs[jb];
-            const uint32_t matb = __float_as_uint(vb.w);
-            const FluidMat fb = T.fmats[matb];
-            const PairSide sb{f3(xb), f3(vb), xb.w, __fdividef(1.0f, xb.w), a.bps[jb], fb.mass, fb.visc,
-                              fb.bulk, matb, false};
-            const DevInter it = row_i[matb - P.mat_base];
-            const PairGeom G = make_geom<DIM>(si.x, si.v, sb.x, sb.v, it, P.h2, P.kconst, P.eps_hh);
-            PairGrad o;
-            pair_vjp<DIM, true>(G, si, sb, it.dampening, it.friction, wd, wF, o);
-            Fs = add(Fs, o.F);
-            lx = sub(lx, o.lr);
-            lv = sub(lv, o.lvv);
-            lrho += o.ld_self + o.lpt * dpt_i;
-        } else {
-            const uint32_t j = a.st.perm ? a.st.perm[h] : h;
-            if (j == i) return;
-            const float4 xj = a.st.pd[j];
-            const float4 vj = a.st.vm[j];
-            const uint32_t matj = __float_as_uint(vj.w);
-            const FluidMat fj = T.fmats[matj];
-            const uint32_t sidj = a.sid[j];
-            const float4 ej = EQ[j], wj = W[j];
+    const FluidMat* const fmats = T.fmats + P.mat_base;
+    const DevInter* const row_i = T.inter + P.inter_base + li * P.nmat;
+    const float h2 = P.h2, kc = P.kconst, eps_hh = P.eps_hh;
+    float3 lx = make_float3(0.f, 0.f, 0.f), lv = lx;
+    float lrho = 0.0f, force = 0.0f;
+    uint32_t* const list = s_list[gi];
+    Scan::run(xi, valid && finite3(xi), P, ScanArrays{a.code, a.st.start, a.bstart, a.n}, list,
+                               s_seg[gi], [&](uint32_t ev) {
+#pragma unroll 1
+        for (uint32_t e = lane; e < ev; e += LANES) {
+            const uint32_t j = list[e];
+            if (j == k) continue;
+            float4 xj, vj, wj, ej;
+            load8_at(a.rec + 4 * (size_t)j, xj, vj);
+            load8_at(a.rec + 4 * (size_t)j + 2, wj, ej);
+            const float rx = xj.x - xi.x, ry = xj.y - xi.y, rz = DIM == 3 ? xj.z - xi.z : 0.0f;
+            if (!(h2 - (rx * rx + ry * ry + rz * rz) > 0.0f)) continue;
+            const uint32_t idj = __float_as_uint(vj.w), matj = idj & kAdjMat;
+            const FluidMat fj = fmats[matj];
             const PairSide sj{f3(xj), f3(vj), xj.w, ej.z, ej.x, fj.mass, fj.visc, fj.bulk, matj,
-                              sidj != kInvalid && fj.stiff != 0u};
-            const DevInter it = row_i[matj - P.mat_base];  // symmetric: also the neighbor's entry
-            const PairGeom G = make_geom<DIM>(si.x, si.v, sj.x, sj.v, it, P.h2, P.kconst, P.eps_hh);
+                              (idj & kAdjElastic) != 0u};
+            const DevInter it = row_i[matj];  // symmetric: also the neighbor's entry
+            const PairGeom G = make_geom<DIM>(si.x, si.v, sj.x, sj.v, it, h2, kc, eps_hh);
             PairGrad o;
-            pair_vjp<DIM, false>(G, si, sj, it.dampening, it.friction, wd, wF, o);
-            Fs = add(Fs, o.F);
+            const bool boundary = j >= a.n;  // its weights are zero
+            const float3 wFj = f3(wj);
+            pair_vjp<DIM>(G, si, sj, boundary, it.dampening, boundary ? 0.0f : wd * sj.m + wj.w * si.m, wF, wFj, o);
             lx = sub(lx, o.lr);
             lv = sub(lv, o.lvv);
-            lrho += o.ld_self + o.lpt * dpt_i;
-            // the neighbor's own pair, in which this particle is the neighbor
-            pair_vjp<DIM, false>(flipped(G), sj, si, it.dampening, it.friction, wj.w, f3(wj), o);
+            lrho += o.ld + o.lpt * dpt_i;
+            force += o.force;
+            if (!G.contact) continue;
+            contact_vjp<DIM>(G, si, sj, boundary, it.friction, wF, o);
+            lx = sub(lx, o.lr);
+            lv = sub(lv, o.lvv);
+            force += o.force;
+            if (boundary) continue;
+            // the neighbor's own term, in which this particle is the neighbor
+            contact_vjp<DIM>(flipped(G), sj, si, false, it.friction, wFj, o);
             lx = add(lx, o.lr);
             lv = add(lv, o.lvv);
-            lrho += o.ld_nbr + o.lpt * dpt_i;
+            lrho += o.ld;
         }
-    };
-    if (finite3(xi)) {
-        for (uint32_t done = 0;;) {
-            uint32_t total = 0, cnt = 0;  // hits seen in this scan, hits listed
-            auto take = [&](uint32_t h) {
-                if (total >= done && cnt < (uint32_t)kAdjCap) my[cnt++ * kT] = h;
-                ++total;
-            };
-            for_search_rows<DIM>(xi, P, [&](uint32_t c0, uint32_t c1) {
-                for (uint32_t jb = a.bstart[c0]; jb < a.bstart[c1]; ++jb) {
-                    const float4 xb = a.bxs[jb];
-                    const float rx = xb.x - xi.x, ry = xb.y - xi.y, rz = DIM == 3 ? xb.z - xi.z : 0.0f;
-                    if (P.h2 - (rx * rx + ry * ry + rz * rz) > 0.0f) take(jb | kHitBoundary);
-                }
-                for (uint32_t k = a.st.start[c0]; k < a.st.start[c1]; ++k) {
-                    const float4 xj = a.xs[k];
-                    const float rx = xj.x - xi.x, ry = xj.y - xi.y, rz = DIM == 3 ? xj.z - xi.z : 0.0f;
-                    if (P.h2 - (rx * rx + ry * ry + rz * rz) > 0.0f) take(k);
-                }
-            });
-            for (uint32_t e = 0; e < cnt; ++e) eval(my[e * kT]);
-            done += cnt;
-            if (done >= total) break;
-        }
-    }
-    lrho -= dot(wF, Fs) * ei.z;  // k_v = F / rho
+    });
+    lx = make_float3(group_sum<LANES>(lx.x), group_sum<LANES>(lx.y), group_sum<LANES>(lx.z));
+    lv = make_float3(group_sum<LANES>(lv.x), group_sum<LANES>(lv.y), group_sum<LANES>(lv.z));
+    force = group_sum<LANES>(force);
+    lrho = group_sum<LANES>(lrho);
+    if (!valid || lane != 0) return;
+    lrho -= force * ei.z;  // k_v = F / rho
+    // dx/dt = v (twice for solids in the solid branch)
+    const bool solid_term = a.solid_branch && (id & kAdjElastic) && P.solid_branch;
+    lv = add(lv, mul(solid_term ? 2.0f : 1.0f, f3(a.mux[k])));
     if (DIM == 2) {
         lx.z = 0.0f;
         lv.z = 0.0f;
     }
-    float4 lp = a.lam_pd[i], lw = a.lam_vm[i];
-    lp.x += lx.x;
-    lp.y += lx.y;
-    lp.z += lx.z;
-    lp.w += lrho;
-    lw.x += lv.x;
-    lw.y += lv.y;
-    lw.z += lv.z;
+    const uint32_t i = a.st.perm ? a.st.perm[k] : k;
+    float4 lp = make_float4(lx.x, lx.y, lx.z, lrho), lw = make_float4(lv.x, lv.y, lv.z, 0.0f);
+    if (a.solid_branch) {  // after the solid kernels
+        lp = axpy4(1.0f, a.lam_pd[i], lp);
+        lw = axpy4(1.0f, a.lam_vm[i], lw);
+    }
     a.lam_pd[i] = lp;
     a.lam_vm[i] = lw;
 }
@@ -676,15 +736,18 @@ __device__ inline void sh_rate_vjp(const M3& C, const M3& dC, int two_m, const M
     }
 }
 
-// Hourglass pair term of `self` (solid.rs:430-443 as k_solid_forces evaluates
-// it) and its VJP for weight w: forward force f, dL/d(dx) with dx = x_nbr -
-// x_self, dL/de (e = 0.5 (F_self + F_nbr) dX - dx), dL/d rho_self, rho_nbr.
+// Hourglass pair term of `a` with `b` (solid.rs:430-443 as k_solid_forces
+// evaluates it) and that of `b` with `a`, differentiated at once: the second is
+// the first with dx, dX and e negated, so both are the first's vector-Jacobian
+// product for the difference of the weights (w of `a`, wb of `b`).  force: w
+// times the forward force on `a`; dL/d(dx) with dx = x_b - x_a, dL/de (e = 0.5
+// (F_a + F_b) dX - dx) and dL/d rho_a.
 struct HgGrad {
-    float3 f, ldx, le;
-    float lda, ldb;
+    float3 ldx, le;
+    float ld, force;
 };
 __device__ __forceinline__ void hg_vjp(float3 dx, float3 dX, const M3& Fa, const M3& Fb, float da, float db, float m,
-                                       float kern, const SceneP& P, float3 w, HgGrad& o) {
+                                       float kern, const SceneP& P, float3 w, float3 wb, HgGrad& o) {
     M3 Fs;
 #pragma unroll
     for (int r = 0; r < 3; ++r)
@@ -700,14 +763,14 @@ __device__ __forceinline__ void hg_vjp(float3 dx, float3 dX, const M3& Fa, const
     const float sh = a1 * b1 * c1 * kern;
     const float den = l + P.eps_h;
     const float u = sh / den;
-    o.f = mul(-u, dx);
-    const float lu = -dot(w, dx);
-    float3 ldx = mul(-u, w);
+    o.force = -u * dot(w, dx);
+    const float3 W = sub(w, wb);
+    const float lu = -dot(W, dx);
+    float3 ldx = mul(-u, W);
     const float lsh = lu / den;
     const float lden = -lu * u / den;
     const float la1 = lsh * b1 * c1 * kern, lb1 = lsh * a1 * c1 * kern, lc1 = lsh * a1 * b1 * kern;
-    o.lda = -la1 * a1 / da;
-    o.ldb = -la1 * a1 / db;
+    o.ld = -la1 * a1 / da;
     const float led = lb1 * 0.5f / lh;
     float ll = -lb1 * b1 / lh - lc1 * c1 * c1 * 2.0f * l + lden;
     const float3 le = mul(led, dx);
@@ -718,9 +781,12 @@ __device__ __forceinline__ void hg_vjp(float3 dx, float3 dX, const M3& Fa, const
     o.le = le;
 }
 
-// LANES threads share one solid: both reference-list loops are split over
-// them with stride LANES, their partial sums combined by group_sum; lane 0
-// finishes the particle.
+// LANES threads share one solid: the reference list is split over them with
+// stride LANES, their partial sums combined by group_sum; lane 0 finishes the
+// particle.  Bound by the loads of the neighbors' records (160 bytes a pair)
+// at 128 registers a thread.  With a second pass over the list for dF/dt, each
+// hourglass pair's two terms in turn and 4 threads a solid a launch took 51 us
+// for 32,256 solids (now 30), k_adj_strain with one thread a solid 29 (now 13).
 // GENERAL: some solid material has a strain order other than 2 (the log
 // series, square roots and inverses are compiled out otherwise).  PLASTIC:
 // some material is plastic; the plastic strain then enters E and its rate
@@ -728,76 +794,68 @@ __device__ __forceinline__ void hg_vjp(float3 dx, float3 dX, const M3& Fa, const
 // is differentiated, 4 x 4 as the shader holds them.
 template <int LANES, bool GENERAL, bool PLASTIC>
 __global__ void __launch_bounds__(kT) k_adj_solid(AdjArgs a, Tables T) {
+    step_begin();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = t / LANES, lane = t % LANES;
     if (i >= a.ns) return;  // whole groups leave together
-    const float4 xi = a.st.sx[2 * (size_t)i], vi = a.st.sv[i];
+    const SolidPos pi = load_pos(a.st.sx, i);
+    const float4 xi = pi.x;
+    float4 vi, wi;
+    load8(a.sw + 2 * (size_t)i, vi, wi);
+    const uint32_t k1 = a.rl.off[i + 1];
+    uint32_t k = a.rl.off[i] + lane;
     const uint32_t mat = __float_as_uint(vi.w);
     const DevMat mm = T.mats[mat];
     const SceneP& P = T.scenes[mm.scene];
     if (!P.solid_branch) return;
-    const uint32_t slot = a.slot_of[i];
     const float d1 = xi.w, m1 = mm.mass, V1 = m1 / d1;
-    const float3 w = mul(1.0f / d1, f3(a.mu_vm[slot]));
+    const float3 w = f3(wi);
     const float3 wdm = mask_dim(w, P.dim);
     M3 Ai, Fi;
-    const uint2 ci = m3_stress(a.st.AF, i, Ai, Fi);
-    const float3 Xi = f3(a.ref[i]);
-    M3 lA = m3_zero(), lFh = m3_zero();
-    float3 lx = make_float3(0.f, 0.f, 0.f), fs = lx;
-    float lrho = 0.0f;
-    const uint32_t k0 = a.rl.off[i], k1 = a.rl.off[i + 1];
-    for (uint32_t k = k0 + lane; k < k1; k += LANES) {
-        const uint32_t e = a.rl.nbr[k];
-        if (!(e & kSameMatBit)) continue;
-        const uint32_t j = e & ~kSameMatBit;
+    const uint2 ci = m3_stress<false>(a.st.AF, i, Ai, Fi);
+    const float3 Xi = f3(pi.X);
+    const M3 L = m3_cols(a.L + 3 * i);
+    M3 lA = m3_zero(), lFh = m3_zero(), Fd = m3_zero();  // Fd: dF/dt of the stage, recomputed
+    float3 lx = make_float3(0.f, 0.f, 0.f);
+    float lrho = 0.0f, force = 0.0f;
+    for (; k < k1; k += LANES) {
+        const uint32_t e = a.rl.nbr[k], j = e & ~kSameMatBit;
         const SolidPos pj = load_pos_at(a.st.sx, j);
+        float4 vj, wj4;
+        load8_at(a.sw + 2 * (size_t)j, vj, wj4);
         const float3 dX = sub(f3(pj.X), Xi);
-        const float diff = P.h2 - ((dX.x * dX.x + dX.y * dX.y) + dX.z * dX.z);
-        const float3 g = mul(-6.0f * P.kconst * diff * diff, dX);
+        float diff;
+        const float3 g = ref_grad(dX, P, diff);
+        m3_add_outer(Fd, pj.X.w, sub(f3(vj), f3(vi)), m3_vec(L, g));  // X.w = V_j
+        if (!(e & kSameMatBit)) continue;
         const float4 xj = pj.x;
         const float d2 = xj.w;
         const float c = -V1 * (m1 / d2);
         M3 Aj, Fj;
-        const uint2 cj = m3_stress(a.st.AF, j, Aj, Fj);
+        const uint2 cj = m3_stress<true>(a.st.AF, j, Aj, Fj);
         M3 As;
 #pragma unroll
         for (int r = 0; r < 3; ++r)
 #pragma unroll
             for (int cc = 0; cc < 3; ++cc) As.m[r][cc] = Ai.m[r][cc] + Aj.m[r][cc];
         const float3 Ag = m3_vec(As, g);
-        fs = add(fs, mul(c, mask_dim(Ag, P.dim)));
-        m3_add_outer(lA, c, wdm, g);
-        lrho += (-c / d1) * dot(wdm, Ag);
-        // the neighbor's elastic term: f_j += c (A_j + A_i) grad_w(X_i - X_j), the gradient being -g
-        const float3 wj = mul(1.0f / d2, f3(a.mu_vm[a.slot_of[j]]));
-        const float3 wjd = mask_dim(wj, P.dim);
-        m3_add_outer(lA, -c, wjd, g);
-        lrho += (c / d1) * dot(wjd, Ag);
+        force += c * dot(wdm, Ag);
+        // the particle's elastic term and the neighbor's, f_j += c (A_j + A_i)
+        // grad_w(X_i - X_j), whose gradient is -g
+        const float3 wj = f3(wj4);
+        const float3 wdiff = sub(wdm, mask_dim(wj, P.dim));
+        m3_add_outer(lA, c, wdiff, g);
+        lrho += (-c / d1) * dot(wdiff, Ag);
         if (in_stencil(cj, ci)) {
             const float3 dx = sub(f3(xj), f3(xi));
             const float kern = P.kconst * diff * diff * diff;
             HgGrad o;
-            hg_vjp(dx, dX, Fi, Fj, d1, d2, m1, kern, P, w, o);
-            fs = add(fs, o.f);
+            hg_vjp(dx, dX, Fi, Fj, d1, d2, m1, kern, P, w, wj, o);
+            force += o.force;
             lx = sub(lx, o.ldx);
             m3_add_outer(lFh, 0.5f, o.le, dX);
-            lrho += o.lda;
-            hg_vjp(neg(dx), neg(dX), Fj, Fi, d2, d1, m1, kern, P, wj, o);
-            lx = add(lx, o.ldx);
-            m3_add_outer(lFh, -0.5f, o.le, dX);
-            lrho += o.ldb;
+            lrho += o.ld;
         }
-    }
-    // dF/dt of the stage, recomputed from the reference list
-    const M3 L = m3_cols(a.L + 3 * i);
-    M3 Fd = m3_zero();
-    for (uint32_t k = k0 + lane; k < k1; k += LANES) {
-        const uint32_t j = a.rl.nbr[k] & ~kSameMatBit;
-        const float4 vj = a.st.sv[j];
-        const float3 G = m3_vec(L, ref_grad(a.ref, j, Xi, P));
-        const float3 dv = sub(f3(vj), f3(vi));
-        m3_add_outer(Fd, a.ref[j].w, dv, G);  // ref.w = V_j
     }
     if (LANES > 1) {
 #pragma unroll
@@ -809,7 +867,7 @@ __global__ void __launch_bounds__(kT) k_adj_solid(AdjArgs a, Tables T) {
                 Fd.m[r][c] = group_sum<LANES>(Fd.m[r][c]);
             }
         lx = make_float3(group_sum<LANES>(lx.x), group_sum<LANES>(lx.y), group_sum<LANES>(lx.z));
-        fs = make_float3(group_sum<LANES>(fs.x), group_sum<LANES>(fs.y), group_sum<LANES>(fs.z));
+        force = group_sum<LANES>(force);
         lrho = group_sum<LANES>(lrho);
         if (lane != 0) return;
     }
@@ -834,7 +892,7 @@ __global__ void __launch_bounds__(kT) k_adj_solid(AdjArgs a, Tables T) {
             if (active) atomicOr(a.flags, 1u);
         }
     }
-    lrho -= dot(w, fs) / d1;  // k_v = f / rho - g
+    lrho -= force / d1;  // k_v = f / rho - g
     // stress chain: C = F^T F (padded with ones past dim), dC = dF^T F + F^T dF,
     // E = seth_hill(C), dE/dt = seth_hill_rate(C, dC) (any strain order),
     // S = Hooke(E; n, s) + Hooke(dE/dt; n_d, s_d), sigma = F S^T, A = sigma L
@@ -983,8 +1041,8 @@ __global__ void __launch_bounds__(kT) k_adj_solid(AdjArgs a, Tables T) {
     m3_acc(lF, m3_mul(Fd, lR));
     const M3 lFd = m3_mul(Fi, m3_t(lR));
     m3_acc(lF, lFh);
-    m3_store_cols(lF, a.lamF + 3 * i);
-    m3_store_cols(lFd, a.lamFd + 3 * i);
+    // k_adj_strain reads lF and dF/dt's adjoint only as (lF L) g and (lFd L) g
+    m3_store_pair(a.lamM, i, m3_mul(lF, L), m3_mul(lFd, L));
     // summed over every stage of every step in double: the per-stage terms
     // change sign as the bar oscillates, and a float sum would lose the
     // difference to rounding
@@ -992,6 +1050,7 @@ __global__ void __launch_bounds__(kT) k_adj_solid(AdjArgs a, Tables T) {
     gsum.x += (double)gn;
     gsum.y += (double)gs;
     a.g_stiff[i] = gsum;
+    const uint32_t slot = a.slot_of[i];
     float4 lp = a.lam_pd[slot];
     lp.x += lx.x;
     lp.y += lx.y;
@@ -1002,33 +1061,52 @@ __global__ void __launch_bounds__(kT) k_adj_solid(AdjArgs a, Tables T) {
 
 // F_i = sum_j V_j (x_j - x_i) (x) L_i gradW_ij and dF/dt likewise with v:
 // gather the adjoints of F and dF/dt of the particle and of its reference
-// neighbors into dL/dx and dL/dv.
+// neighbors into dL/dx and dL/dv.  In F_j this particle enters with V_i and
+// L_j gradW(X_i - X_j) = -L_j g, so with M = lF L both add up to
+// -(V_j M_i + V_i M_j) g.
+template <int LANES>
 __global__ void __launch_bounds__(kT) k_adj_strain(AdjArgs a, Tables T) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.ns) return;
+    step_begin();
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = t / LANES, lane = t % LANES;
+    if (i >= a.ns) return;  // whole groups leave together
     const uint32_t mat = __float_as_uint(a.st.sv[i].w);
+    const uint32_t k1 = a.rl.off[i + 1];
+    uint32_t k = a.rl.off[i] + lane;
     const DevMat& mm = T.mats[mat];
     const SceneP& P = T.scenes[mm.scene];
     if (!P.solid_branch) return;
-    const uint32_t slot = a.slot_of[i];
-    const M3 Li = m3_cols(a.L + 3 * i);
-    const M3 lFi = m3_cols(a.lamF + 3 * i), lFdi = m3_cols(a.lamFd + 3 * i);
-    const float Vri = mm.vol0;
-    const float3 Xi = f3(a.ref[i]);
+    M3 Mi, Mdi;
+    m3_stress<false>(a.lamM, i, Mi, Mdi);
+    const float4 Xi4 = a.st.sx[2 * (size_t)i + 1];
+    const float3 Xi = f3(Xi4);
+    const float Vi = Xi4.w;
     float3 lx = make_float3(0.f, 0.f, 0.f), lv = lx;
-    for (uint32_t k = a.rl.off[i]; k < a.rl.off[i + 1]; ++k) {
-        const uint32_t j = a.rl.nbr[k] & ~kSameMatBit;
-        const float3 g = ref_grad(a.ref, j, Xi, P);
-        const float4 g4 = make_float4(g.x, g.y, g.z, a.ref[j].w);  // ref.w = V_j
-        const float3 G = m3_vec(Li, g);
-        lx = sub(lx, mul(g4.w, m3_vec(lFi, G)));
-        lv = sub(lv, mul(g4.w, m3_vec(lFdi, G)));
-        // in F_j this particle enters with V_i and L_j gradW(X_i - X_j) = -L_j g
-        const M3 Lj = m3_cols(a.L + 3 * j);
-        const float3 Gj = neg(m3_vec(Lj, g));
-        lx = add(lx, mul(Vri, m3_vec(m3_cols(a.lamF + 3 * j), Gj)));
-        lv = add(lv, mul(Vri, m3_vec(m3_cols(a.lamFd + 3 * j), Gj)));
+    auto pair = [&](float4 X, const M3& Mj, const M3& Mdj) {
+        float diff;
+        const float3 g = ref_grad(sub(f3(X), Xi), P, diff);
+        lx = sub(lx, add(mul(X.w, m3_vec(Mi, g)), mul(Vi, m3_vec(Mj, g))));
+        lv = sub(lv, add(mul(X.w, m3_vec(Mdi, g)), mul(Vi, m3_vec(Mdj, g))));
+    };
+    for (; k + LANES < k1; k += 2 * LANES) {
+        const uint32_t j0 = a.rl.nbr[k] & ~kSameMatBit, j1 = a.rl.nbr[k + LANES] & ~kSameMatBit;
+        const float4 X0 = a.st.sx[2 * (size_t)j0 + 1], X1 = a.st.sx[2 * (size_t)j1 + 1];
+        M3 M0, Md0, M1, Md1;
+        m3_stress<true>(a.lamM, j0, M0, Md0);
+        m3_stress<true>(a.lamM, j1, M1, Md1);
+        pair(X0, M0, Md0);
+        pair(X1, M1, Md1);
     }
+    if (k < k1) {
+        const uint32_t j = a.rl.nbr[k] & ~kSameMatBit;
+        M3 Mj, Mdj;
+        m3_stress<true>(a.lamM, j, Mj, Mdj);
+        pair(a.st.sx[2 * (size_t)j + 1], Mj, Mdj);
+    }
+    lx = make_float3(group_sum<LANES>(lx.x), group_sum<LANES>(lx.y), group_sum<LANES>(lx.z));
+    lv = make_float3(group_sum<LANES>(lv.x), group_sum<LANES>(lv.y), group_sum<LANES>(lv.z));
+    if (lane != 0) return;
+    const uint32_t slot = a.slot_of[i];
     float4 lp = a.lam_pd[slot], lw = a.lam_vm[slot];
     lp.x += lx.x;
     lp.y += lx.y;
@@ -1040,15 +1118,23 @@ __global__ void __launch_bounds__(kT) k_adj_strain(AdjArgs a, Tables T) {
     a.lam_vm[slot] = lw;
 }
 
-struct Later {
-    const float4* pd[4];
-    const float4* vm[4];
-    float c[4];
-    int n;
-};
+using Later = AdjLater;
 
-__device__ __forceinline__ float4 axpy4(float c, float4 x, float4 y) {
-    return make_float4(y.x + c * x.x, y.y + c * x.y, y.z + c * x.z, y.w + c * x.w);
+// lam_n = lam_{n+1} + sum_s lam_{Y_s} of one Runge-Kutta step, in caller order
+// (slot i holds caller id orig[i]), in place.
+__global__ void k_adj_finish(uint32_t n, const uint32_t* orig, float4* lc_p, float4* lc_v, Later L) {
+    step_begin();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t c = orig[i];
+    float4 p = lc_p[c], v = lc_v[c];
+    for (int t = 0; t < L.n; ++t) {
+        p = axpy4(1.0f, L.pd[t][i], p);
+        v = axpy4(1.0f, L.vm[t][i], v);
+    }
+    v.w = 0.0f;
+    lc_p[c] = p;
+    lc_v[c] = v;
 }
 
 __global__ void k_adj_weights(uint32_t n, float cb, const float4* __restrict__ lp, const float4* __restrict__ lv,
@@ -1129,41 +1215,45 @@ __global__ void k_adj_perm(uint32_t n, const uint32_t* __restrict__ orig, const 
 
 }  // namespace
 
+namespace {
+template <int DIM>
+void launch_adj_fluid(const AdjArgs& a, const Tables& T, cudaStream_t st) {
+    if (a.n <= kAdjFew) launch_step(k_adj_fluid<DIM, 8>, nblocks(a.n, kT / 8), kT, 0, st, a, T);
+    else launch_step(k_adj_fluid<DIM, 2>, nblocks(a.n, kT / 2), kT, 0, st, a, T);
+}
+template <int LANES>
+void launch_adj_solid(const AdjArgs& a, const Tables& T, cudaStream_t st) {
+    const uint32_t nb = nblocks(a.ns, kT / LANES);
+    if (a.st.ep) {
+        if (a.all_order2) launch_step(k_adj_solid<LANES, false, true>, nb, kT, 0, st, a, T);
+        else launch_step(k_adj_solid<LANES, true, true>, nb, kT, 0, st, a, T);
+    } else {
+        if (a.all_order2) launch_step(k_adj_solid<LANES, false, false>, nb, kT, 0, st, a, T);
+        else launch_step(k_adj_solid<LANES, true, false>, nb, kT, 0, st, a, T);
+    }
+}
+}  // namespace
+
 int launch_adjoint_stage(const AdjArgs& a, const Tables& T, int kdim, cudaStream_t st) {
     int launches = 0;
+    if (a.n == 0) return 0;
+    launch_step(k_adj_prep, nblocks(a.n + a.nb, 256), 256, 0, st, a, T);
+    ++launches;
     if (a.solid_branch && a.ns > 0) {
-        const uint32_t nb = nblocks(a.ns * kAdjSolidLanes, kT);
-        if (a.st.ep) {
-            if (a.all_order2) k_adj_solid<kAdjSolidLanes, false, true><<<nb, kT, 0, st>>>(a, T);
-            else k_adj_solid<kAdjSolidLanes, true, true><<<nb, kT, 0, st>>>(a, T);
-        } else {
-            if (a.all_order2) k_adj_solid<kAdjSolidLanes, false, false><<<nb, kT, 0, st>>>(a, T);
-            else k_adj_solid<kAdjSolidLanes, true, false><<<nb, kT, 0, st>>>(a, T);
-        }
-        k_adj_strain<<<nblocks(a.ns, kT), kT, 0, st>>>(a, T);
+        if (a.ns <= kAdjFewSolids) launch_adj_solid<8>(a, T, st);
+        else launch_adj_solid<2>(a, T, st);
+        launch_step(k_adj_strain<kAdjStrainLanes>, nblocks(a.ns, kT / kAdjStrainLanes), kT, 0, st, a, T);
         launches += 2;
     }
-    if (a.n > 0) {
-        k_adj_prep<<<nblocks(a.n, 256), 256, 0, st>>>(a, T, a.w, a.eq);
-        if (kdim == 2) k_adj_fluid<2><<<nblocks(a.n, kT), kT, 0, st>>>(a, T, a.w, a.eq);
-        else k_adj_fluid<3><<<nblocks(a.n, kT), kT, 0, st>>>(a, T, a.w, a.eq);
-        launches += 2;
-    }
-    return launches;
+    if (kdim == 2) launch_adj_fluid<2>(a, T, st);
+    else launch_adj_fluid<3>(a, T, st);
+    return launches + 1;
 }
 
-int adjoint_stage_weights(uint32_t n, float cb, const float4* lam_pd, const float4* lam_vm, int nlater,
-                          const float* ca, const float4* const* lamY_pd, const float4* const* lamY_vm,
-                          float4* mu_pd, float4* mu_vm, cudaStream_t st) {
+int adjoint_step_finish(uint32_t n, const uint32_t* orig, float4* lc_p, float4* lc_v, const AdjLater& L,
+                        cudaStream_t st) {
     if (n == 0) return 0;
-    Later L{};
-    L.n = nlater < 4 ? nlater : 4;
-    for (int t = 0; t < L.n; ++t) {
-        L.pd[t] = lamY_pd[t];
-        L.vm[t] = lamY_vm[t];
-        L.c[t] = ca[t];
-    }
-    k_adj_weights<<<nblocks(n, 256), 256, 0, st>>>(n, cb, lam_pd, lam_vm, L, mu_pd, mu_vm);
+    launch_step(k_adj_finish, nblocks(n, 256), 256, 0, st, n, orig, lc_p, lc_v, L);
     return 1;
 }
 

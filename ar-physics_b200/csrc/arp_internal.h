@@ -408,13 +408,28 @@ struct AdjStage {
     const uint32_t* contact_bound;  // [2] self-contact gate of the stage
     const float4* ep;          // [4*ns] plastic strain of the stage (columns), null without plastic materials
 };
+// Later stages' adjoints (storage order) and their weights.
+struct AdjLater {
+    const float4* pd[4];
+    const float4* vm[4];
+    float c[4];
+    int n;
+};
 struct AdjArgs {
     AdjStage st;
+    // Runge-Kutta: mu = cb lam_{n+1} + sum_t later.c[t] later[t], with lam_{n+1}
+    // in caller order (lc_p, lc_v; orig[slot] = caller id), is formed by the
+    // stage's first kernel; with lc_p null, mu_pd / mu_vm hold it already.
+    const float4* lc_p;
+    const float4* lc_v;
+    const uint32_t* orig;
+    float cb;
+    AdjLater later;
     const uint32_t* sid;       // slot -> solid id
     const uint32_t* slot_of;   // solid id -> slot
     const float4* mu_pd;       // adjoint of the stage derivative k_s, storage order: (x, y, z, rho)
     const float4* mu_vm;       // (vx, vy, vz, 0)
-    float4* lam_pd;            // adjoint of the stage state Y_s (accumulated)
+    float4* lam_pd;            // adjoint of the stage state Y_s (written)
     float4* lam_vm;
     const float4* bxs;         // boundary, cell order
     const float4* bvs;
@@ -424,14 +439,16 @@ struct AdjArgs {
     const float4* L;
     SolidRefList rl;
     const float2* stiff;       // per-solid stiffness override or null
-    float4* lamF;              // [3*ns] adjoint of F (columns), scratch
-    float4* lamFd;             // [3*ns] adjoint of dF/dt
+    float4* lamM;              // [6*ns] scratch: adjoints of F and dF/dt, each times L, as stress records
+    float4* sw;                // [2*ns] scratch: velocity, mu_v / rho of each solid
     double2* g_stiff;          // [ns] accumulated dL/d(normal, shear) stiffness
     uint32_t* flags;           // bit 0: an active self-contact pair (not differentiated)
-    float4* w;                 // [n] scratch: per-particle weights of the stage
-    float4* eq;                // [n] scratch: per-particle state-equation terms
-    float4* xs;                // [n] scratch: the stage positions in cell order
-    uint32_t n, ns;
+    // scratch: the stage's mobile particles in cell order, then the boundary
+    float4* rec;               // [4 (n + nb)]: position, density; velocity, id bits; weights (mu_v / rho, mu_rho);
+                               // (p / rho^2, its derivative in rho, 1 / rho, mu_x.x) -- see k_adj_prep
+    float4* mux;               // [n] position part of mu
+    uint32_t* code;            // [n + nb] quantised positions, readable kScanPad entries past the end
+    uint32_t n, nb, ns;
     int solid_branch;
     int all_order2;            // every solid material has strain order 2
     const float4* mu_ep;       // [4*ns] adjoint of the stage's plastic-strain rate (columns), or null
@@ -454,10 +471,9 @@ int verlet_adjoint_weights(uint32_t n, const float4* lsp, const float4* lsv, con
                            float h, float4* mp, float4* mv, cudaStream_t st);
 int verlet_kick_drift_adjoint(uint32_t n, float4* lp, float4* lv, float h, float dt, float4* lfp, float4* lfv,
                               cudaStream_t st);
-// mu = cb * lam_next + sum_t ca[t] * lamY[t] over the given later stages.
-int adjoint_stage_weights(uint32_t n, float cb, const float4* lam_pd, const float4* lam_vm, int nlater,
-                          const float* ca, const float4* const* lamY_pd, const float4* const* lamY_vm,
-                          float4* mu_pd, float4* mu_vm, cudaStream_t st);
+// lam_n = lam_{n+1} + sum_s lam_{Y_s} in caller order, in place.
+int adjoint_step_finish(uint32_t n, const uint32_t* orig, float4* lc_p, float4* lc_v, const AdjLater& L,
+                        cudaStream_t st);
 // lam_out = lam_next + sum_s lamY[s]
 int adjoint_step_sum(uint32_t n, const float4* lam_pd, const float4* lam_vm, int stages,
                      const float4* const* lamY_pd, const float4* const* lamY_vm, float4* out_pd, float4* out_vm,

@@ -26,7 +26,7 @@
 // order the oracle uses.
 #include <algorithm>
 
-#include "grid.cuh"
+#include "group_scan.cuh"
 #include "launch.cuh"
 #include "warp.cuh"
 
@@ -344,36 +344,6 @@ __device__ __forceinline__ const SceneP& init_self(uint32_t k, const FluidArgs& 
     return P;
 }
 
-// The rows of search cells around a particle: row q (ascending z, then y; the
-// order of for_search_rows) spans `width` cells from search_row(q) on.
-struct SearchRows {
-    int y, z, x0, ry, nrows;
-    uint32_t width;
-};
-template <int DIM>
-__device__ __forceinline__ SearchRows search_rows(float4 x, bool scan, const SceneP& P) {
-    constexpr int RZ = 1 + (int)(kSearchHalve >> 2 & 1u);
-    const Grid& g = P.sgrid;
-    const CellCoord c = scan ? cell_coord(x, g) : CellCoord{0, 0, 0};
-    const int rx = 1 + (int)P.halved[0];
-    SearchRows r;
-    r.ry = 1 + (int)P.halved[1];
-    r.y = c.y - r.ry;
-    r.z = DIM == 3 ? c.z - RZ : c.z;
-    r.x0 = max(c.x - rx, 0);
-    r.width = (uint32_t)(min(c.x + rx, (int)g.sub[0] - 1) - r.x0) + 1u;
-    r.nrows = scan ? (2 * r.ry + 1) * (DIM == 3 ? 2 * RZ + 1 : 1) : 0;
-    return r;
-}
-// First cell of row q, or kInvalid outside the grid.
-__device__ __forceinline__ uint32_t search_row(const SearchRows& r, int q, const SceneP& P) {
-    const int qz = r.ry == 1 ? q / 3 : q / 5;
-    const int y = r.y + q - qz * (2 * r.ry + 1), z = r.z + qz;
-    const Grid& g = P.sgrid;
-    if (y < 0 || y >= (int)g.sub[1] || z < 0 || z >= (int)g.sub[2]) return kInvalid;
-    return P.cell_base + (uint32_t)r.x0 + (uint32_t)y * g.sub[0] + (uint32_t)z * g.sub[0] * g.sub[1];
-}
-
 // How the terms of a particle's hits are added up, in every form: hit e of the
 // candidate order goes to partial sum e mod 4, each partial sum adds its hits
 // in order, and the total is (p0 + p1) + (p2 + p3); contact terms likewise in
@@ -643,36 +613,23 @@ __global__ void __launch_bounds__(BLOCK, kBlocksPerSM * 128 / BLOCK) k_fluid(Flu
 // Bound: the latency of the chain of dependent loads of one particle, and whether
 // all blocks are resident at once: 8 blocks per SM with 16 lanes (16.5 us for 9,072
 // particles, 18.9 with 7), 7 with 4 and 8 (35.5 us for 32,256, 37 with 8, 42 with 6).
-//   * The bounds of all search rows are read at once, one row per lane, and
-//     turned into a list of non-empty segments of consecutive candidates
-//     (boundary, then mobile, row by row: the candidate order of the block
-//     form), so the scan is one flat loop with U loads in flight per lane.
-//   * Hits are compacted in candidate order by ballots into the particle's list
-//     in shared memory; when a list of the warp could fill up, the warp
-//     evaluates whole rounds of LANES hits of each and goes on.
+//   * Candidates are scanned and hits listed by the lanes together (GroupScan).
 //   * Each lane evaluates one hit at a time; with more than four lanes the terms
 //     go through shared memory to the lanes that hold the partial sums (partial
 //     sum lane mod 4, 16 / LANES components each).
-constexpr int kGroupList = 96;   // list entries per particle
 constexpr int kGroupBlock = 128;
 
 template <int DIM, int LANES>
 __global__ void __launch_bounds__(kGroupBlock, LANES == 16 ? 8 : 7) k_fluid_group(FluidArgs a, Tables T, StageCoefs c, StageBuffers b) {
     constexpr int NG = kGroupBlock / LANES;       // particles per block
-    constexpr int U = LANES >= 16 ? 2 : 4;        // candidate loads in flight per lane
-    constexpr int RZ = 1 + (int)(kSearchHalve >> 2 & 1u);
-    constexpr int MAXROWS = 5 * (DIM == 3 ? 2 * RZ + 1 : 1);
     constexpr int CPL = 16 / LANES;               // components of the partial sum a lane holds
     static_assert(LANES == 4 || LANES == 8 || LANES == 16, "four partial sums of four components over the lanes");
-    static_assert(kGroupList >= 2 * U * LANES, "the list holds what one scan iteration can add");
     __shared__ uint32_t s_list[NG][kGroupList];
-    __shared__ uint2 s_seg[NG][2 * MAXROWS];      // (end, first index - first number) of each segment
+    __shared__ uint2 s_seg[NG][2 * GroupScan<DIM, LANES>::MAXROWS];
     __shared__ float4 s_term[LANES > 4 ? NG : 1][LANES];
     constexpr unsigned FULL = 0xFFFFFFFFu;
-    constexpr unsigned GM = (1u << LANES) - 1u;
     step_begin();
     const uint32_t lane = threadIdx.x % LANES, gi = threadIdx.x / LANES;
-    const uint32_t gshift = (threadIdx.x & 31u) & ~(uint32_t)(LANES - 1);
     const uint32_t kk = blockIdx.x * NG + gi;
     const bool valid = kk < a.n;
     const uint32_t k = valid ? kk : a.n - 1u;  // idle groups of the last block follow the last particle, without candidates
@@ -680,44 +637,7 @@ __global__ void __launch_bounds__(kGroupBlock, LANES == 16 ? 8 : 7) k_fluid_grou
     const SceneP& P = init_self(k, a, T, nullptr, kInvalid, s);
     const float4 xi = make_float4(s.x.x, s.x.y, s.x.z, 0.0f);
     const PairK K{P.h2, -6.0f * P.kconst, P.eps_hh};
-    const uint32_t own = own_code(xi, P);
     uint32_t* const list = s_list[gi];
-    uint2* const seg = s_seg[gi];
-
-    // segments of candidates, numbered 0 .. total over all rows
-    uint32_t total = 0, nseg = 0;
-    {
-        const SearchRows rows = search_rows<DIM>(xi, valid && finite3(xi), P);
-#pragma unroll
-        for (int q0 = 0; q0 < MAXROWS; q0 += LANES) {
-            const int q = q0 + (int)lane;
-            const uint32_t c0 = q < rows.nrows ? search_row(rows, q, P) : kInvalid;
-            uint32_t bb = 0, lb = 0, jb = 0, lm = 0;
-            if (c0 != kInvalid) {
-                const uint32_t c1 = c0 + rows.width;
-                bb = a.bstart[c0];
-                lb = a.bstart[c1] - bb;
-                jb = a.start[c0];
-                lm = a.start[c1] - jb;
-            }
-            uint32_t len = lb + lm, cnt = (lb ? 1u : 0u) + (lm ? 1u : 0u);
-#pragma unroll
-            for (int o = 1; o < LANES; o <<= 1) {
-                const uint32_t l2 = __shfl_up_sync(FULL, len, o, LANES), c2 = __shfl_up_sync(FULL, cnt, o, LANES);
-                if ((int)lane >= o) {
-                    len += l2;
-                    cnt += c2;
-                }
-            }
-            const uint32_t first = total + len - lb - lm;
-            uint32_t w = nseg + cnt - (lb ? 1u : 0u) - (lm ? 1u : 0u);
-            if (lb) seg[w++] = make_uint2(first + lb, a.n + bb - first);
-            if (lm) seg[w] = make_uint2(first + lb + lm, jb - first - lb);
-            total += __shfl_sync(FULL, len, LANES - 1, LANES);
-            nseg += __shfl_sync(FULL, cnt, LANES - 1, LANES);
-        }
-    }
-    __syncwarp();
 
     // components (lane / 4) * CPL + i of partial sum lane mod 4: (density rate,
     // force) and (unused, contact force)
@@ -745,35 +665,8 @@ __global__ void __launch_bounds__(kGroupBlock, LANES == 16 ? 8 : 7) k_fluid_grou
         }
     };
     bool any_con = false;
-    uint32_t t0 = 0, cnt = 0, si = 0;  // candidates tested, hits listed, the lane's current segment
-    for (;;) {
-        while (__any_sync(FULL, t0 < total)) {
-            uint32_t jj[U], code[U];
-            bool in[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const uint32_t t = t0 + (uint32_t)(u * LANES) + lane;
-                in[u] = t < total;
-                jj[u] = code[u] = 0u;
-                if (in[u]) {
-                    uint2 sg = seg[si];
-                    while (t >= sg.x) sg = seg[++si];  // the last segment ends at total > t
-                    jj[u] = sg.y + t;
-                    code[u] = a.code[jj[u]];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const bool h = in[u] && code_test(code[u], own) < 0;
-                const unsigned m = __ballot_sync(FULL, h) >> gshift & GM;
-                if (h) list[cnt + __popc(m & ((1u << lane) - 1u))] = jj[u];
-                cnt += __popc(m);
-            }
-            t0 += U * LANES;
-            if (__any_sync(FULL, cnt > (uint32_t)(kGroupList - U * LANES))) break;
-        }
-        __syncwarp();
-        const uint32_t ev = t0 < total ? cnt & ~(uint32_t)(LANES - 1) : cnt;
+    GroupScan<DIM, LANES>::run(xi, valid && finite3(xi), P, ScanArrays{a.code, a.start, a.bstart, a.n}, list, s_seg[gi],
+                               [&](uint32_t ev) {
         uint32_t bits = 0;
 #pragma unroll 1
         for (uint32_t e0 = 0; __any_sync(FULL, e0 < ev); e0 += LANES) {
@@ -800,13 +693,7 @@ __global__ void __launch_bounds__(kGroupBlock, LANES == 16 ? 8 : 7) k_fluid_grou
                 add(con, make_float4(0.f, t.c.x, t.c.y, t.c.z));
             }
         }
-        if (!__any_sync(FULL, t0 < total)) break;
-        const uint32_t rest = cnt - ev;  // fewer than LANES
-        const uint32_t keep = lane < rest ? list[ev + lane] : 0u;
-        __syncwarp();
-        if (lane < rest) list[lane] = keep;
-        cnt = rest;
-    }
+    });
 #pragma unroll
     for (int i = 0; i < CPL; ++i) {
         acc[i] = sum_partials(acc[i]);

@@ -173,10 +173,12 @@ struct Tape {
 struct AdjointPool {
     std::vector<StepRecord> recs;       // one segment of recording steps
     std::vector<Checkpoint> spare;      // checkpoints of ended tapes, reused
-    DevBuf<float4> lc_p, lc_v, ls_p, ls_v, out_p, out_v, mu_p, mu_v, w, e, xs;
+    DevBuf<float4> lc_p, lc_v, ls_p, ls_v, out_p, out_v, mu_p, mu_v;
     DevBuf<float4> io;  // [2n] the caller's 8-float-per-particle gradients, on the device
     DevBuf<float4> lY_p[kMaxStages], lY_v[kMaxStages];
-    DevBuf<float4> lamF, lamFd;
+    DevBuf<float4> rec, mux;  // a stage's particles in cell order
+    DevBuf<uint32_t> code;
+    DevBuf<float4> lamM, sw;  // solid order
     DevBuf<float4> lam_ep, out_ep, mu_ep, lY_ep[kMaxStages];  // adjoint of the plastic strain (solid order)
     DevBuf<double2> gst;
     DevBuf<uint32_t> flags;
@@ -2330,14 +2332,16 @@ arp_status arp_tape_backward(arp_sim* sim, const float* dl_dstate, float* grad_s
     const size_t nn = std::max(n, 1u);
     auto fit = [](auto& b, size_t count) -> cudaError_t { return b.n >= count ? cudaSuccess : b.alloc(count); };
     for (DevBuf<float4>* b :
-         {&P.lc_p, &P.lc_v, &P.ls_p, &P.ls_v, &P.out_p, &P.out_v, &P.mu_p, &P.mu_v, &P.w, &P.e, &P.xs})
+         {&P.lc_p, &P.lc_v, &P.ls_p, &P.ls_v, &P.out_p, &P.out_v, &P.mu_p, &P.mu_v, &P.mux})
         CUDA_TRY(fit(*b, nn));
     for (int q = 0; q < S; ++q) {
         CUDA_TRY(fit(P.lY_p[q], nn));
         CUDA_TRY(fit(P.lY_v[q], nn));
     }
-    CUDA_TRY(fit(P.lamF, 3 * size_t(std::max(ns, 1u))));
-    CUDA_TRY(fit(P.lamFd, 3 * size_t(std::max(ns, 1u))));
+    CUDA_TRY(fit(P.rec, 4 * (nn + sim->nb)));
+    CUDA_TRY(fit(P.code, nn + sim->nb + kScanPad));
+    CUDA_TRY(fit(P.lamM, 6 * size_t(std::max(ns, 1u))));
+    CUDA_TRY(fit(P.sw, 2 * size_t(std::max(ns, 1u))));
     CUDA_TRY(fit(P.gst, std::max(ns, 1u)));
     const bool plastic = sim->any_plastic && sim->solid_branch() && ns > 0;
     const size_t ne = 4 * size_t(std::max(ns, 1u));
@@ -2349,7 +2353,7 @@ arp_status arp_tape_backward(arp_sim* sim, const float* dl_dstate, float* grad_s
     CUDA_TRY(fit(P.flags, 1));
     CUDA_TRY(fit(P.io, 2 * nn));
     DevBuf<float4>&lc_p = P.lc_p, &lc_v = P.lc_v, &ls_p = P.ls_p, &ls_v = P.ls_v, &out_p = P.out_p,
-                  &out_v = P.out_v, &mu_p = P.mu_p, &mu_v = P.mu_v, &lamF = P.lamF, &lamFd = P.lamFd;
+                  &out_v = P.out_v, &mu_p = P.mu_p, &mu_v = P.mu_v;
     DevBuf<float4>* lY_p = P.lY_p;
     DevBuf<float4>* lY_v = P.lY_v;
     DevBuf<double2>& gst = P.gst;
@@ -2360,10 +2364,18 @@ arp_status arp_tape_backward(arp_sim* sim, const float* dl_dstate, float* grad_s
         CUDA_TRY(cudaMemcpyAsync(P.io.p, dl_dstate, n * 2 * sizeof(float4), cudaMemcpyHostToDevice, st));
         sim->launches += adjoint_unpack(n, P.io.p, lc_p.p, lc_v.p, st);
     }
-    // lam_Y += J_f(Y)^T mu for stage q of a recorded step
-    auto stage_vjp = [&](const StepRecord& R, int q, const float4* mup, const float4* muv, float4* lyp, float4* lyv,
-                         const float4* muep, float4* lyep) {
+    // lam_Y = J_f(Y)^T mu for stage q of a recorded step; mu is given (mup, muv) or, with
+    // mup null, formed from the step's adjoint in caller order and the later stages'
+    auto stage_vjp = [&](const StepRecord& R, int q, const float4* mup, const float4* muv, float cb,
+                         const AdjLater& later, float4* lyp, float4* lyv, const float4* muep, float4* lyep) {
         AdjArgs a{};
+        if (!mup) {
+            a.lc_p = lc_p.p;
+            a.lc_v = lc_v.p;
+            a.orig = R.orig.p;
+            a.cb = cb;
+            a.later = later;
+        }
         a.st.pd = R.pd[q].p;
         a.st.vm = R.vm[q].p;
         a.st.perm = R.has_perm[q] ? R.perm[q].p : nullptr;
@@ -2387,14 +2399,15 @@ arp_status arp_tape_backward(arp_sim* sim, const float* dl_dstate, float* grad_s
         a.L = sim->L.p;
         a.rl = SolidRefList{sim->rl_off.p, sim->rl_nbr.p, sim->rl_gw.p, sim->rl_nnz};
         a.stiff = sim->have_stiff ? sim->stiff.p : nullptr;
-        a.lamF = lamF.p;
-        a.lamFd = lamFd.p;
+        a.lamM = P.lamM.p;
+        a.sw = P.sw.p;
         a.g_stiff = gst.p;
         a.flags = flags.p;
-        a.w = P.w.p;
-        a.eq = P.e.p;
-        a.xs = P.xs.p;
+        a.rec = P.rec.p;
+        a.mux = P.mux.p;
+        a.code = P.code.p;
         a.n = n;
+        a.nb = sim->nb;
         a.ns = ns;
         a.solid_branch = sb ? 1 : 0;
         a.all_order2 = sim->all_order2 ? 1 : 0;
@@ -2432,11 +2445,7 @@ arp_status arp_tape_backward(arp_sim* sim, const float* dl_dstate, float* grad_s
             sim->launches += adjoint_stage_weights_all(4 * ns, vh, P.lam_ep.p, 1, &one, lfe, P.mu_ep.p, st);
             CUDA_TRY(cudaMemsetAsync(P.lY_ep[0].p, 0, 4 * size_t(ns) * sizeof(float4), st));
         }
-        if (n) {
-            CUDA_TRY(cudaMemsetAsync(lY_p[0].p, 0, n * sizeof(float4), st));
-            CUDA_TRY(cudaMemsetAsync(lY_v[0].p, 0, n * sizeof(float4), st));
-        }
-        stage_vjp(R, 0, mu_p.p, mu_v.p, lY_p[0].p, lY_v[0].p, P.mu_ep.p, P.lY_ep[0].p);
+        stage_vjp(R, 0, mu_p.p, mu_v.p, 0.0f, AdjLater{}, lY_p[0].p, lY_v[0].p, P.mu_ep.p, P.lY_ep[0].p);
         const float4* yp[1] = {lY_p[0].p};
         const float4* yv[1] = {lY_v[0].p};
         sim->launches += adjoint_step_sum(n, ls_p.p, ls_v.p, 1, yp, yv, out_p.p, out_v.p, st);
@@ -2453,12 +2462,8 @@ arp_status arp_tape_backward(arp_sim* sim, const float* dl_dstate, float* grad_s
         // position part is zero), in the storage order of that evaluation
         const StepRecord& R0 = P.prime;
         sim->launches += adjoint_gather(n, R0.orig.p, P.lf_p.p, P.lf_v.p, mu_p.p, mu_v.p, st);
-        if (n) {
-            CUDA_TRY(cudaMemsetAsync(lY_p[0].p, 0, n * sizeof(float4), st));
-            CUDA_TRY(cudaMemsetAsync(lY_v[0].p, 0, n * sizeof(float4), st));
-        }
         if (plastic) CUDA_TRY(cudaMemsetAsync(P.lY_ep[0].p, 0, 4 * size_t(ns) * sizeof(float4), st));
-        stage_vjp(R0, 0, mu_p.p, mu_v.p, lY_p[0].p, lY_v[0].p, P.lf_ep.p, P.lY_ep[0].p);
+        stage_vjp(R0, 0, mu_p.p, mu_v.p, 0.0f, AdjLater{}, lY_p[0].p, lY_v[0].p, P.lf_ep.p, P.lY_ep[0].p);
         sim->launches += adjoint_scatter(n, R0.orig.p, lY_p[0].p, lY_v[0].p, out_p.p, out_v.p, st);
         const float4* op[1] = {out_p.p};
         const float4* ov[1] = {out_v.p};
@@ -2491,49 +2496,40 @@ arp_status arp_tape_backward(arp_sim* sim, const float* dl_dstate, float* grad_s
                 status = verlet_step_vjp(R, t == 0 && P.prime_recorded);
                 continue;
             }
-            sim->launches += adjoint_gather(n, R.orig.p, lc_p.p, lc_v.p, ls_p.p, ls_v.p, st);
+            static_assert(kMaxStages <= 4, "AdjLater");
             for (int q = S - 1; q >= 0; --q) {
-                float ca[kMaxStages];
-                const float4* lp[kMaxStages];
-                const float4* lv[kMaxStages];
-                int nl = 0;
+                AdjLater later{};
                 for (int u = q + 1; u < S; ++u)
                     if (sim->tab.a[u][q] != 0.0) {
-                        ca[nl] = (float)(sim->tab.a[u][q] * (double)sim->dt_sub);
-                        lp[nl] = lY_p[u].p;
-                        lv[nl] = lY_v[u].p;
-                        ++nl;
+                        later.c[later.n] = (float)(sim->tab.a[u][q] * (double)sim->dt_sub);
+                        later.pd[later.n] = lY_p[u].p;
+                        later.vm[later.n] = lY_v[u].p;
+                        ++later.n;
                     }
                 const float cb = (float)(sim->tab.b[q] * (double)sim->dt_sub);
-                sim->launches += adjoint_stage_weights(n, cb, ls_p.p, ls_v.p, nl, ca, lp, lv, mu_p.p, mu_v.p, st);
                 if (plastic) {  // the same weights for the plastic strain's record
                     const float4* le[kMaxStages];
                     int ne_later = 0;
                     for (int u = q + 1; u < S; ++u)
                         if (sim->tab.a[u][q] != 0.0) le[ne_later++] = P.lY_ep[u].p;
-                    sim->launches += adjoint_stage_weights_all(4 * ns, cb, P.lam_ep.p, ne_later, ca, le, P.mu_ep.p, st);
+                    sim->launches += adjoint_stage_weights_all(4 * ns, cb, P.lam_ep.p, ne_later, later.c, le, P.mu_ep.p, st);
                     CUDA_TRY(cudaMemsetAsync(P.lY_ep[q].p, 0, 4 * size_t(ns) * sizeof(float4), st));
                 }
-                if (n) {
-                    cudaMemsetAsync(lY_p[q].p, 0, n * sizeof(float4), st);
-                    cudaMemsetAsync(lY_v[q].p, 0, n * sizeof(float4), st);
-                }
-                stage_vjp(R, q, mu_p.p, mu_v.p, lY_p[q].p, lY_v[q].p, P.mu_ep.p, P.lY_ep[q].p);
+                stage_vjp(R, q, nullptr, nullptr, cb, later, lY_p[q].p, lY_v[q].p, P.mu_ep.p, P.lY_ep[q].p);
             }
-            const float4* yp[kMaxStages];
-            const float4* yv[kMaxStages];
+            AdjLater all{};
+            all.n = S;
             for (int q = 0; q < S; ++q) {
-                yp[q] = lY_p[q].p;
-                yv[q] = lY_v[q].p;
+                all.pd[q] = lY_p[q].p;
+                all.vm[q] = lY_v[q].p;
             }
-            sim->launches += adjoint_step_sum(n, ls_p.p, ls_v.p, S, yp, yv, out_p.p, out_v.p, st);
+            sim->launches += adjoint_step_finish(n, R.orig.p, lc_p.p, lc_v.p, all, st);
             if (plastic) {
                 const float4* ye[kMaxStages];
                 for (int q = 0; q < S; ++q) ye[q] = P.lY_ep[q].p;
                 sim->launches += adjoint_step_sum_all(4 * ns, P.lam_ep.p, S, ye, P.out_ep.p, st);
                 std::swap(P.lam_ep, P.out_ep);
             }
-            sim->launches += adjoint_scatter(n, R.orig.p, out_p.p, out_v.p, lc_p.p, lc_v.p, st);
         }
         if (status == ARP_OK) {
             cudaError_t e = cudaStreamSynchronize(st);
