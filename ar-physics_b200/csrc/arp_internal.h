@@ -372,6 +372,7 @@ struct RenderCfg {
     float ca, sa, tx, ty, tz;      // view matrix terms
     float render_h;
     float kconst;                  // poly6 constant the fragment shader weighs alpha with
+    float kinv_hi, kinv_lo;        // 1 / kconst in two floats
     int lighting;
     float light[3], lcol[3], amb, dif, spec;
     const float4* c1;              // per material: low-density colour
@@ -390,8 +391,9 @@ uint32_t render_tile_size();
 int render_bin_count(const float4* PR, const float4* PC, const RenderCfg& c, uint32_t* counts, cudaStream_t st);
 int render_bin_scatter(const float4* PR, const float4* PC, const RenderCfg& c, const uint32_t* start,
                        uint32_t* fill, uint32_t* list, cudaStream_t st);
-int render_composite(const float4* PR, const float4* PC, const RenderCfg& c, const uint32_t* start,
-                     const uint32_t* list, uint8_t* rgb, cudaStream_t st);
+// sorts the bins' ids (list) by draw order, then composites
+int render_composite(const float4* PR, const float4* PC, const RenderCfg& c, const uint32_t* start, uint32_t* list,
+                     uint8_t* rgb, cudaStream_t st);
 int render_lit(const float4* PR, const float4* PC, const float4* PP, const RenderCfg& c, unsigned long long* zkey,
                uint8_t* rgb, cudaStream_t st);
 

@@ -301,7 +301,7 @@ struct arp_sim {
     struct RenderBufs {
         DevBuf<float4> PR, PC, PP, c1, c2, c3;
         DevBuf<float> d0;
-        DevBuf<uint32_t> counts, start, fill, list, bsums;
+        DevBuf<uint32_t> counts, start, list, bsums;
         DevBuf<unsigned long long> zkey;
         DevBuf<uint8_t> rgb;
     } rbuf;
@@ -2182,6 +2182,8 @@ arp_status arp_sim_render_rgb24(arp_sim* sim, const arp_view* view, const arp_re
     c.tz = -view->scale + 1.0f;
     c.render_h = style->render_h;
     c.kconst = norm_const_f32(3, 3.0f);  // normalization_constant(3, 3) in the fragment shader
+    c.kinv_hi = 1.0f / c.kconst;
+    c.kinv_lo = (float)(1.0 / (double)c.kconst - (double)c.kinv_hi);
     c.lighting = style->lighting ? 1 : 0;
     for (int k = 0; k < 3; ++k) {
         c.light[k] = style->light_pos[k];
@@ -2231,17 +2233,15 @@ arp_status arp_sim_render_rgb24(arp_sim* sim, const arp_view* view, const arp_re
         if (K + 1 > (1ull << 31)) return fail(ARP_ERR_UNSUPPORTED, "too many sprite bins for this frame size");
         CUDA_TRY(fit(R.counts, K + 1));
         CUDA_TRY(fit(R.start, K + 1));
-        CUDA_TRY(fit(R.fill, K + 1));
         CUDA_TRY(fit(R.bsums, scan_block_sums_needed((uint32_t)(K + 1))));
         CUDA_TRY(cudaMemsetAsync(R.counts.p, 0, (K + 1) * sizeof(uint32_t), st));
-        CUDA_TRY(cudaMemsetAsync(R.fill.p, 0, (K + 1) * sizeof(uint32_t), st));
         sim->launches += render_bin_count(R.PR.p, R.PC.p, c, R.counts.p, st);
-        sim->launches += exclusive_scan(R.counts.p, (uint32_t)(K + 1), R.start.p, R.bsums.p, st);
+        sim->launches += exclusive_scan(R.counts.p, (uint32_t)(K + 1), R.start.p, R.bsums.p, st);  // clears the counts
         uint32_t total = 0;
         CUDA_TRY(cudaMemcpyAsync(&total, R.start.p + K, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
         CUDA_TRY(fit(R.list, std::max(total, 1u)));
-        sim->launches += render_bin_scatter(R.PR.p, R.PC.p, c, R.start.p, R.fill.p, R.list.p, st);
+        sim->launches += render_bin_scatter(R.PR.p, R.PC.p, c, R.start.p, R.counts.p, R.list.p, st);
         sim->launches += render_composite(R.PR.p, R.PC.p, c, R.start.p, R.list.p, R.rgb.p, st);
     } else {
         CUDA_TRY(fit(R.zkey, (size_t)width * height));
