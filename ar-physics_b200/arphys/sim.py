@@ -300,7 +300,7 @@ class FluidSim:
         st.n_materials = len(colors)
         st.colors = ptr(colors)
         st.densities = ptr(dens)
-        out = np.zeros((height, width, 3), np.uint8)
+        out = np.empty((height, width, 3), np.uint8)  # every pixel is written
         check(self._L.arp_sim_render_rgb24(self._h, ctypes.byref(v), ctypes.byref(st), int(width), int(height),
                                            ptr(out)))
         return out
