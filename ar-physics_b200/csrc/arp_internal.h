@@ -164,6 +164,7 @@ struct StageCoefs {
     float c_acc;        // b[stage] * dt
     int acc_first;      // 1 when no earlier stage contributed to acc
     int kick;           // 1: a velocity-Verlet kick, which leaves positions as they are
+    float half, full;   // velocity Verlet: dt / 2 and dt of the next step's kick and drift
 };
 
 struct StageBuffers {
@@ -181,7 +182,9 @@ struct StageBuffers {
     const float4* prev1_vm;
     const float4* prev2_pd;
     const float4* prev2_vm;
-    CellBins bin;            // where the next state is counted into cells (count null: it is not)
+    float4* drift_pd;        // velocity Verlet: the next step's kicked and drifted state (null: not formed)
+    float4* drift_vm;
+    CellBins bin;            // where the next (or the drifted) state is counted into cells (count null: it is not)
 };
 
 // Record `msg` as the calling thread's last error and return `code`.
@@ -214,6 +217,8 @@ struct GridBuffers {
 inline CellBins cell_bins(const GridBuffers& gb) { return CellBins{gb.key, gb.rank, gb.count, gb.coord}; }
 int bin_cells(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
               GridBuffers& gb, uint32_t* zero2, cudaStream_t st);
+// clears the counts if a state was scattered and never ordered
+void clear_cells(const Tables& T, GridBuffers& gb, cudaStream_t st);
 int scatter_cells(uint32_t n, const Tables& T, GridBuffers& gb, uint32_t* zero2, cudaStream_t st);
 int order_cells(const Tables& T, GridBuffers& gb, cudaStream_t st);
 int build_grid(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
@@ -343,6 +348,7 @@ struct SolidArgs {
     float4* ep_next;          // stage / step output
     float4* ep_acc;
     float4* ep_store;         // k of this stage, or null
+    float4* ep_kick;          // velocity Verlet: the next step's kicked plastic strain, or null (may be ep0)
     const float4* ep_prev0;   // stored k_0, k_1, k_2
     const float4* ep_prev1;
     const float4* ep_prev2;

@@ -239,11 +239,24 @@ __device__ __forceinline__ void add_hit_contact(Acc& acc, uint32_t j, const Self
     add_contact(acc, contact_terms<DIM>(s, g, rj.x.w, m.mass, mat2, rubs, it[mat2]));
 }
 
+// Velocity Verlet, first half of a step (kick, then drift): v' = v + (dt/2) a,
+// rho' = rho + (dt/2) drho/dt, x' = x + dt v', with (a, drho/dt) the derivative
+// record of the state (its position part is not used).  Each sum is formed as
+// y + (0 + c k), the order of the stage epilogue.
+__device__ __forceinline__ float4 kick_drift(float4 p, float4 v, float4 fp, float4 fv, float half, float full,
+                                             float4& vh) {
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    vh = comb(v, axpy(half, fv, z), true);  // w holds the material bits
+    const float rho = __fadd_rn(p.w, __fadd_rn(0.0f, __fmul_rn(half, fp.w)));
+    const float4 dx = axpy(full, make_float4(vh.x, vh.y, vh.z, 0.0f), z);
+    return make_float4(__fadd_rn(p.x, dx.x), __fadd_rn(p.y, dx.y), __fadd_rn(p.z, dx.z), rho);
+}
+
 // The derivative record of one particle (fluid.rs:243-247, plus the solid
 // term when active) and the Runge-Kutta stage epilogue: the store of k, the
 // b-weighted accumulator and the next stage state of sorted particle k, in its
-// storage slot.  With b.bin.count the new state is counted into its search
-// cell on the way (the first pass of the grid build that follows, which then
+// storage slot.  With b.drift_pd the next velocity-Verlet step's kick and drift
+// follow.  With b.bin.count the new state is counted into its search cell on the way (the first pass of the grid build that follows, which then
 // need not read the positions again).
 __device__ __forceinline__ void stage_epilogue(const FluidArgs& a, const Tables& T, const StageCoefs& c,
                                                const StageBuffers& b, uint32_t k, const Acc& acc) {
@@ -291,7 +304,7 @@ __device__ __forceinline__ void stage_epilogue(const FluidArgs& a, const Tables&
         accp = b.acc_pd[slot];
         accv = b.acc_vm[slot];
     }
-    float4 np;
+    float4 np, nv;
     if (c.last) {
         np = comb(y0p, accp, false);
         if (c.kick) {  // a velocity-Verlet kick moves no particle: positions come from the drift
@@ -299,8 +312,7 @@ __device__ __forceinline__ void stage_epilogue(const FluidArgs& a, const Tables&
             np.y = y0p.y;
             np.z = y0p.z;
         }
-        b.next_pd[slot] = np;
-        b.next_vm[slot] = comb(y0v, accv, true);
+        nv = comb(y0v, accv, true);
     } else {
         float4 tp = make_float4(0.f, 0.f, 0.f, 0.f), tv = make_float4(0.f, 0.f, 0.f, 0.f);
         if (c.c_prev0 != 0.0f) {
@@ -320,8 +332,15 @@ __device__ __forceinline__ void stage_epilogue(const FluidArgs& a, const Tables&
             tv = axpy(c.c_self, kvm, tv);
         }
         np = comb(y0p, tp, false);
-        b.next_pd[slot] = np;
-        b.next_vm[slot] = comb(y0v, tv, true);
+        nv = comb(y0v, tv, true);
+    }
+    b.next_pd[slot] = np;
+    b.next_vm[slot] = nv;
+    if (b.drift_pd) {  // a force evaluation of its own leaves the state as it is
+        const float4 vh = c.last ? nv : y0v;
+        np = kick_drift(c.last ? np : y0p, vh, kpd, kvm, c.half, c.full, nv);
+        b.drift_pd[slot] = np;
+        b.drift_vm[slot] = nv;
     }
     if (b.bin.count) bin_particle(np, P, T.ncells, slot, b.bin);
 }
@@ -707,12 +726,10 @@ __global__ void __launch_bounds__(kGroupBlock, LANES == 16 ? 8 : 7) k_fluid_grou
     if (valid && lane == 0) stage_epilogue(a, T, c, b, k, sum);
 }
 
-// Velocity Verlet, first half of a step (kick, then drift), in storage
-// order: v' = v + (dt/2) a, rho' = rho + (dt/2) drho/dt, x' = x + dt v', with
-// (a, drho/dt) the derivative record kept from the previous force evaluation
-// (its position part is not used).  Each sum is formed as y + (0 + c k), the
-// order of the stage epilogue.  The drifted state is counted into its search
-// cells on the way.
+// The kick and drift of a state that no step has written, in storage order; the
+// drifted state is counted into its search cells on the way.  A step that ends
+// with a force evaluation forms the next one's in its epilogue: as a launch of
+// its own it cost 4 of 47 us per step of 16,899 particles.
 __global__ void k_verlet_kick_drift(const float4* pd, const float4* vm,
                                     const float4* fpd, const float4* fvm, uint32_t n,
                                     float half, float full, float4* out_pd, float4* out_vm,
@@ -720,12 +737,9 @@ __global__ void k_verlet_kick_drift(const float4* pd, const float4* vm,
     step_begin();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const float4 p = pd[k], v = vm[k], fp = fpd[k], fv = fvm[k];
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 vh = comb(v, axpy(half, fv, z), true);  // w holds the material bits
-    const float rho = __fadd_rn(p.w, __fadd_rn(0.0f, __fmul_rn(half, fp.w)));
-    const float4 dx = axpy(full, make_float4(vh.x, vh.y, vh.z, 0.0f), z);
-    const float4 np = make_float4(__fadd_rn(p.x, dx.x), __fadd_rn(p.y, dx.y), __fadd_rn(p.z, dx.z), rho);
+    const float4 v = vm[k];
+    float4 vh;
+    const float4 np = kick_drift(pd[k], v, fpd[k], fvm[k], half, full, vh);
     out_pd[k] = np;
     out_vm[k] = vh;
     bin_particle(np, T.scenes[T.mats[__float_as_uint(v.w)].scene], T.ncells, k, bin);

@@ -709,10 +709,7 @@ cudaError_t noalloc_scratch(uint32_t** out) {
 int bin_cells(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
               GridBuffers& gb, uint32_t* zero2, cudaStream_t st) {
     int launches = 0;
-    // a state that was scattered and then replaced never reached the ordering,
-    // which clears the counts
-    if (gb.scattered) cudaMemsetAsync(gb.count, 0, (size_t(T.ncells) + 2) * sizeof(uint32_t), st);
-    gb.scattered = false;
+    clear_cells(T, gb, st);
     if (n > 0) {
         // a single scene needs no material to find the scene: skip that read
         const bool one = T.nscenes == 1;
@@ -721,6 +718,13 @@ int bin_cells(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint
         ++launches;
     }
     return launches + scatter_cells(n, T, gb, zero2, st);
+}
+
+void clear_cells(const Tables& T, GridBuffers& gb, cudaStream_t st) {
+    // a state that was scattered and then replaced never reached the ordering,
+    // which clears the counts
+    if (gb.scattered) cudaMemsetAsync(gb.count, 0, (size_t(T.ncells) + 2) * sizeof(uint32_t), st);
+    gb.scattered = false;
 }
 
 int scatter_cells(uint32_t n, const Tables& T, GridBuffers& gb, uint32_t* zero2, cudaStream_t st) {

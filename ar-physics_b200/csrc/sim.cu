@@ -285,10 +285,11 @@ struct arp_sim {
     DevBuf<uint32_t> contact_bound;
     int fluid_variant = 0;
     uint32_t grid_cap = 0;
-    // gb holds the state Y counted and scattered into cells (all but the order
-    // inside them): the last stage of a Runge-Kutta step does that for the next
-    // step's grid.
-    // False whenever Y or the grid buffers have changed otherwise.
+    // gb holds the state counted and scattered into cells (all but the order
+    // inside them), as the last stage of a step leaves it for the next step: the
+    // state Y or, for velocity Verlet, the kicked and drifted one, which X holds
+    // (ep_s[0] the kicked plastic strain).  False whenever Y, X or the grid
+    // buffers have changed otherwise.
     bool binned = false;
     // solids
     DevBuf<float4> ref, L, AF, ksol;
@@ -723,6 +724,25 @@ arp_status restore_checkpoint(arp_sim* S, const Checkpoint& c) {
     return ARP_OK;
 }
 
+// Count the state into cells and scatter it, where the step before has not: the
+// current one or, for velocity Verlet's steps (not for a force evaluation at the
+// current state), the kicked and drifted one, in X, with the plastic strain's
+// kick.
+void bin_state(arp_sim* S, bool prime) {
+    uint32_t* const zero2 = S->solid_branch() ? S->contact_bound.p : nullptr;
+    if (!S->verlet() || prime) {
+        S->launches += bin_cells(S->Y.pd.p, S->Y.vm.p, nullptr, S->n, S->tables, S->gb, zero2, S->stream);
+        return;
+    }
+    const float half = (float)(S->tab.b[0] * (double)S->dt_sub);
+    clear_cells(S->tables, S->gb, S->stream);
+    S->launches += verlet_kick_drift(S->Y.pd.p, S->Y.vm.p, S->vforce.pd.p, S->vforce.vm.p, S->n, half, S->dt_sub,
+                                     S->X.pd.p, S->X.vm.p, S->tables, cell_bins(S->gb), S->stream);
+    S->launches += scatter_cells(S->n, S->tables, S->gb, zero2, S->stream);
+    if (S->solid_branch() && S->any_plastic)
+        S->launches += verlet_kick4(S->ep.p, S->ep_force.p, 4 * S->ns, half, S->ep_s[0].p, S->stream);
+}
+
 // One integrator step.  With `prime` (velocity Verlet only) it instead
 // evaluates the forces at the current state and keeps their derivative
 // record for the next step's kick, the force evaluation of the reference's
@@ -758,21 +778,17 @@ arp_status do_step(arp_sim* S, bool prime = false) {
     // 1. sort y0 into cell order
     arp_sim::Mark mk{};
     mark(S, mk, 0);
-    // a state is counted into cells where it is written: by the fluid kernel's
-    // epilogue, or by velocity Verlet's kick and drift (storage order, into X;
-    // the grid and the force evaluation then see the drifted state)
+    // a state is counted into cells where it is written, by the fluid kernel's
+    // epilogue; for velocity Verlet the kicked and drifted one (storage order, in
+    // X), which the grid and the force evaluation see
     const CellBins bins = cell_bins(S->gb);
     uint32_t* const zero2 = sb ? S->contact_bound.p : nullptr;  // cleared with each stage's sort
     const float4* src_pd = S->Y.pd.p;
     const float4* src_vm = S->Y.vm.p;
+    if (!S->binned || prime) bin_state(S, prime);
     if (verlet && !prime) {
-        S->launches += verlet_kick_drift(S->Y.pd.p, S->Y.vm.p, S->vforce.pd.p, S->vforce.vm.p, n, half, S->dt_sub,
-                                         S->X.pd.p, S->X.vm.p, S->tables, bins, st);
-        S->launches += scatter_cells(n, S->tables, S->gb, zero2, st);
         src_pd = S->X.pd.p;
         src_vm = S->X.vm.p;
-    } else if (!S->binned) {
-        S->launches += bin_cells(src_pd, src_vm, nullptr, n, S->tables, S->gb, zero2, st);
     }
     S->binned = false;
     // the stage-0 solid copies and the solid -> slot map come out of the same gather
@@ -807,10 +823,7 @@ arp_status do_step(arp_sim* S, bool prime = false) {
     const float4* cur_vm = S->Y.vm.p;
     const float4* cur_ep = S->ep.p;
     const float4* ep_base = S->ep.p;  // the step's y0 of the plastic strain
-    if (verlet && !prime && sb && S->any_plastic) {
-        S->launches += verlet_kick4(S->ep.p, S->ep_force.p, 4 * ns, half, S->ep_s[0].p, st);
-        ep_base = cur_ep = S->ep_s[0].p;
-    }
+    if (verlet && !prime && sb && S->any_plastic) ep_base = cur_ep = S->ep_s[0].p;  // kicked with the state
     for (int s = 0; s < tab.stages; ++s) {
         const bool last = !prime && s == tab.stages - 1;
         StageCoefs c{};
@@ -827,6 +840,8 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         c.c_acc = prime ? 0.0f : (float)(tab.b[s] * (double)S->dt_sub);
         c.acc_first = acc_started ? 0 : 1;
         c.kick = verlet ? 1 : 0;
+        c.half = half;
+        c.full = S->dt_sub;
         if (c.c_acc != 0.0f) acc_started = true;
         bool store_k = false;
         for (int t = s + 2; t < tab.stages; ++t)
@@ -898,6 +913,8 @@ arp_status do_step(arp_sim* S, bool prime = false) {
             a.sv = S->sv.p;
             a.sc = S->sc.p;
             a.stiff = S->have_stiff ? S->stiff.p : nullptr;
+            a.ep_kick = verlet ? S->ep_s[0].p : nullptr;
+            if (R && S->any_plastic) CUDA_TRY(keep(R->ep[s], a.ep, 4 * size_t(ns), st));
             sl = launch_solid(a, S->tables, c, st);
             S->launches += sl;
             cur_ep = a.ep_next;
@@ -906,7 +923,6 @@ arp_status do_step(arp_sim* S, bool prime = false) {
                 CUDA_TRY(keep(R->sx[s], (const float4*)S->sx.p, 2 * size_t(ns), st));
                 CUDA_TRY(keep(R->sv[s], (const float4*)S->sv.p, ns, st));
                 CUDA_TRY(keep(R->cb[s], (const uint32_t*)S->contact_bound.p, 2, st));
-                if (S->any_plastic) CUDA_TRY(keep(R->ep[s], a.ep, 4 * size_t(ns), st));
             }
         }
         mark(S, mk, 2);
@@ -926,10 +942,11 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         B.next_pd = next_pd;
         B.next_vm = next_vm;
         // the next state's cells: the next stage's grid, or the next step's
-        const bool bin_next = !verlet && !prime;
-        B.bin = bin_next ? bins : CellBins{};
+        B.drift_pd = verlet ? S->X.pd.p : nullptr;
+        B.drift_vm = verlet ? S->X.vm.p : nullptr;
+        B.bin = bins;
         int fl = launch_fluid(f, S->tables, S->kdim, c, B, S->fluid_variant, st);
-        if (bin_next) fl += scatter_cells(n, S->tables, S->gb, zero2, st);
+        fl += scatter_cells(n, S->tables, S->gb, zero2, st);
         S->launches += fl;
         mark(S, mk, 3);
         if (S->profiling) {
@@ -950,7 +967,7 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         if (sb && S->any_plastic) std::swap(S->ep, S->ep_t);  // without plastic materials ep stays zero
     }
     if (verlet) S->vforce_valid = true;
-    S->binned = !verlet && !prime;
+    S->binned = true;
     if (S->profiling) S->prof_steps++;
     return check_launch("step");
 }
@@ -1643,9 +1660,8 @@ arp_status arp_sim_step(arp_sim* sim, uint32_t nsteps) {
         if (graphed && sim->verlet() && !sim->vforce_valid) ARP_TRY(do_step(sim, true));
         // likewise the graph replays only steps that find their state counted
         // into cells by the step before
-        if (graphed && !sim->verlet() && !sim->binned) {
-            sim->launches += bin_cells(sim->Y.pd.p, sim->Y.vm.p, nullptr, sim->n, sim->tables, sim->gb,
-                                       sim->solid_branch() ? sim->contact_bound.p : nullptr, sim->stream);
+        if (graphed && !sim->binned) {
+            bin_state(sim, false);
             sim->binned = true;
         }
         if (graphed) ARP_TRY(graph_step(sim));
@@ -1902,6 +1918,7 @@ arp_status arp_sim_device_state(arp_sim* sim, arp_device_view* out) {
     out->vel_mat = sim->Y.vm.p;
     out->orig_id = sim->orig.p;
     out->n = sim->n;
+    sim->binned = false;  // the next step reads the state anew
     return ARP_OK;
 }
 

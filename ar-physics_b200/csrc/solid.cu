@@ -474,8 +474,10 @@ __global__ void __launch_bounds__(kThreads) k_solid_stress(SolidArgs a, Tables T
         } else if (c.last) {
             acc = a.ep_acc[o];
         }
+        float4 e = y0;
         if (c.last) {
-            a.ep_next[o] = add4(y0, acc);
+            e = add4(y0, acc);
+            a.ep_next[o] = e;
         } else {
             float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
             if (c.c_prev0 != 0.0f) t = lin4(c.c_prev0, a.ep_prev0[o], t);
@@ -484,6 +486,8 @@ __global__ void __launch_bounds__(kThreads) k_solid_stress(SolidArgs a, Tables T
             if (c.c_self != 0.0f) t = lin4(c.c_self, kv[cc], t);
             a.ep_next[o] = add4(y0, t);
         }
+        if (a.ep_kick)  // the next velocity-Verlet step's kick
+            a.ep_kick[o] = add4(e, lin4(c.half, kv[cc], make_float4(0.f, 0.f, 0.f, 0.f)));
     }
 }
 
