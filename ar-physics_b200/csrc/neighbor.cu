@@ -410,14 +410,15 @@ __device__ void sort_block_runs(const uint32_t* start, uint32_t ncells, uint32_t
 // hold at most kStage slots and none is longer than kWarpRun, the slots are
 // staged in shared memory and every thread ranks its slot among its cell's by
 // counting the smaller ones (a handful of shared-memory reads for the few
-// particles of a search cell); f(position, slot) is called for each.  Other
-// blocks are sorted in global memory first.  Insertion sorts in global memory,
-// one thread per cell, took 14 us per stage of the 1 M-particle scene.
+// particles of a search cell); store(position, slot, load(slot)) is called for
+// each.  A thread's first slot is loaded (and its cell, `key(slot)`) before the
+// block's barrier, so those reads overlap the wait and the ranking.  Other blocks
+// are sorted in global memory first.  Insertion sorts in global memory, one
+// thread per cell, took 14 us per stage of the 1 M-particle scene.
 constexpr uint32_t kStage = kBlockRun;
-// `key(slot)` is the slot's cell.
-template <class Key, class F>
+template <class Key, class Load, class Store>
 __device__ __forceinline__ void order_block(const uint32_t* start, uint32_t ncells, uint32_t* perm, uint32_t* tmp,
-                                            Key&& key, F&& f) {
+                                            Key&& key, Load&& load, Store&& store) {
     __shared__ uint32_t buf[kStage];
     __shared__ uint32_t cstart[kThreads + 1];
     const uint32_t c0 = blockIdx.x * kThreads;
@@ -430,21 +431,39 @@ __device__ __forceinline__ void order_block(const uint32_t* start, uint32_t ncel
     const uint32_t p0 = cstart[0], m = cstart[kThreads] - p0;
     if (m == 0u) return;
     if (!lengthy && m <= kStage) {
-        for (uint32_t t = threadIdx.x; t < m; t += kThreads) buf[t] = perm[p0 + t];
+        const uint32_t t0 = threadIdx.x;
+        uint32_t q0 = 0;
+        decltype(load(0u)) r0{};
+        if (t0 < m) {
+            const uint32_t v = perm[p0 + t0];
+            buf[t0] = v;
+            q0 = key(v);
+            r0 = load(v);
+        }
+        for (uint32_t t = t0 + kThreads; t < m; t += kThreads) buf[t] = perm[p0 + t];
         __syncthreads();
-        for (uint32_t t = threadIdx.x; t < m; t += kThreads) {
+        for (uint32_t t = t0; t < m; t += kThreads) {
             const uint32_t v = buf[t];
-            const uint32_t q = key(v) - c0;
+            if (t != t0) {
+                q0 = key(v);
+                r0 = load(v);
+            }
+            const uint32_t q = q0 - c0;
             const uint32_t b = cstart[q] - p0, e = cstart[q + 1] - p0;
             uint32_t at = b;
             for (uint32_t j = b; j < e; ++j) at += buf[j] < v ? 1u : 0u;
-            f(p0 + at, v);
+            store(p0 + at, v, r0);
         }
         return;
     }
     sort_block_runs(start, ncells, perm, tmp, buf);
-    for (uint32_t t = threadIdx.x; t < m; t += kThreads) f(p0 + t, perm[p0 + t]);
+    for (uint32_t t = threadIdx.x; t < m; t += kThreads) {
+        const uint32_t v = perm[p0 + t];
+        store(p0 + t, v, load(v));
+    }
 }
+
+struct Nothing {};
 
 __global__ void __launch_bounds__(kThreads) k_order(const uint32_t* start, uint32_t ncells, uint32_t* perm,
                                                     uint32_t* tmp, const uint32_t* key,
@@ -452,8 +471,8 @@ __global__ void __launch_bounds__(kThreads) k_order(const uint32_t* start, uint3
     step_begin();
     const uint32_t c = blockIdx.x * kThreads + threadIdx.x;
     if (count && c < ncells + 2u) count[c] = 0u;  // ready for the next histogram
-    order_block(start, ncells, perm, tmp, [&](uint32_t v) { return key[v]; },
-                [&](uint32_t at, uint32_t v) { perm[at] = v; });
+    order_block(start, ncells, perm, tmp, [&](uint32_t v) { return key[v]; }, [](uint32_t) { return Nothing{}; },
+                [&](uint32_t at, uint32_t v, Nothing) { perm[at] = v; });
 }
 
 __global__ void k_gather(const uint32_t* __restrict__ perm, uint32_t n, const float4* __restrict__ a_in,
@@ -496,24 +515,22 @@ struct GatherArgs {
     DevStats* stats;
     PairOut out;
 };
-__device__ __forceinline__ void gather_one(const GatherArgs& g, const Tables& T, uint32_t k, uint32_t s) {
-    const float4 pd = g.pd_in[s];
-    const float4 vm = g.vm_in[s];
-    if (g.pd_out) g.pd_out[k] = pd;
-    if (g.vm_out) g.vm_out[k] = vm;
-    if (g.sol.sx) {
-        const uint32_t sid = g.sol.sid_of_slot[s];
-        if (sid != kInvalid) {
-            g.sol.sx[2 * (size_t)sid] = pd;
-            g.sol.sv[sid] = vm;
-            g.sol.sc[sid] = g.sol.coord_of_slot[s];
-            if (g.sol.slot_of) g.sol.slot_of[sid] = k;
-        }
-    }
-    if (g.a_out) g.a_out[k] = g.a_in[s];
-    if (g.b_out) g.b_out[k] = g.b_in[s];
-    const uint32_t mat = __float_as_uint(vm.w);
-    const DevMat& m = T.mats[mat];
+struct Gathered {
+    float4 pd, vm;
+    float ps;  // p / rho^2
+    uint32_t code, local, sid, a, b;
+    uint2 coord;
+};
+__device__ __forceinline__ Gathered gather_load(const GatherArgs& g, const Tables& T, uint32_t s) {
+    Gathered r{};
+    r.pd = g.pd_in[s];
+    r.vm = g.vm_in[s];
+    r.sid = g.sol.sx ? g.sol.sid_of_slot[s] : kInvalid;
+    if (r.sid != kInvalid) r.coord = g.sol.coord_of_slot[s];
+    if (g.a_out) r.a = g.a_in[s];
+    if (g.b_out) r.b = g.b_in[s];
+    const float4 pd = r.pd;
+    const DevMat& m = T.mats[__float_as_uint(r.vm.w)];
     if (g.stats) {
         if (!finite3(pd)) {
             atomicAdd(&g.stats->nonfinite_positions, 1u);
@@ -527,34 +544,52 @@ __device__ __forceinline__ void gather_one(const GatherArgs& g, const Tables& T,
         }
     }
     const float p = eos_pressure(m.state_eq, pd.w, m.sound_speed, m.target_den);
-    const float ps = p / (pd.w * pd.w);
-    if (g.ps_out) g.ps_out[k] = ps;
+    r.ps = p / (pd.w * pd.w);
     if (g.out.rec) {
-        g.out.rec[2 * (size_t)k] = pd;
-        g.out.rec[2 * (size_t)k + 1] = make_float4(vm.x, vm.y, vm.z, ps);
-        g.out.code[k] = scan_code(pd, T.scenes[m.scene]);
-        g.out.mat8[k] = (uint8_t)m.local;
-        if (g.out.mat) g.out.mat[k] = mat;
+        r.code = scan_code(pd, T.scenes[m.scene]);
+        r.local = m.local;
+    }
+    return r;
+}
+__device__ __forceinline__ void gather_store(const GatherArgs& g, uint32_t k, const Gathered& r) {
+    if (g.pd_out) g.pd_out[k] = r.pd;
+    if (g.vm_out) g.vm_out[k] = r.vm;
+    if (r.sid != kInvalid) {
+        g.sol.sx[2 * (size_t)r.sid] = r.pd;
+        g.sol.sv[r.sid] = r.vm;
+        g.sol.sc[r.sid] = r.coord;
+        if (g.sol.slot_of) g.sol.slot_of[r.sid] = k;
+    }
+    if (g.a_out) g.a_out[k] = r.a;
+    if (g.b_out) g.b_out[k] = r.b;
+    if (g.ps_out) g.ps_out[k] = r.ps;
+    if (g.out.rec) {
+        g.out.rec[2 * (size_t)k] = r.pd;
+        g.out.rec[2 * (size_t)k + 1] = make_float4(r.vm.x, r.vm.y, r.vm.z, r.ps);
+        g.out.code[k] = r.code;
+        g.out.mat8[k] = (uint8_t)r.local;
+        if (g.out.mat) g.out.mat[k] = __float_as_uint(r.vm.w);
     }
 }
 
 __global__ void k_gather_state(const uint32_t* __restrict__ perm, uint32_t n, GatherArgs g, Tables T) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) gather_one(g, T, k, perm ? perm[k] : k);
+    if (k < n) gather_store(g, k, gather_load(g, T, perm ? perm[k] : k));
 }
 
-// Orders the block's cells and gathers the state of their particles.  Also,
-// with `stats`, the occupancy counters of the reference cells.
-__global__ void __launch_bounds__(kThreads) k_order_gather(const uint32_t* start, uint32_t ncells,
+// Orders the block's cells and gathers the state of their particles.  With
+// `stats` the grid is twice as long: the second half takes the occupancy counters
+// of the reference cells, a chain of reads of its own that would double the
+// latency of the ordering in a scene that leaves SMs idle.
+__global__ void __launch_bounds__(kThreads) k_order_gather(const uint32_t* start, uint32_t ncells, uint32_t nblocks,
                                                            uint32_t* perm, uint32_t* tmp,
                                                            const uint32_t* key,
                                                            uint32_t* count,
                                                            const uint32_t* boundary_start, DevStats* stats,
                                                            GatherArgs g, Tables T) {
     step_begin();
-    const uint32_t c = blockIdx.x * kThreads + threadIdx.x;
-    if (c < ncells + 2u) count[c] = 0u;  // ready for the next histogram
-    if (stats) {
+    if (blockIdx.x >= nblocks) {
+        const uint32_t c = (blockIdx.x - nblocks) * kThreads + threadIdx.x;
         const uint32_t occ = c < ncells ? reference_cell_occupancy(c, start, boundary_start, T) : 0u;
         const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, occ);
         const uint32_t over = __popc(__ballot_sync(0xFFFFFFFFu, occ > kBucketSlots));
@@ -562,11 +597,15 @@ __global__ void __launch_bounds__(kThreads) k_order_gather(const uint32_t* start
             if (most > 0u) atomicMax(&stats->max_cell_occupancy, most);
             if (over > 0u) atomicAdd(&stats->overflow_cells, over);
         }
+        return;
     }
+    const uint32_t c = blockIdx.x * kThreads + threadIdx.x;
+    if (c < ncells + 2u) count[c] = 0u;  // ready for the next histogram
     order_block(start, ncells, perm, tmp, [&](uint32_t v) { return key[v]; },
-                [&](uint32_t at, uint32_t v) {
+                [&](uint32_t v) { return gather_load(g, T, v); },
+                [&](uint32_t at, uint32_t v, const Gathered& r) {
                     perm[at] = v;
-                    gather_one(g, T, at, v);
+                    gather_store(g, at, r);
                 });
 }
 
@@ -679,7 +718,7 @@ __global__ void __launch_bounds__(kThreads) k_order_noalloc(const float4* pos, G
                     const float4 p = pos[v];
                     return finite3(p) ? cell_id(cell_coord(p, grid), grid) : grid.ncells;
                 },
-                [&](uint32_t at, uint32_t v) { perm[at] = v; });
+                [](uint32_t) { return Nothing{}; }, [&](uint32_t at, uint32_t v, Nothing) { perm[at] = v; });
 }
 
 // Device address of g_noalloc_scratch, looked up once per device with that
@@ -757,9 +796,9 @@ int order_gather(const Tables& T, GridBuffers& gb, const uint32_t* boundary_star
                  uint32_t* b_out, cudaStream_t st, const SolidScatter& sol, DevStats* stats, const PairOut& out) {
     gb.scattered = false;
     const GatherArgs g{pd_in, vm_in, pd_out, vm_out, a_in, b_in, a_out, b_out, nullptr, sol, stats, out};
-    launch_step(k_order_gather, blocks_for(T.ncells + 2, kThreads), kThreads, 0, st, gb.start, T.ncells, gb.perm, gb.rank,
-                                                                            gb.key, gb.count, boundary_start,
-                                                                            stats, g, T);
+    const uint32_t nb = blocks_for(T.ncells + 2, kThreads);
+    launch_step(k_order_gather, stats ? 2 * nb : nb, kThreads, 0, st, gb.start, T.ncells, nb, gb.perm, gb.rank, gb.key,
+                gb.count, boundary_start, stats, g, T);
     return 1;
 }
 
