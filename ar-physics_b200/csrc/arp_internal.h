@@ -403,6 +403,18 @@ int render_composite(const float4* PR, const float4* PC, const RenderCfg& c, con
 int render_lit(const float4* PR, const float4* PC, const float4* PP, const RenderCfg& c, unsigned long long* zkey,
                uint8_t* rgb, cudaStream_t st);
 
+// Device arrays copied by one launch (a stage's record, a checkpoint): whole
+// 4-byte words, no array both read and written.
+struct CopyList {
+    static constexpr int kMost = 12;
+    const uint32_t* src[kMost];
+    uint32_t* dst[kMost];
+    uint32_t first_block[kMost + 1];  // blocks [first_block[q], first_block[q + 1]) copy array q
+    uint64_t words[kMost];
+    int n;
+};
+int copy_arrays(CopyList& list, cudaStream_t st);
+
 // ---- adjoint (reverse mode of one integrator step) ------------------------------
 // Quantities of one RK stage saved by a recording forward step.
 struct AdjStage {

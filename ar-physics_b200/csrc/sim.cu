@@ -665,15 +665,40 @@ void populate(void* p, size_t bytes) {
 #endif
 }
 
-// Device-to-device copy into a buffer grown to fit.
+// Adds a device-to-device copy to a list, into a buffer grown to fit.
 template <class T>
-cudaError_t keep(DevBuf<T>& dst, const T* src, size_t count, cudaStream_t st) {
+cudaError_t keep(CopyList& l, DevBuf<T>& dst, const T* src, size_t count) {
+    static_assert(sizeof(T) % 4 == 0, "whole words");
     if (dst.n < std::max<size_t>(count, 1)) {
         cudaError_t e = dst.alloc(count);
         if (e != cudaSuccess) return e;
     }
     if (count == 0) return cudaSuccess;
-    return cudaMemcpyAsync(dst.p, src, count * sizeof(T), cudaMemcpyDeviceToDevice, st);
+    if (l.n == CopyList::kMost) return cudaErrorInvalidValue;
+    l.src[l.n] = reinterpret_cast<const uint32_t*>(src);
+    l.dst[l.n] = reinterpret_cast<uint32_t*>(dst.p);
+    l.words[l.n++] = count * (sizeof(T) / 4);
+    return cudaSuccess;
+}
+
+// The current state into `c`.
+arp_status keep_state(arp_sim* S, Checkpoint& c) {
+    CopyList l{};
+    const size_t n = S->n, ne = 4 * size_t(S->ns);
+    CUDA_TRY(keep(l, c.pd, (const float4*)S->Y.pd.p, n));
+    CUDA_TRY(keep(l, c.vm, (const float4*)S->Y.vm.p, n));
+    CUDA_TRY(keep(l, c.orig, (const uint32_t*)S->orig.p, n));
+    CUDA_TRY(keep(l, c.sid, (const uint32_t*)S->sid.p, n));
+    if (S->any_plastic) CUDA_TRY(keep(l, c.ep, (const float4*)S->ep.p, ne));
+    c.fvalid = S->verlet() && S->vforce_valid;
+    if (c.fvalid) {
+        CUDA_TRY(keep(l, c.fpd, (const float4*)S->vforce.pd.p, n));
+        CUDA_TRY(keep(l, c.fvm, (const float4*)S->vforce.vm.p, n));
+        if (S->any_plastic) CUDA_TRY(keep(l, c.fep, (const float4*)S->ep_force.p, ne));
+    }
+    S->launches += copy_arrays(l, S->stream);
+    c.time = S->time;
+    return ARP_OK;
 }
 
 arp_status save_checkpoint(arp_sim* S) {
@@ -682,44 +707,29 @@ arp_status save_checkpoint(arp_sim* S) {
         c = std::move(S->adj.spare.back());
         S->adj.spare.pop_back();
     }
-    CUDA_TRY(keep(c.pd, (const float4*)S->Y.pd.p, S->n, S->stream));
-    CUDA_TRY(keep(c.vm, (const float4*)S->Y.vm.p, S->n, S->stream));
-    CUDA_TRY(keep(c.orig, (const uint32_t*)S->orig.p, S->n, S->stream));
-    CUDA_TRY(keep(c.sid, (const uint32_t*)S->sid.p, S->n, S->stream));
-    if (S->any_plastic) CUDA_TRY(keep(c.ep, (const float4*)S->ep.p, 4 * size_t(S->ns), S->stream));
-    c.fvalid = S->verlet() && S->vforce_valid;
-    if (c.fvalid) {
-        CUDA_TRY(keep(c.fpd, (const float4*)S->vforce.pd.p, S->n, S->stream));
-        CUDA_TRY(keep(c.fvm, (const float4*)S->vforce.vm.p, S->n, S->stream));
-        if (S->any_plastic) CUDA_TRY(keep(c.fep, (const float4*)S->ep_force.p, 4 * size_t(S->ns), S->stream));
-    }
-    c.time = S->time;
+    ARP_TRY(keep_state(S, c));
     S->tape->ckpts.push_back(std::move(c));
     return ARP_OK;
 }
 
 arp_status restore_checkpoint(arp_sim* S, const Checkpoint& c) {
-    const size_t n = S->n;
+    CopyList l{};
+    const size_t n = S->n, ne = 4 * size_t(S->ns);
     S->binned = false;
-    if (n) {
-        CUDA_TRY(cudaMemcpyAsync(S->Y.pd.p, c.pd.p, n * sizeof(float4), cudaMemcpyDeviceToDevice, S->stream));
-        CUDA_TRY(cudaMemcpyAsync(S->Y.vm.p, c.vm.p, n * sizeof(float4), cudaMemcpyDeviceToDevice, S->stream));
-        CUDA_TRY(cudaMemcpyAsync(S->orig.p, c.orig.p, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, S->stream));
-        CUDA_TRY(cudaMemcpyAsync(S->sid.p, c.sid.p, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, S->stream));
-    }
-    if (S->any_plastic && S->ns)
-        CUDA_TRY(cudaMemcpyAsync(S->ep.p, c.ep.p, 4 * size_t(S->ns) * sizeof(float4), cudaMemcpyDeviceToDevice,
-                                 S->stream));
+    CUDA_TRY(keep(l, S->Y.pd, (const float4*)c.pd.p, n));
+    CUDA_TRY(keep(l, S->Y.vm, (const float4*)c.vm.p, n));
+    CUDA_TRY(keep(l, S->orig, (const uint32_t*)c.orig.p, n));
+    CUDA_TRY(keep(l, S->sid, (const uint32_t*)c.sid.p, n));
+    if (S->any_plastic && S->ns) CUDA_TRY(keep(l, S->ep, (const float4*)c.ep.p, ne));
     if (S->verlet()) {
         S->vforce_valid = c.fvalid;
-        if (c.fvalid && n) {
-            CUDA_TRY(cudaMemcpyAsync(S->vforce.pd.p, c.fpd.p, n * sizeof(float4), cudaMemcpyDeviceToDevice, S->stream));
-            CUDA_TRY(cudaMemcpyAsync(S->vforce.vm.p, c.fvm.p, n * sizeof(float4), cudaMemcpyDeviceToDevice, S->stream));
+        if (c.fvalid) {
+            CUDA_TRY(keep(l, S->vforce.pd, (const float4*)c.fpd.p, n));
+            CUDA_TRY(keep(l, S->vforce.vm, (const float4*)c.fvm.p, n));
+            if (S->any_plastic && S->ns) CUDA_TRY(keep(l, S->ep_force, (const float4*)c.fep.p, ne));
         }
-        if (c.fvalid && S->any_plastic && S->ns)
-            CUDA_TRY(cudaMemcpyAsync(S->ep_force.p, c.fep.p, 4 * size_t(S->ns) * sizeof(float4),
-                                     cudaMemcpyDeviceToDevice, S->stream));
     }
+    S->launches += copy_arrays(l, S->stream);
     S->time = c.time;
     return ARP_OK;
 }
@@ -806,11 +816,6 @@ arp_status do_step(arp_sim* S, bool prime = false) {
     std::swap(S->Y, S->T);
     std::swap(S->orig, S->orig_r);
     std::swap(S->sid, S->sid_r);
-    if (R) {
-        CUDA_TRY(keep(R->orig, (const uint32_t*)S->orig.p, n, st));
-        CUDA_TRY(keep(R->sid, (const uint32_t*)S->sid.p, n, st));
-        CUDA_TRY(keep(R->slot_of, (const uint32_t*)S->slot_of.p, ns, st));
-    }
     uint64_t nl = S->launches - l0;
 
     StageBuffers B{};
@@ -876,14 +881,6 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         float4* next_pd = last ? S->T.pd.p : S->S[s % 2].pd.p;
         float4* next_vm = last ? S->T.vm.p : S->S[s % 2].vm.p;
         mark(S, mk, 1);
-        if (R) {
-            CUDA_TRY(keep(R->pd[s], cur_pd, n, st));
-            CUDA_TRY(keep(R->vm[s], cur_vm, n, st));
-            CUDA_TRY(keep(R->start[s], (const uint32_t*)S->gb.start, size_t(S->ncells) + 2, st));
-            R->has_perm[s] = s > 0;
-            if (s > 0) CUDA_TRY(keep(R->perm[s], (const uint32_t*)S->gb.perm, n, st));
-        }
-
         uint64_t sl = 0;
         if (sb) {
             SolidArgs a{};
@@ -914,16 +911,34 @@ arp_status do_step(arp_sim* S, bool prime = false) {
             a.sc = S->sc.p;
             a.stiff = S->have_stiff ? S->stiff.p : nullptr;
             a.ep_kick = verlet ? S->ep_s[0].p : nullptr;
-            if (R && S->any_plastic) CUDA_TRY(keep(R->ep[s], a.ep, 4 * size_t(ns), st));
+            if (R && S->any_plastic) {  // a Verlet step's kick writes over it
+                CopyList l{};
+                CUDA_TRY(keep(l, R->ep[s], a.ep, 4 * size_t(ns)));
+                S->launches += copy_arrays(l, st);
+            }
             sl = launch_solid(a, S->tables, c, st);
             S->launches += sl;
             cur_ep = a.ep_next;
-            if (R) {
-                CUDA_TRY(keep(R->AF[s], (const float4*)S->AF.p, 6 * size_t(ns), st));
-                CUDA_TRY(keep(R->sx[s], (const float4*)S->sx.p, 2 * size_t(ns), st));
-                CUDA_TRY(keep(R->sv[s], (const float4*)S->sv.p, ns, st));
-                CUDA_TRY(keep(R->cb[s], (const uint32_t*)S->contact_bound.p, 2, st));
+        }
+        if (R) {  // what the stage's kernels read, before the next grid takes its place
+            CopyList l{};
+            if (s == 0) {
+                CUDA_TRY(keep(l, R->orig, (const uint32_t*)S->orig.p, n));
+                CUDA_TRY(keep(l, R->sid, (const uint32_t*)S->sid.p, n));
+                CUDA_TRY(keep(l, R->slot_of, (const uint32_t*)S->slot_of.p, ns));
             }
+            CUDA_TRY(keep(l, R->pd[s], cur_pd, n));
+            CUDA_TRY(keep(l, R->vm[s], cur_vm, n));
+            CUDA_TRY(keep(l, R->start[s], (const uint32_t*)S->gb.start, size_t(S->ncells) + 2));
+            R->has_perm[s] = s > 0;
+            if (s > 0) CUDA_TRY(keep(l, R->perm[s], (const uint32_t*)S->gb.perm, n));
+            if (sb) {
+                CUDA_TRY(keep(l, R->AF[s], (const float4*)S->AF.p, 6 * size_t(ns)));
+                CUDA_TRY(keep(l, R->sx[s], (const float4*)S->sx.p, 2 * size_t(ns)));
+                CUDA_TRY(keep(l, R->sv[s], (const float4*)S->sv.p, ns));
+                CUDA_TRY(keep(l, R->cb[s], (const uint32_t*)S->contact_bound.p, 2));
+            }
+            S->launches += copy_arrays(l, st);
         }
         mark(S, mk, 2);
 
@@ -2346,18 +2361,7 @@ arp_status arp_tape_backward(arp_sim* sim, const float* dl_dstate, float* grad_s
     AdjointPool& P = sim->adj;
     // the forward state is put back when the pass ends
     Checkpoint& now = P.now;
-    CUDA_TRY(keep(now.pd, (const float4*)sim->Y.pd.p, n, st));
-    CUDA_TRY(keep(now.vm, (const float4*)sim->Y.vm.p, n, st));
-    CUDA_TRY(keep(now.orig, (const uint32_t*)sim->orig.p, n, st));
-    CUDA_TRY(keep(now.sid, (const uint32_t*)sim->sid.p, n, st));
-    if (sim->any_plastic) CUDA_TRY(keep(now.ep, (const float4*)sim->ep.p, 4 * size_t(ns), st));
-    now.fvalid = sim->verlet() && sim->vforce_valid;
-    if (now.fvalid) {
-        CUDA_TRY(keep(now.fpd, (const float4*)sim->vforce.pd.p, n, st));
-        CUDA_TRY(keep(now.fvm, (const float4*)sim->vforce.vm.p, n, st));
-        if (sim->any_plastic) CUDA_TRY(keep(now.fep, (const float4*)sim->ep_force.p, 4 * size_t(ns), st));
-    }
-    now.time = sim->time;
+    ARP_TRY(keep_state(sim, now));
     // adjoint buffers: caller order (lc), storage order (ls, out), per stage (lY), stage weights (mu)
     const size_t nn = std::max(n, 1u);
     auto fit = [](auto& b, size_t count) -> cudaError_t { return b.n >= count ? cudaSuccess : b.alloc(count); };
