@@ -411,16 +411,22 @@ __device__ void sort_block_runs(const uint32_t* start, uint32_t ncells, uint32_t
 // staged in shared memory and every thread ranks its slot among its cell's by
 // counting the smaller ones (a handful of shared-memory reads for the few
 // particles of a search cell); store(position, slot, load(slot)) is called for
-// each.  A thread's first slot is loaded (and its cell, `key(slot)`) before the
-// block's barrier, so those reads overlap the wait and the ranking.  Other blocks
-// are sorted in global memory first.  Insertion sorts in global memory, one
-// thread per cell, took 14 us per stage of the 1 M-particle scene.
+// each.  A slot's cell is `key[slot]` or, with key null, marked by the cell's own
+// thread at its positions (the allocation-free build, which keeps no keys, read
+// the position again: 12.4 us for 1 M particles, 9.6 marked; with the gather the
+// marks' shared memory costs 3 us a stage at 1 M, and the key is there).  A
+// thread's first slot is loaded before the block's barrier, so those reads
+// overlap the wait and the ranking.  Other blocks are sorted in global memory
+// first.  Insertion sorts in global memory, one thread per cell, took 14 us per
+// stage of the 1 M-particle scene.
 constexpr uint32_t kStage = kBlockRun;
-template <class Key, class Load, class Store>
+template <bool KEYS, class Load, class Store>
 __device__ __forceinline__ void order_block(const uint32_t* start, uint32_t ncells, uint32_t* perm, uint32_t* tmp,
-                                            Key&& key, Load&& load, Store&& store) {
+                                            const uint32_t* key, Load&& load, Store&& store) {
     __shared__ uint32_t buf[kStage];
     __shared__ uint32_t cstart[kThreads + 1];
+    __shared__ uint8_t cell[KEYS ? 4 : kStage];  // of the block's kThreads
+    static_assert(kThreads <= 256, "cells in 8 bits");
     const uint32_t c0 = blockIdx.x * kThreads;
     const uint32_t c = c0 + threadIdx.x;
     // cells 0 .. ncells (the last is the non-finite bucket), start has ncells + 2 entries
@@ -437,18 +443,20 @@ __device__ __forceinline__ void order_block(const uint32_t* start, uint32_t ncel
         if (t0 < m) {
             const uint32_t v = perm[p0 + t0];
             buf[t0] = v;
-            q0 = key(v);
+            if (KEYS) q0 = key[v];
             r0 = load(v);
         }
         for (uint32_t t = t0 + kThreads; t < m; t += kThreads) buf[t] = perm[p0 + t];
+        if (!KEYS)
+            for (uint32_t p = s0; p < s1; ++p) cell[p - p0] = (uint8_t)threadIdx.x;
         __syncthreads();
         for (uint32_t t = t0; t < m; t += kThreads) {
             const uint32_t v = buf[t];
             if (t != t0) {
-                q0 = key(v);
+                if (KEYS) q0 = key[v];
                 r0 = load(v);
             }
-            const uint32_t q = q0 - c0;
+            const uint32_t q = KEYS ? q0 - c0 : cell[t];
             const uint32_t b = cstart[q] - p0, e = cstart[q + 1] - p0;
             uint32_t at = b;
             for (uint32_t j = b; j < e; ++j) at += buf[j] < v ? 1u : 0u;
@@ -466,12 +474,12 @@ __device__ __forceinline__ void order_block(const uint32_t* start, uint32_t ncel
 struct Nothing {};
 
 __global__ void __launch_bounds__(kThreads) k_order(const uint32_t* start, uint32_t ncells, uint32_t* perm,
-                                                    uint32_t* tmp, const uint32_t* key,
+                                                    uint32_t* tmp,
                                                     uint32_t* count) {
     step_begin();
     const uint32_t c = blockIdx.x * kThreads + threadIdx.x;
     if (count && c < ncells + 2u) count[c] = 0u;  // ready for the next histogram
-    order_block(start, ncells, perm, tmp, [&](uint32_t v) { return key[v]; }, [](uint32_t) { return Nothing{}; },
+    order_block<false>(start, ncells, perm, tmp, nullptr, [](uint32_t) { return Nothing{}; },
                 [&](uint32_t at, uint32_t v, Nothing) { perm[at] = v; });
 }
 
@@ -582,8 +590,7 @@ __global__ void k_gather_state(const uint32_t* __restrict__ perm, uint32_t n, Ga
 // of the reference cells, a chain of reads of its own that would double the
 // latency of the ordering in a scene that leaves SMs idle.
 __global__ void __launch_bounds__(kThreads) k_order_gather(const uint32_t* start, uint32_t ncells, uint32_t nblocks,
-                                                           uint32_t* perm, uint32_t* tmp,
-                                                           const uint32_t* key,
+                                                           uint32_t* perm, uint32_t* tmp, const uint32_t* key,
                                                            uint32_t* count,
                                                            const uint32_t* boundary_start, DevStats* stats,
                                                            GatherArgs g, Tables T) {
@@ -601,8 +608,7 @@ __global__ void __launch_bounds__(kThreads) k_order_gather(const uint32_t* start
     }
     const uint32_t c = blockIdx.x * kThreads + threadIdx.x;
     if (c < ncells + 2u) count[c] = 0u;  // ready for the next histogram
-    order_block(start, ncells, perm, tmp, [&](uint32_t v) { return key[v]; },
-                [&](uint32_t v) { return gather_load(g, T, v); },
+    order_block<true>(start, ncells, perm, tmp, key, [&](uint32_t v) { return gather_load(g, T, v); },
                 [&](uint32_t at, uint32_t v, const Gathered& r) {
                     perm[at] = v;
                     gather_store(g, at, r);
@@ -709,18 +715,6 @@ __global__ void k_scatter_noalloc(const float4* pos, uint32_t n, Grid grid,
     perm[start[k] + rank[i]] = i;
 }
 
-__global__ void __launch_bounds__(kThreads) k_order_noalloc(const float4* pos, Grid grid,
-                                                            const uint32_t* start, uint32_t* perm,
-                                                            uint32_t* tmp) {
-    step_begin();
-    order_block(start, grid.ncells, perm, tmp,
-                [&](uint32_t v) {
-                    const float4 p = pos[v];
-                    return finite3(p) ? cell_id(cell_coord(p, grid), grid) : grid.ncells;
-                },
-                [](uint32_t) { return Nothing{}; }, [&](uint32_t at, uint32_t v, Nothing) { perm[at] = v; });
-}
-
 // Device address of g_noalloc_scratch, looked up once per device with that
 // device current (host code may not use the symbol itself as an address).
 constexpr int kMaxDevices = 64;
@@ -786,8 +780,8 @@ int scatter_cells(uint32_t n, const Tables& T, GridBuffers& gb, uint32_t* zero2,
 
 int order_cells(const Tables& T, GridBuffers& gb, cudaStream_t st) {
     gb.scattered = false;
-    launch_step(k_order, blocks_for(T.ncells + 2, kThreads), kThreads, 0, st, gb.start, T.ncells, gb.perm, gb.rank, gb.key,
-                                                                     gb.count);
+    launch_step(k_order, blocks_for(T.ncells + 2, kThreads), kThreads, 0, st, gb.start, T.ncells, gb.perm, gb.rank,
+                gb.count);
     return 1;
 }
 
@@ -915,7 +909,7 @@ extern "C" arp_status arp_grid_build_noalloc(const void* pos_den, uint32_t n, co
     if (n > 0) launch_step(k_rank_noalloc, blocks_for(n, kThreads), kThreads, 0, st, pos, n, g, cell_start, rank);
     exclusive_scan(cell_start, len, cell_start, tile_sums, st);  // in place: counts become starts
     if (n > 0) launch_step(k_scatter_noalloc, blocks_for(n, kThreads), kThreads, 0, st, pos, n, g, cell_start, rank, perm);
-    if (n > 0) launch_step(k_order_noalloc, blocks_for(g.ncells + 1, kThreads), kThreads, 0, st, pos, g, cell_start, perm, rank);
+    if (n > 0) launch_step(k_order, blocks_for(g.ncells + 1, kThreads), kThreads, 0, st, cell_start, g.ncells, perm, rank, nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(ARP_ERR_CUDA, std::string("grid build launch: ") + cudaGetErrorString(e));
     return ARP_OK;
