@@ -343,7 +343,9 @@ __global__ void __launch_bounds__(kCompWarps * 32) k_rp_composite(const float4* 
 }
 
 // Lighting: the nearest covering sprite of each pixel (depth LESS, the first
-// drawn on ties): min over (window depth bits, draw order).
+// drawn on ties): min over (window depth bits, draw order).  Bound by the
+// atomics: with one for every covered pixel, and both offsets divided for every
+// pixel, 62 us for 314,000 sprites 64 layers deep; 42 now.
 __global__ void k_rp_depth(const float4* __restrict__ PR, const float4* __restrict__ PC, RenderCfg c,
                            unsigned long long* __restrict__ zkey) {
     const uint32_t prim = blockIdx.x * blockDim.x + threadIdx.x;
@@ -354,11 +356,25 @@ __global__ void k_rp_depth(const float4* __restrict__ PR, const float4* __restri
     const int i0 = max(0, (int)floorf(r.x - R)), i1 = min((int)c.W - 1, (int)ceilf(r.x + R));
     const int j0 = max(0, (int)floorf(r.y - R)), j1 = min((int)c.H - 1, (int)ceilf(r.y + R));
     const unsigned long long key = ((unsigned long long)__float_as_uint(r.w) << 32) | prim;
-    for (int j = j0; j <= j1; ++j)
-        for (int i = i0; i <= i1; ++i) {
-            float dx, dy, r2;
-            if (covers(c, r, i + 0.5f, j + 0.5f, dx, dy, r2)) atomicMin(&zkey[(size_t)j * c.W + i], key);
+    constexpr int W = 8;  // columns at a time
+    for (int ib = i0; ib <= i1; ib += W) {
+        float dx2[W];
+#pragma unroll
+        for (int u = 0; u < W; ++u) {
+            const float f = ib + u + 0.5f;
+            const float dx = ib + u <= i1 && in_square(c, r.x, f) ? sprite_dx(c, r, f) : INFINITY;
+            dx2[u] = __fmul_rn(dx, dx);
         }
+        for (int j = j0; j <= j1; ++j) {
+            if (!in_square(c, r.y, j + 0.5f)) continue;
+            const float dy = sprite_dy(c, r, j + 0.5f), dy2 = __fmul_rn(dy, dy);
+            if (!(dy2 <= 1.0f)) continue;  // no pixel of the row is covered
+            unsigned long long* const z = zkey + (size_t)j * c.W + ib;
+#pragma unroll
+            for (int u = 0; u < W; ++u)  // most sprites lie behind what a pixel already holds
+                if (__fadd_rn(dx2[u], dy2) <= 1.0f && key < __ldcg(z + u)) atomicMin(z + u, key);
+        }
+    }
 }
 
 __global__ void k_rp_shade(const float4* __restrict__ PR, const float4* __restrict__ PC,
