@@ -395,7 +395,7 @@ __device__ __forceinline__ float sum_partials(float v) {  // over the lanes that
 // read from the positions, took 352 us per stage of the 1,048,576-particle
 // fluid and bar scene (RK2, 222 M warp instructions, 69 M wavefronts) and two
 // more launches for the particles whose lists overflowed; this takes 292 us
-// (202 M, 59 M), the next state's cell keys included.  On the way: 4 threads per
+// (205 M, 59 M), the next state's cell keys included.  On the way: 4 threads per
 // particle alone 372 us; + quantised candidates 345 us; + 32-byte records 330 us;
 // + the next row's bounds and a second hit's record in flight 292 us.
 // kBlocksPerSM 128-thread blocks per SM (72 registers): 8 (64 registers, spills)

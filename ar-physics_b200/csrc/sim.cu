@@ -1289,9 +1289,9 @@ arp_status allocate(arp_sim* S) {
 }
 
 // ---- autotuner -----------------------------------------------------------------
-// Chooses the fluid kernel's launch shape (hit-list capacity, one tile per
-// block or persistent tile queue) by timing every variant on the live stage-0
-// state.  All variants evaluate the same pairs in the same order, so the
+// Chooses the fluid kernel's launch shape (the block form with a block size and
+// hit-list capacity, or the group form with 4, 8 or 16 threads per particle) by
+// timing them on the live stage-0 state.  All variants evaluate the same pairs in the same order, so the
 // choice changes speed, never results.  Choices are cached per (kernel
 // dimension, log2 particle count, quarter-octave of h / particle spacing).
 // Sizes at which a form cannot win are left out: the group form above

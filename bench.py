@@ -271,9 +271,9 @@ def run_batched(torch, stream, rank=0, world=1, steps_batch=200, rounds_loop=10,
     blocks and elastic blocks): stepped as one batch (one set of launches per
     stage) and as a loop over 256 separate simulations, both on one GPU and
     both replaying each step from a CUDA graph.  The batch is timed over the
-    configuration's 200 steps with the autotuner's launch shape; every
-    persistent tile-queue shape of the fluid kernel is timed beside it over
-    the same 200 steps from the same state.  With N ranks the scenes are
+    configuration's 200 steps with the autotuner's launch shape; any
+    launch shape that takes tiles from a persistent queue (today none does) is
+    timed beside it over the same 200 steps from the same state.  With N ranks the scenes are
     sharded (scenes.partition_scenes, by particle count) and each rank steps
     its share; every time is the slowest rank's, and rates count all 256
     scenes."""
@@ -646,7 +646,7 @@ def run_ours(args, rank, world, local_rank):
 
     peak, peak_kind = load_peaks()
     fl = prof["stages"]
-    fluid_ms = prof["fluid_ms"] / fl if fl else float("nan")  # per stage: tile kernel + overflow kernel
+    fluid_ms = prof["fluid_ms"] / fl if fl else float("nan")  # per stage: the fluid kernel, the next grid's scan and scatter
     alg_bytes = 96.0 * sc.n  # per stage: read y_s 32 B + read y0 32 B + write y_{s+1} 32 B per particle
     achieved = alg_bytes / (fluid_ms / 1000.0) / 1e9
     traffic = load_traffic().get(f"fluid_{args.config}")
