@@ -297,6 +297,7 @@ struct FluidArgs {
     const float4* ksol;      // per-solid solid-term acceleration (nullptr when the solid branch is off)
     uint32_t n;
     int solid_branch;
+    int beside_solids;       // the solid kernels were launched just before: only the epilogue waits for them
 };
 // Launch shapes of the fluid kernel the autotuner chooses between: threads
 // per block and hit-list capacity of the block form (one thread per particle

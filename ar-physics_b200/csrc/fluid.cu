@@ -398,6 +398,11 @@ __device__ __forceinline__ float sum_partials(float v) {  // over the lanes that
 // (205 M, 59 M), the next state's cell keys included.  On the way: 4 threads per
 // particle alone 372 us; + quantised candidates 345 us; + 32-byte records 330 us;
 // + the next row's bounds and a second hit's record in flight 292 us.
+// Only the epilogue reads what the solid kernels write, so behind those
+// (a.beside_solids) a block waits there instead of at its start, and the pair
+// sums fill the SMs that the solid kernels' last blocks leave: ten RK2 steps of
+// the 1,048,576-particle scene 10,021 -> 9,905 us, 48 batched scenes 10,082 ->
+// 9,955, 16,899 particles under velocity Verlet 563 -> 550.
 // kBlocksPerSM 128-thread blocks per SM (72 registers): 8 (64 registers, spills)
 // take 6 % more, 6 (80 registers) 2 % more.
 constexpr int kBlocksPerSM = 7;
@@ -410,7 +415,7 @@ __global__ void __launch_bounds__(BLOCK, kBlocksPerSM * 128 / BLOCK) k_fluid(Flu
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint32_t* const lists = reinterpret_cast<uint32_t*>(smem_raw);
     PairMat* const sm = reinterpret_cast<PairMat*>(smem_raw + sizeof(uint32_t) * STRIDE * BLOCK);
-    step_begin();
+    if (!a.beside_solids) step_begin();
     const uint32_t k0 = blockIdx.x * BLOCK;
     const uint32_t scene0 = T.mats[a.mat[k0]].scene;  // k0 < n: one block per started tile
     {
@@ -619,6 +624,7 @@ __global__ void __launch_bounds__(BLOCK, kBlocksPerSM * 128 / BLOCK) k_fluid(Flu
         w = my + (open ? cnt - ev : 0u);
         wend = my + CAP - TAIL;
     }
+    step_begin();
     if (valid) stage_epilogue(a, T, c, b, k, acc);
 }
 
@@ -647,7 +653,7 @@ __global__ void __launch_bounds__(kGroupBlock, LANES == 16 ? 8 : 7) k_fluid_grou
     __shared__ uint2 s_seg[NG][2 * GroupScan<DIM, LANES>::MAXROWS];
     __shared__ float4 s_term[LANES > 4 ? NG : 1][LANES];
     constexpr unsigned FULL = 0xFFFFFFFFu;
-    step_begin();
+    if (!a.beside_solids) step_begin();
     const uint32_t lane = threadIdx.x % LANES, gi = threadIdx.x / LANES;
     const uint32_t kk = blockIdx.x * NG + gi;
     const bool valid = kk < a.n;
@@ -723,6 +729,7 @@ __global__ void __launch_bounds__(kGroupBlock, LANES == 16 ? 8 : 7) k_fluid_grou
     sum.f.x = __shfl_sync(FULL, acc[1 % CPL], 4 * (1 / CPL), LANES);
     sum.f.y = __shfl_sync(FULL, acc[2 % CPL], 4 * (2 / CPL), LANES);
     sum.f.z = __shfl_sync(FULL, acc[3 % CPL], 4 * (3 / CPL), LANES);
+    step_begin();
     if (valid && lane == 0) stage_epilogue(a, T, c, b, k, sum);
 }
 

@@ -24,6 +24,15 @@ __device__ __forceinline__ void step_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Lets the next kernel's blocks in as soon as every block of this one has got here.
+// For a next kernel that has work before its wait: what it reads until then must
+// have been written by kernels that this one's step_begin(), or that of the
+// kernel before, has waited for.  Blocks that wait hold no place that an earlier
+// kernel's block still needs, all of which are resident by then.
+__device__ __forceinline__ void step_let_next() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 template <class... P, class... A>
 void launch_step(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchAttribute at{};

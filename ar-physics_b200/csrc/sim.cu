@@ -954,6 +954,7 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         f.ksol = sb ? S->ksol.p : nullptr;
         f.n = n;
         f.solid_branch = sb ? 1 : 0;
+        f.beside_solids = sl && !R ? 1 : 0;  // a tape's copies lie between the two
         B.next_pd = next_pd;
         B.next_vm = next_vm;
         // the next state's cells: the next stage's grid, or the next step's

@@ -281,6 +281,7 @@ __device__ __forceinline__ T3 stress_order2(const T3& F, const T3& Fd, float lam
 template <bool ORDER2, bool PLASTIC, int LANES>
 __global__ void __launch_bounds__(kThreads) k_solid_stress(SolidArgs a, Tables T, StageCoefs c) {
     step_begin();
+    step_let_next();  // after the wait: the kernels let in rely on the grid being there
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = t / LANES, lane = t % LANES;
     if (i >= a.ns) return;  // whole groups leave together
@@ -497,6 +498,7 @@ __global__ void __launch_bounds__(kThreads) k_solid_stress(SolidArgs a, Tables T
 // kernels took 92 us per stage of 129,024 solids and 36 us for 1,274.
 template <int LANES>
 __global__ void __launch_bounds__(kThreads) k_solid_forces(SolidArgs a, Tables T) {
+    step_let_next();  // the fluid kernel's pair sums need only the grid, which the stress kernel has waited for
     step_begin();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = t / LANES, lane = t % LANES;
