@@ -6,8 +6,8 @@
 // and wait in step_begin() until that kernel has finished and its writes are
 // visible, so the launch itself no longer lies between them.  Every kernel
 // launched this way calls step_begin() first, on every thread and before it
-// reads or writes memory (the next kernel's wait then covers all earlier ones),
-// and reads what other kernels of the step write by ordinary loads (not
+// reads or writes memory (the next kernel's wait then covers all earlier ones;
+// the fluid kernel behind the solid kernels, which let it in, waits later), and reads what other kernels of the step write by ordinary loads (not
 // through the read-only path, whose data must not change while a kernel
 // runs).  Per stage, plain launches / graph replay: 16,384-particle 2D scene (4
 // kernels) 24.8 / 18.1 us without it, 17.1 / 17.3 with it; 16,899-particle 3D
