@@ -1294,11 +1294,17 @@ arp_status allocate(arp_sim* S) {
 // hit-list capacity, or the group form with 4, 8 or 16 threads per particle) by
 // timing them on the live stage-0 state.  All variants evaluate the same pairs in the same order, so the
 // choice changes speed, never results.  Choices are cached per (kernel
-// dimension, log2 particle count, quarter-octave of h / particle spacing).
+// dimension, quarter-octaves of the particle count and of h / particle spacing):
+// how many waves of blocks a group form takes changes within an octave (solids,
+// 31,200: 290 us a step with 16 threads, chosen at 19,496 particles, against 258
+// with 4).  A shape's time is the least of kTuneRounds, since the first launches
+// may run while the clocks still rise.
 // Sizes at which a form cannot win are left out: the group form above
 // kGroupMost particles (126,464 in 3D: 86 us against 62; 1.05 M: 600 against
-// 290), the block form below kBlockLeast (9,072 in 3D: 58 us against 14).
-constexpr uint32_t kGroupMost = 131072, kBlockLeast = 12288;
+// 290), the block form below kBlockLeast (24,706 in 3D: ten steps 1312 us
+// against 986; 22,500 in 2D: 1145 against 899).
+constexpr uint32_t kGroupMost = 131072, kBlockLeast = 24576;
+constexpr int kTuneRounds = 3;
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int>, int> g_tune_cache;
 
@@ -1312,8 +1318,8 @@ std::tuple<int, int, int> tune_key(const arp_sim* S) {
         acc += std::log2((double)H.h / spacing);
     }
     const double ratio = S->n ? acc / S->n : 0.0;
-    const int nbits = S->n ? (int)std::ceil(std::log2((double)S->n)) : 0;
-    return std::make_tuple(S->kdim, nbits, (int)std::lround(4.0 * ratio));
+    const int size = S->n ? (int)std::lround(4.0 * std::log2((double)S->n)) : 0;
+    return std::make_tuple(S->kdim, size, (int)std::lround(4.0 * ratio));
 }
 
 arp_status run_autotune(arp_sim* S, bool force) {
@@ -1372,15 +1378,17 @@ arp_status run_autotune(arp_sim* S, bool force) {
         const FluidVariant& fv = kFluidVariants[v];
         if (fv.lanes ? n > kGroupMost : n < kBlockLeast) continue;
         S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, st);  // warm-up
-        CUDA_TRY(cudaEventRecord(e0, st));
-        for (int r = 0; r < 3; ++r) S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, st);
-        CUDA_TRY(cudaEventRecord(e1, st));
-        CUDA_TRY(cudaEventSynchronize(e1));
-        float ms = 0;
-        CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
-        if (ms < best) {
-            best = ms;
-            best_v = v;
+        for (int round = 0; round < (fv.lanes ? kTuneRounds : 1); ++round) {
+            CUDA_TRY(cudaEventRecord(e0, st));
+            for (int r = 0; r < 3; ++r) S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, st);
+            CUDA_TRY(cudaEventRecord(e1, st));
+            CUDA_TRY(cudaEventSynchronize(e1));
+            float ms = 0;
+            CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
+            if (ms < best) {
+                best = ms;
+                best_v = v;
+            }
         }
     }
     S->ev_free.push_back(e0);
