@@ -291,6 +291,11 @@ struct arp_sim {
     // (ep_s[0] the kicked plastic strain).  False whenever Y, X or the grid
     // buffers have changed otherwise.
     bool binned = false;
+    // A caller has captured steps into a graph of its own, which it may replay at
+    // any time, also after a state was set: from then on every step counts its
+    // state itself, leaves nothing counted for the next, and finds no use in what
+    // the host knows of the counts (`binned`, GridBuffers::scattered).
+    bool standalone = false;
     // solids
     DevBuf<float4> ref, L, AF, ksol;
     DevBuf<float4> ep, ep_t, ep_s[2], ep_acc, ep_kst[4];
@@ -326,7 +331,7 @@ struct arp_sim {
     struct StepGraph {
         cudaGraph_t g = nullptr;
         cudaGraphExec_t exec = nullptr;
-        const void* sig[4] = {nullptr, nullptr, nullptr, nullptr};
+        const void* sig[5] = {};
         uint64_t launches = 0;  // kernels per replay
     };
     bool use_graph = false;
@@ -795,6 +800,10 @@ arp_status do_step(arp_sim* S, bool prime = false) {
     uint32_t* const zero2 = sb ? S->contact_bound.p : nullptr;  // cleared with each stage's sort
     const float4* src_pd = S->Y.pd.p;
     const float4* src_vm = S->Y.vm.p;
+    if (S->standalone) {
+        S->binned = false;
+        S->gb.scattered = true;  // the counts are cleared whatever they hold
+    }
     if (!S->binned || prime) bin_state(S, prime);
     if (verlet && !prime) {
         src_pd = S->X.pd.p;
@@ -831,6 +840,7 @@ arp_status do_step(arp_sim* S, bool prime = false) {
     if (verlet && !prime && sb && S->any_plastic) ep_base = cur_ep = S->ep_s[0].p;  // kicked with the state
     for (int s = 0; s < tab.stages; ++s) {
         const bool last = !prime && s == tab.stages - 1;
+        const bool count_next = !S->standalone || !(last || prime);  // the written state is counted into cells
         StageCoefs c{};
         c.stage = s;
         c.last = last ? 1 : 0;
@@ -910,7 +920,7 @@ arp_status do_step(arp_sim* S, bool prime = false) {
             a.sv = S->sv.p;
             a.sc = S->sc.p;
             a.stiff = S->have_stiff ? S->stiff.p : nullptr;
-            a.ep_kick = verlet ? S->ep_s[0].p : nullptr;
+            a.ep_kick = verlet && count_next ? S->ep_s[0].p : nullptr;
             if (R && S->any_plastic) {  // a Verlet step's kick writes over it
                 CopyList l{};
                 CUDA_TRY(keep(l, R->ep[s], a.ep, 4 * size_t(ns)));
@@ -958,11 +968,11 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         B.next_pd = next_pd;
         B.next_vm = next_vm;
         // the next state's cells: the next stage's grid, or the next step's
-        B.drift_pd = verlet ? S->X.pd.p : nullptr;
-        B.drift_vm = verlet ? S->X.vm.p : nullptr;
-        B.bin = bins;
+        B.drift_pd = verlet && count_next ? S->X.pd.p : nullptr;
+        B.drift_vm = verlet && count_next ? S->X.vm.p : nullptr;
+        B.bin = count_next ? bins : CellBins{};
         int fl = launch_fluid(f, S->tables, S->kdim, c, B, S->fluid_variant, st);
-        fl += scatter_cells(n, S->tables, S->gb, zero2, st);
+        if (count_next) fl += scatter_cells(n, S->tables, S->gb, zero2, st);
         S->launches += fl;
         mark(S, mk, 3);
         if (S->profiling) {
@@ -983,7 +993,8 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         if (sb && S->any_plastic) std::swap(S->ep, S->ep_t);  // without plastic materials ep stays zero
     }
     if (verlet) S->vforce_valid = true;
-    S->binned = true;
+    S->binned = !S->standalone;
+    if (S->standalone) S->gb.scattered = true;  // a captured step has not run: the counts are unknown
     if (S->profiling) S->prof_steps++;
     return check_launch("step");
 }
@@ -1594,12 +1605,15 @@ arp_status arp_sim_fluid_variant(const arp_sim* sim, int* variant, int* block, i
     return ARP_OK;
 }
 
-// The buffer pointers a step's launches depend on and swaps.
-static void step_signature(const arp_sim* S, const void* sig[4]) {
+// The buffer pointers a step's launches depend on and swaps, and whether it
+// counts its state itself.
+constexpr int kSignature = 5;
+static void step_signature(const arp_sim* S, const void* sig[kSignature]) {
     sig[0] = S->Y.pd.p;
     sig[1] = S->orig.p;
     sig[2] = S->sid.p;
     sig[3] = S->ep.p;
+    sig[4] = S->standalone ? S : nullptr;
 }
 
 // Capture one step on the handle's stream into the graph slot `k`; the host
@@ -1644,12 +1658,12 @@ arp_status capture_step_graph(arp_sim* S, int k) {
 // side: the buffer swaps of do_step, time and launch count.
 arp_status graph_step(arp_sim* S) {
     if (S->graph_stream != S->stream) S->drop_graph();
-    const void* sig[4];
+    const void* sig[kSignature];
     step_signature(S, sig);
     int k = -1, free_slot = -1;
     for (int q = 0; q < arp_sim::kStepGraphs; ++q) {
         const auto& G = S->graphs[q];
-        if (G.exec && std::equal(sig, sig + 4, G.sig)) k = q;
+        if (G.exec && std::equal(sig, sig + kSignature, G.sig)) k = q;
         if (!G.exec && free_slot < 0) free_slot = q;
     }
     if (k < 0) {  // capture; do_step's host side happens during the capture
@@ -1675,16 +1689,21 @@ arp_status graph_step(arp_sim* S) {
 
 arp_status arp_sim_step(arp_sim* sim, uint32_t nsteps) {
     ARP_TRY(need_init(sim));
+    // a caller's capture records plain steps
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(sim->stream, &capture) != cudaSuccess) (void)cudaGetLastError();  // launches will tell
+    const bool captured = capture == cudaStreamCaptureStatusActive;
+    if (captured) sim->standalone = true;
     for (uint32_t i = 0; i < nsteps; ++i) {
         const bool sampled = sim->prof_on && sim->prof_phase % sim->prof_every == 0;
-        const bool graphed = sim->use_graph && !sim->tape && !sampled;
+        const bool graphed = sim->use_graph && !sim->tape && !sampled && !captured;
         // velocity Verlet starts from a force evaluation at the current state:
         // plain launches before a graphed step (the graph replays only steps
         // that carry the record); a plain step makes it itself
         if (graphed && sim->verlet() && !sim->vforce_valid) ARP_TRY(do_step(sim, true));
         // likewise the graph replays only steps that find their state counted
         // into cells by the step before
-        if (graphed && !sim->binned) {
+        if (graphed && !sim->binned && !sim->standalone) {
             bin_state(sim, false);
             sim->binned = true;
         }

@@ -404,7 +404,11 @@ arp_status arp_grid_build_noalloc(const void* pos_den, uint32_t n, const arp_aab
 /* ---- streams, profiling, health ------------------------------------------- */
 
 /* Use a caller-owned CUDA stream (cudaStream_t passed as void*); NULL returns
- * to the handle's own stream. */
+ * to the handle's own stream.  Steps taken while the stream is being captured
+ * become part of the caller's graph (an even number of them, since a step
+ * exchanges buffers and two end where they began); from then on the handle's
+ * steps count their state into cells themselves, so that a replay may come at
+ * any time, also after arp_sim_set_particles. */
 arp_status arp_sim_set_stream(arp_sim* sim, void* stream);
 /* (arp_sim_synchronize is declared with the asynchronous exchange above.) */
 /* Per-segment timing (grid build, solid, fluid) with CUDA events between the
