@@ -437,7 +437,7 @@ __global__ void k_adj_prep(AdjArgs a, Tables T) {
     r[1] = make_float4(v.x, v.y, v.z, __uint_as_float(id));
     r[2] = w;
     r[3] = make_float4(pt, dpt, ir, v.w);
-    a.code[k] = scan_code(x, T.scenes[m.scene]);
+    a.code[k] = scan_code(x, T.scenes[m.scene], T.flat);
 }
 
 // LANES threads share one particle, as in the forward kernel's group form: the

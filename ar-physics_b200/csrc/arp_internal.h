@@ -132,6 +132,7 @@ struct Tables {
     uint32_t ncells;                  // total search cells of all scenes (the non-finite bucket follows)
     uint32_t max_nmat;                // largest per-scene material count
     uint32_t nscenes;
+    uint32_t flat;                    // the pair kernels run in two dimensions (every scene flat in z)
 };
 
 // Health counters written by device code.

@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(BLOCK, kBlocksPerSM * 128 / BLOCK) k_fluid(Flu
             const float4 xi = a.rec[2 * (size_t)k];
             const SceneP& P = T.scenes[T.mats[a.mat[k]].scene];
             const SearchRows rows = search_rows<DIM>(xi, finite3(xi), P);
-            const uint32_t own = own_code(xi, P);
+            const uint32_t own = own_code<DIM>(xi, P);
             const uint4* const code4 = reinterpret_cast<const uint4*>(a.code);
             // the bounds of the next row are read while the current one is tested
             uint32_t nb0 = 0, nb1 = 0, nm0 = 0, nm1 = 0;

@@ -83,20 +83,24 @@ __device__ __forceinline__ void bin_particle(float4 p, const SceneP& P, uint32_t
 // h therefore has a sum of squares of at most (63 + 2.345)^2 + 1 = 4271.0; the
 // bound below leaves 2 for the roundings of X in double precision.  Differences past 127
 // wrap, which can only let far candidates through, and the evaluation of a
-// pair tests r < h again.
+// pair tests r < h again.  A flat handle (Tables::flat) measures distances in the
+// plane whatever z a state set later holds, so its codes leave z out.
 constexpr double kCodeUnits = 63.0;
 constexpr int kCodeBound = 4273;
 
 __device__ __forceinline__ uint32_t code_axis(float p, float mn, double inv, double shift) {
     return (uint32_t)__double2ll_rn(((double)p - (double)mn) * inv - shift) & 255u;
 }
-__device__ __forceinline__ uint32_t scan_code(float4 p, const SceneP& P) {
+__device__ __forceinline__ uint32_t scan_code(float4 p, const SceneP& P, uint32_t flat) {
+    const uint32_t z = flat ? 0u : code_axis(p.z, P.grid.min[2], P.code_inv, 0.0);
     return code_axis(p.x, P.grid.min[0], P.code_inv, 0.0) | code_axis(p.y, P.grid.min[1], P.code_inv, 0.0) << 8 |
-           code_axis(p.z, P.grid.min[2], P.code_inv, 0.0) << 16;
+           z << 16;
 }
+template <int DIM>  // 2 for a flat handle
 __device__ __forceinline__ uint32_t own_code(float4 p, const SceneP& P) {
+    const uint32_t z = DIM == 2 ? 0u : code_axis(p.z, P.grid.min[2], P.code_inv, 0.5);
     return code_axis(p.x, P.grid.min[0], P.code_inv, 0.0) | code_axis(p.y, P.grid.min[1], P.code_inv, 0.5) << 8 |
-           code_axis(p.z, P.grid.min[2], P.code_inv, 0.5) << 16;
+           z << 16;
 }
 // Negative when the candidate may lie within h.
 __device__ __forceinline__ int code_test(uint32_t candidate, uint32_t own) {

@@ -69,7 +69,7 @@ struct GroupScan {
         constexpr unsigned GM = LANES == 32 ? FULL : (1u << (LANES & 31)) - 1u;
         const uint32_t lane = threadIdx.x % LANES;
         const uint32_t gshift = (threadIdx.x & 31u) & ~(uint32_t)(LANES - 1);
-        const uint32_t own = own_code(xi, P);
+        const uint32_t own = own_code<DIM>(xi, P);
         // segments (end, first index - first number) of candidates, numbered 0 .. total over all rows
         uint32_t total = 0, nseg = 0;
         const SearchRows rows = search_rows<DIM>(xi, scan, P);

@@ -554,7 +554,7 @@ __device__ __forceinline__ Gathered gather_load(const GatherArgs& g, const Table
     const float p = eos_pressure(m.state_eq, pd.w, m.sound_speed, m.target_den);
     r.ps = p / (pd.w * pd.w);
     if (g.out.rec) {
-        r.code = scan_code(pd, T.scenes[m.scene]);
+        r.code = scan_code(pd, T.scenes[m.scene], T.flat);
         r.local = m.local;
     }
     return r;

@@ -1297,6 +1297,7 @@ arp_status allocate(arp_sim* S) {
     S->tables.ncells = S->ncells;
     S->tables.max_nmat = S->max_nmat;
     S->tables.nscenes = (uint32_t)S->scenes.size();
+    S->tables.flat = S->kdim == 2 ? 1u : 0u;
     return ARP_OK;
 }
 
