@@ -2329,12 +2329,13 @@ arp_status arp_sim_render_rgb24(arp_sim* sim, const arp_view* view, const arp_re
 
 arp_status arp_sim_set_solid_stiffness(arp_sim* sim, const float* normal_shear, uint32_t ns) {
     if (!sim) return fail(ARP_ERR_INVALID_ARG, "sim is null");
+    if (normal_shear && ns != sim->ns)
+        return fail(ARP_ERR_INVALID_ARG, "stiffness count differs from the number of solids");
+    sim->drop_graph();  // a graph's solid kernels read the stiffness they were captured with
     if (!normal_shear) {
         sim->have_stiff = false;
         return ARP_OK;
     }
-    if (ns != sim->ns) return fail(ARP_ERR_INVALID_ARG, "stiffness count differs from the number of solids");
-    sim->drop_graph();
     if (ns) {
         CUDA_TRY(sim->stiff.alloc(ns));
         CUDA_TRY(cudaMemcpyAsync(sim->stiff.p, normal_shear, ns * sizeof(float2), cudaMemcpyHostToDevice,
