@@ -1575,6 +1575,7 @@ arp_status arp_sim_destroy(arp_sim* sim) {
 
 arp_status arp_sim_init(arp_sim* sim) {
     if (!sim) return fail(ARP_ERR_INVALID_ARG, "sim is null");
+    sim->drop_graph();  // initialising again makes the reference lists anew
     ARP_TRY(do_init(sim));
     return run_autotune(sim, false);
 }
