@@ -213,14 +213,15 @@ struct GridBuffers {
 // order_cells.  Each returns the number of kernel launches issued.
 // The scene of item i is mats[material].scene, the material read from
 // vm[i].w (bits) when vm is given, else from mat_u32[i].
-// `zero2` (may be null) points at two counters to clear for the stage's later
+// `zero` (may be null) points at kStageWords words to clear for the stage's later
 // kernels.
+constexpr uint32_t kStageWords = 3;  // SolidArgs::contact_bound
 inline CellBins cell_bins(const GridBuffers& gb) { return CellBins{gb.key, gb.rank, gb.count, gb.coord}; }
 int bin_cells(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
-              GridBuffers& gb, uint32_t* zero2, cudaStream_t st);
+              GridBuffers& gb, uint32_t* zero, cudaStream_t st);
 // clears the counts if a state was scattered and never ordered
 void clear_cells(const Tables& T, GridBuffers& gb, cudaStream_t st);
-int scatter_cells(uint32_t n, const Tables& T, GridBuffers& gb, uint32_t* zero2, cudaStream_t st);
+int scatter_cells(uint32_t n, const Tables& T, GridBuffers& gb, uint32_t* zero, cudaStream_t st);
 int order_cells(const Tables& T, GridBuffers& gb, cudaStream_t st);
 int build_grid(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
                GridBuffers& gb, cudaStream_t st);
@@ -298,7 +299,8 @@ struct FluidArgs {
     const float4* ksol;      // per-solid solid-term acceleration (nullptr when the solid branch is off)
     uint32_t n;
     int solid_branch;
-    int beside_solids;       // the solid kernels were launched just before: only the epilogue waits for them
+    const uint32_t* published;  // the solid kernels were launched just before: a block that finds this word set
+                                // (step_begin_unless) waits for them only in its epilogue; null otherwise
 };
 // Launch shapes of the fluid kernel the autotuner chooses between: threads
 // per block and hit-list capacity of the block form (one thread per particle
@@ -356,7 +358,8 @@ struct SolidArgs {
     const float4* ep_prev2;
     float4* AF;               // [6*ns] stress records (stage scratch, solid_rec.cuh)
     float4* ksol;             // [ns] solid-term acceleration
-    uint32_t* contact_bound;  // [2] max |u_i - u_0| bits, outside-box flag (cleared per stage)
+    uint32_t* contact_bound;  // [kStageWords], cleared per stage: max |u_i - u_0| bits, outside-box flag, and 1 once
+                              // the stage's grid is known to be there (step_publish)
     const float4* rec;        // sorted stage state (current-neighbor loop, see FluidArgs)
     const uint32_t* mat;
     const uint32_t* start;

@@ -399,10 +399,10 @@ __device__ __forceinline__ float sum_partials(float v) {  // over the lanes that
 // particle alone 372 us; + quantised candidates 345 us; + 32-byte records 330 us;
 // + the next row's bounds and a second hit's record in flight 292 us.
 // Only the epilogue reads what the solid kernels write, so behind those
-// (a.beside_solids) a block waits there instead of at its start, and the pair
+// (a.published) a block waits there instead of at its start, and the pair
 // sums fill the SMs that the solid kernels' last blocks leave: ten RK2 steps of
-// the 1,048,576-particle scene 10,021 -> 9,905 us, 48 batched scenes 10,082 ->
-// 9,955, 16,899 particles under velocity Verlet 563 -> 550.
+// the 1,048,576-particle scene 10,067 -> 9,992 us, 48 batched scenes 10,012 ->
+// 9,873, 16,899 particles under velocity Verlet 560 -> 538.
 // kBlocksPerSM 128-thread blocks per SM (72 registers): 8 (64 registers, spills)
 // take 6 % more, 6 (80 registers) 2 % more.
 constexpr int kBlocksPerSM = 7;
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(BLOCK, kBlocksPerSM * 128 / BLOCK) k_fluid(Flu
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint32_t* const lists = reinterpret_cast<uint32_t*>(smem_raw);
     PairMat* const sm = reinterpret_cast<PairMat*>(smem_raw + sizeof(uint32_t) * STRIDE * BLOCK);
-    if (!a.beside_solids) step_begin();
+    step_begin_unless(a.published, kBlocksPerSM * 128 / BLOCK);
     const uint32_t k0 = blockIdx.x * BLOCK;
     const uint32_t scene0 = T.mats[a.mat[k0]].scene;  // k0 < n: one block per started tile
     {
@@ -653,7 +653,7 @@ __global__ void __launch_bounds__(kGroupBlock, LANES == 16 ? 8 : 7) k_fluid_grou
     __shared__ uint2 s_seg[NG][2 * GroupScan<DIM, LANES>::MAXROWS];
     __shared__ float4 s_term[LANES > 4 ? NG : 1][LANES];
     constexpr unsigned FULL = 0xFFFFFFFFu;
-    if (!a.beside_solids) step_begin();
+    step_begin_unless(a.published, LANES == 16 ? 8 : 7);
     const uint32_t lane = threadIdx.x % LANES, gi = threadIdx.x / LANES;
     const uint32_t kk = blockIdx.x * NG + gi;
     const bool valid = kk < a.n;

@@ -159,11 +159,11 @@ __global__ void __launch_bounds__(kThreads) k_scatter(const uint32_t* key,
                                                       const uint32_t* local,
                                                       const uint32_t* sums, uint32_t len,
                                                       uint32_t* start, uint32_t* perm,
-                                                      uint32_t* zero2) {
+                                                      uint32_t* zero) {
     __shared__ uint32_t tile_base[kBaseTiles];
     step_begin();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (zero2 && i < 2u) zero2[i] = 0u;
+    if (zero && i < kStageWords) zero[i] = 0u;
     // loads that do not need the bases first
     const bool mine = i < n;
     const uint32_t c = mine ? key[i] : 0u;
@@ -198,10 +198,10 @@ __global__ void __launch_bounds__(kThreads) k_scatter(const uint32_t* key,
 // The same scatter from finished cell starts (grids of more tiles).
 __global__ void k_scatter_plain(const uint32_t* key, const uint32_t* rank, uint32_t n,
                                 const uint32_t* start, uint32_t* perm,
-                                uint32_t* zero2) {
+                                uint32_t* zero) {
     step_begin();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (zero2 && i < 2u) zero2[i] = 0u;
+    if (zero && i < kStageWords) zero[i] = 0u;
     if (i < n) perm[start[key[i]] + rank[i]] = i;
 }
 
@@ -740,7 +740,7 @@ cudaError_t noalloc_scratch(uint32_t** out) {
 }  // namespace
 
 int bin_cells(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint32_t n, const Tables& T,
-              GridBuffers& gb, uint32_t* zero2, cudaStream_t st) {
+              GridBuffers& gb, uint32_t* zero, cudaStream_t st) {
     int launches = 0;
     clear_cells(T, gb, st);
     if (n > 0) {
@@ -750,7 +750,7 @@ int bin_cells(const float4* pos, const float4* vm, const uint32_t* mat_u32, uint
                                                                   T, cell_bins(gb));
         ++launches;
     }
-    return launches + scatter_cells(n, T, gb, zero2, st);
+    return launches + scatter_cells(n, T, gb, zero, st);
 }
 
 void clear_cells(const Tables& T, GridBuffers& gb, cudaStream_t st) {
@@ -760,21 +760,21 @@ void clear_cells(const Tables& T, GridBuffers& gb, cudaStream_t st) {
     gb.scattered = false;
 }
 
-int scatter_cells(uint32_t n, const Tables& T, GridBuffers& gb, uint32_t* zero2, cudaStream_t st) {
+int scatter_cells(uint32_t n, const Tables& T, GridBuffers& gb, uint32_t* zero, cudaStream_t st) {
     const uint32_t len = T.ncells + 2;  // cells, the non-finite bucket, and the total
     const uint32_t tiles = blocks_for(len, kScanTile);
     if (tiles > kBaseTiles) {
         // exclusive_scan clears the counts
         const int l = exclusive_scan(gb.count, len, gb.start, gb.block_sums, st);
         launch_step(k_scatter_plain, std::max(blocks_for(n, kThreads), 1u), kThreads, 0, st, gb.key, gb.rank, n, gb.start,
-                                                                                    gb.perm, zero2);
+                                                                                    gb.perm, zero);
         return l + 1;
     }
     gb.scattered = true;
     launch_step(k_scan_tiles<false>, tiles, kScanThreads, 0, st, gb.count, len, gb.count, gb.block_sums, true);
     const uint32_t work = std::max(n, (len + 3u) / 4u);
     launch_step(k_scatter, blocks_for(work, kThreads), kThreads, 0, st, gb.key, gb.rank, n, gb.count, gb.block_sums, len,
-                                                               gb.start, gb.perm, zero2);
+                                                               gb.start, gb.perm, zero);
     return 2;
 }
 

@@ -744,16 +744,16 @@ arp_status restore_checkpoint(arp_sim* S, const Checkpoint& c) {
 // current state), the kicked and drifted one, in X, with the plastic strain's
 // kick.
 void bin_state(arp_sim* S, bool prime) {
-    uint32_t* const zero2 = S->solid_branch() ? S->contact_bound.p : nullptr;
+    uint32_t* const zero = S->solid_branch() ? S->contact_bound.p : nullptr;
     if (!S->verlet() || prime) {
-        S->launches += bin_cells(S->Y.pd.p, S->Y.vm.p, nullptr, S->n, S->tables, S->gb, zero2, S->stream);
+        S->launches += bin_cells(S->Y.pd.p, S->Y.vm.p, nullptr, S->n, S->tables, S->gb, zero, S->stream);
         return;
     }
     const float half = (float)(S->tab.b[0] * (double)S->dt_sub);
     clear_cells(S->tables, S->gb, S->stream);
     S->launches += verlet_kick_drift(S->Y.pd.p, S->Y.vm.p, S->vforce.pd.p, S->vforce.vm.p, S->n, half, S->dt_sub,
                                      S->X.pd.p, S->X.vm.p, S->tables, cell_bins(S->gb), S->stream);
-    S->launches += scatter_cells(S->n, S->tables, S->gb, zero2, S->stream);
+    S->launches += scatter_cells(S->n, S->tables, S->gb, zero, S->stream);
     if (S->solid_branch() && S->any_plastic)
         S->launches += verlet_kick4(S->ep.p, S->ep_force.p, 4 * S->ns, half, S->ep_s[0].p, S->stream);
 }
@@ -797,7 +797,7 @@ arp_status do_step(arp_sim* S, bool prime = false) {
     // epilogue; for velocity Verlet the kicked and drifted one (storage order, in
     // X), which the grid and the force evaluation see
     const CellBins bins = cell_bins(S->gb);
-    uint32_t* const zero2 = sb ? S->contact_bound.p : nullptr;  // cleared with each stage's sort
+    uint32_t* const zero = sb ? S->contact_bound.p : nullptr;  // cleared with each stage's sort
     const float4* src_pd = S->Y.pd.p;
     const float4* src_vm = S->Y.vm.p;
     if (S->standalone) {
@@ -964,7 +964,7 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         f.ksol = sb ? S->ksol.p : nullptr;
         f.n = n;
         f.solid_branch = sb ? 1 : 0;
-        f.beside_solids = sl && !R ? 1 : 0;  // a tape's copies lie between the two
+        f.published = sl && !R ? S->contact_bound.p + 2 : nullptr;  // a tape's copies lie between the two
         B.next_pd = next_pd;
         B.next_vm = next_vm;
         // the next state's cells: the next stage's grid, or the next step's
@@ -972,7 +972,7 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         B.drift_vm = verlet && count_next ? S->X.vm.p : nullptr;
         B.bin = count_next ? bins : CellBins{};
         int fl = launch_fluid(f, S->tables, S->kdim, c, B, S->fluid_variant, st);
-        if (count_next) fl += scatter_cells(n, S->tables, S->gb, zero2, st);
+        if (count_next) fl += scatter_cells(n, S->tables, S->gb, zero, st);
         S->launches += fl;
         mark(S, mk, 3);
         if (S->profiling) {
@@ -1223,7 +1223,7 @@ arp_status allocate(arp_sim* S) {
     CUDA_TRY(S->L.alloc(3 * ns));
     CUDA_TRY(S->AF.alloc(6 * ns));
     CUDA_TRY(S->ksol.alloc(ns));
-    CUDA_TRY(S->contact_bound.alloc(2));
+    CUDA_TRY(S->contact_bound.alloc(kStageWords));
     CUDA_TRY(S->ep.alloc(4 * ns));
     CUDA_TRY(S->ep_t.alloc(4 * ns));
     CUDA_TRY(S->sx.alloc(2 * ns));

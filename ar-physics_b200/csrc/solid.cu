@@ -281,6 +281,8 @@ __device__ __forceinline__ T3 stress_order2(const T3& F, const T3& Fd, float lam
 template <bool ORDER2, bool PLASTIC, int LANES>
 __global__ void __launch_bounds__(kThreads) k_solid_stress(SolidArgs a, Tables T, StageCoefs c) {
     step_begin();
+    // a block of its own hands the wait's order on, so that no solid waits for the release
+    if (blockIdx.x == gridDim.x - 1u && threadIdx.x == 0) step_publish(a.contact_bound + 2);
     step_let_next();  // after the wait: the kernels let in rely on the grid being there
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = t / LANES, lane = t % LANES;
@@ -623,17 +625,18 @@ namespace {
 template <int L>
 void launch_solid_lanes(const SolidArgs& a, const Tables& T, const StageCoefs& c, cudaStream_t st) {
     const uint32_t blocks = blocks_for(a.ns * L, kThreads);
-    if (a.all_order2 && !a.any_plastic) launch_step(k_solid_stress<true, false, L>, blocks, kThreads, 0, st, a, T, c);
-    else if (a.all_order2) launch_step(k_solid_stress<true, true, L>, blocks, kThreads, 0, st, a, T, c);
-    else if (!a.any_plastic) launch_step(k_solid_stress<false, false, L>, blocks, kThreads, 0, st, a, T, c);
-    else launch_step(k_solid_stress<false, true, L>, blocks, kThreads, 0, st, a, T, c);
+    const uint32_t more = blocks + 1u;  // and the block that publishes
+    if (a.all_order2 && !a.any_plastic) launch_step(k_solid_stress<true, false, L>, more, kThreads, 0, st, a, T, c);
+    else if (a.all_order2) launch_step(k_solid_stress<true, true, L>, more, kThreads, 0, st, a, T, c);
+    else if (!a.any_plastic) launch_step(k_solid_stress<false, false, L>, more, kThreads, 0, st, a, T, c);
+    else launch_step(k_solid_stress<false, true, L>, more, kThreads, 0, st, a, T, c);
     launch_step(k_solid_forces<L>, blocks, kThreads, 0, st, a, T);
 }
 }  // namespace
 
 int launch_solid(const SolidArgs& a, const Tables& T, const StageCoefs& c, cudaStream_t st) {
     if (a.ns == 0) return 0;
-    if (!a.counters_cleared) cudaMemsetAsync(a.contact_bound, 0, 2 * sizeof(uint32_t), st);
+    if (!a.counters_cleared) cudaMemsetAsync(a.contact_bound, 0, kStageWords * sizeof(uint32_t), st);
     // a.sx (its stage half), a.sv and a.sc were written by the stage's gather (gather_state)
     if (a.ns <= kFewSolids) launch_solid_lanes<4>(a, T, c, st);
     else launch_solid_lanes<2>(a, T, c, st);
