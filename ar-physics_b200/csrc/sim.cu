@@ -1309,14 +1309,20 @@ arp_status allocate(arp_sim* S) {
 // dimension, quarter-octaves of the particle count and of h / particle spacing):
 // how many waves of blocks a group form takes changes within an octave (solids,
 // 31,200: 290 us a step with 16 threads, chosen at 19,496 particles, against 258
-// with 4).  A shape's time is the least of kTuneRounds, since the first launches
-// may run while the clocks still rise.
+// with 4).  A program that makes handles of many sizes therefore tunes up to four
+// times an octave, 35 to 160 launches each time; handles of one size tune once.
+// Every shape that is timed gets the same: a first launch that is not counted,
+// then the least of kTuneRounds rounds of kTuneLaunches launches (of one where
+// only the block form is left and a launch is long), the shapes in turn within a
+// round, so that clocks which still rise meet all of them alike.
 // Sizes at which a form cannot win are left out: the group form above
-// kGroupMost particles (126,464 in 3D: 86 us against 62; 1.05 M: 600 against
-// 290), the block form below kBlockLeast (24,706 in 3D: ten steps 1312 us
-// against 986; 22,500 in 2D: 1145 against 899).
+// kGroupMost particles (us a stage, graphs, group against block; 3D: 53,280
+// particles 64 / 71, 72,450 79 / 74, 140,872 115 / 94; 2D: 32,400 22 / 26, 62,500
+// 31 / 29, 131,044 49 / 36, 250,000 79 / 55), the block form below kBlockLeast
+// (3D: 15,744 particles 35 / 49, 30,800 48 / 68; 2D: 12,100 18 / 26, 25,600
+// 21 / 26).
 constexpr uint32_t kGroupMost = 131072, kBlockLeast = 24576;
-constexpr int kTuneRounds = 3;
+constexpr int kTuneRounds = 3, kTuneLaunches = 3;
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int>, int> g_tune_cache;
 
@@ -1386,13 +1392,15 @@ arp_status run_autotune(arp_sim* S, bool force) {
     cudaEvent_t e0 = take_event(S), e1 = take_event(S);
     float best = 1e30f;
     int best_v = 0;
-    for (int v = 0; v < kNumFluidVariants; ++v) {
-        const FluidVariant& fv = kFluidVariants[v];
-        if (fv.lanes ? n > kGroupMost : n < kBlockLeast) continue;
-        S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, st);  // warm-up
-        for (int round = 0; round < (fv.lanes ? kTuneRounds : 1); ++round) {
+    auto left_out = [&](int v) { return kFluidVariants[v].lanes ? n > kGroupMost : n < kBlockLeast; };
+    for (int v = 0; v < kNumFluidVariants; ++v)
+        if (!left_out(v)) S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, st);  // warm-up
+    const int launches = n > kGroupMost ? 1 : kTuneLaunches;
+    for (int round = 0; round < kTuneRounds; ++round) {
+        for (int v = 0; v < kNumFluidVariants; ++v) {
+            if (left_out(v)) continue;
             CUDA_TRY(cudaEventRecord(e0, st));
-            for (int r = 0; r < 3; ++r) S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, st);
+            for (int r = 0; r < launches; ++r) S->launches += launch_fluid(f, S->tables, S->kdim, c, B, v, st);
             CUDA_TRY(cudaEventRecord(e1, st));
             CUDA_TRY(cudaEventSynchronize(e1));
             float ms = 0;
