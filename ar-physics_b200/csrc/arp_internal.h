@@ -102,10 +102,9 @@ struct SceneP {
     double code_inv;                  // kCodeUnits / h: scale of the quantised positions (scan_code)
 };
 
-// The fields of a material the fluid pair loop reads (32 B).
+// The fields of a material the reverse pass's pair loop reads (16 B).
 struct FluidMat {
-    float mass, c, d0, visc, bulk;
-    uint32_t eos, stiff, pad;
+    float mass, visc, bulk, pad;
 };
 
 // What the fluid pair terms read of a pair of materials (16 B, one load): the
@@ -158,7 +157,6 @@ struct CellBins {
 // k_stage, and on the last stage y_new = y0 + acc.  Stage derivatives that a
 // later stage reads are stored (non-diagonal tableaus only).
 struct StageCoefs {
-    int stage;          // 0-based
     int last;           // 1 when this stage ends the step
     float c_prev0, c_prev1, c_prev2;  // a[stage+1][j] * dt for j < stage
     float c_self;       // a[stage+1][stage] * dt (unused when last)
@@ -200,7 +198,6 @@ struct GridBuffers {
     uint32_t* perm;        // [cap] sorted index -> slot
     uint2* coord;          // [cap] packed cell coordinates of each slot: x | y << 16, z
     uint32_t* block_sums;  // scan partials
-    uint32_t block_sums_cap;
     bool scattered;        // count holds a prefix that the ordering has not cleared yet (a graph replay of a step
                            // begins and ends with the same value)
 };

@@ -6,8 +6,12 @@
 
 namespace arp {
 
-// The rows of search cells around a particle: row q (ascending z, then y; the
-// order of for_search_rows) spans `width` cells from search_row(q) on.
+// The rows of search cells around a particle, 2 cells each way along a halved
+// axis and 1 along the others: row q (ascending z, then y) spans `width` cells
+// from search_row(q) on.  Every particle within h lies in them (search cells are
+// at least h/2 wide on halved axes and h wide on the others).  The rows are not
+// clipped to the sphere: the lanes of a warp walk rows of equal length, which a
+// clip would only make uneven without shortening the longest.
 struct SearchRows {
     int y, z, x0, ry, nrows;
     uint32_t width;

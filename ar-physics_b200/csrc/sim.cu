@@ -432,7 +432,6 @@ arp_status ensure_grid(arp_sim* S, uint32_t cap) {
     S->gb.perm = S->g_perm.p;
     S->gb.coord = S->g_coord.p;
     S->gb.block_sums = S->g_bsums.p;
-    S->gb.block_sums_cap = (uint32_t)S->g_bsums.n;
     return ARP_OK;
 }
 
@@ -842,7 +841,6 @@ arp_status do_step(arp_sim* S, bool prime = false) {
         const bool last = !prime && s == tab.stages - 1;
         const bool count_next = !S->standalone || !(last || prime);  // the written state is counted into cells
         StageCoefs c{};
-        c.stage = s;
         c.last = last ? 1 : 0;
         float cp[3] = {0.f, 0.f, 0.f};
         if (!last) {
@@ -1258,8 +1256,7 @@ arp_status allocate(arp_sim* S) {
     CUDA_TRY(cudaMemcpy(S->d_mats.p, dm.data(), S->M * sizeof(DevMat), cudaMemcpyHostToDevice));
     std::vector<FluidMat> fm(S->M);
     for (uint32_t i = 0; i < S->M; ++i)
-        fm[i] = FluidMat{dm[i].mass, dm[i].sound_speed, dm[i].target_den, dm[i].visc, dm[i].bulk_visc, dm[i].state_eq,
-                         dm[i].stiff, 0u};
+        fm[i] = FluidMat{dm[i].mass, dm[i].visc, dm[i].bulk_visc, 0.0f};
     CUDA_TRY(S->d_fmats.alloc(S->M));
     CUDA_TRY(cudaMemcpy(S->d_fmats.p, fm.data(), S->M * sizeof(FluidMat), cudaMemcpyHostToDevice));
     std::vector<SceneP> sp;
