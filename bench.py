@@ -266,17 +266,15 @@ def cpu_baseline(config, steps=20, warmup=1):
     return json.loads(r.stdout.strip().splitlines()[-1])
 
 
-def run_batched(torch, stream, rank=0, world=1, steps_batch=200, rounds_loop=10, steps_variant=200):
+def run_batched(torch, stream, rank=0, world=1, steps_batch=200, rounds_loop=10):
     """256 independent scenes (2,048-65,536 particles each, own h, fluid
     blocks and elastic blocks): stepped as one batch (one set of launches per
     stage) and as a loop over 256 separate simulations, both on one GPU and
     both replaying each step from a CUDA graph.  The batch is timed over the
-    configuration's 200 steps with the autotuner's launch shape; any
-    launch shape that takes tiles from a persistent queue (today none does) is
-    timed beside it over the same 200 steps from the same state.  With N ranks the scenes are
-    sharded (scenes.partition_scenes, by particle count) and each rank steps
-    its share; every time is the slowest rank's, and rates count all 256
-    scenes."""
+    configuration's 200 steps with the autotuner's launch shape.  With N ranks
+    the scenes are sharded (scenes.partition_scenes, by particle count) and each
+    rank steps its share; every time is the slowest rank's, and rates count all
+    256 scenes."""
     from arphys import FluidSim, scenes
     everything = scenes.batched_scenes()
     mine = scenes.partition_scenes([sc.n + sc.nb for sc in everything], world)[rank]
@@ -297,23 +295,6 @@ def run_batched(torch, stream, rank=0, world=1, steps_batch=200, rounds_loop=10,
     torch.cuda.synchronize()
     t_batch = max_over_ranks(e0.elapsed_time(e1) / 1000.0, "cuda")
     variant = batch.fluid_variant()
-    # the persistent (scene, cell-tile) work-queue shapes, same state, same steps each
-    shapes = {}
-    for v in range(FluidSim.fluid_variant_count()):
-        batch.set_fluid_variant(v)
-        vi = batch.fluid_variant()
-        if not vi["persistent"]:
-            continue
-        batch.set_particles(init)
-        batch.step(2)  # captures this shape's step graphs
-        batch.set_particles(init)
-        e0.record(stream)
-        batch.step(steps_variant)
-        e1.record(stream)
-        torch.cuda.synchronize()
-        shapes[str(v)] = dict(vi, ms_per_step=max_over_ranks(e0.elapsed_time(e1), "cuda") / steps_variant)
-    batch.set_fluid_variant(variant["variant"])
-    best_pers = min(shapes, key=lambda k: shapes[k]["ms_per_step"]) if shapes else None
     # where a batch step goes: a few more steps, untimed, with the library's
     # per-segment events (graph replay off: the events sit between launches)
     batch.set_graph(False)
@@ -350,8 +331,7 @@ def run_batched(torch, stream, rank=0, world=1, steps_batch=200, rounds_loop=10,
             "scene_steps_per_s": batched, "particle_steps_per_s": parts_all * steps_batch / t_batch,
             "ms_per_step": t_batch * 1000.0 / steps_batch,
             "per_scene_loop_scene_steps_per_s": loop, "speedup_vs_per_scene_loop": batched / loop,
-            "fluid_launch_shape": variant, "persistent_shapes": shapes, "best_persistent_shape": best_pers,
-            "segments_ms_per_step": segments,
+            "fluid_launch_shape": variant, "segments_ms_per_step": segments,
             "solids": int(sum(sc.n_solids() for sc in scs)),
             "note": ("no L2 flush: the batch's state (~%d MB) is larger than L2; both the batch and the "
                      "per-scene loop (%d rounds of one step per simulation) replay CUDA graphs"
@@ -650,10 +630,12 @@ def run_ours(args, rank, world, local_rank):
     alg_bytes = 96.0 * sc.n  # per stage: read y_s 32 B + read y0 32 B + write y_{s+1} 32 B per particle
     achieved = alg_bytes / (fluid_ms / 1000.0) / 1e9
     traffic = load_traffic().get(f"fluid_{args.config}")
-    roofline = {"bound": "hbm", "kernel": "k_fluid (fused fluid forces + RK stage update)",
+    roofline = {"bound": "hbm",
+                "kernel": "fluid segment of a stage: k_fluid (fluid forces + RK stage update + next cells), and the "
+                          "next grid's k_scan_tiles and k_scatter",
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_kind": peak_kind, "traffic": traffic, "alg_bytes_per_launch": alg_bytes,
-                "avg_launch_ms": fluid_ms,
+                "avg_segment_ms": fluid_ms,
                 "segments_ms_per_step": {k: prof[k] / max(prof["steps"], 1) for k in
                                          ("neighbor_ms", "solid_ms", "fluid_ms")}}
     stages = fl / max(prof["steps"], 1)
@@ -661,8 +643,9 @@ def run_ours(args, rank, world, local_rank):
     roofline["pairs"] = pair_rate(sc, stages, prof["fluid_ms"] / max(prof["steps"], 1))
     issue = load_issue().get(f"fluid_{args.config}_v{sim.fluid_variant()['variant']}")
     if issue:
-        # the issue roofline: every warp instruction of a launch issued at one
-        # per scheduler per cycle (148 SMs x 4 schedulers at the sampled clock)
+        # the issue roofline: every warp instruction of a launch of k_fluid issued
+        # at one per scheduler per cycle (148 SMs x 4 schedulers at the sampled
+        # clock), over the time of the segment
         mhz = clocks.get("sm_mhz") or 1965.0
         t_issue = issue["warp_instructions"] / (148 * 4 * mhz * 1e6) * 1e3
         lanes = issue["warp_instructions"] * 32.0

@@ -165,9 +165,10 @@ typedef struct arp_sim arp_sim;
 typedef struct arp_profile {
     uint64_t steps;              /* integrator steps since the last read */
     uint64_t launches;           /* kernels launched by the handle since the last read */
-    double neighbor_ms;          /* grid build: keys, histogram, scan, scatter, reorder */
+    double neighbor_ms;          /* grid build: reorder, and the passes before it of a state no step has written */
     double solid_ms;             /* deformation gradient, stress, solid forces */
-    double fluid_ms;             /* fluid forces + fused stage update */
+    double fluid_ms;             /* fluid forces + fused stage update, with the keys and histogram, scan and scatter
+                                    of the state it writes (the next grid build's first passes) */
     double integrate_ms;         /* stand-alone stage arithmetic (non-fused paths) */
     uint64_t fluid_launches;
     uint64_t neighbor_launches;
