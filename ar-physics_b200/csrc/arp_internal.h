@@ -120,6 +120,7 @@ struct PairMat {
 constexpr uint32_t kPairPotential = 0xFFu;    // bits: contact potential id
 constexpr uint32_t kPairElastic1 = 0x100u;    // the particle's own material is elastic
 constexpr uint32_t kPairElastic2 = 0x200u;    // the neighbor's material is elastic
+constexpr uint32_t kPairContact = 0x80000000u;  // the pair has a contact potential
 
 // Kernel-wide view of the batch tables.
 struct Tables {

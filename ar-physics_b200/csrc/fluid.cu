@@ -209,32 +209,27 @@ __device__ __forceinline__ float4 axpy(float c, float4 k, float4 t) {
 // a boundary particle one of at least n.
 
 // Pair terms of neighbor j added to `acc` if j lies within the kernel radius
-// (the scan's test lets a few others through); the pair's material bits are
-// or-ed into `bits`.  r^2 < h^2 is h^2 - r^2 > 0, grad_w's max(.., 0) test:
+// (the scan's test lets a few others through); returns the pair's material bits
+// then, kPairContact the highest, and 0 otherwise.  r^2 < h^2 is h^2 - r^2 > 0, grad_w's max(.., 0) test:
 // without flush-to-zero a difference of finite floats is zero only when they
 // are equal.
 template <int DIM>
-__device__ __forceinline__ void add_hit(Acc& acc, uint32_t j, const PairRec& rj, uint32_t mat2, const Self& s,
-                                        const FluidArgs& a, const PairK& K, uint32_t& bits) {
+__device__ __forceinline__ uint32_t add_hit(Acc& acc, uint32_t j, const PairRec& rj, uint32_t mat2, const Self& s,
+                                            const FluidArgs& a, const PairK& K) {
     const PairMat m = s.pm[mat2];
     const PairGeom g = pair_geom<DIM>(s, rj, K);
     const float4 t = pair_terms<DIM>(s, g, rj.x.w, rj.v.w, j >= a.n, m, K);
-    if (g.r2 < K.h2) {
-        add_terms(acc, t);
-        bits |= m.bits;
-    }
+    const bool in = g.r2 < K.h2;
+    if (in) add_terms(acc, t);
+    return in ? m.bits : 0u;
 }
-// The contact terms of neighbor j, if there are any.  `it`: the interactions of
-// the particle's material.
+// The contact terms of neighbor j, for which add_hit returned kPairContact.  `it`:
+// the interactions of the particle's material.
 template <int DIM>
-__device__ __forceinline__ void add_hit_contact(Acc& acc, uint32_t j, const Self& s, const FluidArgs& a,
-                                                const DevInter* it, const PairK& K) {
-    const uint32_t mat2 = a.mat8[j];
+__device__ __forceinline__ void add_hit_contact(Acc& acc, uint32_t j, const PairRec& rj, uint32_t mat2, const Self& s,
+                                                const FluidArgs& a, const DevInter* it, const PairK& K) {
     const PairMat m = s.pm[mat2];
-    if ((m.bits & kPairPotential) == ARP_CONTACT_ZERO) return;
-    const PairRec rj = load_hit(a.rec, j);
     const PairGeom g = pair_geom<DIM>(s, rj, K);
-    if (!(g.r2 < K.h2)) return;
     const bool rubs = j >= a.n || (m.bits & (kPairElastic1 | kPairElastic2));
     add_contact(acc, contact_terms<DIM>(s, g, rj.x.w, m.mass, mat2, rubs, it[mat2]));
 }
@@ -564,23 +559,29 @@ __global__ void __launch_bounds__(BLOCK, kBlocksPerSM * 128 / BLOCK) k_fluid(Flu
                 Self s;
                 const SceneP& P = init_self(ko, a, T, sm, scene0, s);
                 const PairK K{P.h2, -6.0f * P.kconst, P.eps_hh};
-                uint32_t bits = 0;
+                uint32_t rubbing = 0;  // a bit for each of the thread's hits: the pair has a contact potential
+                static_assert(CAP / kPartials <= 32, "32 bits");
 #pragma unroll 1
                 for (uint32_t e = q; e < n_ev; e += 2 * kPartials) {  // two hits' loads in flight
                     const bool two = e + kPartials < n_ev;
                     const uint32_t j0 = lists[list + e], j1 = two ? lists[list + e + kPartials] : ko;
                     const PairRec r0 = load_hit(a.rec, j0), r1 = load_hit(a.rec, j1);
                     const uint32_t m0 = a.mat8[j0], m1 = a.mat8[j1];
-                    if (j0 != ko) add_hit<DIM>(part, j0, r0, m0, s, a, K, bits);
-                    if (j1 != ko) add_hit<DIM>(part, j1, r1, m1, s, a, K, bits);
+                    const uint32_t c0 = j0 != ko ? add_hit<DIM>(part, j0, r0, m0, s, a, K) : 0u;
+                    rubbing = __funnelshift_l(c0, rubbing, 1);
+                    const uint32_t c1 = j1 != ko ? add_hit<DIM>(part, j1, r1, m1, s, a, K) : 0u;
+                    rubbing = __funnelshift_l(c1, rubbing, 1);
                 }
-                if (bits & kPairPotential) {
+                if (rubbing) {
                     const DevInter* const it = T.inter + P.inter_base + s.mat * P.nmat;
+                    rubbing <<= 32u - 2u * ((n_ev - q + 2 * kPartials - 1) / (2 * kPartials));  // bit 31 - i: hit q + 4 i
 #pragma unroll 1
-                    for (uint32_t e = q; e < n_ev; e += kPartials) {
-                        const uint32_t j = lists[list + e];
-                        if (j != ko) add_hit_contact<DIM>(part, j, s, a, it, K);
-                    }
+                    do {
+                        const uint32_t i = (uint32_t)__clz((int)rubbing);
+                        rubbing ^= 0x80000000u >> i;
+                        const uint32_t j = lists[list + q + kPartials * i];
+                        add_hit_contact<DIM>(part, j, load_hit(a.rec, j), a.mat8[j], s, a, it, K);
+                    } while (rubbing);
                 }
             }
             __syncwarp();
@@ -692,28 +693,34 @@ __global__ void __launch_bounds__(kGroupBlock, LANES == 16 ? 8 : 7) k_fluid_grou
     bool any_con = false;
     GroupScan<DIM, LANES>::run(xi, valid && finite3(xi), P, ScanArrays{a.code, a.start, a.bstart, a.n}, list, s_seg[gi],
                                [&](uint32_t ev) {
-        uint32_t bits = 0;
+        uint32_t rubbing = 0, e0 = 0;  // a bit for each of the lane's hits: the pair has a contact potential
+        static_assert(kGroupList / LANES <= 32, "32 bits");
 #pragma unroll 1
-        for (uint32_t e0 = 0; __any_sync(FULL, e0 < ev); e0 += LANES) {
+        for (; __any_sync(FULL, e0 < ev); e0 += LANES) {
             Acc t;
+            uint32_t c = 0u;
             t.den = 0.0f;
             t.f = make_float3(0.f, 0.f, 0.f);
             if (e0 + lane < ev) {
                 const uint32_t j = list[e0 + lane];
-                if (j != k) add_hit<DIM>(t, j, load_hit(a.rec, j), a.mat8[j], s, a, K, bits);
+                if (j != k) c = add_hit<DIM>(t, j, load_hit(a.rec, j), a.mat8[j], s, a, K);
             }
+            rubbing = __funnelshift_l(c, rubbing, 1);
             add(acc, make_float4(t.den, t.f.x, t.f.y, t.f.z));
         }
-        if (__any_sync(FULL, (bits & kPairPotential) != 0u)) {
+        if (__any_sync(FULL, rubbing != 0u)) {
             any_con = true;
             const DevInter* const it = T.inter + P.inter_base + s.mat * P.nmat;
+            rubbing <<= 32u - e0 / LANES;
 #pragma unroll 1
-            for (uint32_t e0 = 0; __any_sync(FULL, e0 < ev); e0 += LANES) {
+            for (uint32_t e = lane; __any_sync(FULL, rubbing != 0u); e += LANES, rubbing <<= 1) {
+                const bool mine = (rubbing & kPairContact) != 0u;  // the highest
+                if (!__any_sync(FULL, mine)) continue;
                 Acc t;
                 t.c = make_float3(0.f, 0.f, 0.f);
-                if (e0 + lane < ev) {
-                    const uint32_t j = list[e0 + lane];
-                    if (j != k) add_hit_contact<DIM>(t, j, s, a, it, K);
+                if (mine) {
+                    const uint32_t j = list[e];
+                    add_hit_contact<DIM>(t, j, load_hit(a.rec, j), a.mat8[j], s, a, it, K);
                 }
                 add(con, make_float4(0.f, t.c.x, t.c.y, t.c.z));
             }
