@@ -586,17 +586,23 @@ __global__ void k_gather_state(const uint32_t* __restrict__ perm, uint32_t n, Ga
 }
 
 // Orders the block's cells and gathers the state of their particles.  With
-// `stats` the grid is twice as long: the second half takes the occupancy counters
-// of the reference cells, a chain of reads of its own that would double the
-// latency of the ordering in a scene that leaves SMs idle.
+// `stats` and up to kCountBeside blocks the grid is twice as long: the second half
+// takes the occupancy counters of the reference cells, a chain of reads of its own
+// that would double the latency of the ordering in a scene that leaves SMs idle.
+// In larger grids, most of whose blocks are empty, each block counts its own
+// cells: twice as many blocks cost more than the chain (us a stage, beside / by
+// itself: 4,820 blocks of a batch 33 / 37, 8,790 29 / 27, 55,962 161 / 128).
+// `count` (null: the scan has done it) is cleared on the way.
+constexpr uint32_t kCountBeside = 8192;
 __global__ void __launch_bounds__(kThreads) k_order_gather(const uint32_t* start, uint32_t ncells, uint32_t nblocks,
                                                            uint32_t* perm, uint32_t* tmp, const uint32_t* key,
                                                            uint32_t* count,
                                                            const uint32_t* boundary_start, DevStats* stats,
                                                            GatherArgs g, Tables T) {
     step_begin();
-    if (blockIdx.x >= nblocks) {
-        const uint32_t c = (blockIdx.x - nblocks) * kThreads + threadIdx.x;
+    const bool counts = blockIdx.x >= nblocks;
+    const uint32_t c = (counts ? blockIdx.x - nblocks : blockIdx.x) * kThreads + threadIdx.x;
+    if (counts || (stats && gridDim.x == nblocks)) {
         const uint32_t occ = c < ncells ? reference_cell_occupancy(c, start, boundary_start, T) : 0u;
         const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, occ);
         const uint32_t over = __popc(__ballot_sync(0xFFFFFFFFu, occ > kBucketSlots));
@@ -604,10 +610,9 @@ __global__ void __launch_bounds__(kThreads) k_order_gather(const uint32_t* start
             if (most > 0u) atomicMax(&stats->max_cell_occupancy, most);
             if (over > 0u) atomicAdd(&stats->overflow_cells, over);
         }
-        return;
+        if (counts) return;
     }
-    const uint32_t c = blockIdx.x * kThreads + threadIdx.x;
-    if (c < ncells + 2u) count[c] = 0u;  // ready for the next histogram
+    if (count && c < ncells + 2u) count[c] = 0u;  // ready for the next histogram
     order_block<true>(start, ncells, perm, tmp, key, [&](uint32_t v) { return gather_load(g, T, v); },
                 [&](uint32_t at, uint32_t v, const Gathered& r) {
                     perm[at] = v;
@@ -778,21 +783,28 @@ int scatter_cells(uint32_t n, const Tables& T, GridBuffers& gb, uint32_t* zero, 
     return 2;
 }
 
-int order_cells(const Tables& T, GridBuffers& gb, cudaStream_t st) {
+// the counts for an ordering to clear: none where the scan has cleared them
+static uint32_t* take_counts(GridBuffers& gb) {
+    uint32_t* const count = gb.scattered ? gb.count : nullptr;
     gb.scattered = false;
+    return count;
+}
+
+int order_cells(const Tables& T, GridBuffers& gb, cudaStream_t st) {
+    uint32_t* const count = take_counts(gb);
     launch_step(k_order, blocks_for(T.ncells + 2, kThreads), kThreads, 0, st, gb.start, T.ncells, gb.perm, gb.rank,
-                gb.count);
+                count);
     return 1;
 }
 
 int order_gather(const Tables& T, GridBuffers& gb, const uint32_t* boundary_start, const float4* pd_in, float4* pd_out,
                  const float4* vm_in, float4* vm_out, const uint32_t* a_in, uint32_t* a_out, const uint32_t* b_in,
                  uint32_t* b_out, cudaStream_t st, const SolidScatter& sol, DevStats* stats, const PairOut& out) {
-    gb.scattered = false;
+    uint32_t* const count = take_counts(gb);
     const GatherArgs g{pd_in, vm_in, pd_out, vm_out, a_in, b_in, a_out, b_out, nullptr, sol, stats, out};
     const uint32_t nb = blocks_for(T.ncells + 2, kThreads);
-    launch_step(k_order_gather, stats ? 2 * nb : nb, kThreads, 0, st, gb.start, T.ncells, nb, gb.perm, gb.rank, gb.key,
-                gb.count, boundary_start, stats, g, T);
+    launch_step(k_order_gather, stats && nb <= kCountBeside ? 2 * nb : nb, kThreads, 0, st, gb.start, T.ncells, nb, gb.perm, gb.rank, gb.key,
+                count, boundary_start, stats, g, T);
     return 1;
 }
 
