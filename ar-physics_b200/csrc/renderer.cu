@@ -346,9 +346,18 @@ __global__ void __launch_bounds__(kCompWarps * 32) k_rp_composite(const float4* 
 // drawn on ties): min over (window depth bits, draw order).  Bound by the
 // atomics: with one for every covered pixel, and both offsets divided for every
 // pixel, 62 us for 314,000 sprites 64 layers deep; 42 now.
+// LANES threads take the rows of one sprite in turn: a thread that walks a large
+// sprite alone waits for what its pixels hold row after row.  Frames (ms), 1 / 8
+// threads, sprites of 15, 32, 100 and 400 pixels: 314,000 at 1080p 0.41 / 0.45,
+// 0.52 / 0.50, 1.6 / 1.2, 17.8 / 11.3; 100 at 720p 0.23 / 0.23, 0.30 / 0.23,
+// 1.0 / 0.35, 15.1 / 2.1 (6.4 with an atomic for every covered pixel).  32
+// threads: 0.57, 0.65, 1.7, 20.0 and 0.23, 0.23, 0.26, 0.85.
+constexpr int kDepthBlock = 128, kDepthLanes = 8;
+constexpr float kDepthAlone = 16.0f;  // sprites up to this size: a thread each
+template <int LANES>
 __global__ void k_rp_depth(const float4* __restrict__ PR, const float4* __restrict__ PC, RenderCfg c,
                            unsigned long long* __restrict__ zkey) {
-    const uint32_t prim = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t prim = blockIdx.x * (kDepthBlock / LANES) + threadIdx.x / LANES;
     if (prim >= c.nprims) return;
     const float4 r = PR[prim];
     if (PC[prim].w == 0.0f || !(r.w < 1.0f) || !(r.w >= 0.0f)) return;
@@ -365,7 +374,7 @@ __global__ void k_rp_depth(const float4* __restrict__ PR, const float4* __restri
             const float dx = ib + u <= i1 && in_square(c, r.x, f) ? sprite_dx(c, r, f) : INFINITY;
             dx2[u] = __fmul_rn(dx, dx);
         }
-        for (int j = j0; j <= j1; ++j) {
+        for (int j = j0 + (int)(threadIdx.x % LANES); j <= j1; j += LANES) {
             if (!in_square(c, r.y, j + 0.5f)) continue;
             const float dy = sprite_dy(c, r, j + 0.5f), dy2 = __fmul_rn(dy, dy);
             if (!(dy2 <= 1.0f)) continue;  // no pixel of the row is covered
@@ -453,7 +462,10 @@ int render_lit(const float4* PR, const float4* PC, const float4* PP, const Rende
                uint8_t* rgb, cudaStream_t st) {
     int launches = 0;
     if (c.nprims) {
-        k_rp_depth<<<nblk(c.nprims, 128), 128, 0, st>>>(PR, PC, c, zkey);
+        if (c.S <= kDepthAlone)
+            k_rp_depth<1><<<nblk(c.nprims, kDepthBlock), kDepthBlock, 0, st>>>(PR, PC, c, zkey);
+        else
+            k_rp_depth<kDepthLanes><<<nblk(c.nprims, kDepthBlock / kDepthLanes), kDepthBlock, 0, st>>>(PR, PC, c, zkey);
         ++launches;
     }
     k_rp_shade<<<nblk(c.W * c.H, 256), 256, 0, st>>>(PR, PC, PP, c, zkey, rgb);
