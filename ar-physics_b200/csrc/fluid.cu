@@ -149,8 +149,11 @@ __device__ __forceinline__ float4 pair_terms(const Self& s, const PairGeom& g, f
 // The contact potential and friction of one pair (fluid.rs:176-199).  Few
 // pairs have one, and its registers would cost every pair a quarter of the
 // resident warps (94 registers against 64), so contacts are evaluated in a
-// second walk over the hits, taken only where some hit has one, and have sums
-// of their own.
+// second walk, over the hits that the first has marked, and have sums of their
+// own.  A second walk over all hits wherever some had one took 65 us for 97,336
+// particles with a contact in every pair (58 now, 47 without contacts) and 62 of
+// 81 us a stage in a scene where a bar touches fluid (53 of 72 now); two marked
+// hits' loads in flight spill.
 template <int DIM>
 __device__ __forceinline__ float3 contact_terms(const Self& s, const PairGeom& g, float d2, float mass2, uint32_t mat2,
                                                 bool rubs, const DevInter& it) {
@@ -210,9 +213,9 @@ __device__ __forceinline__ float4 axpy(float c, float4 k, float4 t) {
 
 // Pair terms of neighbor j added to `acc` if j lies within the kernel radius
 // (the scan's test lets a few others through); returns the pair's material bits
-// then, kPairContact the highest, and 0 otherwise.  r^2 < h^2 is h^2 - r^2 > 0, grad_w's max(.., 0) test:
-// without flush-to-zero a difference of finite floats is zero only when they
-// are equal.
+// then, kPairContact the highest, and 0 otherwise.  r^2 < h^2 is h^2 - r^2 > 0,
+// grad_w's max(.., 0) test: without flush-to-zero a difference of finite floats is
+// zero only when they are equal.
 template <int DIM>
 __device__ __forceinline__ uint32_t add_hit(Acc& acc, uint32_t j, const PairRec& rj, uint32_t mat2, const Self& s,
                                             const FluidArgs& a, const PairK& K) {
@@ -384,15 +387,16 @@ __device__ __forceinline__ float sum_partials(float v) {  // over the lanes that
 // sums in the tail of the lists of unfinished particles and scans on, so a
 // particle may have any number of hits.
 //
-// Bound: L1 data wavefronts (70 % of peak) and issue slots (64 %), with L1 and
-// L2 latency behind them (4.6 warps per issue on the long scoreboard); DRAM is
+// Bound: L1 data wavefronts (71 % of peak) and issue slots (65 %), with L1 and
+// L2 latency behind them (4.4 warps per issue on the long scoreboard); DRAM is
 // idle.  What it replaced, one thread per particle over 16-byte candidates
 // read from the positions, took 352 us per stage of the 1,048,576-particle
 // fluid and bar scene (RK2, 222 M warp instructions, 69 M wavefronts) and two
-// more launches for the particles whose lists overflowed; this takes 292 us
-// (205 M, 59 M), the next state's cell keys included.  On the way: 4 threads per
+// more launches for the particles whose lists overflowed; this takes 281 us
+// (208 M, 58 M), the next state's cell keys included.  On the way: 4 threads per
 // particle alone 372 us; + quantised candidates 345 us; + 32-byte records 330 us;
-// + the next row's bounds and a second hit's record in flight 292 us.
+// + the next row's bounds and a second hit's record in flight 292 us; + contacts
+// walked where they are 281.
 // Only the epilogue reads what the solid kernels write, so behind those
 // (a.published) a block waits there instead of at its start, and the pair
 // sums fill the SMs that the solid kernels' last blocks leave: ten RK2 steps of

@@ -1281,8 +1281,8 @@ arp_status allocate(arp_sim* S) {
                 o.mass = b.mass;
                 o.visc = is_stiff(a) || b.immobile ? 0.0f : a.visc + b.visc;
                 o.bulk = b.immobile ? 0.0f : i == j ? a.bulk_visc + b.bulk_visc : x.dampening;
-                o.bits = std::min(x.potential, kPairPotential) | (x.potential != ARP_CONTACT_ZERO ? kPairContact : 0u) | (is_stiff(a) ? kPairElastic1 : 0u) |
-                         (is_stiff(b) ? kPairElastic2 : 0u);
+                o.bits = std::min(x.potential, kPairPotential) | (is_stiff(a) ? kPairElastic1 : 0u) |
+                         (is_stiff(b) ? kPairElastic2 : 0u) | (x.potential != ARP_CONTACT_ZERO ? kPairContact : 0u);
             }
     CUDA_TRY(S->d_pmats.alloc(pm.size()));
     CUDA_TRY(cudaMemcpy(S->d_pmats.p, pm.data(), pm.size() * sizeof(PairMat), cudaMemcpyHostToDevice));

@@ -33,8 +33,8 @@ constexpr int kThreads = 128;
 // threads per solid: 4 hold one partial sum each, 2 hold two.  Four threads
 // halve the chain of dependent loads of one solid, which is what a scene with
 // few solids waits for; two repeat less of the work per solid.  Stress and force
-// kernels per stage (events on both sides), 4 / 2 threads: 1,274 solids 21 / 24 us,
-// 9,072 24 / 28, 15,872 24 / 28, 32,256 34 / 32, 129,024 96 / 82.
+// kernels per stage (events on both sides), 4 / 2 threads: 1,274 solids 17.4 / 19.7
+// us, 9,072 19.4 / 21.5, 15,872 21.6 / 23.5, 32,256 31.8 / 29.6, 129,024 93.5 / 77.5.
 constexpr uint32_t kFewSolids = 24576;
 constexpr uint32_t kSameMat = 0x80000000u;
 // The stage kernels recompute gradW(dX) and W(dX) of each reference pair from

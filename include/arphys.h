@@ -482,10 +482,10 @@ arp_status arp_sim_set_solid_stiffness(arp_sim* sim, const float* normal_shear, 
  * re-runs each segment from its checkpoint recording the stage states, then
  * applies the hand-written adjoint of every stage (neighbor sets reused, not
  * differentiated) in reverse.  CUDA-graph replay is off while a tape records.
- * Refused (ARP_ERR_UNSUPPORTED) for plastic materials, strain orders other
- * than 2 and contact friction; a self-contact pair found active during the
- * backward pass makes it return ARP_ERR_UNSUPPORTED after filling the outputs
- * (that term is not differentiated). */
+ * Plastic materials, every strain order and contact friction are
+ * differentiated; a self-contact pair found active during the backward pass
+ * makes it return ARP_ERR_UNSUPPORTED after filling the outputs (that term is
+ * not). */
 arp_status arp_tape_begin(arp_sim* sim, uint32_t checkpoint_every);
 arp_status arp_tape_end(arp_sim* sim);
 arp_status arp_tape_steps(const arp_sim* sim, uint64_t* steps);
